@@ -7,29 +7,8 @@
 // the caller layout [B][S][N][H][D] through strided TMA tensor maps: no
 // transposes, no head-dim padding.
 //
-// One persistent CTA per SM walks work items (b*s, q-tile of 128 rows, h), h
-// fastest so that CTAs running side by side touch the same 128-byte lines of
-// q/k/v.  Per item it streams kv tiles of 128 residues (NG = 2 softmax groups):
-//
-//   warp 8  (producer)  TMA: Q tile (double buffered; one buffer at D = 128), then per
-//                       kv tile K, V, the [128 x 128] bf16 pair-bias tile (D <= 64)
-//                       and the mask row into a ring of stages
-//   warp 9  (S issuer)  tcgen05.mma S_g = Q K[64g:64g+64, :]^T into tensor memory for
-//                       each softmax group g, a tile ahead of the softmax (two buffers)
-//   warp 10 (PV issuer) PV_g (+)= P_g V[64g:64g+64, :] with P_g read from tensor
-//                       memory; the accumulator stays in tensor memory for the item.
-//                       The groups share no barrier inside an item, so they drift
-//                       apart and one group's exp2 phase overlaps the other's FMA phase
-//   warps 0-3, 4-7      two softmax groups.  Group g owns kv columns 64g..64g+63
-//                       of every tile and runs its own online softmax over them
-//                       (thread = one q row): x = S*scale*log2e + bias*log2e +
-//                       mask*log2e, running max, exp2, P (bf16) back into tensor
-//                       memory; when the row maximum rises the accumulator is
-//                       rescaled in place.  After an item each group publishes its
-//                       (m, l); each group then merges, normalises and stores half of
-//                       the head-dim columns of O, reading both groups' accumulators.
-//                       That epilogue is deferred into the next item's first tile, so
-//                       the last PV of an item is never waited for idly.
+// One persistent CTA per SM walks work items (b*s, q-tile of 128 rows, h), h fastest.  D <= 64: two or
+// three items at a time, as independent streams (below).  D = 96 and 128: evo_fwd_wide.cuh.
 //
 // LSE is stored in natural log (tk_evoattention.cu:330-334).
 #include "evo_host.cuh"
@@ -37,89 +16,20 @@
 
 namespace evo {
 
-// How far the running row maximum may fall behind before the accumulator in tensor memory is
-// rescaled.  0 = the exact online softmax: the largest P of a row is exp2(0) = 1, which bf16
-// represents exactly, so a row dominated by one logit carries no rounding error from its main
-// term.  A lag of 8 (P up to 256, the rescale then almost never runs) measured 2 % faster but
-// put a 2^-9 relative error on exactly those main terms: 10x the dBias error at heavy-tailed
-// logits (0.033 against 0.0035 max-abs at B=1, S=48, N=768, H=8, D=32, bias std 2).
-#ifndef EVO_FWD_LAZY
-#define EVO_FWD_LAZY 0.0f
-#endif
-// Softmax groups per CTA.  A group is four warps (thread = one q row) that own kv columns
-// g*CW .. g*CW+CW-1 (CW = 128 / NG) of every tile and run their own online softmax over them; the
-// groups' partial results are merged in the epilogue.  NG = 2 is the general form.  NG = 4 (D = 32
-// only: tensor memory holds four accumulators of 32 columns, not of 64) puts four softmax warps on
-// every scheduler, so that two of them can keep the exp2 unit saturated while the other two are in
-// the fused-multiply-add pass of their tile.
-template <int DH, int NG>
-struct FwdCfg {
-    static_assert(NG == 2 || NG == 4, "two or four softmax groups");
-    static constexpr int CW = TILE / NG;                       // kv columns per group
-    static constexpr int NSW = NG * 4;                         // softmax warps
-    // + an epilogue warpgroup (warps NSW .. NSW+3: warp & 3 is its quarter of the tensor-memory
-    // lanes) + a warpgroup of producer, S issuer, PV issuer and one idle warp
-    static constexpr int THREADS = (NSW + 8) * 32;
-    // setmaxnreg budgets (one value per warpgroup): the CTA's register pool is the launch count (the
-    // cap ptxas derives from the launch bound) times the threads; an increase that the pool cannot
-    // satisfy blocks for ever
-    static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
-    // Measured at B=1, S=512, N=384, H=8, D=32 (forward kernel): 208/40/40 0.392 ms, 200/56/56 0.393,
-    // 200/72/40 0.383, 192/72/56 0.376, 192/64/64 0.370, 184/72/72 0.383, 176/80/80 0.378.
-#ifndef EVO_FWD_RS
-#define EVO_FWD_RS 192
-#define EVO_FWD_RE 64
-#define EVO_FWD_RO 64
-#endif
-    static constexpr int REGS_SOFTMAX = (NG == 2) ? EVO_FWD_RS : 96;
-    static constexpr int REGS_EPI = (NG == 2) ? EVO_FWD_RE : 40;
-    static constexpr int REGS_OTHER = (NG == 2) ? EVO_FWD_RO : 40;
-    static_assert((REGS_SOFTMAX * NSW + REGS_EPI * 4 + REGS_OTHER * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
-    static constexpr int STAGES = (DH == 32) ? 3 : 2;
-    static constexpr uint32_t ROWT = RowTile<DH>::BYTES;          // one [128][DH] bf16 tile
-    // D = 128 is short of shared and tensor memory: one Q buffer instead of two, the bias slice of
-    // a thread read straight from global memory instead of a staged tile, and P (bf16) written
-    // over the S columns it was computed from (S of tile j+2 then waits for PV of tile j).
-    static constexpr bool WIDE = (DH == 128);
-    static constexpr int NQ = WIDE ? 1 : 2;                        // Q buffers
-    static constexpr uint32_t BIAS_BYTES = WIDE ? 0 : SQ_BYTES;
-    // one stage: K tile, V tile, bias tile (two [128][64] halves), raw bf16 mask row
-    static constexpr uint32_t ST_K = 0, ST_V = ROWT, ST_BIAS = 2 * ROWT, ST_MASK = 2 * ROWT + BIAS_BYTES;
-    static constexpr uint32_t STAGE_STRIDE = 2 * ROWT + BIAS_BYTES + 1024;
-    static constexpr uint32_t OFF_Q = 0;                           // NQ buffers
-    static constexpr uint32_t OFF_STAGE = OFF_Q + NQ * ROWT;
-    // O staging: one row tile, written by the epilogue warpgroup, sent out by TMA
-    static constexpr uint32_t OFF_O = OFF_STAGE + STAGES * STAGE_STRIDE;
-    // exchange of the groups' (m, l) per row: [item parity][group][128 rows]
-    static constexpr uint32_t OFF_XCH = OFF_O + ROWT;
-    static constexpr uint32_t OFF_WMASK = OFF_XCH + 2 * NG * 128 * 8;      // NSW warps x CW floats
-    static constexpr uint32_t OFF_BARS = OFF_WMASK + NSW * CW * 4;
-    static constexpr uint32_t NUM_BARS = 4 + 2 * STAGES + 4 * NG + 2 * NG + 2 * NG + 3 + 2;
-    static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;   // + alignment slack
-    static constexpr uint32_t TMEM_S = 0;                          // two buffers: + (tile & 1) * 128 + g * CW
-    static constexpr uint32_t TMEM_PV = 256;                       // + g * DH
-    static constexpr uint32_t TMEM_P = 256 + NG * DH;              // + g * CW/2: CW bf16 per lane (not WIDE)
-    static constexpr uint32_t TMEM_COLS = 512;
-    static_assert(WIDE ? (TMEM_PV + NG * DH <= TMEM_COLS) : (TMEM_P + 64 <= TMEM_COLS), "tensor memory budget");
-    // tensor-memory column (without the lane part) of group w's P of running tile g
-    __device__ static __forceinline__ uint32_t p_col(int w, int g) {
-        return WIDE ? TMEM_S + (g & 1) * 128 + CW * w : TMEM_P + w * (CW / 2);
-    }
-    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-    static_assert(OFF_STAGE % 1024 == 0 && STAGE_STRIDE % 1024 == 0 && OFF_O % 1024 == 0, "tile alignment");
-};
-
 struct FwdParams {
     int B, S, N, H;
     int Dt;            // true head dim (16 runs on the D = 32 kernel: loads zero-filled, stores clipped)
     int KB;            // contraction blocks of 16 head-dim columns that hold data: ceil(Dt / 16)
     int QT;            // q tiles (= kv tiles) per row: ceil(N / 128)
-    int total_items;   // B*S*QT*H
+    int shared_bias;   // D <= 64: the streams of a CTA work on rows of the same q tile and share its bias tiles
+    int NG;            // D <= 64: rows per batch, or groups of G rows if the bias tiles are shared
+    int total_items;   // B*S*QT*H, or B*SG*QT*H
     float c1;          // scale * log2(e)
+    float scale, inv_scale;
     const __nv_bfloat16* mask;   // [B*S][N]
     const __nv_bfloat16* bias;   // [B][H][N][N] (read directly when the bias tile is not staged)
     float* lse;                  // [B*S][H][N]
+    __nv_bfloat16* o;            // activation layout `lay`
     __nv_bfloat16* o_resid;      // activation layout `lay`, or nullptr
     const __nv_bfloat16* gate;   // activation layout `lay`, or nullptr: pre-activation gate logits
     __nv_bfloat16* o_gated;      // activation layout `lay` (with gate): O * sigmoid(gate)
@@ -127,511 +37,529 @@ struct FwdParams {
     unsigned int* status;
 };
 
-// STRIDED: the activation tensors are views with the strides of p.lay; otherwise they are
-// contiguous and the residual's address is formed from N and H alone.  (The generic address
-// arithmetic, in the epilogue, cost 4-10 % of the kernel when it was the only version: the
-// contiguous case keeps its own instantiation.)
-// GATED: the epilogue also writes sigmoid(gate) * O (its own instantiation: the extra loads and
-// arithmetic, even behind a uniform branch, cost the plain kernel 5 %).
-template <int DH, bool STRIDED, int NG, bool GATED>
-__global__ void __launch_bounds__((FwdCfg<DH, NG>::THREADS), 1)
+}  // namespace evo
+#include "evo_fwd_wide.cuh"
+namespace evo {
+
+// ---------------------------------------------------------------------------
+// D <= 64: independent item streams.
+//
+// What bounds the kernel at D = 32 is not one unit but the hand-offs: every arrive/wait pair costs
+// about 130 clocks, an MMA about 130 more until its commit is seen, and a softmax warp that crosses
+// four of them per [128 x 64] tile spends as long waiting as computing.  So a CTA runs G streams that
+// share nothing but the bias tiles, the tensor core and the issue slots.  Stream s has four softmax
+// warps (thread = one q row, all 128 columns of a tile), its own Q, K, V buffers and tensor-memory
+// columns, and one MMA warp; it is a serial chain
+//
+//   S' = Q K^T + mask block  ->  softmax of the tile  ->  PV (+)= P V  ->  next tile
+//
+// with two waits per softmax warp and tile; while one stream waits, the others compute.
+//
+//   D = 32 (G = 3): three warps per scheduler.  x = S' * scale + bias goes back into the S columns
+//     and is read again for the exp2 pass (tensor memory moves two columns per clock), so a thread
+//     needs no 128 registers for it; P (bf16) overwrites the columns already read, and S' of the
+//     next tile follows PV of this one.
+//   D = 64 (G = 2; three accumulators of 64 columns do not fit beside three S tiles): x stays in
+//     registers, P has columns of its own, so S' of the next tile runs during the exp2 pass.
+//
+// Bias tiles travel through a ring.  SHARED: the streams of a CTA work on G rows of S at the same
+// (b, h, q tile), so one tile serves G streams; otherwise (few rows per batch, or too few items to
+// fill the SMs G at a time) every stream has its own items and its own ring slot.
+//
+// Measured against the kernel with two groups of 64 columns on one item (which runs D = 128): B=1, S=512,
+// N=384, H=8, D=32 0.371 -> 0.323 ms; S=256, N=768 0.650 -> 0.560; S=256, N=1024, H=4, D=64 0.690 -> 0.580.
+// A step takes about 2400 clocks of a CTA: 1024 for its exponentials, 1000 issue slots.  Also tried: the
+// epilogue on a warpgroup of its own (its registers cost the softmax warps more than it saves, 0.42 ms),
+// two streams in the exp2 pass at a time (0.365), none taking turns (0.39), two streams at D = 32 (0.375).
+//
+// The mask rides in an extra contraction block (evo_tiles.cuh, "EXTRA TILE"): the producer turns 128
+// mask values into a [128][8] tile (m/scale in three bf16 parts, exact to fp32), columns past N get
+// -1e38.  The base of the exponentials: x in natural units, P = exp2(x log2e - m log2e).
+// ---------------------------------------------------------------------------
+template <int DH>
+struct FwdCfg {
+    static constexpr int G = (DH == 32) ? 3 : 2;               // item streams
+    static constexpr bool HOLD = (G == 2);                     // x in registers, P in its own columns
+    // every fourth column pair of the exp2 pass on the fused-multiply-add pipe: D = 32 (B=1, S=512, N=384,
+    // H=8) 0.334 -> 0.323 ms; D = 64, whose warps have no issue slots to spare, 0.58 -> 0.63 ms
+    static constexpr int POLY_EVERY = (DH == 32) ? 4 : 0;
+    static constexpr int NSW = 4 * G;                          // softmax warps
+    static constexpr int W_PROD = NSW;                         // producer, then G MMA warps (one warpgroup)
+    static constexpr int THREADS = (NSW + 4) * 32;
+    // setmaxnreg budgets: the CTA's register pool is the launch count (the cap ptxas derives from the
+    // launch bound) times the threads; an increase that the pool cannot satisfy blocks for ever
+    static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
+    static constexpr int REGS_SOFTMAX = (G == 3) ? 144 : 208;
+    static constexpr int REGS_OTHER = (G == 3) ? 80 : 88;
+    static_assert((REGS_SOFTMAX * NSW + REGS_OTHER * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
+    static constexpr uint32_t ROWT = RowTile<DH>::BYTES;       // one [128][DH] bf16 tile
+    static constexpr int NQ = (DH == 32) ? 2 : 1;              // Q buffers per stream
+    static constexpr int NK = HOLD ? 2 : 1;                    // K (and mask tile) buffers per stream
+    static constexpr int NR = G;                               // bias tiles in the ring
+    static constexpr uint32_t ST_Q = 0, ST_K = NQ * ROWT, ST_V = ST_K + NK * ROWT, ST_XK = ST_V + ROWT;
+    static constexpr uint32_t STREAM_BYTES = ST_XK + NK * XT_BYTES;
+    static constexpr uint32_t OFF_BIAS = 0;                    // ring of bias tiles: two [128][64] halves each
+    static constexpr uint32_t OFF_STREAM = NR * SQ_BYTES;
+    // constant extra tiles, above every tile that refers to the zero tile
+    static constexpr uint32_t OFF_XQ = OFF_STREAM + G * STREAM_BYTES;       // rows (1, 1, 1, 0, ...)
+    static constexpr uint32_t OFF_ZERO = OFF_XQ + XT_BYTES;
+    static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
+    static constexpr int BARS = 21;                            // barriers of a stream (FwdBars)
+    static constexpr uint32_t OFF_MISC = OFF_BARS + (G * BARS + 2 * NR) * 8;
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;   // + alignment slack
+    static constexpr uint32_t TMEM_S = 0;                      // + 128 s
+    static constexpr uint32_t TMEM_PV = 128 * G;               // + DH s
+    static constexpr uint32_t TMEM_P = HOLD ? TMEM_PV + DH * G : TMEM_S;   // + 64 s, or the S columns of stream s
+    static constexpr uint32_t TMEM_COLS = 512;
+    static_assert((HOLD ? TMEM_P + 64 * G : TMEM_PV + DH * G) <= TMEM_COLS, "tensor memory budget");
+    __device__ static __forceinline__ uint32_t p_col(int s) { return TMEM_P + s * (HOLD ? 64 : 128); }
+    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+    static_assert(STREAM_BYTES % 1024 == 0, "tile alignment");
+};
+
+// The barriers of one stream.
+struct FwdBars {
+    uint64_t *q_full, *q_empty;      // [NQ]
+    uint64_t *k_full, *k_empty;      // [NK]: K and mask tile
+    uint64_t *v_full;
+    uint64_t *s_full, *s_free;       // S' complete / read (HOLD)
+    uint64_t *p_ready, *pv_done;     // P written / PV complete
+    uint64_t *turn;                 // [2][4] by tile parity: warp w of the stream has left its exp2 pass
+    __device__ __forceinline__ FwdBars(uint64_t* b)
+        : q_full(b), q_empty(b + 2), k_full(b + 4), k_empty(b + 6), v_full(b + 8), s_full(b + 9), s_free(b + 10),
+          p_ready(b + 11), pv_done(b + 12), turn(b + 13) {}
+};
+
+// A stream's walk over its items: coordinates in mixed radix (head, q tile, row or group of rows, batch),
+// advanced without a division (a division costs a warp about a hundred clocks, on the stream's chain).
+struct FwdStep {
+    int h, qt, g, b;
+    __device__ __forceinline__ FwdStep(int w, const FwdParams& p) {
+        h = w % p.H; w /= p.H;
+        qt = w % p.QT; w /= p.QT;
+        g = w % p.NG; b = w / p.NG;
+    }
+};
+struct FwdItem {
+    int h, qt, row, b;       // row of S: with groups, G apart
+    __device__ __forceinline__ void next(const FwdStep& d, int rows, int rstep, const FwdParams& p) {
+        h += d.h;
+        int c = h >= p.H;
+        h -= c ? p.H : 0;
+        qt += d.qt + c;
+        c = qt >= p.QT;
+        qt -= c ? p.QT : 0;
+        row += (d.g + c) * rstep;
+        c = row >= rows;
+        row -= c ? rows : 0;
+        b += d.b + c;
+    }
+    __device__ __forceinline__ bool valid(const FwdParams& p) const { return b < p.B && row < p.S; }
+    __device__ __forceinline__ int bs(const FwdParams& p) const { return b * p.S + row; }
+};
+
+// v as three bf16 parts (24 significant bits), in the layout of words 0 and 1 of an extra-tile row
+__device__ __forceinline__ uint2 split3_bf16(float v) {
+    v = fminf(fmaxf(v, -1e38f), 1e38f);
+    const float a = __bfloat162float(__float2bfloat16_rn(v));
+    const float b = __bfloat162float(__float2bfloat16_rn(v - a));
+    const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn((v - a) - b));
+    return make_uint2(pack_bf16(a, b), c);
+}
+
+// Four lanes of a quad hold four 16-byte chunks each of their own row: afterwards lane t of the quad
+// holds chunk t of the quad's rows 0..3, so that a store instruction covers whole 64-byte segments.
+__device__ __forceinline__ void quad_transpose(uint4 (&c)[4]) {
+    const bool b0 = threadIdx.x & 1u, b1 = threadIdx.x & 2u;
+    auto swap_pair = [](uint4& lo, uint4& hi, bool up, int mask) {
+        uint4 snd = up ? lo : hi;
+        snd.x = __shfl_xor_sync(0xffffffffu, snd.x, mask);
+        snd.y = __shfl_xor_sync(0xffffffffu, snd.y, mask);
+        snd.z = __shfl_xor_sync(0xffffffffu, snd.z, mask);
+        snd.w = __shfl_xor_sync(0xffffffffu, snd.w, mask);
+        lo = up ? snd : lo;
+        hi = up ? hi : snd;
+    };
+    swap_pair(c[0], c[1], b0, 1);
+    swap_pair(c[2], c[3], b0, 1);
+    swap_pair(c[0], c[2], b1, 2);
+    swap_pair(c[1], c[3], b1, 2);
+}
+
+// STRIDED: the output-side tensors are views with the strides of p.lay (otherwise contiguous, with
+// addresses formed from N, H and Dt alone).  GATED: the epilogue also writes sigmoid(gate) * O.
+template <int DH, bool STRIDED, bool GATED>
+__global__ void __launch_bounds__(FwdCfg<DH>::THREADS, 1)
 evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias,
-               const __grid_constant__ CUtensorMap tm_o, const FwdParams p) {
-    using C = FwdCfg<DH, NG>;
+               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias, const FwdParams p) {
+    using C = FwdCfg<DH>;
     using RT = RowTile<DH>;
-    constexpr int ST = C::STAGES, CW = C::CW, NSW = C::NSW;
-    constexpr int W_EPI = NSW, W_PROD = NSW + 4, W_S = NSW + 5, W_PV = NSW + 6;
+    using RD = RowDesc<DH>;
+    constexpr int G = C::G, NSW = C::NSW, NQ = C::NQ, NK = C::NK, NR = C::NR;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BARS);
-    uint64_t* q_full = bars;                 // [2]
-    uint64_t* q_empty = bars + 2;            // [2]
-    uint64_t* kv_full = bars + 4;            // [ST]
-    uint64_t* kv_empty = kv_full + ST;       // [ST]
-    uint64_t* s_full = kv_empty + ST;        // [2 * NG]: softmax group + NG * S buffer
-    uint64_t* s_free = s_full + 2 * NG;      // [2 * NG]
-    uint64_t* p_ready = s_free + 2 * NG;     // [NG] per softmax group
-    uint64_t* pv_full = p_ready + NG;        // [NG]
-    uint64_t* xch_ready = pv_full + NG;      // [item parity][group]: the group's final (m, l) of an item are written
-    uint64_t* acc_full = xch_ready + 2 * NG; // every PV MMA of an item is complete
-    uint64_t* acc_free = acc_full + 1;       // the epilogue has read the item's accumulators and (m, l)
-    uint64_t* e_bar = acc_free + 1;          // rendezvous of the four epilogue warps
-    uint64_t* xu_done = e_bar + 1;           // [2]: a half of the groups has finished the exp2 pass of a tile
+    uint64_t* bias_full = bars + G * C::BARS;            // [NR]
+    uint64_t* bias_empty = bias_full + NR;               // [NR]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // uniform: what derives from it stays in uniform registers
     const int lane = tid & 31;
     const int NT = p.QT;
+    const bool shared_bias = p.shared_bias != 0;
     WaitCtx wc{abort_flag, p.status};
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
-        for (int i = 0; i < ST; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], NSW + 1); }
-        for (int i = 0; i < 2 * NG; ++i) {
-            mbar_init(&s_full[i], 1); mbar_init(&s_free[i], C::WIDE ? 1 : 4); mbar_init(&xch_ready[i], 4);
+        tmem_slot[3] = 0;                   // the flag of the waits before exit: never set
+        for (int s = 0; s < G; ++s) {
+            const FwdBars b(bars + s * C::BARS);
+            for (int i = 0; i < NQ; ++i) { mbar_init(&b.q_full[i], 1); mbar_init(&b.q_empty[i], 1); }
+            for (int i = 0; i < NK; ++i) { mbar_init(&b.k_full[i], 1); mbar_init(&b.k_empty[i], 1); }
+            mbar_init(b.v_full, 1);
+            mbar_init(b.s_full, 1); mbar_init(b.s_free, 4);
+            mbar_init(b.p_ready, 4); mbar_init(b.pv_done, 1);
+            for (int i = 0; i < 8; ++i) mbar_init(&b.turn[i], 1);
         }
-        for (int i = 0; i < NG; ++i) { mbar_init(&p_ready[i], 4); mbar_init(&pv_full[i], 1); }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_free, 4);
-        mbar_init(e_bar, 4);
-        for (int i = 0; i < 2; ++i) mbar_init(&xu_done[i], NSW / 2);
+        for (int i = 0; i < NR; ++i) { mbar_init(&bias_full[i], 1); mbar_init(&bias_empty[i], shared_bias ? NSW : 4); }
         fence_mbar_init();
-        fence_async_smem();
     }
-    if (warp == W_S) {
+    if (warp == C::W_PROD) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
+        if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_bias); }
     }
-    if (warp == W_PROD && lane == 0) {
-        prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
-        prefetch_tmap(&tm_bias); prefetch_tmap(&tm_o);
+    if (tid < 128) {
+        *reinterpret_cast<uint4*>(smem + C::OFF_XQ + tid * 16) = make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u);
+        *reinterpret_cast<uint4*>(smem + C::OFF_ZERO + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
-    EVO_TRACE_INIT();
+    fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    EVO_TS(t_kernel);
 
-    const int first = blockIdx.x;
-    const int stride = gridDim.x;
-    const int n_items = (p.total_items > first) ? (p.total_items - first + stride - 1) / stride : 0;
-
-    // item index -> (bs, qt, h); h fastest, then q tile, then row
-    auto decode = [&](int it, int& bs, int& qt, int& h) {
-        const int w = first + it * stride;
-        h = w % p.H;
-        const int r = w / p.H;
-        qt = r % p.QT;
-        bs = r / p.QT;
+    // Items.  h fastest, then q tile, then row (or group of G rows), so that CTAs side by side touch the
+    // same 128-byte lines of q/k/v.  Every stream counts the same number of items; the last ones of a
+    // stream, or rows of a group past S, may be missing.
+    const int first = blockIdx.x, stride = gridDim.x;
+    const int per_cta = stride * (shared_bias ? 1 : G);
+    const int n_items = (p.total_items > first) ? (p.total_items - first + per_cta - 1) / per_cta : 0;
+    // rows count in steps of G within a batch if they are taken in groups: row r of the group sits at g * G + r
+    const int rstep = shared_bias ? G : 1;
+    auto items_of = [&](int s) -> FwdItem {
+        const FwdStep w(first + (shared_bias ? 0 : s * stride), p);
+        return FwdItem{w.h, w.qt, w.g * rstep + (shared_bias ? s : 0), w.b};
+    };
+    const FwdStep step(per_cta, p);
+    auto advance = [&](FwdItem& x, int s) {
+        const int shift = shared_bias ? s : 0;
+        x.row -= shift;
+        x.next(step, p.NG * rstep, rstep, p);
+        x.row += shift;
+    };
+    // ring slot and phase parity of the bias tile of tile r of stream s
+    auto bias_slot = [&](int s, int r, int& slot, uint32_t& ph) {
+        slot = shared_bias ? r % NR : s;
+        ph = static_cast<uint32_t>(shared_bias ? r / NR : r) & 1u;
     };
 
-    if (warp >= NSW + 4) {
+    if (warp >= C::W_PROD) {
         reg_dec<C::REGS_OTHER>();
-        if (warp == W_PROD) {
-            if (lane == 0) {
-                // ------------------------------ producer ------------------------------
-                bool ok = true;
-                int g = 0;   // running kv-tile counter across items
-                for (int it = 0; it < n_items && ok; ++it) {
-                    int bs, qt, h;
-                    decode(it, bs, qt, h);
-                    const int b = bs / p.S;
-                    const int qb = it % C::NQ;
-                    if (it >= C::NQ) ok = mbar_wait(&q_empty[qb], ((it / C::NQ) - 1) & 1, wc, 0x10);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(&q_full[qb], C::ROWT);
-                    tma_load_row_tile<DH>(smem + C::OFF_Q + qb * C::ROWT, &tm_q, &q_full[qb], h, qt * TILE, bs);
-                    for (int j = 0; j < NT; ++j, ++g) {
-                        const int st = g % ST;
-                        if (g >= ST) ok = mbar_wait(&kv_empty[st], ((g / ST) - 1) & 1, wc, 0x11);
-                        if (!ok) break;
-                        uint8_t* sb = smem + C::OFF_STAGE + st * C::STAGE_STRIDE;
-                        const int ncol = (p.N - j * TILE < TILE) ? (p.N - j * TILE) : TILE;   // multiple of 8
-                        mbar_arrive_expect_tx(&kv_full[st], 2 * C::ROWT + C::BIAS_BYTES + ncol * 2);
-                        tma_load_row_tile<DH>(sb + C::ST_K, &tm_k, &kv_full[st], h, j * TILE, bs);
-                        tma_load_row_tile<DH>(sb + C::ST_V, &tm_v, &kv_full[st], h, j * TILE, bs);
-                        if (!C::WIDE) {
-                            tma_load_4d(sb + C::ST_BIAS, &tm_bias, &kv_full[st], j * TILE, qt * TILE, h, b);
-                            tma_load_4d(sb + C::ST_BIAS + SQ_SUB_BYTES, &tm_bias, &kv_full[st], j * TILE + 64, qt * TILE, h, b);
-                        }
-                        bulk_load(sb + C::ST_MASK, p.mask + static_cast<size_t>(bs) * p.N + j * TILE, ncol * 2, &kv_full[st]);
-                    }
-                }
-                // Drain: every load issued above has landed before the CTA exits.
-                const int issued = g;
-                for (int k = (issued > ST ? issued - ST : 0); k < issued; ++k)
-                    (void)mbar_wait(&kv_full[k % ST], (k / ST) & 1, wc, 0x12);
-                for (int it = (n_items > C::NQ ? n_items - C::NQ : 0); it < n_items; ++it)
-                    (void)mbar_wait(&q_full[it % C::NQ], (it / C::NQ) & 1, wc, 0x13);
-            }
-        } else if (warp == W_S) {
-            // ------------------------------ S issuer ------------------------------
-            // S_w = Q K[CW w : CW w + CW, :]^T for every softmax group w of every tile, one tile ahead
-            // of the softmax (two S buffers).  The warp runs its loop with all lanes (uniform control
-            // flow keeps the operand descriptors in uniform registers) and elects one lane to issue.
-            constexpr uint32_t IDESC_S = make_idesc_bf16(128, CW, 0, 0);
-            const uint32_t aQ = smem_u32(smem + C::OFF_Q), aSt = smem_u32(smem + C::OFF_STAGE);
+        if (warp == C::W_PROD) {
+            // ------------------------------ producer ------------------------------
+            // Round r holds tile r of every stream (item r / NT, kv tile r % NT): the bias tile, then Q per
+            // item, K and the mask tile.  (V is fetched by the stream's MMA warp, the first to know that its
+            // buffer is free.)  The warp runs with all lanes and elects one to issue.
+            int used[G], qn[G];      // tiles and items of the stream so far
+            FwdItem item[3] = {items_of(0), items_of(1), items_of(2)};      // the first G of them are walked
+#pragma unroll
+            for (int s = 0; s < G; ++s) used[s] = qn[s] = 0;
             bool ok = true;
-            int g = 0;
+            int r = 0;
             for (int it = 0; it < n_items && ok; ++it) {
-                const int qb = it % C::NQ;
-                for (int j = 0; j < NT && ok; ++j, ++g) {
-                    const int st = g % ST;
-                    if (j == 0) ok = warp_all(mbar_wait(&q_full[qb], (it / C::NQ) & 1, wc, 0x20));
-                    if (ok) ok = warp_all(mbar_wait(&kv_full[st], (g / ST) & 1, wc, 0x21));
+                for (int j = 0; j < NT && ok; ++j, ++r) {
 #pragma unroll
-                    for (int w = 0; w < NG; ++w) {
-                        const int sb = w + NG * (g & 1);
-                        if (ok && g >= 2) ok = warp_all(mbar_wait(&s_free[sb], ((g >> 1) - 1) & 1, wc, 0x22));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            // K rows CW w .. of the tile: that many rows further into the K-major tile
-                            const uint32_t kt = aSt + st * C::STAGE_STRIDE + C::ST_K + w * CW * RT::ROW_BYTES;
-#pragma unroll
-                            for (int kb = 0; kb < RT::KBLOCKS; ++kb)
-                                if (kb < p.KB)      // blocks past the true head dim are zero-filled: skipped
-                                    umma_ss(tmem + C::TMEM_S + (g & 1) * 128 + CW * w, RT::kmajor(aQ + qb * C::ROWT, kb),
-                                            RT::kmajor(kt, kb), IDESC_S, kb > 0);
-                            umma_commit(&s_full[sb]);
-                            // Q is free once every group's S of the item's last tile is issued
-                            if (w == NG - 1 && j == NT - 1) umma_commit(&q_empty[qb]);
-                        }
-                        __syncwarp();
-                    }
-                }
-            }
-        } else if (warp == W_PV) {
-            // ------------------------------ PV issuer ------------------------------
-            // PV_w (+)= P_w V[CW w : CW w + CW, :] with P_w read from tensor memory; the accumulator of a
-            // group stays in tensor memory for the whole item (the first tile overwrites it).
-            const uint32_t IDESC_PV = make_idesc_bf16(128, 16 * p.KB, 0, 1);   // N = the head-dim columns that hold data
-            const uint32_t aSt = smem_u32(smem + C::OFF_STAGE);
-            bool ok = true;
-            int g = 0;
-            for (int it = 0; it < n_items && ok; ++it) {
-                for (int j = 0; j < NT && ok; ++j, ++g) {
-                    const int st = g % ST;
-                    // the first PV of an item overwrites the accumulators: the epilogue has read the previous item's
-                    if (j == 0 && it > 0) ok = warp_all(mbar_wait(acc_free, (it - 1) & 1, wc, 0x24));
-#pragma unroll
-                    for (int w = 0; w < NG; ++w) {
-                        if (ok) ok = warp_all(mbar_wait(&p_ready[w], g & 1, wc, 0x23));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-#pragma unroll
-                            for (int kk = 0; kk < CW / 16; ++kk)
-                                umma_ts(tmem + C::TMEM_PV + w * DH, tmem + C::p_col(w, g) + kk * 8,
-                                        RT::mnmajor(aSt + st * C::STAGE_STRIDE + C::ST_V, (CW / 16) * w + kk), IDESC_PV,
-                                        (kk > 0 || j > 0) ? 1u : 0u);
-                            umma_commit(&pv_full[w]);
-                            if (C::WIDE) umma_commit(&s_free[w + NG * (g & 1)]);   // P sat in this S buffer
-                            if (w == NG - 1) umma_commit(&kv_empty[st]);   // every group's PV of the tile issued
-                            if (w == NG - 1 && j == NT - 1) umma_commit(acc_full);   // ... and of the item
-                        }
-                        __syncwarp();
-                    }
-                }
-            }
-        }
-    } else if (warp >= W_EPI) {
-        reg_dec<C::REGS_EPI>();
-        // ------------------------------ epilogue warpgroup ------------------------------
-        // Finishes item k while the softmax groups are already in item k+1: merges the groups'
-        // partial results (split-kv merge), normalises, writes O through shared memory and TMA, the
-        // log-sum-exp, the rounding residual and the gated output.  Thread = one q row; warp e reads
-        // tensor-memory lanes 32e .. 32e+31.
-        const int row = tid & 127;
-        const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-        const uint32_t aO = smem_u32(smem + C::OFF_O);
-        const uint32_t aXch = smem_u32(smem + C::OFF_XCH);
-        bool ok = true;
-        uint32_t e_phase = 0;
-        auto epi_sync = [&]() -> bool {      // rendezvous of the four epilogue warps (bounded)
-            __syncwarp();
-            if (lane == 0) mbar_arrive(e_bar);
-            const bool r = warp_all(mbar_wait(e_bar, e_phase, wc, 0x30));
-            e_phase ^= 1u;
-            return r;
-        };
-        constexpr int EC = 16;               // head-dim columns per pass (register budget)
-        for (int it = 0; it < n_items && ok; ++it) {
-            int bs, qt, h;
-            decode(it, bs, qt, h);
-            EVO_TS(t_epi);
-            const int qrow = qt * TILE + row;
-            size_t act_off;
-            if constexpr (STRIDED)
-                act_off = bs * p.lay.row + qrow * p.lay.n + h * p.lay.h;
-            else
-                act_off = ((static_cast<size_t>(bs) * p.N + qrow) * p.H + h) * DH;
-            // every group's (m, l) of the item, then every PV MMA of the item
-            float gm[NG], gl[NG];
-#pragma unroll
-            for (int og = 0; og < NG; ++og) {
-                if (ok) ok = warp_all(mbar_wait(&xch_ready[(it & 1) * NG + og], (it >> 1) & 1, wc, 0x35));
-                if (!ok) break;
-                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(gm[og]), "=f"(gl[og])
-                             : "r"(aXch + (((it & 1) * NG + og) * 128 + row) * 8));
-            }
-            if (ok) ok = warp_all(mbar_wait(acc_full, it & 1, wc, 0x37));
-            if (!ok) break;
-            tc_fence_after();
-            float mt = gm[0];
-#pragma unroll
-            for (int og = 1; og < NG; ++og) mt = fmaxf(mt, gm[og]);
-            const float ms = (mt == -INFINITY) ? 0.f : mt;
-            float gf[NG], lt = 0.f;
-#pragma unroll
-            for (int og = 0; og < NG; ++og) { gf[og] = ex2(gm[og] - ms); lt += gl[og] * gf[og]; }
-            const float inv = 1.f / lt;
-#pragma unroll
-            for (int og = 0; og < NG; ++og) gf[og] *= inv;
-            // the previous item's TMA store must have finished reading the staging tile
-            if (row == 0) tma_wait_group_read<0>();
-            if (!epi_sync()) { ok = false; break; }
-#pragma unroll
-            for (int hc = 0; hc < DH / EC; ++hc) {
-                float outv[EC];
-#pragma unroll
-                for (int e = 0; e < EC; ++e) outv[e] = 0.f;
-#pragma unroll
-                for (int og = 0; og < NG; ++og) {
-                    float part[EC];
-                    tmem_ld_f32<EC>(lane_base + C::TMEM_PV + og * DH + hc * EC, part);
-#pragma unroll
-                    for (int e = 0; e < EC; ++e) outv[e] = fmaf(part[e], gf[og], outv[e]);
-                }
-                if (hc == DH / EC - 1) {
-                    // accumulators and (m, l) are read: the next item's first PV may overwrite them
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_free);
-                }
-#pragma unroll
-                for (int c8l = 0; c8l < EC / 8; ++c8l) {
-                    const int col = hc * EC + c8l * 8;                 // first head-dim column of this 16-byte chunk
-                    uint4 v;
-                    v.x = pack_bf16(outv[c8l * 8 + 0], outv[c8l * 8 + 1]);
-                    v.y = pack_bf16(outv[c8l * 8 + 2], outv[c8l * 8 + 3]);
-                    v.z = pack_bf16(outv[c8l * 8 + 4], outv[c8l * 8 + 5]);
-                    v.w = pack_bf16(outv[c8l * 8 + 6], outv[c8l * 8 + 7]);
-                    sts128(aO + (col / RT::BOX_D) * RT::SUB_BYTES + swz_off<RT::ROW_BYTES>(row, (col % RT::BOX_D) / 8), v);
-                    if (qrow < p.N && col < p.Dt) {
-                        if (p.o_resid != nullptr) {
-                            // rounding residual of O, straight to global memory
-                            const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-                            uint32_t rw[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                rw[e] = pack_bf16(outv[c8l * 8 + 2 * e] - bf16_lo(vw[e]),
-                                                  outv[c8l * 8 + 2 * e + 1] - bf16_hi(vw[e]));
-                            *reinterpret_cast<uint4*>(p.o_resid + act_off + col) = make_uint4(rw[0], rw[1], rw[2], rw[3]);
-                        }
-                        if constexpr (GATED) {
-                            // O * sigmoid(gate), from the unrounded O
-                            const uint4 g4 = __ldg(reinterpret_cast<const uint4*>(p.gate + act_off + col));
-                            const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
-                            uint32_t ow[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
-                                const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
-                                ow[e] = pack_bf16(outv[c8l * 8 + 2 * e] * s0, outv[c8l * 8 + 2 * e + 1] * s1);
+                    for (int s = 0; s < G; ++s) {
+                        if (!ok || !item[s].valid(p)) continue;
+                        const int bs = item[s].bs(p), qt = item[s].qt, h = item[s].h;
+                        const FwdBars b(bars + s * C::BARS);
+                        uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
+                        // four mask values per lane, requested before the waits
+                        const int c = j * TILE + 4 * lane;
+                        uint2 mw = make_uint2(0u, 0u);
+                        if (c < p.N) mw = __ldg(reinterpret_cast<const uint2*>(p.mask + static_cast<size_t>(bs) * p.N + c));
+                        if (j == 0) {
+                            const int qb = qn[s] % NQ, use = qn[s] / NQ;
+                            if (qn[s]++ >= NQ) ok = warp_all(mbar_wait(&b.q_empty[qb], (use - 1) & 1, wc, 0x10));
+                            if (ok && elect_one()) {
+                                mbar_arrive_expect_tx(&b.q_full[qb], C::ROWT);
+                                tma_load_row_tile<DH>(sb + C::ST_Q + qb * C::ROWT, &tm_q, &b.q_full[qb], h, qt * TILE, bs);
                             }
-                            *reinterpret_cast<uint4*>(p.o_gated + act_off + col) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                            __syncwarp();
+                        }
+                        if (!ok) continue;
+                        const int n = used[s]++, kb = n % NK;
+                        if (n >= NK) ok = warp_all(mbar_wait(&b.k_empty[kb], ((n / NK) - 1) & 1, wc, 0x11));
+                        if (!ok) continue;
+                        if (elect_one()) {
+                            mbar_expect_tx(&b.k_full[kb], C::ROWT);
+                            tma_load_row_tile<DH>(sb + C::ST_K + kb * C::ROWT, &tm_k, &b.k_full[kb], h, j * TILE, bs);
+                        }
+                        __syncwarp();
+                        const float mv[4] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y)};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const uint2 w = split3_bf16(c < p.N ? mv[e] * p.inv_scale : -1e38f);
+                            *reinterpret_cast<uint4*>(sb + C::ST_XK + kb * XT_BYTES + (4 * lane + e) * 16) = make_uint4(w.x, w.y, 0u, 0u);
+                        }
+                        fence_async_smem();
+                        __syncwarp();
+                        if (elect_one()) mbar_arrive(&b.k_full[kb]);
+                        __syncwarp();
+                        // the bias tile: once per round if the streams share it (stream 0 always has the item)
+                        if (!shared_bias || s == 0) {
+                            int slot; uint32_t ph;
+                            bias_slot(s, r, slot, ph);
+                            if (r >= (shared_bias ? NR : 1)) ok = warp_all(mbar_wait(&bias_empty[slot], ph ^ 1u, wc, 0x14));
+                            if (ok && elect_one()) {
+                                uint8_t* bt = smem + C::OFF_BIAS + slot * SQ_BYTES;
+                                                                mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
+                                tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, item[s].b);
+                                tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, item[s].b);
+                            }
+                            __syncwarp();
                         }
                     }
                 }
-            }
-            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ms * LN2 + __logf(lt);
-            fence_async_smem();
-            if (!epi_sync()) { ok = false; break; }
-            if (row == 0) {
 #pragma unroll
-                for (int sub = 0; sub < RT::SUBS; ++sub)
-                    if (sub * RT::BOX_D < p.Dt)
-                        tma_store_4d(&tm_o, smem + C::OFF_O + sub * RT::SUB_BYTES, sub * RT::BOX_D, h, qt * TILE, bs);
-                tma_commit_group();
+                for (int s = 0; s < G; ++s) advance(item[s], s);
             }
-            EVO_TE(t_epi, p.status, 0x79);
+            // the last loads have landed before the CTA exits (also if a wait gave up)
+            const WaitCtx dc{tmem_slot + 3, p.status};
+#pragma unroll
+            for (int s = 0; s < G; ++s) {
+                const FwdBars b(bars + s * C::BARS);
+                for (int k = (used[s] > NK ? used[s] - NK : 0); k < used[s]; ++k) (void)mbar_wait(&b.k_full[k % NK], (k / NK) & 1, dc, 0x12);
+                for (int k = (qn[s] > NQ ? qn[s] - NQ : 0); k < qn[s]; ++k) (void)mbar_wait(&b.q_full[k % NQ], (k / NQ) & 1, dc, 0x13);
+            }
+        } else if (warp - C::W_PROD - 1 < G) {
+            // ------------------------------ MMA warp of one stream ------------------------------
+            const int s = warp - C::W_PROD - 1;
+            const FwdBars b(bars + s * C::BARS);
+            constexpr uint32_t IDESC_S = make_idesc_bf16(128, 128, 0, 0);
+            const uint32_t IDESC_PV = make_idesc_bf16(128, 16 * p.KB, 0, 1);   // N = the head-dim columns that hold data
+            uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
+            const uint32_t aS = smem_u32(sb), aZero = smem_u32(smem + C::OFF_ZERO);
+            const uint64_t d_xq = xt_desc(smem_u32(smem + C::OFF_XQ), aZero);
+            const uint32_t v_lo = RD::mnmajor_lo(aS + C::ST_V);
+            const uint32_t t_s = tmem + C::TMEM_S + 128 * s, t_pv = tmem + C::TMEM_PV + DH * s, t_p = tmem + C::p_col(s);
+            bool ok = true;
+            FwdItem cur = items_of(s);         // the item whose V tiles are being loaded
+            int qn = 0;                        // items whose S' tiles have all been issued
+            // S' of tile n (kv tile j of item qn): what it waits for, and the issue
+            auto wait_s = [&](int n, int j) {
+                if (j == 0) ok = warp_all(mbar_wait(&b.q_full[qn % NQ], (qn / NQ) & 1, wc, 0x20));
+                if (ok) ok = warp_all(mbar_wait(&b.k_full[n % NK], (n / NK) & 1, wc, 0x21));
+            };
+            auto issue_s = [&](int n, int j) {
+                const int kb = n % NK;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t q_lo = RD::kmajor_lo(aS + C::ST_Q + (qn % NQ) * C::ROWT), k_lo = RD::kmajor_lo(aS + C::ST_K + kb * C::ROWT);
+#pragma unroll
+                    for (int kk = 0; kk < RT::KBLOCKS; ++kk)
+                        if (kk < p.KB)          // blocks past the true head dim are zero-filled: skipped
+                            umma_ss(t_s, RD::kmajor(q_lo, kk), RD::kmajor(k_lo, kk), IDESC_S, kk > 0);
+                    umma_ss(t_s, d_xq, xt_desc(aS + C::ST_XK + kb * XT_BYTES, aZero), IDESC_S, 1u);
+                    umma_commit(b.s_full);
+                    umma_commit(&b.k_empty[kb]);
+                    if (j == NT - 1) umma_commit(&b.q_empty[qn % NQ]);
+                }
+                __syncwarp();
+                if (j == NT - 1) ++qn;
+            };
+            auto load_v = [&](int j) {         // of the item `cur`
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(b.v_full, C::ROWT);
+                    tma_load_row_tile<DH>(sb + C::ST_V, &tm_v, b.v_full, cur.h, j * TILE, cur.bs(p));
+                }
+                __syncwarp();
+            };
+            auto issue_pv = [&](int n, int j) {
+                ok = warp_all(mbar_wait(b.v_full, n & 1, wc, 0x24));
+                if (ok) ok = warp_all(mbar_wait(b.p_ready, n & 1, wc, 0x23));
+                if (!ok) return;
+                tc_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk)
+                        umma_ts(t_pv, t_p + kk * 8, RD::mnmajor(v_lo, kk), IDESC_PV, (kk > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(b.pv_done);
+                }
+                __syncwarp();
+            };
+            // with rows in groups, the last group of a batch may lack this stream's row: skipped
+            int it = 0;
+            auto skip_missing = [&]() -> bool {
+                bool any = false;
+                for (; it < n_items && !cur.valid(p); ++it, any = true) advance(cur, s);
+                return any;
+            };
+            (void)skip_missing();
+            int j = 0, loaded = 0;
+            if (it < n_items) { load_v(0); loaded = 1; wait_s(0, 0); if (ok) issue_s(0, 0); }
+            bool more = it < n_items;
+            for (int n = 0; more && ok; ++n) {
+                int j1 = j + 1;                // the tile after this one
+                bool gap = false;              // items are missing before it
+                if (j1 == NT) { j1 = 0; ++it; advance(cur, s); gap = skip_missing(); }
+                more = it < n_items;
+                // S' of the next tile: its columns are free once the softmax has read them (HOLD), or once
+                // PV of this tile, which reads P from them, is complete.  Behind a gap Q and K do not come
+                // before the softmax has finished this item and passed the missing one's bias tiles on.
+                const bool early = C::HOLD && more && !gap;
+                auto s_free = [&]() { if (C::HOLD && ok) ok = warp_all(mbar_wait(b.s_free, n & 1, wc, 0x22)); };
+                if (early) {
+                    wait_s(n + 1, j1);
+                    s_free();
+                    if (!ok) break;
+                    issue_s(n + 1, j1);
+                }
+                issue_pv(n, j);
+                if (!ok) break;
+                if (more) {
+                    if (!early) wait_s(n + 1, j1);            // while PV runs
+                    if (ok) ok = warp_all(mbar_wait(b.pv_done, n & 1, wc, 0x25));
+                    if (!early) s_free();
+                    if (!ok) break;
+                    if (!early) issue_s(n + 1, j1);
+                    load_v(j1);
+                    ++loaded;
+                }
+                j = j1;
+            }
+            if (loaded > 0) (void)mbar_wait(b.v_full, (loaded - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x26);
         }
-        if (row == 0) tma_wait_group<0>();
     } else {
         reg_inc<C::REGS_SOFTMAX>();
-        // ------------------------------ softmax groups ------------------------------
-        const int wg = warp >> 2;            // kv columns CW*wg .. CW*wg+CW-1 of each tile
+        // ------------------------------ softmax warps of one stream ------------------------------
+        const int s = warp >> 2;
+        const FwdBars b(bars + s * C::BARS);
         const int row = tid & 127;           // q row within the tile == TMEM lane
         const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-        const uint32_t aStage = smem_u32(smem + C::OFF_STAGE);
-        const uint32_t aXch = smem_u32(smem + C::OFF_XCH);            // [parity][group][128 rows] (m, l)
-        const uint32_t aWmask = smem_u32(smem + C::OFF_WMASK) + warp * CW * 4;
+        const uint32_t tS = lane_base + C::TMEM_S + 128 * s, tPV = lane_base + C::TMEM_PV + DH * s, tP = lane_base + C::p_col(s);
         const uint32_t scratch_w = smem_u32(tmem_slot + 2);           // a word nobody reads
-        const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
-        // where this group's columns sit in the bias tile (two [128][64] sub-tiles, 16-byte chunks)
-        constexpr int CH0_MASK = 7;
-        const uint32_t bias_sub = ((CW * wg) >> 6) * SQ_SUB_BYTES;
-        const int bias_c0 = ((CW * wg) & 63) >> 3;
-        (void)CH0_MASK;
+        const float2 sc2 = make_float2(p.scale, p.scale), l2e2 = make_float2(LOG2E, LOG2E);
+        // The exp2 pass loads the special-function unit, the passes around it the other pipes.  Left alone
+        // the warps of a scheduler fall into step, all in the same pass at the same time; so the streams
+        // take turns on it, scheduler by scheduler, and a warp hands its turn on halfway through the pass (a
+        // single warp leaves the unit idle while its own multiplies and loads are in the way).
+        uint64_t* turn_mine = &b.turn[warp & 3];
+        uint64_t* turn_prev = &FwdBars(bars + (s > 0 ? s - 1 : G - 1) * C::BARS).turn[warp & 3];
         bool ok = true;
-        int g = 0;
-        float m_used = -INFINITY, l = 0.f;
+        int n = 0, r = 0;                     // tiles of the stream so far, tiles counting missing items
+        auto take_turn = [&]() {
+            // a stream may leave its pass of tile t + 1 before the one that waits for it looks at tile t: two
+            // barriers by tile parity keep the waiter within one phase
+            const int t = s > 0 ? r : r - 1;
+            if (t >= 0) ok = warp_all(mbar_wait(turn_prev + 4 * (t & 1), (t >> 1) & 1, wc, 0x38));
+        };
 
-        for (int it = 0; it < n_items && ok; ++it) {
-            int bs, qt, h;
-            decode(it, bs, qt, h);
-            m_used = -INFINITY;
-            l = 0.f;
-            for (int j = 0; j < NT && ok; ++j, ++g) {
-                const int st = g % ST;
-                const uint32_t sb = aStage + st * C::STAGE_STRIDE;
-                const int sbuf = wg + NG * (g & 1);
-                const uint32_t tS = lane_base + C::TMEM_S + (g & 1) * 128 + CW * wg;
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 0);
-                // without a staged bias tile: this thread's CW bias values of the tile, straight from
-                // global memory, requested before the wait so that they arrive while the MMA runs
-                uint4 bg[C::WIDE ? CW / 8 : 1];
-                if constexpr (C::WIDE) {
-                    const int qrow = qt * TILE + row, col0 = j * TILE + CW * wg;
-                    const __nv_bfloat16* bp =
-                        p.bias + ((static_cast<size_t>(bs / p.S) * p.H + h) * p.N + qrow) * p.N + col0;
-#pragma unroll
-                    for (int c8 = 0; c8 < CW / 8; ++c8) {
-                        bg[c8] = make_uint4(0u, 0u, 0u, 0u);
-                        if (qrow < p.N && col0 + c8 * 8 < p.N) bg[c8] = __ldg(reinterpret_cast<const uint4*>(bp + c8 * 8));
+        FwdItem cur = items_of(s);
+        for (int it = 0; it < n_items && ok; ++it, advance(cur, s)) {
+            if (!cur.valid(p)) {
+                // no such item: hand the bias tiles (if shared) and the turns on
+                for (int j = 0; j < NT && ok; ++j, ++r) {
+                    if (shared_bias) {
+                        int slot; uint32_t ph;
+                        bias_slot(s, r, slot, ph);
+                        ok = warp_all(mbar_wait(&bias_full[slot], ph, wc, 0x36));
+                        if (!ok) break;
+                        if (lane == 0) mbar_arrive(&bias_empty[slot]);
                     }
-                }
-                ok = warp_all(mbar_wait(&s_full[sbuf], (g >> 1) & 1, wc, 0x31));
-                if (!ok) break;
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 1);
-                EVO_TS(t_tile);
-                tc_fence_after();
-                uint32_t sv[2][16];
-                tmem_ld16(tS, sv[0]);
-
-                ok = warp_all(mbar_wait(&kv_full[st], (g / ST) & 1, wc, 0x32));
-                if (!ok) break;
-                uint32_t dep = 0;      // data the release of the stage must wait for
-                {
-                    // this warp's copy of the mask row slice: bf16 -> fp32 * log2e, -inf past N
-                    if constexpr (CW == 64) {
-                        const uint32_t mraw = sb + C::ST_MASK + 2 * CW * wg + 4 * lane;      // two bf16 per lane
-                        uint32_t mw;
-                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(mw) : "r"(mraw));
-                        dep = mw;
-                        const int c = j * TILE + CW * wg + 2 * lane;
-                        const float m0 = (c < p.N) ? bf16_lo(mw) * LOG2E : -INFINITY;
-                        const float m1 = (c + 1 < p.N) ? bf16_hi(mw) * LOG2E : -INFINITY;
-                        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(aWmask + 8 * lane), "f"(m0), "f"(m1) : "memory");
-                    } else {
-                        const uint32_t mraw = sb + C::ST_MASK + 2 * CW * wg + 2 * lane;      // one bf16 per lane
-                        uint16_t mw;
-                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(mw) : "r"(mraw));
-                        dep = mw;
-                        const int c = j * TILE + CW * wg + lane;
-                        const float m0 = (c < p.N) ? __uint_as_float(static_cast<uint32_t>(mw) << 16) * LOG2E : -INFINITY;
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(aWmask + 4 * lane), "f"(m0) : "memory");
-                    }
+                    take_turn();
+                    if (!ok) break;
                     __syncwarp();
+                    if (lane == 0) mbar_arrive(turn_mine + 4 * (r & 1));
                 }
-                // x = S*c1 + (bias*log2e + mask*log2e), in chunks of 16 columns; the tensor-memory
-                // load of chunk ch+1 is in flight during the arithmetic of chunk ch
-                float2 x2[CW / 2];
-                float tmx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains: ILP
-                const uint32_t sbias = sb + C::ST_BIAS + bias_sub;
+                continue;
+            }
+            float m = -INFINITY, l = 0.f;
+            for (int j = 0; j < NT; ++j, ++n, ++r) {
+                int slot; uint32_t ph;
+                bias_slot(s, r, slot, ph);
+                const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + slot * SQ_BYTES;
+                ok = warp_all(mbar_wait(&bias_full[slot], ph, wc, 0x32));      // usually there already
+                if (ok) ok = warp_all(mbar_wait(b.s_full, n & 1, wc, 0x31));
+                if (!ok) break;
+                tc_fence_after();
+                // pass 1: x = S' * scale + bias and the row maximum, 32 columns at a time
+                float2 xh[C::HOLD ? 64 : 1];
+                float tmx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                uint32_t sv[2][32];
+                tmem_ld32(tS, sv[0]);
 #pragma unroll
-                for (int ch = 0; ch < CW / 16; ++ch) {
-                    const int cb = ch & 1;
+                for (int ch = 0; ch < 4; ++ch) {
+                    uint32_t (&cv)[32] = sv[ch & 1];
+                    uint4 bv[4];
+#pragma unroll
+                    for (int q4 = 0; q4 < 4; ++q4) bv[q4] = lds128(aBias + sq_chunk_off(row, ch * 4 + q4));
                     tmem_wait_ld();
-                    if (ch + 1 < CW / 16) {
-                        tmem_ld16(tS + 16 * (ch + 1), sv[cb ^ 1]);
-                    } else if (!C::WIDE) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&s_free[sbuf]);
-                    }
-                    uint4 b0, b1;
-                    if constexpr (C::WIDE) {
-                        b0 = bg[2 * ch];
-                        b1 = bg[2 * ch + 1];
-                    } else {
-                        b0 = lds128(sbias + swz_off<128>(row, bias_c0 + 2 * ch));
-                        b1 = lds128(sbias + swz_off<128>(row, bias_c0 + 2 * ch + 1));
-                        dep ^= b0.x ^ b1.x;
-                    }
-                    const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-                    float2 mm[8];
+                    if (ch < 3) tmem_ld32(tS + 32 * (ch + 1), sv[(ch + 1) & 1]);
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4) {
-                        const float4 mv = lds128f(aWmask + 64 * ch + 16 * q4);
-                        mm[2 * q4] = make_float2(mv.x, mv.y);
-                        mm[2 * q4 + 1] = make_float2(mv.z, mv.w);
-                    }
+                        const uint32_t bw[4] = {bv[q4].x, bv[q4].y, bv[q4].z, bv[q4].w};
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float2 t2 = ffma2(bf16x2_f2(bw[k]), l2e2, mm[k]);
-                        const float2 xx = ffma2(u2f2(sv[cb][2 * k], sv[cb][2 * k + 1]), c1x2, t2);
-                        x2[ch * 8 + k] = xx;
-                        tmx[k & 3] = fmax3(tmx[k & 3], xx.x, xx.y);
+                        for (int e = 0; e < 4; ++e) {
+                            const int k = q4 * 4 + e;
+                            const float2 x = ffma2(u2f2(cv[2 * k], cv[2 * k + 1]), sc2, bf16x2_f2(bw[e]));
+                            tmx[e] = fmax3(tmx[e], x.x, x.y);
+                            if constexpr (C::HOLD) {
+                                xh[ch * 16 + k] = x;
+                            } else {
+                                cv[2 * k] = __float_as_uint(x.x);
+                                cv[2 * k + 1] = __float_as_uint(x.y);
+                            }
+                        }
                     }
+                    if constexpr (!C::HOLD) tmem_st32(tS + 32 * ch, cv);
                 }
-                mbar_release_after_loads(&kv_empty[st], dep, scratch_w);      // bias tile and mask row are read
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 2);
-
                 const float tmax = fmaxf(fmaxf(tmx[0], tmx[1]), fmaxf(tmx[2], tmx[3]));
-                const float m_new = fmaxf(m_used, tmax);
-                // When the running maximum rises (by more than EVO_FWD_LAZY), the accumulator in
-                // tensor memory and the row sum are rescaled; otherwise the tensor core simply keeps
-                // accumulating into the same tile.
-                const bool need = (j > 0) && (m_new - m_used > EVO_FWD_LAZY);
-                const float m_old = m_used;
-                if (j == 0 || need) m_used = m_new;
-                const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
-                // The exp2 pass loads the special-function unit, the passes around it the other pipes.
-                // Left alone the groups run in lockstep, all in the same pass at the same time.  At
-                // D = 32 the two halves of the groups take turns instead: the first half runs the exp2
-                // pass of tile g, then the second half runs its own, while the other half is in the
-                // fused-multiply-add pass of its next tile or in its epilogue.  The first half waits
-                // for the second half's pass of the previous tile, the second for the first's pass of
-                // this tile.  (At D = 64 taking turns measured 7 % slower: 0.736 against 0.686 ms at B=1, S=256, N=1024, H=4.)
-#ifdef EVO_FWD_NO_PINGPONG
-                constexpr bool PINGPONG = false;
-#else
-                constexpr bool PINGPONG = (DH == 32);
-#endif
-                const int half = wg / (NG / 2);
-                if (PINGPONG && (half == 1 || g > 0)) {
-                    ok = warp_all(mbar_wait(&xu_done[half ^ 1], (half == 1 ? g : g - 1) & 1, wc, 0x38));
-                    if (!ok) break;
-                }
-                // P = exp2(x - m), packed to bf16 pairs; row sum in two packed chains
-                uint32_t pk[CW / 2];
-                float rsum;
-                {
-                    const float2 nm2 = make_float2(-m_safe, -m_safe);
-                    float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-                    for (int c = 0; c < CW / 2; ++c) {
-                        const float2 d2 = fadd2(x2[c], nm2);
-                        const float2 p2 = make_float2(ex2(d2.x), ex2(d2.y));
-                        rs[c & 1] = fadd2(rs[c & 1], p2);
-                        pk[c] = pack_bf16(p2.x, p2.y);
-                    }
-                    rsum = (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
-                }
-                if (PINGPONG) {
-                    // hand the unit over; the store orders the arrive behind the last exp2 of the pass
+                if constexpr (C::HOLD) {
+                    tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) {
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(scratch_w), "r"(pk[CW / 2 - 1]) : "memory");
-                        mbar_arrive(&xu_done[half]);
+                    if (lane == 0) mbar_arrive(b.s_free);
+                }
+                // the maximum depends on every bias value read: the producer may refill the tile
+                mbar_release_after_loads(&bias_empty[slot], __float_as_uint(tmax), scratch_w);
+
+                // the exact online softmax: the largest P of a row is exp2(0) = 1, which bf16 represents
+                // exactly.  When the maximum rises, accumulator and row sum are rescaled.
+                const float m_new = fmaxf(m, tmax);
+                const bool need = (j > 0) && (m_new > m);
+                const float m_old = m;
+                m = m_new;
+                const float ms = (m == -INFINITY) ? 0.f : m;
+                const float nm = -ms * LOG2E;
+                if constexpr (C::HOLD) {
+                    // P's columns are free and the accumulator is at rest once the previous PV is complete
+                    if (n > 0) {
+                        ok = warp_all(mbar_wait(b.pv_done, (n - 1) & 1, wc, 0x33));
+                        if (!ok) break;
+                        tc_fence_after();
                     }
                 }
-
-                // The P columns in tensor memory are free, and the accumulator may be rescaled, once
-                // the previous tile's PV MMA is done.
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 3);
-                if (g > 0) {
-                    ok = warp_all(mbar_wait(&pv_full[wg], (g - 1) & 1, wc, 0x33));
-                    if (!ok) break;
-                    tc_fence_after();
-                }
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 4);
                 if (__any_sync(0xffffffffu, need)) {
-                    // rescale this group's accumulator (lanes that need nothing scale by 1)
-                    const float alpha = need ? ex2(m_old - m_safe) : 1.0f;
+                    const float alpha = need ? ex2(fmaf(m_old, LOG2E, nm)) : 1.0f;
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
                         uint32_t r[32];
-                        tmem_ld32(lane_base + C::TMEM_PV + wg * DH + c * 32, r);
+                        tmem_ld32(tPV + c * 32, r);
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
@@ -639,47 +567,143 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             r[i] = __float_as_uint(v2.x);
                             r[i + 1] = __float_as_uint(v2.y);
                         }
-                        tmem_st32(lane_base + C::TMEM_PV + wg * DH + c * 32, r);
+                        tmem_st32(tPV + c * 32, r);
                     }
                     l *= alpha;
                 }
-                l += rsum;
-                // P (bf16 pairs) into this group's columns of tensor memory
-                if constexpr (CW == 64) tmem_st32(lane_base + C::p_col(wg, g), pk);
-                else tmem_st16(lane_base + C::p_col(wg, g), pk);
+                take_turn();
+                if (!ok) break;
+                // pass 2: P = exp2(x log2e - m log2e), row sum, bf16 pairs into tensor memory
+                const float2 nm2 = make_float2(nm, nm);
+                float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                if constexpr (!C::HOLD) {
+                    tmem_wait_st();                     // x is written
+                    tmem_ld32(tS, sv[0]);
+                }
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch) {
+                    uint32_t pk[16];
+                    if constexpr (!C::HOLD) {
+                        tmem_wait_ld();
+                        if (ch < 3) tmem_ld32(tS + 32 * (ch + 1), sv[(ch + 1) & 1]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        const float2 x = C::HOLD ? xh[C::HOLD ? ch * 16 + k : 0]
+                                                 : u2f2(sv[ch & 1][2 * k], sv[ch & 1][2 * k + 1]);
+                        const float2 d2 = ffma2(x, l2e2, nm2);
+                        const float2 p2 = use_poly<C::POLY_EVERY>(k) ? ex2_poly2<5>(d2) : make_float2(ex2(d2.x), ex2(d2.y));
+                        rs[k & 1] = fadd2(rs[k & 1], p2);
+                        pk[k] = pack_bf16(p2.x, p2.y);
+                    }
+                    tmem_st16(tP + 16 * ch, pk);        // behind the columns that pass 2 has read
+                    if (ch == 1) {
+                        // the turn goes on; the store orders the arrive behind the exp2 of this chunk
+                        __syncwarp();
+                        if (lane == 0) {
+                            asm volatile("st.shared.u32 [%0], %1;" ::"r"(scratch_w), "r"(pk[15]) : "memory");
+                            mbar_arrive(turn_mine + 4 * (r & 1));
+                        }
+                    }
+                }
+                l += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&p_ready[wg]);
-                if ((warp & 3) == 0 && wg < 3) EVO_TL(p.status, 5 + wg, g, 5);
-                EVO_TE(t_tile, p.status, 0x78);
+                if (lane == 0) mbar_arrive(b.p_ready);
             }
             if (!ok) break;
-            // publish this group's (m, l) of the item for the other groups' epilogues
-            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(aXch + (((it & 1) * NG + wg) * 128 + row) * 8),
-                         "f"(m_used), "f"(l) : "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&xch_ready[(it & 1) * NG + wg]);
+            // epilogue of the item: every PV of it is complete
+            ok = warp_all(mbar_wait(b.pv_done, (n - 1) & 1, wc, 0x34));
+            if (!ok) break;
+            tc_fence_after();
+            const int bs = cur.bs(p), qt = cur.qt, h = cur.h;
+            const int qrow = qt * TILE + row;
+            const float inv = __frcp_rn(l);
+            // lane t of a quad of rows stores chunk t of each of the four: 64 contiguous bytes per row (from
+            // one thread per row, 16 bytes at a time, the stores cost 1600 clocks per item)
+            const int qrow0 = qt * TILE + (row & ~3);
+            size_t off0, rstep;
+            if constexpr (STRIDED) {
+                off0 = bs * p.lay.row + qrow0 * p.lay.n + h * p.lay.h;
+                rstep = p.lay.n;
+            } else {
+                off0 = ((static_cast<size_t>(bs) * p.N + qrow0) * p.H + h) * p.Dt;
+                rstep = static_cast<size_t>(p.H) * p.Dt;
+            }
+#pragma unroll
+            for (int c = 0; c < DH / 32; ++c) {
+                float o[32];
+                __syncwarp();
+                tmem_ld_f32<32>(tPV + c * 32, o);
+                if (c * 32 >= p.Dt) continue;          // warp-uniform
+                const int col = c * 32 + (lane & 3) * 8;
+                uint4 vo[4], vr[4];
+#pragma unroll
+                for (int c8 = 0; c8 < 4; ++c8) {
+                    uint32_t vw[4], rw[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float o0 = o[c8 * 8 + 2 * e] *= inv, o1 = o[c8 * 8 + 2 * e + 1] *= inv;
+                        vw[e] = pack_bf16(o0, o1);
+                        rw[e] = pack_bf16(o0 - bf16_lo(vw[e]), o1 - bf16_hi(vw[e]));
+                    }
+                    vo[c8] = make_uint4(vw[0], vw[1], vw[2], vw[3]);
+                    vr[c8] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+                }
+                quad_transpose(vo);
+                if (p.o_resid != nullptr) quad_transpose(vr);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (qrow0 + e < p.N && col < p.Dt) {
+                        *reinterpret_cast<uint4*>(p.o + off0 + e * rstep + col) = vo[e];
+                        // rounding residual of O
+                        if (p.o_resid != nullptr) *reinterpret_cast<uint4*>(p.o_resid + off0 + e * rstep + col) = vr[e];
+                    }
+                if constexpr (GATED) {
+                    // O * sigmoid(gate), from the unrounded O: the gate's chunks come in transposed
+                    uint4 vg[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        vg[e] = make_uint4(0u, 0u, 0u, 0u);
+                        if (qrow0 + e < p.N && col < p.Dt) vg[e] = __ldg(reinterpret_cast<const uint4*>(p.gate + off0 + e * rstep + col));
+                    }
+                    __syncwarp();
+                    quad_transpose(vg);
+#pragma unroll
+                    for (int c8 = 0; c8 < 4; ++c8) {
+                        const uint32_t gw[4] = {vg[c8].x, vg[c8].y, vg[c8].z, vg[c8].w};
+                        uint32_t ow[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
+                            const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
+                            ow[e] = pack_bf16(o[c8 * 8 + 2 * e] * s0, o[c8 * 8 + 2 * e + 1] * s1);
+                        }
+                        vg[c8] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                    }
+                    quad_transpose(vg);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (qrow0 + e < p.N && col < p.Dt)
+                            *reinterpret_cast<uint4*>(p.o_gated + off0 + e * rstep + col) = vg[e];
+                }
+            }
+            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ((m == -INFINITY) ? 0.f : m) + __logf(l);
         }
     }
 
-    if (tid == 0) EVO_TE(t_kernel, p.status, 0x7e);
     tc_fence_before();
     __syncthreads();
-    EVO_TRACE_FLUSH(p.status);
-    if (warp == W_S) tmem_dealloc(tmem, C::TMEM_COLS);
+    if (warp == C::W_PROD) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-#ifndef EVO_FWD_NG32
-#define EVO_FWD_NG32 2
-#endif
-
 // lay_in: q, k, v; lay: the output side (o, o_resid, gate, o_gated)
-template <int DH, int NG>
+template <int DH>
 static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout& lay, const void* q, const void* k, const void* v,
                       const void* bias, const void* mask, const void* gate, void* o, void* o_gated, void* o_resid,
                       float* lse, float scale, cudaStream_t st) {
-    using C = FwdCfg<DH, NG>;
+    constexpr bool WIDE = (DH == 128);
     const int BS = d->B * d->S;
     const int QT = (d->N + TILE - 1) / TILE;
 
@@ -690,7 +714,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
-    if ((rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
+    if (WIDE && (rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
 
     FwdParams p;
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
@@ -698,10 +722,13 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.KB = (Dt + 15) / 16;
     p.QT = QT;
     p.total_items = BS * QT * d->H;
-    p.c1 = ((scale > 0.f) ? scale : 1.0f / sqrtf(static_cast<float>(Dt))) * LOG2E;
+    p.scale = (scale > 0.f) ? scale : 1.0f / sqrtf(static_cast<float>(Dt));
+    p.inv_scale = 1.0f / p.scale;
+    p.c1 = p.scale * LOG2E;
     p.mask = static_cast<const __nv_bfloat16*>(mask);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.lse = lse;
+    p.o = static_cast<__nv_bfloat16*>(o);
     p.o_resid = static_cast<__nv_bfloat16*>(o_resid);
     p.gate = static_cast<const __nv_bfloat16*>(gate);
     p.o_gated = static_cast<__nv_bfloat16*>(o_gated);
@@ -711,16 +738,41 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
 
     int sms = 0;
     if ((rc = sm_count(&sms))) return rc;
-    const ActLayout cl = contiguous_layout(d->N, d->H, DH);
-    const bool strided = (lay.row != cl.row || lay.n != cl.n || lay.h != cl.h);
-    auto kernel = gate ? (strided ? evo_fwd_kernel<DH, true, NG, true> : evo_fwd_kernel<DH, false, NG, true>)
-                       : (strided ? evo_fwd_kernel<DH, true, NG, false> : evo_fwd_kernel<DH, false, NG, false>);
-    if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES))))
-        return rc;
-    const int grid = p.total_items < sms ? p.total_items : sms;
-    prof_begin(0, st);
-    kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, to, p);
-    prof_end(0, st);
+    if constexpr (WIDE) {
+        const int grid = p.total_items < sms ? p.total_items : sms;
+        using C = FwdWideCfg<DH, 2>;
+        const ActLayout cl = contiguous_layout(d->N, d->H, DH);
+        const bool strided = (lay.row != cl.row || lay.n != cl.n || lay.h != cl.h);
+        auto kernel = gate ? (strided ? evo_fwd_wide_kernel<DH, true, 2, true> : evo_fwd_wide_kernel<DH, false, 2, true>)
+                           : (strided ? evo_fwd_wide_kernel<DH, true, 2, false> : evo_fwd_wide_kernel<DH, false, 2, false>);
+        if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
+        prof_begin(0, st);
+        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, to, p);
+        prof_end(0, st);
+    } else {
+        using C = FwdCfg<DH>;
+        // Streams share bias tiles (rows taken G at a time) when that leaves no SM with more rounds of work
+        // than separate items would.
+        const int sg = (d->S + C::G - 1) / C::G;
+        const long units = static_cast<long>(d->B) * sg * QT * d->H;
+        const long apart = (static_cast<long>(p.total_items) + static_cast<long>(C::G) * sms - 1) / (static_cast<long>(C::G) * sms);
+        p.shared_bias = 0;
+        p.NG = d->S;
+        if ((units + sms - 1) / sms * 16 <= apart * 17 && p.total_items > sms) {
+            p.shared_bias = 1;
+            p.NG = sg;
+            p.total_items = static_cast<int>(units);
+        }
+        const int grid = p.total_items < sms ? p.total_items : sms;
+        const ActLayout cl = contiguous_layout(d->N, d->H, Dt);
+        const bool strided = (lay.row != cl.row || lay.n != cl.n || lay.h != cl.h);
+        auto kernel = gate ? (strided ? evo_fwd_kernel<DH, true, true> : evo_fwd_kernel<DH, false, true>)
+                           : (strided ? evo_fwd_kernel<DH, true, false> : evo_fwd_kernel<DH, false, false>);
+        if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
+        prof_begin(0, st);
+        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, p);
+        prof_end(0, st);
+    }
     return cuda_err(cudaGetLastError());
 }
 
@@ -765,11 +817,11 @@ extern "C" int evo_fwd_views(const EvoDims* dims, const EvoStrides* s_qkv, const
     if ((rc = evo::ensure_context())) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dims->D <= 32)
-        return evo::launch_fwd<32, EVO_FWD_NG32>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated,
+        return evo::launch_fwd<32>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated,
                                                  o_resid, lse, scale, st);
     if (dims->D <= 64)
-        return evo::launch_fwd<64, 2>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated, o_resid, lse,
+        return evo::launch_fwd<64>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated, o_resid, lse,
                                       scale, st);
-    return evo::launch_fwd<128, 2>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated, o_resid, lse,
+    return evo::launch_fwd<128>(dims, lay_in, lay, q, k, v, pair_bias, res_mask, gate, o, o_gated, o_resid, lse,
                                    scale, st);
 }

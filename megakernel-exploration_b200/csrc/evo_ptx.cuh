@@ -72,6 +72,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  "r"(bytes)
                  : "memory");
 }
+// The transaction count alone, without the arrival: for a phase that other writes complete later.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -519,23 +523,32 @@ __device__ __forceinline__ float ex2(float x) {
 }
 // 2^x for x <= 0 (any magnitude, -inf included) on the fused-multiply-add pipe instead of
 // the special-function unit, two values at a time: x = n + f with n = round(x), f in
-// [-0.5, 0.5]; 2^f by a cubic (minimax, relative error 7.5e-5, far below the bf16 rounding
-// the result goes through); 2^n by adding n to the exponent field.  Adding 1.5 * 2^23
+// [-0.5, 0.5]; 2^f by a polynomial that minimises the largest relative error (least squares on
+// Chebyshev nodes, reweighted): degree 3 7.5e-5, far below a bf16 rounding; degree 5 2.3e-7, what
+// ex2.approx itself guarantees.  2^n by adding n to the exponent field.  Adding 1.5 * 2^23
 // rounds to the nearest integer and leaves it in the low mantissa bits.  A loop that is
 // bound by the special-function unit can hand every k-th column pair to this routine so that
-// both pipes work at the same time.  Measured at B=1, S=512, N=384, H=8, D=32: the dBias kernel,
-// whose arithmetic is little more than the exp2, gains 8 % with every fourth pair (0.218 ->
-// 0.200 ms); the forward and the dQ/dK/dV kernel, which are not bound by that unit, gain nothing
-// (every third pair) or lose (every second: 0.441 -> 0.478 ms and 0.480 -> 0.533 ms).
+// both pipes work at the same time; a pair costs about 16 clocks of a scheduler either way.
+template <int DEG>
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
+    static_assert(DEG == 3 || DEG == 5, "degree 3 or 5");
     x.x = fmaxf(x.x, -126.0f);
     x.y = fmaxf(x.y, -126.0f);
     const float2 xf = __fadd2_rn(x, make_float2(12582912.0f, 12582912.0f));
     const float2 n = __fadd2_rn(xf, make_float2(-12582912.0f, -12582912.0f));
     const float2 f = __ffma2_rn(n, make_float2(-1.0f, -1.0f), x);
-    float2 p = __ffma2_rn(f, make_float2(0.0551714588f, 0.0551714588f), make_float2(0.242610862f, 0.242610862f));
-    p = __ffma2_rn(p, f, make_float2(0.693260992f, 0.693260992f));
-    p = __ffma2_rn(p, f, make_float2(0.99992809f, 0.99992809f));
+    float2 p;
+    if constexpr (DEG == 3) {
+        p = __ffma2_rn(f, make_float2(0.0551714588f, 0.0551714588f), make_float2(0.242610862f, 0.242610862f));
+        p = __ffma2_rn(p, f, make_float2(0.693260992f, 0.693260992f));
+        p = __ffma2_rn(p, f, make_float2(0.99992809f, 0.99992809f));
+    } else {
+        p = __ffma2_rn(f, make_float2(0.001327647013f, 0.001327647013f), make_float2(0.009675540961f, 0.009675540961f));
+        p = __ffma2_rn(p, f, make_float2(0.05550713092f, 0.05550713092f));
+        p = __ffma2_rn(p, f, make_float2(0.2402212024f, 0.2402212024f));
+        p = __ffma2_rn(p, f, make_float2(0.693146944f, 0.693146944f));
+        p = __ffma2_rn(p, f, make_float2(1.000000119f, 1.000000119f));
+    }
     float2 r;
     r.x = __uint_as_float(__float_as_uint(p.x) + (__float_as_uint(xf.x) << 23));
     r.y = __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(xf.y) << 23));
