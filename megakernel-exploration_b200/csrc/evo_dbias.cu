@@ -33,11 +33,8 @@
 
 namespace evo {
 
-// every fourth column pair takes its exp2 on the fused-multiply-add pipe (see ex2_poly2)
-#ifndef EVO_DBIAS_POLY_EVERY
-#define EVO_DBIAS_POLY_EVERY 4
-#endif
-constexpr int DBIAS_POLY_EVERY = EVO_DBIAS_POLY_EVERY;
+// Every third column pair takes its exp2 on the fused-multiply-add pipe (see ex2_poly2).
+constexpr int DBIAS_POLY_EVERY = 3;
 
 template <int DH, int NG>
 struct DbCfg {
@@ -48,10 +45,8 @@ struct DbCfg {
     // (the per-thread cap ptxas derives from the launch bound, times THREADS); an
     // increase blocks until the pool has room, for ever if it never can.
     static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
-    // measured (B=1, S=512, N=384, H=8, D=32 / B=1, S=256, N=1024, H=4, D=64): 224/56 0.200 / 0.394 ms,
-    // 216/72 0.195 / 0.380, 208/88 0.213 / 0.409
-    static constexpr int REGS_COMPUTE = (NG == 2) ? 216 : 112;
-    static constexpr int REGS_OTHER = (NG == 2) ? 72 : 32;
+    static constexpr int REGS_COMPUTE = 112;
+    static constexpr int REGS_OTHER = 32;
     static_assert(REGS_COMPUTE * NCW * 32 + REGS_OTHER * 128 <= REGS_LAUNCH * THREADS, "register pool");
     // D <= 64: a stage holds the four operand tiles of a step.  D = 128 (four tiles are 128 KB):
     // a stage holds ONE operand pair, (Q, K) of a step or (dO, V) of a step, alternately; each of
@@ -62,7 +57,6 @@ struct DbCfg {
     static constexpr uint32_t ST_Q = 0, ST_DO = (SPLIT == 2) ? 0 : ROWT;
     static constexpr uint32_t ST_K = (SPLIT == 2) ? ROWT : 2 * ROWT, ST_V = (SPLIT == 2) ? ROWT : 3 * ROWT;
     static constexpr uint32_t ST_XQ = (4 / SPLIT) * ROWT, ST_XK = ST_XQ + XT_BYTES;     // extra tiles of the step
-    static constexpr uint32_t STAGE_TX = 4 * ROWT + 2 * XT_BYTES;            // SPLIT == 1
     static constexpr uint32_t STAGE_STRIDE = (4 / SPLIT) * ROWT + 2 * XT_BYTES;
     // constant extra tiles, above every stage (the zero tile must sit above the tiles that refer to it)
     static constexpr uint32_t OFF_XDP = QS * STAGE_STRIDE;                    // column selector of -delta
@@ -122,7 +116,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 2); }
+        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 2); mbar_init(&st_empty[i], 2); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sdp_full[i], 2); mbar_init(&sdp_free[i], NCW); }
         fence_mbar_init();
         fence_async_smem();
@@ -167,45 +161,51 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
     if (warp >= NCW) {
         reg_dec<C::REGS_OTHER>();
-        if (warp == NCW) {
-            if (lane == 0) {
-                // ------------------------------ producer ------------------------------
-                bool ok = true;
-                int gs = 0;
-                for (int it = 0; it < n_items && ok; ++it) {
-                    const DbItem x = decode(it);
-                    for (int n = 0; n < x.ns && ok; ++n, ++gs) {
-                        const int bs = x.b * p.S + x.s0 + n;
-                        const size_t ro = (static_cast<size_t>(bs) * p.H + x.h) * p.NTP + x.i * TILE;
+        if (warp == NCW || warp == NCW + 3) {
+            // ------------------------------ producers ------------------------------
+            // One warp loads the q-side tiles (Q, dO, extra tile of the q rows), the other the kv-side tiles
+            // (K, V, extra tile of the kv rows) of every stage; each warp runs the loop with all lanes and
+            // elects one to issue.  A bulk load costs its issuer about 60 clocks and a stage's bookkeeping
+            // about 300: from one divergent thread the six loads of a step took longer than its arithmetic.
+            const bool kv_side = (warp != NCW);
+            const CUtensorMap* tm_s = kv_side ? &tm_k : &tm_q;
+            const CUtensorMap* tm_dp = kv_side ? &tm_v : &tm_do;
+            bool ok = true;
+            int ld = 0, st = 0;
+            uint32_t ph = 1;                 // parity of the release that frees stage st for this load
+            for (int it = 0; it < n_items && ok; ++it) {
+                const DbItem x = decode(it);
+                const int n0 = (kv_side ? x.j : x.i) * TILE;
+                int bs = x.b * p.S + x.s0;
+                // extra tiles: [B*S][H][NTP] for the q rows, [B*S][NTP] for the kv rows
+                const __nv_bfloat16* xp = kv_side ? p.xk + (static_cast<size_t>(bs) * p.NTP + n0) * 8
+                                                  : p.xq + ((static_cast<size_t>(bs) * p.H + x.h) * p.NTP + n0) * 8;
+                const size_t xstep = static_cast<size_t>(kv_side ? 1 : p.H) * p.NTP * 8;
+                for (int n = 0; n < x.ns && ok; ++n, ++bs, xp += xstep) {
 #pragma unroll
-                        for (int hf = 0; hf < C::SPLIT; ++hf) {
-                            const int ld = gs * C::SPLIT + hf;        // running load counter
-                            const int st = ld % QS;
-                            if (ld >= QS) ok = mbar_wait(&st_empty[st], ((ld / QS) - 1) & 1, wc, 0x82);
-                            if (!ok) break;
+                    for (int hf = 0; hf < C::SPLIT; ++hf, ++ld) {
+                        if (ld >= QS) ok = warp_all(mbar_wait(&st_empty[st], ph, wc, 0x82));
+                        if (!ok) break;
+                        if (elect_one()) {
                             uint8_t* sb = smem + st * C::STAGE_STRIDE;
                             const bool with_s = (C::SPLIT == 1 || hf == 0), with_dp = (C::SPLIT == 1 || hf == 1);
-                            mbar_arrive_expect_tx(&st_full[st], C::SPLIT == 1 ? C::STAGE_TX
-                                                                             : 2 * C::ROWT + (hf == 0 ? 2 : 1) * XT_BYTES);
-                            if (with_s) {
-                                tma_load_row_tile<DH>(sb + C::ST_Q, &tm_q, &st_full[st], x.h, x.i * TILE, bs);
-                                tma_load_row_tile<DH>(sb + C::ST_K, &tm_k, &st_full[st], x.h, x.j * TILE, bs);
-                                bulk_load(sb + C::ST_XK, p.xk + (static_cast<size_t>(bs) * p.NTP + x.j * TILE) * 8,
-                                          XT_BYTES, &st_full[st]);
-                            }
-                            if (with_dp) {
-                                tma_load_row_tile<DH>(sb + C::ST_DO, &tm_do, &st_full[st], x.h, x.i * TILE, bs);
-                                tma_load_row_tile<DH>(sb + C::ST_V, &tm_v, &st_full[st], x.h, x.j * TILE, bs);
-                            }
-                            bulk_load(sb + C::ST_XQ, p.xq + ro * 8, XT_BYTES, &st_full[st]);
+                            // the extra tile of the kv rows belongs to S' alone, that of the q rows to both products
+                            const bool with_x = with_s || !kv_side;
+                            mbar_arrive_expect_tx(&st_full[st], (with_s + with_dp) * C::ROWT + with_x * XT_BYTES);
+                            if (with_s)
+                                tma_load_row_tile<DH>(sb + (kv_side ? C::ST_K : C::ST_Q), tm_s, &st_full[st], x.h, n0, bs);
+                            if (with_dp)
+                                tma_load_row_tile<DH>(sb + (kv_side ? C::ST_V : C::ST_DO), tm_dp, &st_full[st], x.h, n0, bs);
+                            if (with_x) bulk_load(sb + (kv_side ? C::ST_XK : C::ST_XQ), xp, XT_BYTES, &st_full[st]);
                         }
+                        __syncwarp();
+                        if (++st == QS) { st = 0; ph ^= 1u; }
                     }
                 }
-                // the most recent loads have landed before the CTA exits
-                const int loads = gs * C::SPLIT;
-                for (int k = (loads > QS ? loads - QS : 0); k < loads; ++k)
-                    (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, wc, 0x83);
             }
+            // the most recent loads have landed before the CTA exits
+            for (int k = (ld > QS ? ld - QS : 0); k < ld; ++k)
+                (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, wc, 0x83);
         } else if (warp == NCW + 1 || warp == NCW + 2) {
             // ------------------------------ mma issuers ------------------------------
             // warp NCW+1 issues S' = Q K^T + extra block, warp NCW+2 issues dP' = dO V^T + extra
@@ -365,15 +365,16 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (warp == NCW + 1) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-#ifndef EVO_DBIAS_GROUPS
-#define EVO_DBIAS_GROUPS 2
-#endif
+// Four groups of 32 columns: a step's arithmetic alone takes a CTA 1010 clocks with four warps per
+// scheduler and 1545 with two of 64 columns, which cannot hide their own latencies (B=1, S=512, N=384, H=8,
+// D=32: 0.193 -> 0.177 ms; B=1, S=256, N=1024, H=4, D=64: 0.383 -> 0.371).
+constexpr int DBIAS_GROUPS = 4;
 
 template <int DH>
 static int launch_dbias_t(const EvoDims* d, const ActLayout& lay, const ActLayout& lay_do, const void* q, const void* k, const void* v, const void* bias,
                           const void* d_o, const void* xq, const void* xk,
                           float* dbias, float scale, int sms, cudaStream_t st) {
-    constexpr int NG = EVO_DBIAS_GROUPS;
+    constexpr int NG = DBIAS_GROUPS;
     using C = DbCfg<DH, NG>;
     const int BS = d->B * d->S;
     const int NT = (d->N + TILE - 1) / TILE;
