@@ -199,6 +199,28 @@ int evo_bwd_views(const EvoDims* dims, const EvoStrides* s_qkv, const EvoStrides
                   void* d_gate, float* dbias, void* workspace, size_t workspace_bytes, float scale,
                   unsigned phases, int reserved_sms, void* stream);
 
+/* The backward with every option in one structure: evo_bwd_views plus the type of d_pair_bias.
+ * With dbias_bf16, dbias is bf16 [B][H][N][N] (the sum over S is still formed in fp32 and
+ * rounded once; the reference rounds in a separate pass, evo_h100/tk_evo_attention_layer.py:176),
+ * and both phases must be requested. */
+typedef struct EvoBwdArgs {
+    EvoDims dims;
+    const EvoStrides *s_qkv, *s_out, *s_grad;   /* NULL = contiguous */
+    const void *q, *k, *v, *pair_bias, *res_mask, *gate, *o, *o_resid;
+    const float* lse;
+    const void* d_out;
+    void *dq, *dk, *dv, *d_gate, *dbias;
+    int dbias_bf16;
+    void* workspace;
+    size_t workspace_bytes;
+    float scale;
+    unsigned phases;
+    int reserved_sms;
+    void* stream;
+} EvoBwdArgs;
+int evo_bwd_ex(const EvoBwdArgs* args);
+size_t evo_bwd_ex_workspace_bytes(const EvoDims* dims, int gated, int dbias_bf16);
+
 /* Reads (and clears) the device status word that kernels set when a bounded
  * wait gives up.  Synchronises the device.  Returns EVO_OK, EVO_ERR_DEVICE_WAIT
  * (raw word in *raw if non-NULL) or EVO_ERR_CUDA.  The reference has no

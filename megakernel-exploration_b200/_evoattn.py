@@ -51,6 +51,8 @@ SYMBOLS = {
     "evo_bwd_gated": (C.c_int, [C.POINTER(EvoDims), C.POINTER(EvoStrides)] + [C.c_void_p] * 16
                       + [C.c_size_t, C.c_float, C.c_uint, C.c_int, C.c_void_p]),
     "evo_bwd_gated_workspace_bytes": (C.c_size_t, [C.POINTER(EvoDims)]),
+    "evo_bwd_ex": (C.c_int, [C.c_void_p]),                       # called from the native operator
+    "evo_bwd_ex_workspace_bytes": (C.c_size_t, [C.POINTER(EvoDims), C.c_int, C.c_int]),
     "evo_bwd_workspace_bytes": (C.c_size_t, [C.POINTER(EvoDims)]),
     "evo_bwd": (C.c_int, [C.POINTER(EvoDims)] + [C.c_void_p] * 14 + [C.c_size_t, C.c_float, C.c_void_p]),
     "evo_bwd_static_scratch_capacity": (C.c_size_t, []),

@@ -12,11 +12,12 @@
 //   1. bwd_prep_kernel    delta and the extra tiles through which the main kernels add
 //                         (mask - LSE) / scale to S and -delta to dP inside the tensor
 //                         core (evo_tiles.cuh, "EXTRA TILE"), padded to whole tiles so
-//                         the main kernels need no edge predicates
+//                         the main kernels need no edge predicates; zeroes the accumulators
 //   2. evo_dbias_kernel   dBias (evo_dbias.cu): one CTA per pair-bias tile keeps its
 //                         sum over the S rows in registers, no reduction traffic
 //   3. evo_bwd_kernel     dQ, dK, dV (below)
-//   4. cvt_dq_kernel      fp32 dQ accumulator -> bf16 dQ in the caller layout
+//   4. bwd_finish_kernel  fp32 dQ accumulator -> bf16 dQ in the caller layout (and dBias,
+//                         summed over slices of S in fp32, to bf16 if the caller wants that)
 //
 // evo_bwd_kernel: one persistent CTA per SM walks items (chunk of RC consecutive
 // S rows, head h, kv tile j of 128 residues); per item it walks steps
@@ -128,7 +129,7 @@ struct BwdParams {
     const __nv_bfloat16* xq;   // [B*S][H][NTP][8] extra tiles of the q rows  (bwd_prep_kernel)
     const __nv_bfloat16* xk;   // [B*S][NTP][8]    extra tiles of the kv rows
     const __nv_bfloat16* bias; // [B][H][N][N] (read directly when the bias tile is not staged)
-    float* dbias;              // [B][H][N][N] (written by this kernel only when S = 1)
+    void* dbias;               // [B][H][N][N], fp32 or bf16 (written by this kernel only when S = 1)
     __nv_bfloat16* dk;    // activation layout `lay`
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
@@ -140,9 +141,10 @@ struct BwdItem {
 };
 
 // DBIAS_HERE (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
-// fp32 dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
+// dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
 // per item) is not launched.
-template <int DH, bool DBIAS_HERE>
+enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2 };
+template <int DH, int DBIAS_HERE>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -562,16 +564,28 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         pkd[ch * 8 + k] = pack_bf16(ds2.x, ds2.y);
                         dsv[k] = ds2;
                     }
-                    if constexpr (DBIAS_HERE) {
+                    if constexpr (DBIAS_HERE != DBIAS_NO) {
                         // one S row: this step's dS tile is the dBias tile (q tile n, kv tile j)
                         const int qrow = (n / x.nr) * TILE + row, c0 = x.j * TILE + 64 * wg + 16 * ch;
                         if (qrow < p.N) {
-                            float* out = p.dbias + ((static_cast<size_t>(x.b) * p.H + x.h) * p.N + qrow) * p.N + c0;
+                            const size_t at = ((static_cast<size_t>(x.b) * p.H + x.h) * p.N + qrow) * p.N + c0;
+                            if constexpr (DBIAS_HERE == DBIAS_F32) {
+                                float* out = static_cast<float*>(p.dbias) + at;
 #pragma unroll
-                            for (int q4 = 0; q4 < 4; ++q4)
-                                if (c0 + q4 * 4 < p.N)
-                                    *reinterpret_cast<float4*>(out + q4 * 4) =
-                                        make_float4(dsv[2 * q4].x, dsv[2 * q4].y, dsv[2 * q4 + 1].x, dsv[2 * q4 + 1].y);
+                                for (int q4 = 0; q4 < 4; ++q4)
+                                    if (c0 + q4 * 4 < p.N)
+                                        *reinterpret_cast<float4*>(out + q4 * 4) =
+                                            make_float4(dsv[2 * q4].x, dsv[2 * q4].y, dsv[2 * q4 + 1].x, dsv[2 * q4 + 1].y);
+                            } else {
+                                // the bf16 pairs are the ones the MMAs read
+                                __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.dbias) + at;
+#pragma unroll
+                                for (int q8 = 0; q8 < 2; ++q8)
+                                    if (c0 + q8 * 8 < p.N)
+                                        *reinterpret_cast<uint4*>(out + q8 * 8) =
+                                            make_uint4(pkd[ch * 8 + q8 * 4], pkd[ch * 8 + q8 * 4 + 1], pkd[ch * 8 + q8 * 4 + 2],
+                                                       pkd[ch * 8 + q8 * 4 + 3]);
+                            }
                         }
                     }
                 }
@@ -634,109 +648,161 @@ __device__ __forceinline__ uint32_t split_bf16(float v) {
 // sig = sigmoid(gate), writes the gradient that enters the attention, bf16(d_o * sig), to do_att
 // (contiguous [B*S][N][H][Dt], what the main kernels read as their dO) and the gate's gradient
 // d_o * O * sig * (1 - sig) to d_gate, and takes delta from the rounded do_att.
-template <int DH>
-__global__ void bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ o_resid,
-                                const __nv_bfloat16* __restrict__ d_o, const float* __restrict__ lse,
-                                const __nv_bfloat16* __restrict__ mask, uint4* __restrict__ xq,
-                                uint4* __restrict__ xk, float inv_scale, int BS, int N, int H,
-                                int NTP, ActLayout lay, int Dt, const __nv_bfloat16* __restrict__ gate,
-                                __nv_bfloat16* __restrict__ do_att, __nv_bfloat16* __restrict__ d_gate) {
+//
+// Bound by DRAM: it reads O, its residual and dO once and also zeroes the accumulators of the later
+// kernels (`zero`, n_zero 16-byte words), which saves two memset launches.  Dt / 8 lanes share a row
+// (one 16-byte chunk each) and rows are walked in the order they lie in memory, so that a warp's loads
+// are contiguous.
+struct PrepParams {
+    const __nv_bfloat16 *o, *o_resid, *d_o, *mask, *gate;
+    const float* lse;
+    uint4 *xq, *xk;
+    __nv_bfloat16 *do_att, *d_gate;
+    uint4* zero[2];
+    size_t n_zero[2];
+    float inv_scale;
+    int BS, N, H, NTP, Dt;
+    ActLayout lay;
+};
+template <int LANES>      // lanes per row: the power of two at or above Dt / 8
+__global__ void __launch_bounds__(256) bwd_prep_kernel(const PrepParams p) {
     constexpr uint32_t ONES = 0x3f803f80u;     // bf16 (1, 1)
-    const size_t rows = static_cast<size_t>(BS) * N * H;
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    for (size_t idx = t0; idx < rows; idx += gstride) {
-        const int h = static_cast<int>(idx % H);
-        const size_t bn = idx / H;
-        const int n = static_cast<int>(bn % N);
-        const size_t bs = bn / N;
-        const size_t off = bs * lay.row + static_cast<size_t>(n) * lay.n + static_cast<size_t>(h) * lay.h;
-        const uint4* po = reinterpret_cast<const uint4*>(o + off);
-        const uint4* pr = o_resid ? reinterpret_cast<const uint4*>(o_resid + off) : nullptr;
-        const uint4* pd = reinterpret_cast<const uint4*>(d_o + off);
-        const uint4* pg = gate ? reinterpret_cast<const uint4*>(gate + off) : nullptr;
+    const int N = p.N, H = p.H, NTP = p.NTP;
+    const size_t rows = static_cast<size_t>(p.BS) * N * H;
+    const int c = static_cast<int>(t0 % LANES);      // this lane's chunk of eight head-dim columns
+    const bool have = c * 8 < p.Dt;
+    // which of the two outer axes lies closer together in memory
+    const bool n_inner = p.lay.n <= p.lay.row;
+    const uint32_t inner = n_inner ? N : p.BS;
+    const size_t rstride = gstride / LANES;
+    // (whole warps run the same number of iterations: the shuffles need all lanes)
+    for (size_t r0 = (t0 - (threadIdx.x & 31)) / LANES; r0 < rows; r0 += rstride) {
+        const size_t r = r0 + (threadIdx.x & 31) / LANES;
+        const bool live = r < rows;
         float s = 0.f;
-#pragma unroll
-        for (int c = 0; c < DH / 8; ++c) {
-            if (c * 8 >= Dt) break;
-            const uint4 a = po[c];
-            uint4 b = pd[c];
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-            uint32_t rw[4] = {0u, 0u, 0u, 0u};
-            if (pr) {
-                const uint4 rr = pr[c];
-                rw[0] = rr.x; rw[1] = rr.y; rw[2] = rr.z; rw[3] = rr.w;
+        size_t ro = 0, lo = 0;
+        if (live) {
+            size_t bn;
+            uint32_t h, in_, out_;
+            if (rows < 0x80000000ull) {              // 32-bit divisions where they suffice
+                const uint32_t r32 = static_cast<uint32_t>(r), b32 = r32 / H;
+                h = r32 - b32 * H;
+                out_ = b32 / inner;
+                in_ = b32 - out_ * inner;
+            } else {
+                bn = r / H;
+                h = static_cast<uint32_t>(r - bn * H);
+                out_ = static_cast<uint32_t>(bn / inner);
+                in_ = static_cast<uint32_t>(bn - static_cast<size_t>(out_) * inner);
             }
-            if (pg) {
-                const uint4 g4 = pg[c];
-                const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, dw[4] = {b.x, b.y, b.z, b.w};
-                uint32_t aw2[4], gg[4];
+            const size_t bs = n_inner ? out_ : in_, n = n_inner ? in_ : out_;
+            const size_t off = bs * p.lay.row + n * p.lay.n + h * p.lay.h + c * 8;
+            ro = (bs * H + h) * NTP + n;
+            lo = (bs * H + h) * N + n;
+            if (have) {
+                const uint4 a = __ldg(reinterpret_cast<const uint4*>(p.o + off));
+                uint4 b = __ldg(reinterpret_cast<const uint4*>(p.d_o + off));
+                const uint4 rr = p.o_resid ? __ldg(reinterpret_cast<const uint4*>(p.o_resid + off)) : make_uint4(0u, 0u, 0u, 0u);
+                const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, rw[4] = {rr.x, rr.y, rr.z, rr.w};
+                if (p.gate) {
+                    const uint4 g4 = __ldg(reinterpret_cast<const uint4*>(p.gate + off));
+                    const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, dw[4] = {b.x, b.y, b.z, b.w};
+                    uint32_t aw2[4], gg[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
+                        const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
+                        const float d0 = bf16_lo(dw[e]), d1 = bf16_hi(dw[e]);
+                        const float o0 = bf16_lo(aw[e]) + bf16_lo(rw[e]), o1 = bf16_hi(aw[e]) + bf16_hi(rw[e]);
+                        aw2[e] = pack_bf16(d0 * s0, d1 * s1);
+                        gg[e] = pack_bf16(d0 * o0 * s0 * (1.0f - s0), d1 * o1 * s1 * (1.0f - s1));
+                    }
+                    b = make_uint4(aw2[0], aw2[1], aw2[2], aw2[3]);
+                    *reinterpret_cast<uint4*>(p.do_att + ((bs * N + n) * H + h) * static_cast<size_t>(p.Dt) + c * 8) = b;
+                    *reinterpret_cast<uint4*>(p.d_gate + off) = make_uint4(gg[0], gg[1], gg[2], gg[3]);
+                }
+                const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
-                    const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
-                    const float d0 = bf16_lo(dw[e]), d1 = bf16_hi(dw[e]);
-                    const float o0 = bf16_lo(aw[e]) + bf16_lo(rw[e]), o1 = bf16_hi(aw[e]) + bf16_hi(rw[e]);
-                    aw2[e] = pack_bf16(d0 * s0, d1 * s1);
-                    gg[e] = pack_bf16(d0 * o0 * s0 * (1.0f - s0), d1 * o1 * s1 * (1.0f - s1));
+                    s = fmaf(bf16_lo(aw[e]) + bf16_lo(rw[e]), bf16_lo(bw[e]), s);
+                    s = fmaf(bf16_hi(aw[e]) + bf16_hi(rw[e]), bf16_hi(bw[e]), s);
                 }
-                b = make_uint4(aw2[0], aw2[1], aw2[2], aw2[3]);
-                reinterpret_cast<uint4*>(do_att + ((bs * N + n) * H + h) * static_cast<size_t>(Dt))[c] = b;
-                reinterpret_cast<uint4*>(d_gate + off)[c] = make_uint4(gg[0], gg[1], gg[2], gg[3]);
-            }
-            const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                s = fmaf(bf16_lo(aw[e]) + bf16_lo(rw[e]), bf16_lo(bw[e]), s);
-                s = fmaf(bf16_hi(aw[e]) + bf16_hi(rw[e]), bf16_hi(bw[e]), s);
             }
         }
-        const size_t ro = (bs * H + h) * NTP + n;
-        xq[ro] = make_uint4(ONES, split_bf16(-lse[(bs * H + h) * N + n] * inv_scale), split_bf16(-s), 0u);
+#pragma unroll
+        for (int d = 1; d < LANES; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (live && c == 0) p.xq[ro] = make_uint4(ONES, split_bf16(-p.lse[lo] * p.inv_scale), split_bf16(-s), 0u);
     }
     // padding of the per-row tiles, and the per-column tiles
     const int pad = NTP - N;
-    const size_t npad = static_cast<size_t>(BS) * H * pad;
+    const size_t npad = static_cast<size_t>(p.BS) * H * pad;
     for (size_t idx = t0; idx < npad; idx += gstride) {
         const size_t bh = idx / pad;
         const int n = N + static_cast<int>(idx % pad);
-        xq[bh * NTP + n] = make_uint4(ONES, split_bf16(-1e30f), 0u, 0u);
+        p.xq[bh * NTP + n] = make_uint4(ONES, split_bf16(-1e30f), 0u, 0u);
     }
-    const size_t nmask = static_cast<size_t>(BS) * NTP;
+    const size_t nmask = static_cast<size_t>(p.BS) * NTP;
     for (size_t idx = t0; idx < nmask; idx += gstride) {
         const size_t bs = idx / NTP;
         const int n = static_cast<int>(idx % NTP);
-        const float m = (n < N) ? __bfloat162float(mask[bs * N + n]) * inv_scale : -1e30f;
-        xk[idx] = make_uint4(split_bf16(m), ONES, 0u, 0u);
+        const float m = (n < N) ? __bfloat162float(p.mask[bs * N + n]) * p.inv_scale : -1e30f;
+        p.xk[idx] = make_uint4(split_bf16(m), ONES, 0u, 0u);
     }
+#pragma unroll
+    for (int z = 0; z < 2; ++z)
+        for (size_t i = t0; i < p.n_zero[z]; i += gstride) p.zero[z][i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// fp32 accumulator [B*S][N][H][D] (contiguous) -> bf16 dQ in the activation layout, 8 elements per thread
+// The results that were accumulated in fp32, in their final type: dQ ([B*S][N][H][DH] contiguous) -> bf16 in
+// the activation layout, and dBias -> bf16 if the caller wants it so.  Eight elements per thread.
+struct FinishParams {
+    const float* dq_acc;
+    __nv_bfloat16* dq;
+    size_t n8;                 // groups of eight of dq_acc
+    int N, H, Dt;
+    ActLayout lay;
+    const float* dbias_acc;    // nullptr: dBias is final already
+    __nv_bfloat16* dbias;
+    size_t nb8;
+};
+__device__ __forceinline__ uint4 cvt8(const float* src) {
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(src)), b = __ldcs(reinterpret_cast<const float4*>(src) + 1);
+    return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+}
 template <int DH>
-__global__ void cvt_dq_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n8, int N, int H,
-                              ActLayout lay, int Dt) {
+__global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += gstride) {
-        const float4 a = reinterpret_cast<const float4*>(src)[2 * i];
-        const float4 b = reinterpret_cast<const float4*>(src)[2 * i + 1];
-        uint4 u;
-        u.x = pack_bf16(a.x, a.y); u.y = pack_bf16(a.z, a.w);
-        u.z = pack_bf16(b.x, b.y); u.w = pack_bf16(b.z, b.w);
+    const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (size_t i = t0; i < p.n8; i += gstride) {
         const size_t rowi = i / (DH / 8);                 // (bs, n, h) of this group of eight
         const int d8 = static_cast<int>(i % (DH / 8));
-        if (d8 * 8 >= Dt) continue;
-        const int h = static_cast<int>(rowi % H);
-        const size_t bn = rowi / H;
-        const size_t off = (bn / N) * lay.row + (bn % N) * lay.n + static_cast<size_t>(h) * lay.h + d8 * 8;
-        *reinterpret_cast<uint4*>(dst + off) = u;
+        if (d8 * 8 >= p.Dt) continue;
+        const uint4 u = cvt8(p.dq_acc + 8 * i);
+        size_t bs, n, h;
+        if (p.n8 < 0x80000000ull) {
+            const uint32_t r32 = static_cast<uint32_t>(rowi), b32 = r32 / p.H, s32 = b32 / p.N;
+            h = r32 - b32 * p.H;
+            n = b32 - s32 * p.N;
+            bs = s32;
+        } else {
+            const size_t bn = rowi / p.H;
+            h = rowi - bn * p.H;
+            bs = bn / p.N;
+            n = bn - bs * p.N;
+        }
+        *reinterpret_cast<uint4*>(p.dq + bs * p.lay.row + n * p.lay.n + h * p.lay.h + d8 * 8) = u;
     }
+    if (p.dbias_acc)
+        for (size_t i = t0; i < p.nb8; i += gstride) reinterpret_cast<uint4*>(p.dbias)[i] = cvt8(p.dbias_acc + 8 * i);
 }
 
 struct BwdWorkspace {
-    size_t off_xq, off_xk, off_dq, off_do, total;
+    size_t off_xq, off_xk, off_dq, off_do, off_db, total;
 };
 
-static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false) {
+static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false, bool dbias_bf16 = false) {
     const size_t BS = static_cast<size_t>(d->B) * d->S;
     const size_t NTP = static_cast<size_t>((d->N + TILE - 1) / TILE) * TILE;
     auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
@@ -746,7 +812,9 @@ static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false) {
     w.off_dq = up(w.off_xk + BS * NTP * 16);
     const size_t dh = d->D <= 32 ? 32 : (d->D <= 64 ? 64 : 128);
     w.off_do = up(w.off_dq + BS * d->N * d->H * dh * 4);                         // fp32 dQ accumulator, kernel width
-    w.total = gated ? up(w.off_do + BS * d->N * d->H * d->D * 2) : w.off_do;     // bf16 d_out * sigmoid(gate)
+    w.off_db = gated ? up(w.off_do + BS * d->N * d->H * d->D * 2) : w.off_do;    // bf16 d_out * sigmoid(gate)
+    // fp32 dBias of a caller that wants bf16 (one S row needs none: dBias is not a sum)
+    w.total = (dbias_bf16 && d->S > 1) ? up(w.off_db + static_cast<size_t>(d->B) * d->H * d->N * d->N * 4) : w.off_db;
     return w;
 }
 
@@ -755,12 +823,12 @@ template <int DH>
 static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout& lay_out, const ActLayout& lay_grad,
                       const void* q, const void* k, const void* v, const void* bias,
                       const void* mask, const void* o, const void* o_resid, const float* lse, const void* d_o_in,
-                      void* dq, void* dk, void* dv, float* dbias, uint8_t* ws, float scale, unsigned phases,
-                      int reserved_sms, cudaStream_t st, const void* gate = nullptr, void* d_gate = nullptr) {
+                      void* dq, void* dk, void* dv, void* dbias_out, bool dbias_bf16, uint8_t* ws, float scale, unsigned phases,
+                      int reserved_sms, cudaStream_t st, const void* gate, void* d_gate) {
     using C = BwdCfg<DH>;
     const int BS = d->B * d->S;
     const int NT = (d->N + TILE - 1) / TILE;
-    const BwdWorkspace w = bwd_workspace(d, gate != nullptr);
+    const BwdWorkspace w = bwd_workspace(d, gate != nullptr, dbias_bf16);
     // with a gate the kernels read the gradient entering the attention from the workspace (contiguous)
     const void* d_o = gate ? static_cast<const void*>(ws + w.off_do) : d_o_in;
     const ActLayout lay_do = gate ? contiguous_layout(d->N, d->H, d->D) : lay_out;
@@ -800,26 +868,48 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = sm_count(&sms))) return rc;
 
     const size_t dq_bytes = static_cast<size_t>(BS) * d->N * d->H * DH * 4;
-    const size_t db_bytes = static_cast<size_t>(d->B) * d->H * d->N * d->N * 4;
+    const size_t db_elems = static_cast<size_t>(d->B) * d->H * d->N * d->N;
 
     // one S row and the whole backward in this call: the dQ/dK/dV kernel writes dBias (= dS) itself
-    const bool dbias_here = (d->S == 1) && (phases & EVO_BWD_PHASE_DBIAS) && (phases & EVO_BWD_PHASE_DQKV);
-    p.dbias = dbias;
+    const bool both = (phases & EVO_BWD_PHASE_DBIAS) && (phases & EVO_BWD_PHASE_DQKV);
+    const bool dbias_here = (d->S == 1) && both;
+    p.dbias = dbias_out;
+    // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
+    const int slices = dbias_slices(d, sms);
+    float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
+    const bool convert_dbias = dbias_bf16 && !dbias_here && slices > 1;
     if (phases & EVO_BWD_PHASE_DBIAS) {
-        if (!dbias_here && (rc = cuda_err(cudaMemsetAsync(dbias, 0, db_bytes, st)))) return rc;
-        bwd_prep_kernel<DH><<<sms * 8, 256, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(o_resid),
-            static_cast<const __nv_bfloat16*>(d_o_in), lse, static_cast<const __nv_bfloat16*>(mask), xq, xk,
-            1.0f / p.scale, BS, d->N, d->H, p.NTP, lay_out, Dt, static_cast<const __nv_bfloat16*>(gate),
-            reinterpret_cast<__nv_bfloat16*>(ws + w.off_do), static_cast<__nv_bfloat16*>(d_gate));
+        PrepParams r;
+        r.o = static_cast<const __nv_bfloat16*>(o);
+        r.o_resid = static_cast<const __nv_bfloat16*>(o_resid);
+        r.d_o = static_cast<const __nv_bfloat16*>(d_o_in);
+        r.mask = static_cast<const __nv_bfloat16*>(mask);
+        r.gate = static_cast<const __nv_bfloat16*>(gate);
+        r.lse = lse;
+        r.xq = xq;
+        r.xk = xk;
+        r.do_att = reinterpret_cast<__nv_bfloat16*>(ws + w.off_do);
+        r.d_gate = static_cast<__nv_bfloat16*>(d_gate);
+        r.zero[0] = reinterpret_cast<uint4*>(dbias_acc);
+        r.n_zero[0] = (!dbias_here && slices > 1) ? db_elems / 4 : 0;
+        r.zero[1] = reinterpret_cast<uint4*>(dq_acc);
+        r.n_zero[1] = both ? dq_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
+        r.inv_scale = 1.0f / p.scale;
+        r.BS = BS; r.N = d->N; r.H = d->H; r.NTP = p.NTP; r.Dt = Dt;
+        r.lay = lay_out;
+        constexpr int LANES = DH / 8;
+        if (Dt <= 16) bwd_prep_kernel<2><<<sms * 8, 256, 0, st>>>(r);
+        else bwd_prep_kernel<LANES><<<sms * 8, 256, 0, st>>>(r);
         if ((rc = cuda_err(cudaGetLastError()))) return rc;
-        if (!dbias_here && (rc = launch_dbias(d, lay_in, lay_do, q, k, v, bias, d_o, xq, xk, dbias, scale, sms, st)))
+        if (!dbias_here && (rc = launch_dbias(d, tq, tk, tv, tdo, bias, xq, xk, dbias_acc,
+                                              (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, st)))
             return rc;
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
 
-    if ((rc = cuda_err(cudaMemsetAsync(dq_acc, 0, dq_bytes, st)))) return rc;
-    auto kernel = dbias_here ? evo_bwd_kernel<DH, true> : evo_bwd_kernel<DH, false>;
+    if (!both && (rc = cuda_err(cudaMemsetAsync(dq_acc, 0, dq_bytes, st)))) return rc;
+    auto kernel = !dbias_here ? evo_bwd_kernel<DH, DBIAS_NO>
+                              : (dbias_bf16 ? evo_bwd_kernel<DH, DBIAS_BF16> : evo_bwd_kernel<DH, DBIAS_F32>);
     if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES))))
         return rc;
     // SMs left to other work (a collective on another stream) while this kernel runs
@@ -831,7 +921,16 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     prof_end(1, st);
     if ((rc = cuda_err(cudaGetLastError()))) return rc;
 
-    cvt_dq_kernel<DH><<<sms * 8, 256, 0, st>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), dq_bytes / 32, d->N, d->H, lay_grad, Dt);
+    FinishParams f;
+    f.dq_acc = dq_acc;
+    f.dq = static_cast<__nv_bfloat16*>(dq);
+    f.n8 = dq_bytes / 32;
+    f.N = d->N; f.H = d->H; f.Dt = Dt;
+    f.lay = lay_grad;
+    f.dbias_acc = convert_dbias ? dbias_acc : nullptr;
+    f.dbias = static_cast<__nv_bfloat16*>(dbias_out);
+    f.nb8 = db_elems / 8;
+    bwd_finish_kernel<DH><<<sms * 8, 256, 0, st>>>(f);
     return cuda_err(cudaGetLastError());
 }
 
@@ -936,37 +1035,43 @@ extern "C" int evo_bwd_views(const EvoDims* dims, const EvoStrides* s_qkv, const
                              const void* o_resid, const float* lse, const void* d_o, void* dq, void* dk, void* dv,
                              void* d_gate, float* dbias, void* workspace, size_t workspace_bytes, float scale,
                              unsigned phases, int reserved_sms, void* stream) {
+    if (!dims) return EVO_ERR_NULL_PTR;
+    const EvoBwdArgs a{*dims, s_qkv, s_out, s_grad, q, k, v, pair_bias, res_mask, gate, o, o_resid, lse, d_o, dq, dk, dv,
+                       d_gate, dbias, 0, workspace, workspace_bytes, scale, phases, reserved_sms, stream};
+    return evo_bwd_ex(&a);
+}
+
+extern "C" size_t evo_bwd_ex_workspace_bytes(const EvoDims* dims, int gated, int dbias_bf16) {
+    if (evo::check_dims(dims) != EVO_OK) return 0;
+    return evo::bwd_workspace(dims, gated != 0, dbias_bf16 != 0).total;
+}
+
+extern "C" int evo_bwd_ex(const EvoBwdArgs* a) {
+    if (!a) return EVO_ERR_NULL_PTR;
+    const EvoDims* dims = &a->dims;
     int rc = evo::check_dims(dims);
     if (rc) return rc;
-    if (!(phases & (EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV))) return EVO_ERR_BAD_DIMS;
+    const unsigned both = EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV;
+    if (!(a->phases & both)) return EVO_ERR_BAD_DIMS;
+    if (a->dbias_bf16 && (a->phases & both) != both) return EVO_ERR_BAD_DIMS;
     evo::ActLayout lay, lay_out, lay_grad;
-    if ((rc = evo::layout_from_strides(dims, s_qkv, &lay))) return rc;
-    if ((rc = evo::layout_from_strides(dims, s_out, &lay_out))) return rc;
-    if ((rc = evo::layout_from_strides(dims, s_grad, &lay_grad))) return rc;
-    if (!q || !k || !v || !pair_bias || !res_mask || !o || !lse || !d_o || !dq || !dk || !dv || !dbias ||
-        !workspace)
-        return EVO_ERR_NULL_PTR;
-    if ((gate == nullptr) != (d_gate == nullptr)) return EVO_ERR_NULL_PTR;
-    const uintptr_t all = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
-                          reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(pair_bias) |
-                          reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(d_o) |
-                          reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
-                          reinterpret_cast<uintptr_t>(dv) | reinterpret_cast<uintptr_t>(dbias) |
-                          reinterpret_cast<uintptr_t>(lse) | reinterpret_cast<uintptr_t>(o_resid) |
-                          reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(d_gate);
+    if ((rc = evo::layout_from_strides(dims, a->s_qkv, &lay))) return rc;
+    if ((rc = evo::layout_from_strides(dims, a->s_out, &lay_out))) return rc;
+    if ((rc = evo::layout_from_strides(dims, a->s_grad, &lay_grad))) return rc;
+    const void* need[] = {a->q, a->k, a->v, a->pair_bias, a->res_mask, a->o, a->lse, a->d_out, a->dq, a->dk, a->dv, a->dbias, a->workspace};
+    uintptr_t all = reinterpret_cast<uintptr_t>(a->o_resid) | reinterpret_cast<uintptr_t>(a->gate) | reinterpret_cast<uintptr_t>(a->d_gate);
+    for (const void* ptr : need) {
+        if (!ptr) return EVO_ERR_NULL_PTR;
+        if (ptr != a->workspace && ptr != a->res_mask) all |= reinterpret_cast<uintptr_t>(ptr);
+    }
+    if ((a->gate == nullptr) != (a->d_gate == nullptr)) return EVO_ERR_NULL_PTR;
     if (all & 15u) return EVO_ERR_ALIGNMENT;
-    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) ||
-        workspace_bytes < evo::bwd_workspace(dims, gate != nullptr).total)
+    if ((reinterpret_cast<uintptr_t>(a->workspace) & 255u) ||
+        a->workspace_bytes < evo::bwd_workspace(dims, a->gate != nullptr, a->dbias_bf16 != 0).total)
         return EVO_ERR_WORKSPACE;
     if ((rc = evo::ensure_context())) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    uint8_t* ws = static_cast<uint8_t*>(workspace);
-    if (dims->D <= 32)
-        return evo::launch_bwd<32>(dims, lay, lay_out, lay_grad, q, k, v, pair_bias, res_mask, o, o_resid, lse, d_o, dq, dk, dv, dbias,
-                                   ws, scale, phases, reserved_sms, st, gate, d_gate);
-    if (dims->D <= 64)
-        return evo::launch_bwd<64>(dims, lay, lay_out, lay_grad, q, k, v, pair_bias, res_mask, o, o_resid, lse, d_o, dq, dk, dv, dbias,
-                                   ws, scale, phases, reserved_sms, st, gate, d_gate);
-    return evo::launch_bwd<128>(dims, lay, lay_out, lay_grad, q, k, v, pair_bias, res_mask, o, o_resid, lse, d_o, dq, dk, dv, dbias, ws,
-                                scale, phases, reserved_sms, st, gate, d_gate);
+    auto launch = dims->D <= 32 ? evo::launch_bwd<32> : (dims->D <= 64 ? evo::launch_bwd<64> : evo::launch_bwd<128>);
+    return launch(dims, lay, lay_out, lay_grad, a->q, a->k, a->v, a->pair_bias, a->res_mask, a->o, a->o_resid, a->lse,
+                  a->d_out, a->dq, a->dk, a->dv, a->dbias, a->dbias_bf16 != 0, static_cast<uint8_t*>(a->workspace), a->scale,
+                  a->phases, a->reserved_sms, static_cast<cudaStream_t>(a->stream), a->gate, a->d_gate);
 }

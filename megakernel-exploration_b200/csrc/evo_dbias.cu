@@ -81,6 +81,7 @@ struct DbParams {
     const __nv_bfloat16* xk;     // [B*S][NTP][8]    extra tiles: per-column terms
     const __nv_bfloat16* bias;   // [B][H][N][N]
     float* dbias;                // [B][H][N][N]
+    __nv_bfloat16* dbias16;      // with one slice: bf16 result instead of the fp32 one, or nullptr
     unsigned int* status;
 };
 
@@ -340,6 +341,15 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // the finished tile: plain stores when this CTA saw every S row, else atomics
             if (qrow < p.N) {
                 float* out = p.dbias + tile_off;
+                if (p.dbias16) {
+#pragma unroll
+                    for (int c8 = 0; c8 < CW / 8; ++c8)
+                        if (col0 + c8 * 8 < p.N)
+                            *reinterpret_cast<uint4*>(p.dbias16 + tile_off + c8 * 8) =
+                                make_uint4(pack_bf16(acc[c8 * 4].x, acc[c8 * 4].y), pack_bf16(acc[c8 * 4 + 1].x, acc[c8 * 4 + 1].y),
+                                           pack_bf16(acc[c8 * 4 + 2].x, acc[c8 * 4 + 2].y), pack_bf16(acc[c8 * 4 + 3].x, acc[c8 * 4 + 3].y));
+                    continue;
+                }
 #pragma unroll
                 for (int c4 = 0; c4 < CW / 4; ++c4) {
                     if (col0 + c4 * 4 < p.N) {
@@ -370,24 +380,10 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 // D=32: 0.193 -> 0.177 ms; B=1, S=256, N=1024, H=4, D=64: 0.383 -> 0.371).
 constexpr int DBIAS_GROUPS = 4;
 
-template <int DH>
-static int launch_dbias_t(const EvoDims* d, const ActLayout& lay, const ActLayout& lay_do, const void* q, const void* k, const void* v, const void* bias,
-                          const void* d_o, const void* xq, const void* xk,
-                          float* dbias, float scale, int sms, cudaStream_t st) {
-    constexpr int NG = DBIAS_GROUPS;
-    using C = DbCfg<DH, NG>;
-    const int BS = d->B * d->S;
+// Slices of S: enough items to fill the SMs evenly, each long enough that the
+// per-item set-up (bias load, pipeline fill, tile write) stays small.
+int dbias_slices(const EvoDims* d, int sms) {
     const int NT = (d->N + TILE - 1) / TILE;
-
-    CUtensorMap tq, tk, tv, tdo;
-    int rc;
-    if ((rc = make_tmap_qkv(&tq, q, BS, d->N, d->H, d->D, TILE, lay, RowTile<DH>::BOX_D))) return rc;
-    if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, d->D, TILE, lay, RowTile<DH>::BOX_D))) return rc;
-    if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, d->D, TILE, lay, RowTile<DH>::BOX_D))) return rc;
-    if ((rc = make_tmap_qkv(&tdo, d_o, BS, d->N, d->H, d->D, TILE, lay_do, RowTile<DH>::BOX_D))) return rc;
-
-    // Slices of S: enough items to fill the SMs evenly, each long enough that the
-    // per-item set-up (bias load, pipeline fill, tile write) stays small.
     const long base = static_cast<long>(d->B) * d->H * NT * NT;
     int best_z = 1;
     long best_cost = -1;
@@ -399,23 +395,33 @@ static int launch_dbias_t(const EvoDims* d, const ActLayout& lay, const ActLayou
         const long cost = waves * (sl + 6);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_z = zz; }
     }
+    return best_z;
+}
 
+template <int DH>
+static int launch_dbias_t(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                          const CUtensorMap& tdo, const void* bias, const void* xq, const void* xk, float* dbias,
+                          void* dbias16, int slices, float scale, int sms, cudaStream_t st) {
+    constexpr int NG = DBIAS_GROUPS;
+    using C = DbCfg<DH, NG>;
+    const int NT = (d->N + TILE - 1) / TILE;
     DbParams p;
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
     p.NT = NT; p.NTP = NT * TILE;
     p.KB = (d->D + 15) / 16;
-    p.SL = (d->S + best_z - 1) / best_z;
+    p.SL = (d->S + slices - 1) / slices;
     p.Z = (d->S + p.SL - 1) / p.SL;
-    p.total_items = static_cast<int>(base * p.Z);
-    const float sc = (scale > 0.f) ? scale : 1.0f / sqrtf(static_cast<float>(d->D));
-    p.c1 = sc * LOG2E;
+    p.total_items = d->B * d->H * NT * NT * p.Z;
+    p.c1 = scale * LOG2E;
     p.xq = static_cast<const __nv_bfloat16*>(xq);
     p.xk = static_cast<const __nv_bfloat16*>(xk);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.dbias = dbias;
+    p.dbias16 = static_cast<__nv_bfloat16*>(dbias16);
     p.status = status_word();
     if (!p.status) return EVO_ERR_CUDA;
 
+    int rc;
     if ((rc = set_max_smem_once(reinterpret_cast<const void*>(evo_dbias_kernel<DH, NG>),
                                 static_cast<int>(C::SMEM_BYTES))))
         return rc;
@@ -426,14 +432,11 @@ static int launch_dbias_t(const EvoDims* d, const ActLayout& lay, const ActLayou
     return cuda_err(cudaGetLastError());
 }
 
-int launch_dbias(const EvoDims* d, const ActLayout& lay, const ActLayout& lay_do, const void* q, const void* k, const void* v, const void* bias,
-                 const void* d_o, const void* xq, const void* xk, float* dbias,
-                 float scale, int sms, cudaStream_t st) {
-    if (d->D <= 32)
-        return launch_dbias_t<32>(d, lay, lay_do, q, k, v, bias, d_o, xq, xk, dbias, scale, sms, st);
-    if (d->D <= 64)
-        return launch_dbias_t<64>(d, lay, lay_do, q, k, v, bias, d_o, xq, xk, dbias, scale, sms, st);
-    return launch_dbias_t<128>(d, lay, lay_do, q, k, v, bias, d_o, xq, xk, dbias, scale, sms, st);
+int launch_dbias(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                 const void* bias, const void* xq, const void* xk, float* dbias, void* dbias16, int slices, float scale, int sms,
+                 cudaStream_t st) {
+    auto f = d->D <= 32 ? launch_dbias_t<32> : (d->D <= 64 ? launch_dbias_t<64> : launch_dbias_t<128>);
+    return f(d, tq, tk, tv, tdo, bias, xq, xk, dbias, dbias16, slices, scale, sms, st);
 }
 
 }  // namespace evo

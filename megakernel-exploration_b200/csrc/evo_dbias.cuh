@@ -5,11 +5,15 @@
 
 namespace evo {
 
-// dbias [B][H][N][N] fp32 must be zeroed on `st` before the call.  xq and xk are the
-// extra tiles the prep kernel writes (see evo_bwd.cu): bf16 [B*S][H][NTP][8] with the
-// per-row terms and bf16 [B*S][NTP][8] with the per-column terms.
-// `lay` gives the strides of q, k, v, `lay_do` those of d_o.
-int launch_dbias(const EvoDims* d, const ActLayout& lay, const ActLayout& lay_do, const void* q, const void* k, const void* v, const void* bias,
-                 const void* d_o, const void* xq, const void* xk, float* dbias, float scale, int sms, cudaStream_t st);
+// Slices of S that the launcher cuts the sum into (1: every dBias tile is one CTA's whole sum).
+int dbias_slices(const EvoDims* d, int sms);
+
+// dbias [B][H][N][N] fp32 must be zeroed on `st` before the call if there are several slices; with
+// one, dbias16 (bf16, may be nullptr) is written instead if given.  tq, tk, tv, tdo: row-tile maps of
+// q, k, v, d_o.  xq and xk are the extra tiles the prep kernel writes (see evo_bwd.cu): bf16
+// [B*S][H][NTP][8] with the per-row terms and bf16 [B*S][NTP][8] with the per-column terms.
+int launch_dbias(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                 const void* bias, const void* xq, const void* xk, float* dbias, void* dbias16, int slices, float scale, int sms,
+                 cudaStream_t st);
 
 }  // namespace evo

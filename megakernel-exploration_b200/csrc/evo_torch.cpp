@@ -1,0 +1,265 @@
+// The operator's host path in native code: one call per forward, one autograd node for the
+// backward, over the C ABI of libevoattn.so (include/evoattn.h).
+//
+// What it replaces is the Python body of TKEvoAttention.forward / backward for the plain case --
+// CUDA tensors, a head dim the library takes as it is, no process group (tk_evo_attention_layer.py
+// keeps that body for everything else).  At small sizes the step is host work: through Python,
+// ctypes and torch's Python autograd node a forward + backward took 200 us of host time around
+// 35 us of kernels.
+//
+// `apply` returns None for a call it does not handle (the Python body then runs, or raises the
+// reference's own assertion); it never falls back to another implementation of the math.
+#include <torch/extension.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include "../../include/evoattn.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+bool supported_dim(int64_t d) { return d == 16 || d == 32 || d == 64 || d == 96 || d == 128; }
+
+bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0; }
+
+void check(int rc, const char* what) {
+    if (rc == EVO_OK) return;
+    std::string detail = evo_strerror(rc);
+    if (rc == EVO_ERR_CUDA) detail += " (cudaError " + std::to_string(evo_last_cuda_error()) + ")";
+    if (rc == EVO_ERR_TENSOR_MAP) detail += std::string(" (") + evo_last_error_detail() + ")";
+    TORCH_CHECK(false, "libevoattn: ", what, " failed with ", rc, ": ", detail);
+}
+
+// Where q, k and v lie, and where the tensors this call allocates go.
+struct Layout {
+    bool in_view = false;      // q, k, v are read through `in`; otherwise contiguous
+    bool out_view = false;     // o and the gradients carry the strides of q; otherwise contiguous
+    EvoStrides in{};
+    int64_t strides[5]{};      // of q
+};
+
+// q, k, v bf16 views with the same strides, contiguous head dim, steps of 16 bytes and (B, N_SEQ)
+// flattenable can be read in place.  If the strides tile the storage without holes (a permutation of a
+// contiguous tensor), outputs take them as well; a view with holes (sliced out of a fused projection)
+// or with overlap does not qualify for that, one with overlap for neither.
+Layout classify(const Tensor& q, const Tensor& k, const Tensor& v) {
+    Layout l;
+    if (q.is_contiguous()) return l;
+    if (q.scalar_type() != at::kBFloat16 || k.scalar_type() != at::kBFloat16 || v.scalar_type() != at::kBFloat16) return l;
+    const auto st = q.strides();
+    if (k.strides() != st || v.strides() != st || st[4] != 1) return l;
+    const auto sz = q.sizes();
+    for (int i = 0; i < 4; ++i)
+        if (sz[i] > 1 && (st[i] <= 0 || st[i] % 8 != 0)) return l;
+    if (sz[0] > 1 && sz[1] > 1 && st[0] != sz[1] * st[1]) return l;
+    int order[5] = {0, 1, 2, 3, 4};
+    std::sort(order, order + 5, [&](int a, int b) { return st[a] != st[b] ? st[a] < st[b] : sz[a] < sz[b]; });
+    bool dense = true;
+    int64_t span = 1;
+    for (int a : order) {
+        if (sz[a] <= 1) continue;
+        if (st[a] < span) return l;      // overlap
+        if (st[a] != span) dense = false;
+        span = st[a] * sz[a];
+    }
+    if (!aligned(q) || !aligned(k) || !aligned(v)) return l;
+    l.in_view = true;
+    l.out_view = dense;
+    l.in = EvoStrides{st[0], st[1], st[2], st[3]};
+    for (int i = 0; i < 5; ++i) l.strides[i] = st[i];
+    return l;
+}
+
+Tensor bf16_contiguous(const Tensor& t) {
+    return (t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16)).contiguous();
+}
+
+Tensor empty_like_act(const Tensor& q, const Layout& l) {
+    if (l.out_view)
+        return at::detail::empty_strided_cuda(q.sizes(), at::IntArrayRef(l.strides, 5), at::kBFloat16, q.device());
+    return at::detail::empty_cuda(q.sizes(), at::kBFloat16, q.device(), std::nullopt);
+}
+
+// `t` in the layout of the outputs, copied only if it is not there already.
+Tensor as_output(const Tensor& t, const Tensor& q, const Layout& l) {
+    if (l.out_view) {
+        if (t.scalar_type() == at::kBFloat16 && t.strides() == at::IntArrayRef(l.strides, 5) && aligned(t)) return t;
+        Tensor c = empty_like_act(q, l);
+        c.copy_(t);
+        return c;
+    }
+    Tensor c = bf16_contiguous(t);
+    if (!aligned(c)) c = c.clone();
+    return c;
+}
+
+struct Call {
+    Tensor q, k, v, bias, mask, gate;      // gate: undefined without one
+    Layout lay;
+    EvoDims dims;
+    float scale;
+    at::ScalarType bias_type;
+};
+
+struct Forward {
+    Tensor out, o, o_resid, lse;           // out: o, or the gated output
+};
+
+Forward run_forward(const Call& c, bool need_grad) {
+    const c10::cuda::CUDAGuard guard(c.q.device());
+    Forward f;
+    f.o = empty_like_act(c.q, c.lay);
+    Tensor gated;
+    if (c.gate.defined()) gated = empty_like_act(c.q, c.lay);
+    // rounding residual of O, kept for the backward only (accurate delta -> accurate dBias)
+    if (need_grad) f.o_resid = empty_like_act(c.q, c.lay);
+    f.lse = at::detail::empty_cuda({c.dims.B, c.dims.S, c.dims.H, c.dims.N}, at::kFloat, c.q.device(), std::nullopt);
+    check(evo_fwd_views(&c.dims, c.lay.in_view ? &c.lay.in : nullptr, c.lay.out_view ? &c.lay.in : nullptr, c.q.const_data_ptr(),
+                        c.k.const_data_ptr(), c.v.const_data_ptr(), c.bias.const_data_ptr(), c.mask.const_data_ptr(),
+                        c.gate.defined() ? c.gate.const_data_ptr() : nullptr, f.o.data_ptr(),
+                        gated.defined() ? gated.data_ptr() : nullptr, need_grad ? f.o_resid.data_ptr() : nullptr,
+                        static_cast<float*>(f.lse.data_ptr()), c.scale, c10::cuda::getCurrentCUDAStream().stream()),
+          "evo_fwd_views");
+    f.out = gated.defined() ? gated : f.o;
+    return f;
+}
+
+// The backward's autograd node.  Edges: q, k, v, pair_bias, gate (the bf16, laid-out forms of them that
+// the kernels read are what is saved).
+struct EvoBackward : public torch::autograd::Node {
+    SavedVariable q, k, v, bias, mask, gate, o, o_resid, lse;
+    bool gated = false;
+    Layout lay;
+    EvoDims dims{};
+    float scale = 0.f;
+    at::ScalarType bias_type = at::kBFloat16;
+
+    std::string name() const override { return "TKEvoAttentionBackward"; }
+
+    void release_variables() override {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        for (SavedVariable* x : {&q, &k, &v, &bias, &mask, &gate, &o, &o_resid, &lse}) x->reset_data();
+    }
+
+    variable_list apply(variable_list&& grads) override {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        const at::NoGradGuard no_grad;
+        const auto self = getptr();
+        const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack(), mask_ = mask.unpack();
+        const Tensor o_ = o.unpack(self), resid_ = o_resid.unpack(), lse_ = lse.unpack(), gate_ = gated ? gate.unpack() : Tensor();
+        const c10::cuda::CUDAGuard guard(q_.device());
+        const Tensor d_out = grads[0].defined() ? as_output(grads[0], q_, lay) : empty_like_act(q_, lay).zero_();
+        Tensor dq = empty_like_act(q_, lay), dk = empty_like_act(q_, lay), dv = empty_like_act(q_, lay), d_gate;
+        if (gated) d_gate = empty_like_act(q_, lay);
+        const bool bf = bias_type == at::kBFloat16;
+        Tensor dbias = at::detail::empty_cuda({dims.B, 1, dims.H, dims.N, dims.N}, bf ? at::kBFloat16 : at::kFloat, q_.device(),
+                                              std::nullopt);
+        EvoBwdArgs a{};
+        a.dims = dims;
+        a.s_qkv = lay.in_view ? &lay.in : nullptr;
+        a.s_out = a.s_grad = lay.out_view ? &lay.in : nullptr;
+        a.q = q_.const_data_ptr();
+        a.k = k_.const_data_ptr();
+        a.v = v_.const_data_ptr();
+        a.pair_bias = bias_.const_data_ptr();
+        a.res_mask = mask_.const_data_ptr();
+        a.gate = gated ? gate_.const_data_ptr() : nullptr;
+        a.o = o_.const_data_ptr();
+        a.o_resid = resid_.const_data_ptr();
+        a.lse = static_cast<const float*>(lse_.const_data_ptr());
+        a.d_out = d_out.const_data_ptr();
+        a.dq = dq.data_ptr();
+        a.dk = dk.data_ptr();
+        a.dv = dv.data_ptr();
+        a.d_gate = gated ? d_gate.data_ptr() : nullptr;
+        a.dbias = dbias.data_ptr();
+        a.dbias_bf16 = bf;
+        a.workspace_bytes = evo_bwd_ex_workspace_bytes(&dims, gated, bf);
+        const Tensor ws = at::detail::empty_cuda({static_cast<int64_t>(a.workspace_bytes)}, at::kByte, q_.device(), std::nullopt);
+        a.workspace = ws.data_ptr();
+        a.scale = scale;
+        a.phases = EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV;
+        a.stream = c10::cuda::getCurrentCUDAStream().stream();
+        check(evo_bwd_ex(&a), "evo_bwd_ex");
+        if (!bf && bias_type != at::kFloat) dbias = dbias.to(bias_type);
+        return {dq, dk, dv, dbias, d_gate};
+    }
+};
+
+// bias16: pair_bias itself if it is bf16, else its bf16 copy (the caller casts once per version of the tensor).
+std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& res_mask, const Tensor& pair_bias,
+                            const Tensor& bias16, const std::optional<Tensor>& gate) {
+    if (Q.dim() != 5 || !Q.is_cuda()) return std::nullopt;
+    const auto sz = Q.sizes();
+    const int64_t B = sz[0], S = sz[1], N = sz[2], H = sz[3], D = sz[4];
+    if (K.sizes() != sz || V.sizes() != sz || !supported_dim(D) || N % 8 != 0 || N <= 0 || B <= 0 || S <= 0 || H <= 0) return std::nullopt;
+    if (res_mask.sizes() != at::IntArrayRef({B, S, 1, 1, N}) || pair_bias.sizes() != at::IntArrayRef({B, 1, H, N, N})) return std::nullopt;
+    if (gate && gate->sizes() != sz) return std::nullopt;
+    const auto dev = Q.device();
+    if (K.device() != dev || V.device() != dev || res_mask.device() != dev || pair_bias.device() != dev || bias16.device() != dev)
+        return std::nullopt;
+    if (gate && gate->device() != dev) return std::nullopt;
+    if (B > INT32_MAX || S > INT32_MAX || N > INT32_MAX || H > INT32_MAX) return std::nullopt;
+
+    const bool need_grad = at::GradMode::is_enabled() &&
+                           (Q.requires_grad() || K.requires_grad() || V.requires_grad() || pair_bias.requires_grad() ||
+                            (gate && gate->requires_grad()));
+    Call c;
+    {
+        const at::NoGradGuard no_grad;
+        c.lay = classify(Q, K, V);
+        if (c.lay.in_view) {
+            c.q = Q; c.k = K; c.v = V;
+        } else {
+            c.q = bf16_contiguous(Q);
+            c.k = bf16_contiguous(K);
+            c.v = bf16_contiguous(V);
+        }
+        c.bias = bf16_contiguous(bias16);      // the caller's cast of an fp32 bias, or the bf16 bias itself
+        c.mask = bf16_contiguous(res_mask);
+        if (!aligned(c.q) || !aligned(c.k) || !aligned(c.v) || !aligned(c.bias) || !aligned(c.mask)) return std::nullopt;
+        if (gate) c.gate = as_output(*gate, c.q, c.lay);
+        c.dims = EvoDims{static_cast<int32_t>(B), static_cast<int32_t>(S), static_cast<int32_t>(N), static_cast<int32_t>(H),
+                         static_cast<int32_t>(D)};
+        c.scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(D)));
+        c.bias_type = pair_bias.scalar_type();
+        if (!need_grad) return run_forward(c, false).out;
+    }
+    Forward f;
+    {
+        const at::NoGradGuard no_grad;
+        f = run_forward(c, true);
+    }
+    const std::shared_ptr<EvoBackward> node(new EvoBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(Q, K, V, pair_bias, gate ? *gate : Tensor()));
+    node->q = SavedVariable(c.q, false);
+    node->k = SavedVariable(c.k, false);
+    node->v = SavedVariable(c.v, false);
+    node->bias = SavedVariable(c.bias, false);
+    node->mask = SavedVariable(c.mask, false);
+    node->gated = c.gate.defined();
+    if (node->gated) node->gate = SavedVariable(c.gate, false);
+    node->o_resid = SavedVariable(f.o_resid, false);
+    node->lse = SavedVariable(f.lse, false);
+    node->lay = c.lay;
+    node->dims = c.dims;
+    node->scale = c.scale;
+    node->bias_type = c.bias_type;
+    torch::autograd::set_history(f.out, node);
+    node->o = SavedVariable(f.o, /*is_output=*/!node->gated);
+    return f.out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("apply", &apply, "EvoAttention with its autograd node; None if the call is not one of the plain kind");
+}

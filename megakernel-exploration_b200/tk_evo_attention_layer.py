@@ -19,8 +19,8 @@ Differences from the reference, all internal:
     transposes and no zero-padding of D (reference layer.py:81-102,112-113);
   * head dims 16, 32 and 64 run without any padding copy (16 on the D=32 kernels,
     whose loads zero-fill and whose stores clip the missing columns); other D <= 64
-    are zero-padded up to the next of those here; D=96/128 raise ValueError (the
-    reference pads them to 128, layer.py:47-56);
+    are zero-padded up to the next of those here; 96 runs on the D=128 kernels in the
+    same way (the reference pads it to 128, layer.py:47-56);
   * d_pair_bias is accumulated in fp32 and returned in the dtype of pair_bias
     (the reference rounds it to bf16 first, layer.py:176);
   * an optional sixth argument `process_group` shards the independent N_SEQ axis
@@ -197,8 +197,40 @@ def _device_ctx(t: torch.Tensor):
     return torch.cuda.device(t.device)
 
 
+_native_apply = None
+
+
+def _native():
+    """apply() of _evo_torch.so, the operator's host path in native code (csrc/evo_torch.cpp)."""
+    global _native_apply
+    if _native_apply is None:
+        _evoattn.lib()                      # the kernels' library, with its own check and error message
+        import _evo_torch
+        _native_apply = _evo_torch.apply
+    return _native_apply
+
+
 class TKEvoAttention(torch.autograd.Function):
-    """Evo / triangle attention: softmax(Q K^T / sqrt(D) + pair_bias + res_mask) V."""
+    """Evo / triangle attention: softmax(Q K^T / sqrt(D) + pair_bias + res_mask) V.
+
+    apply() hands the plain case (CUDA tensors, a head dim the library takes as it is, no process group)
+    to the native host path, which runs the same launches from C++: a forward + backward took 200 us of
+    host time through the Python body below, which serves every other case (padded head dims, the
+    sharded backward with its all-reduce, and all argument errors)."""
+
+    @classmethod
+    def apply(cls, *args):
+        if (5 <= len(args) <= 7 and (len(args) == 5 or args[5] is None)
+                and isinstance(args[0], torch.Tensor) and args[0].is_cuda):
+            Q, K, V, res_mask, pair_bias = args[:5]
+            if Q.dim() == 5 and pair_bias.dim() == 5:
+                bias = _bias_bf16(pair_bias, Q.shape[0], Q.shape[3], Q.shape[2]) \
+                    if pair_bias.dtype != torch.bfloat16 and pair_bias.shape == (Q.shape[0], 1, Q.shape[3], Q.shape[2], Q.shape[2]) \
+                    else pair_bias
+                out = _native()(Q, K, V, res_mask, pair_bias, bias, args[6] if len(args) == 7 else None)
+                if out is not None:
+                    return out
+        return super().apply(*args)
 
     @staticmethod
     def forward(ctx, Q, K, V, res_mask, pair_bias, process_group=None, gate=None):
