@@ -18,103 +18,18 @@
 //   3. evo_bwd_kernel     dQ, dK, dV (below)
 //   4. bwd_finish_kernel  fp32 dQ accumulator -> bf16 dQ in the caller layout (and dBias,
 //                         summed over slices of S in fp32, to bf16 if the caller wants that)
-//
-// evo_bwd_kernel: one persistent CTA per SM walks items (chunk of RC consecutive
-// S rows, head h, kv tile j of 128 residues); per item it walks steps
-// (q tile i, row r of the chunk), r innermost, so that one pair-bias tile serves
-// RC steps.  dK/dV of every row of the chunk stay in tensor memory for the item.
-//
-//   warps 0-3, 4-7     two compute groups; group g owns kv columns 64g..64g+63
-//                      (thread = one q row).  Per step: P = exp2(S' c1 + bias log2e)
-//                      and dS = P dP' from the two accumulators, kept packed in
-//                      registers until the previous step's dV/dK/dQ MMAs have
-//                      finished reading the P/dS tiles, then written to shared
-//                      memory as MMA operands.
-//   warps 8-11 (drain) warp w owns tensor-memory lanes 32(w-8)..: after every step
-//                      it stages its 32 rows of dQ in its own shared-memory slot and
-//                      issues a TMA reduce-add (fp32) for them; after an item, dK/dV
-//                      go out as bf16 stores.  None of this is on the compute groups'
-//                      path.
-//   warp 12 (producer) TMA per step: Q, dO tiles and the extra tile of the q rows; K, V
-//                      tiles and the extra tile of the kv rows per step (D=32) or per
-//                      item (D>=64); the pair-bias tile per q tile (D<=64)
-//   warps 13, 14, 15   tcgen05.mma issuers, one chain family each, so that no chain
-//                      queues behind another's issue: S' = Q K^T + extra block and
-//                      dP' = dO V^T + extra block of the next step (13);
-//                      dV += P^T dO and dK += dS^T Q (14); dQ = dS K (15).  Each warp
-//                      runs its loop with all lanes and elects one lane to issue.
 #include "evo_dbias.cuh"
 #include "evo_host.cuh"
 #include "evo_ptx.cuh"
 #include "evo_tiles.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 
 namespace evo {
 
-// 4 warpgroups: 2 compute, drain, (producer, mma, 2 idle warps)
-constexpr int BWD_THREADS = 512;
-constexpr int BWD_WARP_DRAIN = 8, BWD_WARP_PRODUCER = 12, BWD_WARP_MMA = 13;   // 13, 14, 15: mma issuers
 constexpr uint32_t BWD_TMEM_COLS = 512;
-// setmaxnreg budgets of the compute warpgroups and of the others, by head dim.  Measured (dQ/dK/dV
-// kernel): D=32 (B=1, S=512, N=384, H=8) 168/88 0.474 ms, 176/80 0.471, 184/72 0.483, 160/96 0.478;
-// D=64 (B=1, S=256, N=1024, H=4) 168/88 1.297 ms, 176/80 1.321, 184/72 1.288, 160/96 1.353.
-template <int DH> constexpr int BWD_REGS_COMPUTE = (DH == 64) ? 184 : 176;
-template <int DH> constexpr int BWD_REGS_OTHER = 256 - BWD_REGS_COMPUTE<DH>;
-// the CTA's register pool is the launch count (cap for 512 threads: 128) times the threads;
-// a setmaxnreg increase that the pool cannot satisfy blocks for ever
-static_assert(BWD_REGS_COMPUTE<32> * 256 + BWD_REGS_OTHER<32> * 256 <= 128 * BWD_THREADS, "register pool");
-
-template <int DH>
-struct BwdCfg {
-    static constexpr int RC = (DH == 32) ? 3 : 1;     // S rows per chunk
-#ifndef EVO_BWD_QS32
-#define EVO_BWD_QS32 3
-#endif
-    static constexpr int QS = (DH == 32) ? EVO_BWD_QS32 : (DH == 64 ? 2 : 1);     // load stages
-    // D=32: K/V travel with every step's stage; D>=64: one resident K/V buffer per item
-    static constexpr bool KV_RESIDENT = (DH >= 64);
-    // D=128 is short of shared and tensor memory: one load stage, the bias slice of a thread read
-    // straight from global memory (no staged tile), and ONE dQ accumulator that shares its tensor
-    // memory columns with S' (S' of step n+1 is issued once dQ of step n is drained).
-    static constexpr bool BIAS_STAGED = (DH <= 64);
-    static constexpr int DQ_BUFS = (DH <= 64) ? 2 : 1;
-    static constexpr int HALF = DH / 2;               // head-dim columns drained per group
-    static constexpr uint32_t ROWT = RowTile<DH>::BYTES;
-    // one stage: Q, dO [, K, V] tiles, then the extra tile of the q rows [and of the kv rows]
-    static constexpr uint32_t ST_Q = 0, ST_DO = ROWT;
-    static constexpr uint32_t ST_K = 2 * ROWT, ST_V = 3 * ROWT;            // streaming only
-    static constexpr uint32_t ST_TILES = KV_RESIDENT ? 2 : 4;
-    static constexpr uint32_t ST_XQ = ST_TILES * ROWT, ST_XK = ST_XQ + XT_BYTES;
-    static constexpr uint32_t STAGE_TX = ST_TILES * ROWT + (KV_RESIDENT ? 1 : 2) * XT_BYTES;
-    static constexpr uint32_t STAGE_STRIDE = ST_TILES * ROWT + 2 * XT_BYTES;
-    // resident K/V buffer: K[RC], V[RC], extra tiles of the kv rows [RC]
-    static constexpr uint32_t KV_BYTES = KV_RESIDENT ? (2 * RC * ROWT + RC * XT_BYTES) : 0;
-    static constexpr uint32_t KV_TX = 2 * ROWT + XT_BYTES;                  // per row of the chunk
-    static constexpr uint32_t OFF_STAGE = 0;
-    static constexpr uint32_t OFF_KV = OFF_STAGE + QS * STAGE_STRIDE;
-    static constexpr uint32_t OFF_BIAS = OFF_KV + KV_BYTES;
-    static constexpr uint32_t OFF_P = OFF_BIAS + (BIAS_STAGED ? SQ_BYTES : 0);
-    static constexpr uint32_t OFF_DS = OFF_P + SQ_BYTES;
-    // per drain warp: dQ slot [32 rows][32 fp32]
-    static constexpr uint32_t WQ_BYTES = 32 * 32 * 4;
-    static constexpr uint32_t OFF_WSTG = OFF_DS + SQ_BYTES;
-    // constant extra tiles, above every tile that refers to the zero tile
-    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WQ_BYTES;            // column selector of -delta
-    static constexpr uint32_t OFF_ZERO = OFF_XDP + XT_BYTES;
-    static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr uint32_t NUM_BARS = 2 * QS + 2 + 2 + 7 + RC + 2;
-    static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + alignment slack
-    static constexpr uint32_t TMEM_S = 0;
-    static constexpr uint32_t TMEM_DP = 128;
-    static constexpr uint32_t TMEM_DQ = (DQ_BUFS == 2) ? 256 : TMEM_S;      // DQ_BUFS accumulators, + (step % DQ_BUFS)*DH
-    static constexpr uint32_t TMEM_DKV = (DQ_BUFS == 2) ? 256 + 2 * DH : 256;   // + r*2*DH (dK), + DH (dV)
-    static_assert(TMEM_DKV + RC * 2 * DH <= BWD_TMEM_COLS, "tensor memory budget");
-    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-    static_assert(OFF_KV % 1024 == 0 && OFF_BIAS % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
-};
 
 struct BwdParams {
     int B, S, N, H;
@@ -122,88 +37,184 @@ struct BwdParams {
     int KB;          // contraction blocks of 16 head-dim columns that hold data: ceil(Dt / 16)
     int NT;          // tiles per row: ceil(N / 128)
     int NTP;         // NT * 128
-    int CPB;         // chunks per batch: ceil(S / RC)
-    int total_items; // B * CPB * H * NT
+    int total_items; // B * S * H, or B * S * H * NT segments
     float scale;     // softmax scale
     float c1;        // scale * log2(e)
     const __nv_bfloat16* xq;   // [B*S][H][NTP][8] extra tiles of the q rows  (bwd_prep_kernel)
     const __nv_bfloat16* xk;   // [B*S][NTP][8]    extra tiles of the kv rows
-    const __nv_bfloat16* bias; // [B][H][N][N] (read directly when the bias tile is not staged)
+    const __nv_bfloat16* bias; // [B][H][N][N]
     void* dbias;               // [B][H][N][N], fp32 or bf16 (written by this kernel only when S = 1)
-    __nv_bfloat16* dk;    // activation layout `lay`
+    float* dq_scratch;         // WHOLE: per CTA scratch_stride 16-byte words, partial sums of dQ
+    size_t scratch_stride;
+    __nv_bfloat16* dq;    // activation layout `lay` (dq: written by this kernel only when WHOLE)
+    __nv_bfloat16* dk;
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
     unsigned int* status;
-};
-
-struct BwdItem {
-    int b, bs0, nr, h, j;
 };
 
 // DBIAS_HERE (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
 // dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
 // per item) is not launched.
 enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2 };
-template <int DH, int DBIAS_HERE>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+
+
+
+}  // namespace evo
+#include "evo_bwd_wide.cuh"
+namespace evo {
+
+// ---------------------------------------------------------------------------
+// dQ, dK, dV.  One persistent CTA per SM walks segments (S row, head h, kv tile j of 128 residues); a
+// segment walks steps (q tile i).  Everything is formed TRANSPOSED, kv rows in the tensor-memory lanes,
+// so that P^T and dS^T are in place as A operands of the products that contract over q, without a trip
+// through shared memory:
+//
+//   S'^T = K Q^T + extra block,  dP'^T = V dO^T + extra block         (evo_tiles.cuh, "EXTRA TILE")
+//   P^T = exp2(S'^T c1 + bias^T log2e),  dS^T = P^T o dP'^T           (thread = one kv row)
+//   dV += P^T dO,  dK += dS^T Q      A from tensor memory: 16 clocks per K = 16 block at N = 32, where an
+//                                    A tile in shared memory costs 40 (it is read at 128 bytes a clock)
+//   dQ = dS K                        A = dS from shared memory (M = q: MN-major), the one tile written there
+//
+// What bounds a step is the work of the compute warps, about 1400 issue slots and 1024 clocks of
+// exponentials per scheduler, and the chain of barriers and products around it.  Sixteen compute warps,
+// because with eight the loads, multiplies and exponentials of a warp hardly overlapped (2000 clocks for
+// the same work).
+//
+//   D = 32: one phase.  P^T and dS^T have columns of their own, so S' and dP' of the next step are formed
+//     during the second half of this one's arithmetic.  (A share of the exponentials on the multiply-add
+//     pipe only costs here: 0.446 -> 0.514 ms.)
+//   D = 64: no columns for P^T and dS^T: they overwrite the columns they were computed from (ALIAS).  Two
+//     phases, P (from S') and dS (from dP'), each with its own barriers, so that the products of one are
+//     formed during the other: dV and S' of the next step while dS is computed, dK, dQ and dP' of the next
+//     step while its P is (B=1, S=256, N=1024, H=4: 1.30 -> 1.11 ms; at D = 32 the extra barriers cost more
+//     than they save).
+//
+//   warps 0-15 (compute)  group g = warp / 4 owns q columns 32g .. 32g+31 of the tile
+//   warps 16-19 (drain)   after every step 32 rows of dQ each, after a segment dK and dV as bf16 stores
+//   warp 20 (producer)    TMA: per step Q, dO, the extra tile of the q rows, the pair-bias tile; per
+//                         segment K, V and the extra tile of the kv rows
+//   warps 21, 22, 23      MMA issuers, one chain family each: S'^T and dP'^T; dV and dK; dQ
+//
+// dQ is a sum over kv tiles.  WHOLE: an item is all NT segments of a (row, head), so one CTA sees the
+// whole sum.  With one or two tiles it stays in tensor memory until the last segment; otherwise the drain
+// warps keep partial sums in a scratch area of the CTA, in L2 (written and added to by bulk copies: loads
+// and stores of their own held up the compute warps' shared-memory accesses), and the last segment's go out
+// as bf16.  Where there are too few items for that, an item is one segment, and the partial sums meet in an
+// fp32 accumulator in memory (TMA reduce-add), which costs a pass to zero it and a pass to convert it.
+//
+// Measured against one kernel with P and dS in shared memory and two compute groups (whole backward):
+// B=1, S=512, N=384, H=8, D=32 0.81 -> 0.71 ms; S=256, N=768 1.40 -> 1.28; S=256, N=1024, H=4, D=64 1.93 ->
+// 1.59; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
+// D = 128: evo_bwd_wide.cuh.
+// ---------------------------------------------------------------------------
+template <int DH, bool WHOLE>
+struct BwdCfg {
+    static constexpr bool ALIAS = (DH == 64);
+    static constexpr bool TWO_PHASE = (DH == 64);
+    static_assert(DH == 32 || DH == 64, "evo_bwd_wide.cuh has D = 128");
+    static constexpr int NG = 4;                       // compute groups
+    static constexpr int CW = TILE / NG;               // q columns per group
+    static constexpr int NCW = 4 * NG;
+    static constexpr int W_DRAIN = NCW, W_PROD = NCW + 4, W_MMA = NCW + 5;
+    static constexpr int THREADS = (NCW + 8) * 32;
+    static constexpr int QS = (DH == 32) ? 3 : 2;      // Q/dO stages
+    static constexpr int NKV = (DH == 32) ? 2 : 1;     // K/V buffers
+    static constexpr int NB = 2;                       // bias tiles
+    static constexpr int DQ_BUFS = 2;
+    static constexpr uint32_t ROWT = RowTile<DH>::BYTES;
+    static constexpr uint32_t ST_Q = 0, ST_DO = ROWT, ST_XQ = 2 * ROWT;
+    static constexpr uint32_t STAGE_BYTES = 2 * ROWT + XT_BYTES;
+    static constexpr uint32_t KV_K = 0, KV_V = ROWT, KV_XK = 2 * ROWT, KV_BYTES = 2 * ROWT + XT_BYTES;
+    static constexpr uint32_t OFF_STAGE = 0;
+    static constexpr uint32_t OFF_KV = OFF_STAGE + QS * STAGE_BYTES;
+    static constexpr uint32_t OFF_BIAS = OFF_KV + NKV * KV_BYTES;
+    static constexpr uint32_t OFF_DS = OFF_BIAS + NB * SQ_BYTES;
+    // per drain warp: WSLOTS slots of [32 rows][32 fp32], for bulk copies of dQ, dK and dV
+    static constexpr uint32_t WQ_BYTES = 32 * 32 * 4;
+    static constexpr int WSLOTS = (DH == 32) ? 2 : 1;
+    static constexpr uint32_t OFF_WSTG = OFF_DS + SQ_BYTES;
+    // constant extra tiles, above every tile that refers to the zero tile
+    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WSLOTS * WQ_BYTES;            // row selector of -delta
+    static constexpr uint32_t OFF_ZERO = OFF_XDP + XT_BYTES;
+    static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
+    static constexpr uint32_t NUM_BARS = 2 * QS + 2 * NKV + 2 * NB + 2 * DQ_BUFS + 9;
+    static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
+    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + alignment slack
+    static constexpr uint32_t TMEM_S = 0, TMEM_DP = 128;
+    static constexpr uint32_t TMEM_P = 256;                                 // not ALIAS: P^T, then dS^T
+    static constexpr uint32_t TMEM_DQ = ALIAS ? 256 : 384;               // DQ_BUFS accumulators
+    static constexpr uint32_t TMEM_DK = TMEM_DQ + 2 * DH, TMEM_DV = TMEM_DK + DH;
+    // column of contraction block kk (16 q) of P^T / dS^T: dense, or inside the columns of its own group
+    __device__ static __forceinline__ uint32_t p_col(int kk) {
+        return ALIAS ? TMEM_S + 32 * (kk >> 1) + 8 * (kk & 1) : TMEM_P + 8 * kk;
+    }
+    __device__ static __forceinline__ uint32_t ds_col(int kk) { return p_col(kk) + (ALIAS ? 128 : 64); }
+    static_assert(TMEM_DV + DH <= BWD_TMEM_COLS, "tensor memory budget");
+    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+    static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
+};
+
+template <int DH, bool WHOLE, int DBIAS_HERE>
+__global__ void __launch_bounds__((BwdCfg<DH, WHOLE>::THREADS), 1)
 evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_dq,
-               const BwdParams p) {
-    using C = BwdCfg<DH>;
+               const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
+    using C = BwdCfg<DH, WHOLE>;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
-    constexpr int RC = C::RC, QS = C::QS;
-    constexpr bool KVR = C::KV_RESIDENT;
+    constexpr int QS = C::QS, NKV = C::NKV, NB = C::NB, DQB = C::DQ_BUFS;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BARS);
     uint64_t* st_full = bars;                  // [QS]
     uint64_t* st_empty = st_full + QS;         // [QS]
-    uint64_t* kv_full = st_empty + QS;         // resident K/V only
-    uint64_t* kv_empty = kv_full + 1;
-    uint64_t* bias_full = kv_empty + 1;
-    uint64_t* bias_empty = bias_full + 1;
-    uint64_t* sdp_full = bias_empty + 1;
-    uint64_t* sdp_free = sdp_full + 1;
-    uint64_t* pds_ready = sdp_free + 1;
-    uint64_t* dq_full = pds_ready + 1;         // [2]
-    uint64_t* dq_free = dq_full + 2;           // [2]
-    uint64_t* dkv_free = dq_free + 2;          // [RC]: accumulators of row r of the chunk are read out
-    uint64_t* tail_done = dkv_free + RC;       // [2] by step parity: both tail issuers' MMAs of a step are complete
+    uint64_t* kv_full = st_empty + QS;         // [NKV]
+    uint64_t* kv_empty = kv_full + NKV;        // [NKV]
+    uint64_t* s_full = kv_empty + NKV;         // [NB]: S' complete and the bias tile landed
+    uint64_t* bias_empty = s_full + NB;        // [NB]
+    uint64_t* dq_full = bias_empty + NB;       // [DQB]
+    uint64_t* dq_free = dq_full + DQB;         // [DQB]
+    uint64_t* dp_full = dq_free + DQB;         // dP' complete
+    uint64_t* s_free = dp_full + 1;            // S', dP' are read (one phase)
+    uint64_t* p_ready = s_free + 1;            // P^T is written (two phases)
+    uint64_t* ds_ready = p_ready + 1;          // dS^T and the dS tile are written
+    uint64_t* dv_done = ds_ready + 1;          // dV of the step is complete
+    uint64_t* dk_done = dv_done + 1;           // dK
+    uint64_t* dq_done = dk_done + 1;           // dQ; one phase: dV, dK and dQ
+    uint64_t* dkv_full = dq_done + 1;          // dK, dV of the segment are complete
+    uint64_t* dkv_free = dkv_full + 1;         // ... and read out
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // uniform
     const int lane = tid & 31;
     const int NT = p.NT;
     WaitCtx wc{abort_flag, p.status};
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 2); }
-        mbar_init(kv_full, 1);
-        mbar_init(kv_empty, 2);
-        for (int i = 0; i < 2; ++i) mbar_init(&tail_done[i], 2);
-        mbar_init(bias_full, 1);
-        mbar_init(bias_empty, 8);
-        mbar_init(sdp_full, 1);
-        mbar_init(sdp_free, 8);
-        mbar_init(pds_ready, 8);
-        for (int i = 0; i < 2; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
-        for (int i = 0; i < RC; ++i) mbar_init(&dkv_free[i], 4);
+        tmem_slot[3] = 0;                      // the flag of the waits before exit: never set
+        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
+        for (int i = 0; i < NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
+        for (int i = 0; i < NB; ++i) { mbar_init(&s_full[i], 2); mbar_init(&bias_empty[i], C::NCW); }
+        for (int i = 0; i < DQB; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
+        for (uint64_t* x : {s_free, p_ready, ds_ready}) mbar_init(x, C::NCW);
+        for (uint64_t* x : {dp_full, dv_done, dk_done, dkv_full}) mbar_init(x, 1);
+        mbar_init(dq_done, C::TWO_PHASE ? 1 : 2);
+        mbar_init(dkv_free, 4);
         fence_mbar_init();
-        fence_async_smem();
     }
-    if (warp == BWD_WARP_MMA) {
+    if (warp == C::W_MMA) {
         tmem_alloc(tmem_slot, BWD_TMEM_COLS);
         tmem_relinquish();
     }
-    if (warp == BWD_WARP_PRODUCER && lane == 0) {
+    if (warp == C::W_PROD && lane == 0) {
         prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do);
-        prefetch_tmap(&tm_bias); prefetch_tmap(&tm_dq);
+        prefetch_tmap(&tm_bias); prefetch_tmap(&tm_dq); prefetch_tmap(&tm_dk); prefetch_tmap(&tm_dv);
     }
     // constant extra tiles: row n of the -delta selector is (0,0,0,0,1,1,0,0); the zero tile
     if (tid < 128) {
@@ -211,412 +222,515 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         *reinterpret_cast<uint4*>(smem + C::OFF_ZERO + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     fence_async_smem();
-    EVO_TRACE_INIT();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    EVO_TS(t_kernel);
 
-    const int first = blockIdx.x;
-    const int stride = gridDim.x;
+    // Segments of this CTA: segment sg is kv tile sg % NT of item sg / NT (WHOLE), or an item of its own.
+    // Item index -> (batch * S + row, head[, kv tile]), the last one fastest.
+    const int first = blockIdx.x, stride = gridDim.x;
     const int n_items = (p.total_items > first) ? (p.total_items - first + stride - 1) / stride : 0;
-
-    // item index -> (batch, first row, rows, head, kv tile); kv tile fastest, then head
-    auto decode = [&](int it) -> BwdItem {
-        BwdItem x;
-        const int w = first + it * stride;
-        x.j = w % NT;
-        const int r1 = w / NT;
-        x.h = r1 % p.H;
-        const int r2 = r1 / p.H;
-        const int c = r2 % p.CPB;
-        x.b = r2 / p.CPB;
-        const int s0 = c * RC;
-        x.nr = (p.S - s0 < RC) ? (p.S - s0) : RC;
-        x.bs0 = x.b * p.S + s0;
-        return x;
+    const int n_segs = WHOLE ? n_items * NT : n_items;
+    const bool resident = WHOLE && NT <= DQB;      // dQ stays in tensor memory for the item
+    auto decode = [&](int sg, int& bs, int& h, int& j) {
+        int w = first + (WHOLE ? sg / NT : sg) * stride;
+        if (WHOLE) {
+            j = sg % NT;
+        } else {
+            j = w % NT;
+            w /= NT;
+        }
+        h = w % p.H;
+        bs = w / p.H;
     };
 
-    if (warp >= BWD_WARP_DRAIN) {
-        reg_dec<BWD_REGS_OTHER<DH>>();
-        if (warp == BWD_WARP_PRODUCER && lane == 0) {
-            // ------------------------------ producer ------------------------------
-            bool ok = true;
-            int gs = 0, gb = 0;
-            for (int it = 0; it < n_items && ok; ++it) {
-                const BwdItem x = decode(it);
-                const int nsteps = NT * x.nr;
-                if (KVR) {
-                    if (it > 0) ok = mbar_wait(kv_empty, (it - 1) & 1, wc, 0x40);
-                    if (!ok) break;
-                    uint8_t* kvb = smem + C::OFF_KV;
-                    mbar_arrive_expect_tx(kv_full, x.nr * C::KV_TX);
-                    for (int r = 0; r < x.nr; ++r) {
-                        tma_load_row_tile<DH>(kvb + r * C::ROWT, &tm_k, kv_full, x.h, x.j * TILE, x.bs0 + r);
-                        tma_load_row_tile<DH>(kvb + (RC + r) * C::ROWT, &tm_v, kv_full, x.h, x.j * TILE, x.bs0 + r);
-                        bulk_load(kvb + 2 * RC * C::ROWT + r * XT_BYTES,
-                                  p.xk + (static_cast<size_t>(x.bs0 + r) * p.NTP + x.j * TILE) * 8, XT_BYTES, kv_full);
-                    }
+    if (warp == C::W_PROD) {
+        // ------------------------------ producer ------------------------------
+        bool ok = true;
+        int gs = 0, n_st = 0, n_bias = 0, n_kv = 0;      // steps; loads issued
+        for (int sg = 0; sg < n_segs && ok; ++sg) {
+            int bs, h, j;
+            decode(sg, bs, h, j);
+            const int b = bs / p.S;
+            const __nv_bfloat16* xq = p.xq + (static_cast<size_t>(bs) * p.H + h) * p.NTP * 8;
+            {
+                const int kb = sg % NKV;
+                if (sg >= NKV) ok = warp_all(mbar_wait(&kv_empty[kb], ((sg / NKV) - 1) & 1, wc, 0x40));
+                if (!ok) break;
+                if (elect_one()) {
+                    uint8_t* kvb = smem + C::OFF_KV + kb * C::KV_BYTES;
+                    mbar_arrive_expect_tx(&kv_full[kb], C::KV_BYTES);
+                    tma_load_row_tile<DH>(kvb + C::KV_K, &tm_k, &kv_full[kb], h, j * TILE, bs);
+                    tma_load_row_tile<DH>(kvb + C::KV_V, &tm_v, &kv_full[kb], h, j * TILE, bs);
+                    bulk_load(kvb + C::KV_XK, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &kv_full[kb]);
                 }
-                for (int n = 0; n < nsteps && ok; ++n, ++gs) {
-                    const int i = n / x.nr, r = n - i * x.nr;
-                    const int st = gs % QS;
-                    if (C::BIAS_STAGED && r == 0) {
-                        if (gb > 0) ok = mbar_wait(bias_empty, (gb - 1) & 1, wc, 0x41);
-                        if (!ok) break;
-                        mbar_arrive_expect_tx(bias_full, SQ_BYTES);
-                        tma_load_4d(smem + C::OFF_BIAS, &tm_bias, bias_full, x.j * TILE, i * TILE, x.h, x.b);
-                        tma_load_4d(smem + C::OFF_BIAS + SQ_SUB_BYTES, &tm_bias, bias_full, x.j * TILE + 64,
-                                    i * TILE, x.h, x.b);
-                        ++gb;
-                    }
-                    if (gs >= QS) ok = mbar_wait(&st_empty[st], ((gs / QS) - 1) & 1, wc, 0x42);
-                    if (!ok) break;
-                    const int bs = x.bs0 + r;
-                    uint8_t* sb = smem + C::OFF_STAGE + st * C::STAGE_STRIDE;
-                    mbar_arrive_expect_tx(&st_full[st], C::STAGE_TX);
-                    tma_load_row_tile<DH>(sb + C::ST_Q, &tm_q, &st_full[st], x.h, i * TILE, bs);
-                    tma_load_row_tile<DH>(sb + C::ST_DO, &tm_do, &st_full[st], x.h, i * TILE, bs);
-                    if (!KVR) {
-                        tma_load_row_tile<DH>(sb + C::ST_K, &tm_k, &st_full[st], x.h, x.j * TILE, bs);
-                        tma_load_row_tile<DH>(sb + C::ST_V, &tm_v, &st_full[st], x.h, x.j * TILE, bs);
-                        bulk_load(sb + C::ST_XK, p.xk + (static_cast<size_t>(bs) * p.NTP + x.j * TILE) * 8, XT_BYTES,
-                                  &st_full[st]);
-                    }
-                    const size_t ro = (static_cast<size_t>(bs) * p.H + x.h) * p.NTP + i * TILE;
-                    bulk_load(sb + C::ST_XQ, p.xq + ro * 8, XT_BYTES, &st_full[st]);
-                }
+                __syncwarp();
+                ++n_kv;
             }
-            // Drain: the most recent loads have landed before the CTA exits.
-            for (int k = (gs > QS ? gs - QS : 0); k < gs; ++k)
-                (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, wc, 0x43);
-            if (gb > 0) (void)mbar_wait(bias_full, (gb - 1) & 1, wc, 0x44);
-            if (KVR && n_items > 0) (void)mbar_wait(kv_full, (n_items - 1) & 1, wc, 0x45);
-        } else if (warp >= BWD_WARP_MMA) {
-            // ------------------------------ mma issuers ------------------------------
-            // Three warps, one chain family each, so that no chain queues behind another one's
-            // issue: warp 13 issues S' and dP' of the next step as soon as the compute groups have
-            // read the previous pair, warp 14 issues dV += P^T dO and dK += dS^T Q, warp 15 issues
-            // dQ = dS K.  Each warp runs its loop with all lanes (uniform control flow: operand
-            // descriptors stay in uniform registers) and elects one lane to issue.
-            constexpr uint32_t IDESC_SDP = make_idesc_bf16(128, 128, 0, 0);
-            // N = the head-dim columns that hold data (the rest of a wider kernel's tile is zero fill)
-            const uint32_t IDESC_DKV = make_idesc_bf16(128, 16 * p.KB, 1, 1);
-            const uint32_t IDESC_DQ = make_idesc_bf16(128, 16 * p.KB, 0, 1);
-            const uint32_t aSt = smem_u32(smem + C::OFF_STAGE), aKV = smem_u32(smem + C::OFF_KV);
-            const uint32_t aZero = smem_u32(smem + C::OFF_ZERO);
-            const int role = warp - BWD_WARP_MMA;          // 0: S/dP, 1: dV/dK, 2: dQ
-            bool ok = true;
-            int gs = 0;
-            for (int it = 0; it < n_items && ok; ++it) {
-                const BwdItem x = decode(it);
-                const int nsteps = NT * x.nr;
-                int i = 0, r = 0;
-                for (int n = 0; n < nsteps && ok; ++n, ++gs) {
-                    const int st = gs % QS;
-                    const uint32_t sb = aSt + st * C::STAGE_STRIDE;
-                    const uint32_t k_tile = KVR ? aKV + r * C::ROWT : sb + C::ST_K;
-                    if (role == 0) {
-                        ok = warp_all(mbar_wait(&st_full[st], (gs / QS) & 1, wc, 0x50));
-                        if (ok && KVR && n == 0) ok = warp_all(mbar_wait(kv_full, it & 1, wc, 0x51));
-                        if (ok && gs > 0) ok = warp_all(mbar_wait(sdp_free, (gs - 1) & 1, wc, 0x52));
-                        // S' shares its columns with the single dQ accumulator: the previous step's dQ is drained
-                        if (ok && C::DQ_BUFS == 1 && gs > 0) ok = warp_all(mbar_wait(&dq_free[0], (gs - 1) & 1, wc, 0x56));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const uint32_t v_tile = KVR ? aKV + (RC + r) * C::ROWT : sb + C::ST_V;
-                            const uint32_t q_lo = RD::kmajor_lo(sb + C::ST_Q), do_lo = RD::kmajor_lo(sb + C::ST_DO);
-                            const uint32_t k_lo = RD::kmajor_lo(k_tile), v_lo = RD::kmajor_lo(v_tile);
-#pragma unroll
-                            for (int kk = 0; kk < RT::KBLOCKS; ++kk) {
-                                if (kk >= p.KB) continue;      // zero-filled blocks past the true head dim
-                                umma_ss(tmem + C::TMEM_S, RD::kmajor(q_lo, kk), RD::kmajor(k_lo, kk), IDESC_SDP, kk > 0);
-                                umma_ss(tmem + C::TMEM_DP, RD::kmajor(do_lo, kk), RD::kmajor(v_lo, kk), IDESC_SDP, kk > 0);
-                            }
-                            // + (mask - LSE) / scale on S, - delta on dP: the extra contraction block
-                            const uint64_t d_xq = xt_desc(sb + C::ST_XQ, aZero);
-                            const uint32_t xk_addr = KVR ? aKV + 2 * RC * C::ROWT + r * XT_BYTES : sb + C::ST_XK;
-                            umma_ss(tmem + C::TMEM_S, d_xq, xt_desc(xk_addr, aZero), IDESC_SDP, 1u);
-                            umma_ss(tmem + C::TMEM_DP, d_xq, xt_desc(smem_u32(smem + C::OFF_XDP), aZero), IDESC_SDP, 1u);
-                            umma_commit(sdp_full);
-                        }
-                        __syncwarp();
-                    } else if (role == 1) {
-                        ok = warp_all(mbar_wait(pds_ready, gs & 1, wc, 0x53));
-                        // the first MMA into row r's dK/dV of an item overwrites them: the previous item's must be out
-                        if (ok && i == 0 && it > 0) ok = warp_all(mbar_wait(&dkv_free[r], (it - 1) & 1, wc, 0x55));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const uint32_t p_mn_lo = SqDesc::mnmajor_lo(smem_u32(smem + C::OFF_P));
-                            const uint32_t ds_mn_lo = SqDesc::mnmajor_lo(smem_u32(smem + C::OFF_DS));
-                            const uint32_t q_lo = RD::mnmajor_lo(sb + C::ST_Q), do_lo = RD::mnmajor_lo(sb + C::ST_DO);
-                            const uint32_t t_dk = tmem + C::TMEM_DKV + r * 2 * DH, t_dv = t_dk + DH;
-                            const uint32_t acc = (i > 0) ? 1u : 0u;
-#pragma unroll
-                            for (int kk = 0; kk < 8; ++kk) {      // two interleaved chains
-                                umma_ss(t_dv, SqDesc::mnmajor(p_mn_lo, kk), RD::mnmajor(do_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
-                                umma_ss(t_dk, SqDesc::mnmajor(ds_mn_lo, kk), RD::mnmajor(q_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
-                            }
-                            umma_commit(&tail_done[gs & 1]);
-                            umma_commit(&st_empty[st]);
-                            if (KVR && n == nsteps - 1) umma_commit(kv_empty);
-                        }
-                        __syncwarp();
-                    } else if (role == 2) {
-                        ok = warp_all(mbar_wait(pds_ready, gs & 1, wc, 0x53));
-                        if (ok && gs >= C::DQ_BUFS)
-                            ok = warp_all(mbar_wait(&dq_free[gs % C::DQ_BUFS], ((gs / C::DQ_BUFS) - 1) & 1, wc, 0x54));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-                            const uint32_t ds_k_lo = SqDesc::kmajor_lo(smem_u32(smem + C::OFF_DS));
-                            const uint32_t k_lo = RD::mnmajor_lo(k_tile);
-                            const uint32_t t_dq = tmem + C::TMEM_DQ + (gs % C::DQ_BUFS) * DH;
-#pragma unroll
-                            for (int kk = 0; kk < 8; ++kk)
-                                umma_ss(t_dq, SqDesc::kmajor(ds_k_lo, kk), RD::mnmajor(k_lo, kk), IDESC_DQ, kk > 0);
-                            umma_commit(&dq_full[gs % C::DQ_BUFS]);
-                            umma_commit(&tail_done[gs & 1]);
-                            umma_commit(&st_empty[st]);
-                            if (KVR && n == nsteps - 1) umma_commit(kv_empty);
-                        }
-                        __syncwarp();
-                    }
-                    if (++r == x.nr) { r = 0; ++i; }
+            for (int i = 0; i < NT && ok; ++i, ++gs) {
+                const int st = gs % QS, bb = gs % NB;
+                uint8_t* sb = smem + C::OFF_STAGE + st * C::STAGE_BYTES;
+                if (gs >= QS) ok = warp_all(mbar_wait(&st_empty[st], ((gs / QS) - 1) & 1, wc, 0x42));
+                if (!ok) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&st_full[st], C::STAGE_BYTES);
+                    tma_load_row_tile<DH>(sb + C::ST_Q, &tm_q, &st_full[st], h, i * TILE, bs);
+                    tma_load_row_tile<DH>(sb + C::ST_DO, &tm_do, &st_full[st], h, i * TILE, bs);
+                    bulk_load(sb + C::ST_XQ, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &st_full[st]);
                 }
+                __syncwarp();
+                ++n_st;
+                if (gs >= NB) ok = warp_all(mbar_wait(&bias_empty[bb], ((gs / NB) - 1) & 1, wc, 0x41));
+                if (!ok) break;
+                if (elect_one()) {
+                    uint8_t* bt = smem + C::OFF_BIAS + bb * SQ_BYTES;
+                    mbar_arrive_expect_tx(&s_full[bb], SQ_BYTES);
+                    tma_load_4d(bt, &tm_bias, &s_full[bb], j * TILE, i * TILE, h, b);
+                    tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &s_full[bb], j * TILE + 64, i * TILE, h, b);
+                }
+                __syncwarp();
+                ++n_bias;
             }
-        } else if (warp < BWD_WARP_DRAIN + 4) {
-            // ------------------------------ drain warps ------------------------------
-            const int wrow0 = (warp & 3) * 32;   // tensor-memory lanes (tile rows) of this warp
-            const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
-            uint8_t* wq = smem + C::OFF_WSTG + (warp & 3) * C::WQ_BYTES;
-            bool ok = true;
-            int gs = 0;
-            for (int it = 0; it < n_items && ok; ++it) {
-                const BwdItem x = decode(it);
-                const int nsteps = NT * x.nr;
-                int i = 0, r = 0;
-                for (int n = 0; n < nsteps && ok; ++n, ++gs) {
-                    const int b = gs % C::DQ_BUFS;
-                    ok = warp_all(mbar_wait(&dq_full[b], (gs / C::DQ_BUFS) & 1, wc, 0x68));
+        }
+        // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
+        // barrier with an MMA commit, which may then never come: a bounded pause instead).
+        const WaitCtx dc{tmem_slot + 3, p.status};
+        for (int k = (n_st > QS ? n_st - QS : 0); k < n_st; ++k) (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, dc, 0x43);
+        for (int k = (n_kv > NKV ? n_kv - NKV : 0); k < n_kv; ++k) (void)mbar_wait(&kv_full[k % NKV], (k / NKV) & 1, dc, 0x45);
+        if (!ok && n_bias > 0)
+            for (int k = 0; k < 64; ++k) __nanosleep(1000);
+    } else if (warp >= C::W_MMA) {
+        // ------------------------------ mma issuers ------------------------------
+        // Each warp runs its loop with all lanes (uniform control flow: operand descriptors stay in
+        // uniform registers) and elects one lane to issue.
+        constexpr uint32_t IDESC_SDP = make_idesc_bf16(128, 128, 0, 0);
+        // N = the head-dim columns that hold data (the rest of a wider kernel's tile is zero fill)
+        const uint32_t IDESC_DKV = make_idesc_bf16(128, 16 * p.KB, 0, 1);
+        const uint32_t IDESC_DQ = make_idesc_bf16(128, 16 * p.KB, 1, 1);
+        const uint32_t aSt = smem_u32(smem + C::OFF_STAGE), aKV = smem_u32(smem + C::OFF_KV);
+        const uint32_t aZero = smem_u32(smem + C::OFF_ZERO);
+        const int role = warp - C::W_MMA;          // 0: S/dP, 1: dV/dK, 2: dQ
+        bool ok = true;
+        int gs = 0;
+        for (int sg = 0; sg < n_segs && ok; ++sg) {
+            const int kb = sg % NKV;
+            const uint32_t kvb = aKV + kb * C::KV_BYTES;
+            for (int i = 0; i < NT && ok; ++i, ++gs) {
+                const int st = gs % QS;
+                const uint32_t sb = aSt + st * C::STAGE_BYTES;
+                if (role == 0) {
+                    ok = warp_all(mbar_wait(&st_full[st], (gs / QS) & 1, wc, 0x50));
+                    if (ok && i == 0) ok = warp_all(mbar_wait(&kv_full[kb], (sg / NKV) & 1, wc, 0x51));
+                    // the columns are read, or (ALIAS) P^T in them is consumed
+                    if (ok && gs > 0) ok = warp_all(mbar_wait(C::ALIAS ? dv_done : s_free, (gs - 1) & 1, wc, 0x52));
                     if (!ok) break;
                     tc_fence_after();
-                    // dQ of this step: tensor memory -> this warp's slot -> fp32 reduce-add
+                    const uint64_t d_xq = xt_desc(sb + C::ST_XQ, aZero);
+                    if (elect_one()) {
+                        const uint32_t q_lo = RD::kmajor_lo(sb + C::ST_Q), k_lo = RD::kmajor_lo(kvb + C::KV_K);
 #pragma unroll
-                    for (int rd = 0; rd < DH / 32; ++rd) {
-                        float dqv[32];
-                        tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
-                        if (rd == DH / 32 - 1) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&dq_free[b]);
-                        }
-                        if (i * TILE + wrow0 < p.N && rd * 32 < p.Dt) {     // warp-uniform
-                            // the slot is free once lane 0's earlier bulk operations have read it
-                            if (lane == 0) tma_wait_group_read<0>();
-                            __syncwarp();
-#pragma unroll
-                            for (int cc = 0; cc < 8; ++cc)
-                                *reinterpret_cast<float4*>(wq + swz_off<128>(lane, cc)) =
-                                    make_float4(dqv[cc * 4 + 0] * p.scale, dqv[cc * 4 + 1] * p.scale,
-                                                dqv[cc * 4 + 2] * p.scale, dqv[cc * 4 + 3] * p.scale);
-                            fence_async_smem();
-                            __syncwarp();
-                            if (lane == 0) {
-                                tma_reduce_add_4d(&tm_dq, wq, rd * 32, x.h, i * TILE + wrow0, x.bs0 + r);
-                                tma_commit_group();
-                            }
-                        }
+                        for (int kk = 0; kk < RT::KBLOCKS; ++kk)
+                            if (kk < p.KB)      // the others are zero-filled blocks past the true head dim
+                                umma_ss(tmem + C::TMEM_S, RD::kmajor(k_lo, kk), RD::kmajor(q_lo, kk), IDESC_SDP, kk > 0);
+                        // + (mask - LSE) / scale: the extra contraction block
+                        umma_ss(tmem + C::TMEM_S, xt_desc(kvb + C::KV_XK, aZero), d_xq, IDESC_SDP, 1u);
+                        if (C::TWO_PHASE) umma_commit(&s_full[gs % NB]);
                     }
-                    if (n == nsteps - 1) {
-                        ok = warp_all(mbar_wait(&tail_done[gs & 1], (gs >> 1) & 1, wc, 0x69));
+                    __syncwarp();
+                    if (C::TWO_PHASE && gs > 0) ok = warp_all(mbar_wait(dk_done, (gs - 1) & 1, wc, 0x59));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t do_lo = RD::kmajor_lo(sb + C::ST_DO), v_lo = RD::kmajor_lo(kvb + C::KV_V);
+#pragma unroll
+                        for (int kk = 0; kk < RT::KBLOCKS; ++kk)
+                            if (kk < p.KB)
+                                umma_ss(tmem + C::TMEM_DP, RD::kmajor(v_lo, kk), RD::kmajor(do_lo, kk), IDESC_SDP, kk > 0);
+                        // - delta
+                        umma_ss(tmem + C::TMEM_DP, xt_desc(smem_u32(smem + C::OFF_XDP), aZero), d_xq, IDESC_SDP, 1u);
+                        umma_commit(C::TWO_PHASE ? dp_full : &s_full[gs % NB]);
+                    }
+                    __syncwarp();
+                } else if (role == 1) {
+                    const uint32_t acc = (i > 0) ? 1u : 0u;
+                    // the first MMA of a segment overwrites dK / dV: the previous one's must be out
+                    if (i == 0 && sg > 0) ok = warp_all(mbar_wait(dkv_free, (sg - 1) & 1, wc, 0x55));
+                    const uint32_t q_lo = RD::mnmajor_lo(sb + C::ST_Q), do_lo = RD::mnmajor_lo(sb + C::ST_DO);
+                    auto dv = [&](int kk) {
+                        umma_ts(tmem + C::TMEM_DV, tmem + C::p_col(kk), RD::mnmajor(do_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
+                    };
+                    auto dk = [&](int kk) {
+                        umma_ts(tmem + C::TMEM_DK, tmem + C::ds_col(kk), RD::mnmajor(q_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
+                    };
+                    if constexpr (C::TWO_PHASE) {
+                        if (ok) ok = warp_all(mbar_wait(p_ready, gs & 1, wc, 0x53));
                         if (!ok) break;
                         tc_fence_after();
-                        // the item's last MMAs are done: dK/dV -> bf16 stores, row by row of the chunk;
-                        // each row's accumulators are handed back as soon as they are read
-                        const int kvrow = x.j * TILE + wrow0 + lane;
+                        if (elect_one()) {
 #pragma unroll
-                        for (int rr = 0; rr < RC; ++rr) {
-                            if (rr < x.nr) {
+                            for (int kk = 0; kk < 8; ++kk) dv(kk);
+                            umma_commit(dv_done);
+                        }
+                        __syncwarp();
+                    }
+                    if (ok) ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5a));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        if constexpr (C::TWO_PHASE) {
 #pragma unroll
-                                for (int t = 0; t < 2; ++t) {      // 0: dK, 1: dV
-                                    const float sc = t ? 1.0f : p.scale;
-                                    __nv_bfloat16* out = (t ? p.dv : p.dk) + (x.bs0 + rr) * p.lay.row +
-                                                         kvrow * p.lay.n + x.h * p.lay.h;
+                            for (int kk = 0; kk < 8; ++kk) dk(kk);
+                            umma_commit(dk_done);
+                        } else {
 #pragma unroll
-                                    for (int hf = 0; hf < DH / 32; ++hf) {
-                                        float v[32];
-                                        tmem_ld_f32<32>(lane_base + C::TMEM_DKV + rr * 2 * DH + t * DH + hf * 32, v);
-                                        if (kvrow < p.N) {
-#pragma unroll
-                                            for (int c8 = 0; c8 < 4; ++c8) {
-                                                if (hf * 32 + c8 * 8 >= p.Dt) continue;
-                                                uint4 u;
-                                                u.x = pack_bf16(v[c8 * 8 + 0] * sc, v[c8 * 8 + 1] * sc);
-                                                u.y = pack_bf16(v[c8 * 8 + 2] * sc, v[c8 * 8 + 3] * sc);
-                                                u.z = pack_bf16(v[c8 * 8 + 4] * sc, v[c8 * 8 + 5] * sc);
-                                                u.w = pack_bf16(v[c8 * 8 + 6] * sc, v[c8 * 8 + 7] * sc);
-                                                *reinterpret_cast<uint4*>(out + hf * 32 + c8 * 8) = u;
-                                            }
-                                        }
-                                    }
-                                }
-                            }
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&dkv_free[rr]);
+                            for (int kk = 0; kk < 8; ++kk) { dv(kk); dk(kk); }      // two interleaved chains
+                            umma_commit(dq_done);
+                        }
+                        umma_commit(&st_empty[st]);
+                        if (i == NT - 1) {
+                            umma_commit(dkv_full);
+                            umma_commit(&kv_empty[kb]);
                         }
                     }
-                    if (++r == x.nr) { r = 0; ++i; }
+                    __syncwarp();
+                } else {
+                    // accumulators: one per step, or (resident) one per q tile of the item
+                    const int j = WHOLE ? sg % NT : 0;
+                    const int ev = resident ? (sg - j) + i : gs;
+                    if (ev >= DQB && !(resident && j > 0)) ok = warp_all(mbar_wait(&dq_free[ev % DQB], ((ev / DQB) - 1) & 1, wc, 0x54));
+                    if (ok) ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5b));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t ds_lo = SqDesc::mnmajor_lo(smem_u32(smem + C::OFF_DS));
+                        const uint32_t k_lo = RD::mnmajor_lo(kvb + C::KV_K);
+                        const uint32_t t_dq = tmem + C::TMEM_DQ + (ev % DQB) * DH;
+                        const uint32_t acc = (resident && j > 0) ? 1u : 0u;
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)
+                            umma_ss(t_dq, SqDesc::mnmajor(ds_lo, kk), RD::mnmajor(k_lo, kk), IDESC_DQ, kk > 0 ? 1u : acc);
+                        umma_commit(dq_done);
+                        if (!resident || j == NT - 1) umma_commit(&dq_full[ev % DQB]);
+                        if (i == NT - 1) umma_commit(&kv_empty[kb]);
+                    }
+                    __syncwarp();
                 }
             }
-            if (lane == 0) tma_wait_group<0>();
         }
-    } else {
-        reg_inc<BWD_REGS_COMPUTE<DH>>();
-        // ------------------------------ compute groups ------------------------------
-        const int wg = warp >> 2;            // kv columns 64*wg .. 64*wg+63 of the tile
-        const int row = tid & 127;           // q row within the tile == TMEM lane
-        const int wrow0 = (warp & 3) * 32;   // first tile row of this warp
+    } else if (warp >= C::W_DRAIN) {
+        // ------------------------------ drain warps ------------------------------
+        const int w4 = warp & 3;
+        const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
-        const uint32_t aP = smem_u32(smem + C::OFF_P) + wg * SQ_SUB_BYTES;
-        const uint32_t aDS = smem_u32(smem + C::OFF_DS) + wg * SQ_SUB_BYTES;
-        const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + wg * SQ_SUB_BYTES;
-        const uint32_t scratch_w = smem_u32(tmem_slot + 2);       // a word nobody reads
+        uint8_t* const wslot = smem + C::OFF_WSTG + w4 * C::WSLOTS * C::WQ_BYTES;
+        // Where the next bulk copy (one group each) is staged, once the copy that used the place last has read it:
+        // two slots in turn, or with one slot its two halves for copies of half its size.
+        int pos = 0;
+        bool last_half = false;
+        auto next_slot = [&](bool half) -> uint8_t* {
+            if (lane == 0) {
+                if (C::WSLOTS == 2 || (half && last_half)) tma_wait_group_read<1>();
+                else tma_wait_group_read<0>();
+            }
+            __syncwarp();
+            last_half = half;
+            pos ^= 1;
+            return wslot + (C::WSLOTS == 2 ? pos * C::WQ_BYTES : (half ? pos * (C::WQ_BYTES / 2) : 0));
+        };
+        // 32 columns of 32 rows as bf16, by a bulk tensor store (which clips rows past N and columns past Dt)
+        auto store_rows = [&](const CUtensorMap* tm, const uint4 (&u)[4], int h, int row0, int col0, int bs) {
+            uint8_t* sl = next_slot(true);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sl + swz_off<64>(lane, c)) = u[c];
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_4d(tm, sl, col0, h, row0, bs);
+                tma_commit_group();
+            }
+        };
+        auto pack_rows = [](uint4 (&u)[4], const float (&v)[32], float sc) {
+#pragma unroll
+            for (int c8 = 0; c8 < 4; ++c8)
+                u[c8] = make_uint4(pack_bf16(v[c8 * 8 + 0] * sc, v[c8 * 8 + 1] * sc), pack_bf16(v[c8 * 8 + 2] * sc, v[c8 * 8 + 3] * sc),
+                                   pack_bf16(v[c8 * 8 + 4] * sc, v[c8 * 8 + 5] * sc), pack_bf16(v[c8 * 8 + 6] * sc, v[c8 * 8 + 7] * sc));
+        };
+        // WHOLE: the partial sums of this CTA, in units of 4 KB: 32 rows x 32 columns as [16-byte word][row]
+        float4* part = reinterpret_cast<float4*>(p.dq_scratch) + static_cast<size_t>(blockIdx.x) * p.scratch_stride;
         bool ok = true;
-        int gs = 0, gb = 0;
-        const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
-
-        uint32_t bias_pk[32];                // this thread's 64 bias values (bf16 pairs)
-
-        for (int it = 0; it < n_items && ok; ++it) {
-            const BwdItem x = decode(it);
-            const int nsteps = NT * x.nr;
-            int r = 0;                       // row of the chunk, innermost
-            for (int n = 0; n < nsteps && ok; ++n, ++gs) {
-                if (!C::BIAS_STAGED && r == 0) {
-                    // this thread's 64 bias values of q tile n / nr, straight from global memory,
-                    // requested before the wait so that they arrive while the MMAs run
-                    const int qrow = (n / x.nr) * TILE + row, col0 = x.j * TILE + 64 * wg;
-                    const __nv_bfloat16* bp = p.bias + ((static_cast<size_t>(x.b) * p.H + x.h) * p.N + qrow) * p.N + col0;
-#pragma unroll
-                    for (int c8 = 0; c8 < 8; ++c8) {
-                        uint4 bv = make_uint4(0u, 0u, 0u, 0u);
-                        if (qrow < p.N && col0 + c8 * 8 < p.N) bv = __ldg(reinterpret_cast<const uint4*>(bp + c8 * 8));
-                        bias_pk[c8 * 4 + 0] = bv.x; bias_pk[c8 * 4 + 1] = bv.y;
-                        bias_pk[c8 * 4 + 2] = bv.z; bias_pk[c8 * 4 + 3] = bv.w;
-                    }
+        int gs = 0;
+        for (int sg = 0; sg < n_segs && ok; ++sg) {
+            int bs, h, j;
+            decode(sg, bs, h, j);
+            for (int i = 0; i < NT && ok; ++i, ++gs) {
+                if (resident && j < NT - 1) continue;          // dQ is still being summed
+                const int ev = resident ? (sg - j) + i : gs, b = ev % DQB;
+                const bool rows = i * TILE + wrow0 < p.N;     // warp-uniform: some row of this warp exists
+                const bool final_sum = WHOLE && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
+                float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
+                float4 old[8];
+                // The bulk copy that last wrote this part of the scratch area, NT >= 3 steps ago, is complete
+                // before the sum is added to or read: at least two were issued after it.
+                if (WHOLE && j > 0 && !resident) {
+                    if (lane == 0) tma_wait_group<2>();
+                    if (add) fence_async_all();
+                    __syncwarp();
                 }
-                ok = warp_all(mbar_wait(sdp_full, gs & 1, wc, 0x63));
+                ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
                 if (!ok) break;
-                EVO_TS(t_cmp);
-                if (C::BIAS_STAGED && r == 0) {
-                    ok = warp_all(mbar_wait(bias_full, gb & 1, wc, 0x64));
-                    if (!ok) break;
-                    uint32_t dep = 0;
-#pragma unroll
-                    for (int c8 = 0; c8 < 8; ++c8) {
-                        const uint4 bv = lds128(aBias + swz_off<128>(row, c8));
-                        bias_pk[c8 * 4 + 0] = bv.x; bias_pk[c8 * 4 + 1] = bv.y;
-                        bias_pk[c8 * 4 + 2] = bv.z; bias_pk[c8 * 4 + 3] = bv.w;
-                        dep ^= bv.x;
-                    }
-                    mbar_release_after_loads(bias_empty, dep, scratch_w);     // the tile now lives in registers
-                    ++gb;
-                }
-
-                // Per element: x = S' c1 + bias log2e (S' already carries mask and -LSE through the
-                // extra contraction block), P = exp2(x), dS = P dP' (dP' already carries -delta).
-                // Chunks of 16 columns; the tensor-memory loads of chunk ch+1 are in flight during
-                // the arithmetic of chunk ch.
-                uint32_t pkp[32], pkd[32];           // P and dS of this thread's 64 columns, bf16 pairs
-                uint32_t sv[2][16], dv[2][16];
                 tc_fence_after();
-                tmem_ld16(lane_base + C::TMEM_S + 64 * wg, sv[0]);
-                tmem_ld16(lane_base + C::TMEM_DP + 64 * wg, dv[0]);
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    const int cb = ch & 1;
-                    tmem_wait_ld();
-                    if (ch < 3) {
-                        tmem_ld16(lane_base + C::TMEM_S + 64 * wg + 16 * (ch + 1), sv[cb ^ 1]);
-                        tmem_ld16(lane_base + C::TMEM_DP + 64 * wg + 16 * (ch + 1), dv[cb ^ 1]);
-                    } else {
+                for (int rd = 0; rd < DH / 32; ++rd) {
+                    float dqv[32];
+                    tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
+                    if (rd == DH / 32 - 1) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(sdp_free);
+                        if (lane == 0) mbar_arrive(&dq_free[b]);
                     }
-                    float2 p2[8];
+                    if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
+                    if (final_sum) {
+                        if (add) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float2 b2 = fmul2(bf16x2_f2(bias_pk[ch * 8 + k]), l2e2);
-                        const float2 x2 = ffma2(u2f2(sv[cb][2 * k], sv[cb][2 * k + 1]), c1x2, b2);
-                        p2[k] = make_float2(ex2(x2.x), ex2(x2.y));
-                    }
-                    float2 dsv[8];
+                            for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + (rd * 8 + c) * 32 + lane);
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float2 ds2 = fmul2(p2[k], u2f2(dv[cb][2 * k], dv[cb][2 * k + 1]));
-                        pkp[ch * 8 + k] = pack_bf16(p2[k].x, p2[k].y);
-                        pkd[ch * 8 + k] = pack_bf16(ds2.x, ds2.y);
-                        dsv[k] = ds2;
-                    }
-                    if constexpr (DBIAS_HERE != DBIAS_NO) {
-                        // one S row: this step's dS tile is the dBias tile (q tile n, kv tile j)
-                        const int qrow = (n / x.nr) * TILE + row, c0 = x.j * TILE + 64 * wg + 16 * ch;
-                        if (qrow < p.N) {
-                            const size_t at = ((static_cast<size_t>(x.b) * p.H + x.h) * p.N + qrow) * p.N + c0;
-                            if constexpr (DBIAS_HERE == DBIAS_F32) {
-                                float* out = static_cast<float*>(p.dbias) + at;
-#pragma unroll
-                                for (int q4 = 0; q4 < 4; ++q4)
-                                    if (c0 + q4 * 4 < p.N)
-                                        *reinterpret_cast<float4*>(out + q4 * 4) =
-                                            make_float4(dsv[2 * q4].x, dsv[2 * q4].y, dsv[2 * q4 + 1].x, dsv[2 * q4 + 1].y);
-                            } else {
-                                // the bf16 pairs are the ones the MMAs read
-                                __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.dbias) + at;
-#pragma unroll
-                                for (int q8 = 0; q8 < 2; ++q8)
-                                    if (c0 + q8 * 8 < p.N)
-                                        *reinterpret_cast<uint4*>(out + q8 * 8) =
-                                            make_uint4(pkd[ch * 8 + q8 * 4], pkd[ch * 8 + q8 * 4 + 1], pkd[ch * 8 + q8 * 4 + 2],
-                                                       pkd[ch * 8 + q8 * 4 + 3]);
+                            for (int c = 0; c < 8; ++c) {
+                                dqv[4 * c] += old[c].x; dqv[4 * c + 1] += old[c].y;
+                                dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
                             }
                         }
+                        uint4 u[4];
+                        pack_rows(u, dqv, p.scale);
+                        store_rows(&tm_dq, u, h, i * TILE + wrow0, rd * 32, bs);
+                        continue;
+                    }
+                    uint8_t* wq = next_slot(false);
+                    const float sc = WHOLE ? 1.0f : p.scale;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        *reinterpret_cast<float4*>(wq + (WHOLE ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
+                            make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (!WHOLE)
+                            tma_reduce_add_4d(&tm_dq, wq, rd * 32, h, i * TILE + wrow0, bs);
+                        else if (j == 0)
+                            bulk_store(ps + rd * 8 * 32, wq, C::WQ_BYTES);
+                        else
+                            bulk_reduce_add_f32(ps + rd * 8 * 32, wq, C::WQ_BYTES);
+                        tma_commit_group();
                     }
                 }
-                EVO_TE(t_cmp, p.status, 0x70);
-
-                // the P / dS tiles are free once the previous step's dV/dK/dQ MMAs are done
-                if (gs > 0) {
-                    ok = warp_all(mbar_wait(&tail_done[(gs - 1) & 1], ((gs - 1) >> 1) & 1, wc, 0x61));
-                    if (!ok) break;
-                }
-                EVO_TS(t_sts);
+            }
+            if (!ok) break;
+            ok = warp_all(mbar_wait(dkv_full, sg & 1, wc, 0x69));
+            if (!ok) break;
+            tc_fence_after();
+            const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
 #pragma unroll
-                for (int c8 = 0; c8 < 8; ++c8) {
-                    const uint32_t off = swz_off<128>(row, c8);
-                    sts128(aP + off, make_uint4(pkp[c8 * 4 + 0], pkp[c8 * 4 + 1], pkp[c8 * 4 + 2], pkp[c8 * 4 + 3]));
-                    sts128(aDS + off, make_uint4(pkd[c8 * 4 + 0], pkd[c8 * 4 + 1], pkd[c8 * 4 + 2], pkd[c8 * 4 + 3]));
+            for (int t = 0; t < 2; ++t) {                   // dK, then dV
+                uint4 u[DH / 32][4];
+#pragma unroll
+                for (int c = 0; c < DH / 32; ++c) {
+                    float v[32];
+                    __syncwarp();
+                    tmem_ld_f32<32>(lane_base + (t ? C::TMEM_DV : C::TMEM_DK) + c * 32, v);
+                    pack_rows(u[c], v, t ? 1.0f : p.scale);
                 }
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(pds_ready);
-                EVO_TE(t_sts, p.status, 0xb3);
-                if (++r == x.nr) r = 0;
+                if (t == 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(dkv_free);
+                }
+#pragma unroll
+                for (int c = 0; c < DH / 32; ++c)
+                    if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[c], h, j * TILE + wrow0, c * 32, bs);
+            }
+        }
+        if (lane == 0) tma_wait_group<0>();
+    } else {
+        // ------------------------------ compute groups ------------------------------
+        const int g = warp >> 2;             // q columns 32g .. 32g+31 of the tile
+        const int row = tid & 127;           // kv row within the tile == TMEM lane
+        const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+        const uint32_t tS = lane_base + C::TMEM_S + 32 * g, tDP = lane_base + C::TMEM_DP + 32 * g;
+        const uint32_t aDS = smem_u32(smem + C::OFF_DS);
+        // this thread's column of the bias tile ([q][kv], swizzled by q & 7), first row of the group
+        const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + (row >> 6) * SQ_SUB_BYTES + 32 * g * 128 + (row & 7) * 2;
+        const uint32_t bchunk = (row & 63) >> 3;
+        const uint32_t scratch_w = smem_u32(tmem_slot + 2);       // a word nobody reads
+        bool ok = true;
+        int gs = 0;
+        const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
+
+        // one S row: a step's dS tile is the dBias tile (q tile i, kv tile j); columns 16 ch .. of this group
+        auto store_dbias = [&](int ch, int i, int j, int bs, int h, const uint32_t (&pkd)[8], const float2 (&dsv)[8]) {
+            if constexpr (DBIAS_HERE != DBIAS_NO) {
+                // one S row: this step's dS tile is the dBias tile (q tile i, kv tile j)
+                const int kv = j * TILE + row, q0 = i * TILE + 32 * g + 16 * ch;
+                const size_t at = ((static_cast<size_t>(bs) * p.H + h) * p.N + q0) * p.N + kv;
+                if constexpr (DBIAS_HERE == DBIAS_F32) {
+                    float* out = static_cast<float*>(p.dbias) + at;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (kv < p.N && q0 + 2 * k < p.N) out[static_cast<size_t>(2 * k) * p.N] = dsv[k].x;
+                        if (kv < p.N && q0 + 2 * k + 1 < p.N) out[static_cast<size_t>(2 * k + 1) * p.N] = dsv[k].y;
+                    }
+                } else {
+                    // lanes 2n and 2n+1 exchange halves: the even one stores both kv of the even q row, the
+                    // odd one those of the odd row
+                    const bool odd = lane & 1;
+                    uint32_t* out = reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.dbias) + at - (odd ? 1 : 0));
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const uint32_t other = __shfl_xor_sync(0xffffffffu, pkd[k], 1);
+                        const uint32_t w = odd ? __byte_perm(other, pkd[k], 0x7632) : __byte_perm(pkd[k], other, 0x5410);
+                        const int q = q0 + 2 * k + (odd ? 1 : 0);
+                        if (kv < p.N && q < p.N) out[static_cast<size_t>(2 * k + (odd ? 1 : 0)) * (p.N >> 1)] = w;
+                    }
+                }
+            }
+        };
+
+        for (int sg = 0; sg < n_segs && ok; ++sg) {
+            int bs = 0, h = 0, j = 0;
+            if constexpr (DBIAS_HERE != DBIAS_NO) decode(sg, bs, h, j);
+            for (int i = 0; i < NT && ok; ++i, ++gs) {
+                const int bb = gs % NB;
+                if constexpr (C::TWO_PHASE) {
+                    // ---- phase P: x = S' c1 + bias log2e (S' already carries mask and -LSE through the extra
+                    // contraction block), P = exp2(x), P^T (bf16) into tensor memory
+                    // (S' of this step waited for dV of the previous one: its columns are free)
+                    ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
+                    if (!ok) break;
+                    tc_fence_after();
+                    float2 p2[16];
+                    uint32_t dep = 0;
+#pragma unroll
+                    for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
+                        uint32_t sv[16], bq[16];
+                        tmem_ld16(tS + 16 * ch, sv);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
+                        tmem_wait_ld();
+                        uint32_t pk[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
+                            const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
+                            const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
+                            p2[8 * ch + k] = e2;
+                            pk[k] = pack_bf16(e2.x, e2.y);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) dep ^= pk[k];      // depends on every bias value read
+                        tmem_st8(lane_base + C::p_col(2 * g + ch), pk);
+                    }
+                    mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(p_ready);
+
+                    // ---- phase dS: dS = P dP' (dP' already carries -delta), dS^T into tensor memory and the tile.
+                    // Both are free once dK and dQ of the previous step are complete.
+                    if (gs == 0)
+                        ok = warp_all(mbar_wait(dp_full, 0, wc, 0x66));
+                    else                           // (dP' of this step waited for dK)
+                        ok = warp_all(mbar_wait_both(dp_full, gs & 1, dq_done, (gs - 1) & 1, wc, 0x66));
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int ch = 0; ch < 2; ++ch) {
+                        uint32_t dv[16];
+                        tmem_ld16(tDP + 16 * ch, dv);
+                        tmem_wait_ld();
+                        uint32_t pkd[8];
+                        float2 dsv[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            dsv[k] = fmul2(p2[8 * ch + k], u2f2(dv[2 * k], dv[2 * k + 1]));
+                            pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
+                        }
+                        tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+                            sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
+                                   make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
+                        store_dbias(ch, i, j, bs, h, pkd, dsv);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(ds_ready);
+                } else {
+                    // One phase: per element x = S' c1 + bias log2e (S' already carries mask and -LSE through the
+                    // extra contraction block), P = exp2(x), dS = P dP' (dP' already carries -delta).
+                    ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
+                    if (!ok) break;
+                    tc_fence_after();
+                    uint32_t dep = 0;
+#pragma unroll
+                    for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
+                        uint32_t sv[16], dv[16], bq[16];
+                        tmem_ld16(tS + 16 * ch, sv);
+                        tmem_ld16(tDP + 16 * ch, dv);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
+                        tmem_wait_ld();
+                        if (ch == 1) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(s_free);
+                        }
+                        uint32_t pkp[8], pkd[8];
+                        float2 dsv[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
+                            const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
+                            const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
+                            dsv[k] = fmul2(e2, u2f2(dv[2 * k], dv[2 * k + 1]));
+                            pkp[k] = pack_bf16(e2.x, e2.y);
+                            pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) dep ^= pkp[k];     // depends on every bias value read
+                        if (ch == 1) {
+                            mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
+                        } else if (gs > 0) {
+                            // P^T, dS^T and the dS tile are free once the previous step's MMAs are done
+                            ok = warp_all(mbar_wait(dq_done, (gs - 1) & 1, wc, 0x61));
+                            if (!ok) break;
+                            tc_fence_after();
+                        }
+                        tmem_st8(lane_base + C::p_col(2 * g + ch), pkp);
+                        tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
+#pragma unroll
+                        for (int c = 0; c < 2; ++c)
+                            sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
+                                   make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
+                        store_dbias(ch, i, j, bs, h, pkd, dsv);
+                    }
+                    if (!ok) break;
+                    tmem_wait_st();
+                    tc_fence_before();
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(ds_ready);
+                }
             }
         }
     }
 
-    if (tid == 0) EVO_TE(t_kernel, p.status, 0x7f);
     tc_fence_before();
     __syncthreads();
-    EVO_TRACE_FLUSH(p.status);
-    if (warp == BWD_WARP_MMA) tmem_dealloc(tmem, BWD_TMEM_COLS);
+    if (warp == C::W_MMA) tmem_dealloc(tmem, BWD_TMEM_COLS);
 }
 
 // ---------------------------------------------------------------------------
@@ -811,7 +925,8 @@ static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false, bool dbi
     w.off_xk = up(w.off_xq + BS * d->H * NTP * 16);
     w.off_dq = up(w.off_xk + BS * NTP * 16);
     const size_t dh = d->D <= 32 ? 32 : (d->D <= 64 ? 64 : 128);
-    w.off_do = up(w.off_dq + BS * d->N * d->H * dh * 4);                         // fp32 dQ accumulator, kernel width
+    // fp32 dQ, kernel width: the accumulator, or the scratch of at most B * S * H CTAs
+    w.off_do = up(w.off_dq + BS * d->H * ((d->N + 31) / 32 * 32) * dh * 4);
     w.off_db = gated ? up(w.off_do + BS * d->N * d->H * d->D * 2) : w.off_do;    // bf16 d_out * sigmoid(gate)
     // fp32 dBias of a caller that wants bf16 (one S row needs none: dBias is not a sum)
     w.total = (dbias_bf16 && d->S > 1) ? up(w.off_db + static_cast<size_t>(d->B) * d->H * d->N * d->N * 4) : w.off_db;
@@ -825,7 +940,6 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
                       const void* mask, const void* o, const void* o_resid, const float* lse, const void* d_o_in,
                       void* dq, void* dk, void* dv, void* dbias_out, bool dbias_bf16, uint8_t* ws, float scale, unsigned phases,
                       int reserved_sms, cudaStream_t st, const void* gate, void* d_gate) {
-    using C = BwdCfg<DH>;
     const int BS = d->B * d->S;
     const int NT = (d->N + TILE - 1) / TILE;
     const BwdWorkspace w = bwd_workspace(d, gate != nullptr, dbias_bf16);
@@ -836,7 +950,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     uint4* xk = reinterpret_cast<uint4*>(ws + w.off_xk);
     float* dq_acc = reinterpret_cast<float*>(ws + w.off_dq);
 
-    CUtensorMap tq, tk, tv, tdo, tb, tdq;
+    CUtensorMap tq, tk, tv, tdo, tb, tdq, tdk, tdv;
     int rc;
     const int Dt = d->D;          // 16 on the D = 32 kernel: boxes of 32 columns over tensors of 16
     if ((rc = make_tmap_qkv(&tq, q, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
@@ -844,14 +958,11 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tdo, d_o, BS, d->N, d->H, Dt, TILE, lay_do, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
-    if ((rc = make_tmap_rows_box(&tdq, dq_acc, 4, BS, d->N, d->H, DH, 32, 32))) return rc;
 
-    BwdParams p;
+    BwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
     p.NT = NT;
     p.NTP = NT * TILE;
-    p.CPB = (d->S + C::RC - 1) / C::RC;
-    p.total_items = d->B * p.CPB * d->H * NT;
     p.scale = (scale > 0.f) ? scale : 1.0f / sqrtf(static_cast<float>(Dt));
     p.Dt = Dt;
     p.KB = (Dt + 15) / 16;
@@ -859,6 +970,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.xq = reinterpret_cast<const __nv_bfloat16*>(xq);
     p.xk = reinterpret_cast<const __nv_bfloat16*>(xk);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
+    p.dq = static_cast<__nv_bfloat16*>(dq);
     p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
     p.lay = lay_grad;          // the kernel's own stores are dK and dV
     p.status = status_word();
@@ -866,6 +978,26 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
 
     int sms = 0;
     if ((rc = sm_count(&sms))) return rc;
+    // SMs left to other work (a collective on another stream) while the dQ/dK/dV kernel runs
+    int use_sms = sms - (reserved_sms > 0 ? reserved_sms : 0);
+    if (use_sms < 1) use_sms = 1;
+    // Whole items (all kv tiles of a row and head) where that costs no more time than single segments: the
+    // rounds of the fullest SM, against those of segments plus the two passes over the fp32 accumulator
+    // (about 1 / (2 NT) of the kernel).
+    const long pairs = static_cast<long>(BS) * d->H;
+    const long t_whole = (pairs + use_sms - 1) / use_sms * NT, t_seg = (pairs * NT + use_sms - 1) / use_sms;
+    const bool whole = NT == 1 || t_whole * 2 * NT <= t_seg * (2 * NT + 1);
+    p.total_items = static_cast<int>(whole ? pairs : pairs * NT);
+    p.dq_scratch = dq_acc;
+    if constexpr (DH <= 64) {
+        // what the drain warps write: boxes of 32 rows x 32 columns (dQ: bf16, or the fp32 accumulator)
+        if (whole) rc = make_tmap_qkv(&tdq, dq, BS, d->N, d->H, Dt, 32, lay_grad, 32);
+        else rc = make_tmap_rows_box(&tdq, dq_acc, 4, BS, d->N, d->H, DH, 32, 32);
+        if (rc || (rc = make_tmap_qkv(&tdk, dk, BS, d->N, d->H, Dt, 32, lay_grad, 32)) ||
+            (rc = make_tmap_qkv(&tdv, dv, BS, d->N, d->H, Dt, 32, lay_grad, 32)))
+            return rc;
+    }
+    p.scratch_stride = static_cast<size_t>((d->N + 31) / 32) * 32 * DH / 4;
 
     const size_t dq_bytes = static_cast<size_t>(BS) * d->N * d->H * DH * 4;
     const size_t db_elems = static_cast<size_t>(d->B) * d->H * d->N * d->N;
@@ -893,7 +1025,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         r.zero[0] = reinterpret_cast<uint4*>(dbias_acc);
         r.n_zero[0] = (!dbias_here && slices > 1) ? db_elems / 4 : 0;
         r.zero[1] = reinterpret_cast<uint4*>(dq_acc);
-        r.n_zero[1] = both ? dq_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
+        r.n_zero[1] = (both && !whole) ? dq_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
         r.inv_scale = 1.0f / p.scale;
         r.BS = BS; r.N = d->N; r.H = d->H; r.NTP = p.NTP; r.Dt = Dt;
         r.lay = lay_out;
@@ -907,24 +1039,38 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
 
-    if (!both && (rc = cuda_err(cudaMemsetAsync(dq_acc, 0, dq_bytes, st)))) return rc;
-    auto kernel = !dbias_here ? evo_bwd_kernel<DH, DBIAS_NO>
-                              : (dbias_bf16 ? evo_bwd_kernel<DH, DBIAS_BF16> : evo_bwd_kernel<DH, DBIAS_F32>);
-    if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES))))
-        return rc;
-    // SMs left to other work (a collective on another stream) while this kernel runs
-    int use_sms = sms - (reserved_sms > 0 ? reserved_sms : 0);
-    if (use_sms < 1) use_sms = 1;
+    if (!both && !whole && (rc = cuda_err(cudaMemsetAsync(dq_acc, 0, dq_bytes, st)))) return rc;
     const int grid = p.total_items < use_sms ? p.total_items : use_sms;
-    prof_begin(1, st);
-    kernel<<<grid, BWD_THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tdo, tb, tdq, p);
-    prof_end(1, st);
-    if ((rc = cuda_err(cudaGetLastError()))) return rc;
+    const int mode = !dbias_here ? DBIAS_NO : (dbias_bf16 ? DBIAS_BF16 : DBIAS_F32);
+    auto run = [&](auto kernel, int threads, uint32_t smem, auto... maps) -> int {
+        const int e = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
+        if (e) return e;
+        prof_begin(1, st);
+        kernel<<<grid, threads, smem, st>>>(maps..., p);
+        prof_end(1, st);
+        return cuda_err(cudaGetLastError());
+    };
+    auto launch = [&](auto whole_c) -> int {
+        constexpr bool W = decltype(whole_c)::value;
+        if constexpr (DH == 128) {
+            using C = BwdWideCfg<DH, W>;
+            auto kernel = mode == DBIAS_NO ? evo_bwd_wide_kernel<DH, W, DBIAS_NO>
+                                           : (mode == DBIAS_BF16 ? evo_bwd_wide_kernel<DH, W, DBIAS_BF16> : evo_bwd_wide_kernel<DH, W, DBIAS_F32>);
+            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
+        } else {
+            using C = BwdCfg<DH, W>;
+            auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<DH, W, DBIAS_NO>
+                                           : (mode == DBIAS_BF16 ? evo_bwd_kernel<DH, W, DBIAS_BF16> : evo_bwd_kernel<DH, W, DBIAS_F32>);
+            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv);
+        }
+    };
+    rc = whole ? launch(std::true_type{}) : launch(std::false_type{});
+    if (rc || (whole && !convert_dbias)) return rc;
 
     FinishParams f;
     f.dq_acc = dq_acc;
     f.dq = static_cast<__nv_bfloat16*>(dq);
-    f.n8 = dq_bytes / 32;
+    f.n8 = whole ? 0 : dq_bytes / 32;
     f.N = d->N; f.H = d->H; f.Dt = Dt;
     f.lay = lay_grad;
     f.dbias_acc = convert_dbias ? dbias_acc : nullptr;

@@ -33,8 +33,9 @@
 
 namespace evo {
 
-// Every third column pair takes its exp2 on the fused-multiply-add pipe (see ex2_poly2).
-constexpr int DBIAS_POLY_EVERY = 3;
+// D = 32, whose arithmetic is little more than the exp2: every fourth column pair takes its exp2 on the
+// fused-multiply-add pipe (see ex2_poly2; 0.187 -> 0.180 ms at B=1, S=512, N=384, H=8).
+template <int DH> constexpr int DBIAS_POLY_EVERY = (DH == 32) ? 4 : 0;
 
 template <int DH, int NG>
 struct DbCfg {
@@ -45,8 +46,8 @@ struct DbCfg {
     // (the per-thread cap ptxas derives from the launch bound, times THREADS); an
     // increase blocks until the pool has room, for ever if it never can.
     static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
-    static constexpr int REGS_COMPUTE = 112;
-    static constexpr int REGS_OTHER = 32;
+    static constexpr int REGS_COMPUTE = (NG == 2) ? 216 : 112;
+    static constexpr int REGS_OTHER = (NG == 2) ? 72 : 32;
     static_assert(REGS_COMPUTE * NCW * 32 + REGS_OTHER * 128 <= REGS_LAUNCH * THREADS, "register pool");
     // D <= 64: a stage holds the four operand tiles of a step.  D = 128 (four tiles are 128 KB):
     // a stage holds ONE operand pair, (Q, K) of a step or (dO, V) of a step, alternately; each of
@@ -328,7 +329,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         const float2 x2 = ffma2(u2f2(sv[cb][2 * k], sv[cb][2 * k + 1]), c1x2, bl2[ch * 8 + k]);
-                        p2[k] = use_poly<DBIAS_POLY_EVERY>(k) ? ex2_poly2<3>(x2) : make_float2(ex2(x2.x), ex2(x2.y));
+                        p2[k] = use_poly<DBIAS_POLY_EVERY<DH>>(k) ? ex2_poly2<3>(x2) : make_float2(ex2(x2.x), ex2(x2.y));
                     }
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
@@ -375,10 +376,11 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (warp == NCW + 1) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-// Four groups of 32 columns: a step's arithmetic alone takes a CTA 1010 clocks with four warps per
-// scheduler and 1545 with two of 64 columns, which cannot hide their own latencies (B=1, S=512, N=384, H=8,
-// D=32: 0.193 -> 0.177 ms; B=1, S=256, N=1024, H=4, D=64: 0.383 -> 0.371).
-constexpr int DBIAS_GROUPS = 4;
+// D <= 64: four groups of 32 columns.  A step's arithmetic alone takes a CTA 1010 clocks with four warps
+// per scheduler and 1545 with two of 64 columns, which cannot hide their own latencies (B=1, S=512, N=384,
+// H=8, D=32: 0.193 -> 0.180 ms; B=1, S=256, N=1024, H=4, D=64: 0.383 -> 0.374).  D = 128 waits for its
+// loads and products either way, and two groups cross fewer barriers (0.157 -> 0.153 ms at B=1, S=128, N=768, H=4).
+template <int DH> constexpr int DBIAS_GROUPS = (DH == 128) ? 2 : 4;
 
 // Slices of S: enough items to fill the SMs evenly, each long enough that the
 // per-item set-up (bias load, pipeline fill, tile write) stays small.
@@ -402,10 +404,10 @@ template <int DH>
 static int launch_dbias_t(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                           const CUtensorMap& tdo, const void* bias, const void* xq, const void* xk, float* dbias,
                           void* dbias16, int slices, float scale, int sms, cudaStream_t st) {
-    constexpr int NG = DBIAS_GROUPS;
+    constexpr int NG = DBIAS_GROUPS<DH>;
     using C = DbCfg<DH, NG>;
     const int NT = (d->N + TILE - 1) / TILE;
-    DbParams p;
+    DbParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
     p.NT = NT; p.NTP = NT * TILE;
     p.KB = (d->D + 15) / 16;

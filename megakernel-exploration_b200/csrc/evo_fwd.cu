@@ -167,25 +167,6 @@ __device__ __forceinline__ uint2 split3_bf16(float v) {
     return make_uint2(pack_bf16(a, b), c);
 }
 
-// Four lanes of a quad hold four 16-byte chunks each of their own row: afterwards lane t of the quad
-// holds chunk t of the quad's rows 0..3, so that a store instruction covers whole 64-byte segments.
-__device__ __forceinline__ void quad_transpose(uint4 (&c)[4]) {
-    const bool b0 = threadIdx.x & 1u, b1 = threadIdx.x & 2u;
-    auto swap_pair = [](uint4& lo, uint4& hi, bool up, int mask) {
-        uint4 snd = up ? lo : hi;
-        snd.x = __shfl_xor_sync(0xffffffffu, snd.x, mask);
-        snd.y = __shfl_xor_sync(0xffffffffu, snd.y, mask);
-        snd.z = __shfl_xor_sync(0xffffffffu, snd.z, mask);
-        snd.w = __shfl_xor_sync(0xffffffffu, snd.w, mask);
-        lo = up ? snd : lo;
-        hi = up ? hi : snd;
-    };
-    swap_pair(c[0], c[1], b0, 1);
-    swap_pair(c[2], c[3], b0, 1);
-    swap_pair(c[0], c[2], b1, 2);
-    swap_pair(c[1], c[3], b1, 2);
-}
-
 // STRIDED: the output-side tensors are views with the strides of p.lay (otherwise contiguous, with
 // addresses formed from N, H and Dt alone).  GATED: the epilogue also writes sigmoid(gate) * O.
 template <int DH, bool STRIDED, bool GATED>
@@ -716,7 +697,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
     if (WIDE && (rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
 
-    FwdParams p;
+    FwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
     p.Dt = Dt;
     p.KB = (Dt + 15) / 16;

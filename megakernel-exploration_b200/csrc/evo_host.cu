@@ -165,11 +165,11 @@ int layout_from_strides(const EvoDims* d, const EvoStrides* s, ActLayout* out) {
     return EVO_OK;
 }
 
-int make_tmap_bias(CUtensorMap* out, const void* base, int B, int H, int N) {
+int make_tmap_bias(CUtensorMap* out, const void* base, int B, int H, int N, int rows) {
     const uint64_t e = 2;
     TmapDim d[4] = {
         {static_cast<uint64_t>(N), 0, 64},
-        {static_cast<uint64_t>(N), N * e, 128},
+        {static_cast<uint64_t>(N), N * e, static_cast<uint32_t>(rows)},
         {static_cast<uint64_t>(H), static_cast<uint64_t>(N) * N * e, 1},
         {static_cast<uint64_t>(B), static_cast<uint64_t>(H) * N * N * e, 1},
     };

@@ -58,8 +58,8 @@ int make_tmap_rows_box(CUtensorMap* out, const void* base, int elem_bytes, int B
                        int box_cols, int rows);
 // fp32 [B][H][N][N] with a box of [rows x box_cols], swizzle by box row bytes.
 int make_tmap_dbias_box(CUtensorMap* out, const void* base, int B, int H, int N, int box_cols, int rows);
-// bf16 [B][H][N][N] viewed as (N, N, H, B); box [128 rows x 64 cols], 128B swizzle.
-int make_tmap_bias(CUtensorMap* out, const void* base, int B, int H, int N);
+// bf16 [B][H][N][N] viewed as (N, N, H, B); box [rows x 64 cols], 128B swizzle.
+int make_tmap_bias(CUtensorMap* out, const void* base, int B, int H, int N, int rows = 128);
 
 int check_dims(const EvoDims* d);
 // Makes the device's primary context current on this thread (see evo_host.cu).

@@ -64,6 +64,9 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void fence_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// The same for any state space, in both directions (reading with ordinary loads what a completed bulk
+// copy wrote to global memory).
+__device__ __forceinline__ void fence_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -213,6 +216,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     return mbar_wait_limited(bar, parity, w, site, EVO_WAIT_LIMIT, EVO_WAIT_NS);
 }
 
+// Two barriers at once: both probes are in flight together, which costs a ready pair one latency.
+__device__ __forceinline__ bool mbar_wait_both(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, const WaitCtx& w, uint32_t site) {
+    const bool ra = mbar_try_wait(a, pa), rb = mbar_try_wait(b, pb);
+    return (ra || mbar_wait(a, pa, w, site)) && (rb || mbar_wait(b, pb, w, site));
+}
+
 // Makes a per-thread flag uniform across the warp (true only if true everywhere),
 // so that .sync.aligned instructions after a bounded wait stay convergent.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
@@ -267,6 +276,11 @@ __device__ __forceinline__ float lds32f(uint32_t saddr) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(saddr));
     return v;
 }
+__device__ __forceinline__ uint32_t lds_u16(uint32_t saddr) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr));
+    return v;
+}
 __device__ __forceinline__ void sts128(uint32_t saddr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -312,6 +326,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
+}
+// Untiled bulk copy and fp32 reduce-add shared -> global, same rules; completion by bulk group.
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                 ::"l"(reinterpret_cast<uint64_t>(dst)), "r"(smem_u32(src)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_add_f32(void* dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+                 ::"l"(reinterpret_cast<uint64_t>(dst)), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* src,
                                              int c0, int c1, int c2, int c3) {
@@ -409,6 +432,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
         ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
           "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
+}
+
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
 }
 
 // Store 32 consecutive 32-bit columns of this thread's lane (counterpart of tmem_ld32).
@@ -580,6 +609,25 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 __device__ __forceinline__ float2 bf16x2_f2(uint32_t w) { return make_float2(bf16_lo(w), bf16_hi(w)); }
 __device__ __forceinline__ float2 u2f2(uint32_t lo, uint32_t hi) {
     return make_float2(__uint_as_float(lo), __uint_as_float(hi));
+}
+
+// Four lanes of a quad hold four 16-byte chunks each of their own row: afterwards lane t of the quad
+// holds chunk t of the quad's rows 0..3, so that a store instruction covers whole 64-byte segments.
+__device__ __forceinline__ void quad_transpose(uint4 (&c)[4]) {
+    const bool b0 = threadIdx.x & 1u, b1 = threadIdx.x & 2u;
+    auto swap_pair = [](uint4& lo, uint4& hi, bool up, int mask) {
+        uint4 snd = up ? lo : hi;
+        snd.x = __shfl_xor_sync(0xffffffffu, snd.x, mask);
+        snd.y = __shfl_xor_sync(0xffffffffu, snd.y, mask);
+        snd.z = __shfl_xor_sync(0xffffffffu, snd.z, mask);
+        snd.w = __shfl_xor_sync(0xffffffffu, snd.w, mask);
+        lo = up ? snd : lo;
+        hi = up ? hi : snd;
+    };
+    swap_pair(c[0], c[1], b0, 1);
+    swap_pair(c[2], c[3], b0, 1);
+    swap_pair(c[0], c[2], b1, 2);
+    swap_pair(c[1], c[3], b1, 2);
 }
 
 // Named barrier over `nthreads` threads (ids 1..15; 0 is __syncthreads).

@@ -1,4 +1,4 @@
-"""Edges of the forward's item streams (D <= 64): rows taken in groups that share bias tiles, with groups
+"""Edges of how the kernels cut a problem into items.  Forward streams (D <= 64): rows taken in groups that share bias tiles, with groups
 cut short at the end of a batch; separate items per stream, with streams that run out; ragged last tiles.
 Tolerance: the operator's parity bar (tests/_util.py)."""
 import pytest
@@ -19,6 +19,31 @@ pytestmark = pytest.mark.gpu
 ])
 def test_forward_streams(B, S, N, H, D):
     q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=B + S + N)
+    got = run_layer(q, k, v, mask, bias, d_o)
+    ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
+    assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
+
+
+# dQ/dK/dV kernel: whole items (every kv tile of a row and head in one CTA) where (rows x heads) fill the 148
+# SMs, single segments where they do not; one and two tiles keep dQ in tensor memory, more go through scratch
+@pytest.mark.parametrize("B,S,N,H,D", [
+    (1, 49, 264, 3, 32),     # whole, three ragged tiles
+    (1, 37, 328, 4, 64),
+    (1, 37, 264, 4, 128),
+    (1, 74, 200, 2, 96),     # two tiles
+    (1, 150, 136, 2, 32),    # ... and several items per CTA
+    (1, 74, 200, 2, 64),
+    (1, 160, 72, 2, 16),     # one tile
+    # one tile at D = 128.  The additive terms of a logit are carried to 16 bits (up to 1e-4 of a row's dS, which
+    # reaches |dO||V| P ~ 40 here); summed over S rows the worst case passes the flat 2e-2 on dBias near S = 300
+    # (0.02001, whichever exp2 the dBias kernel uses), so S stays at half of that
+    (1, 150, 104, 2, 128),
+    (1, 5, 520, 3, 32),      # segments
+    (1, 5, 520, 3, 64),
+    (1, 3, 392, 5, 96),
+])
+def test_backward_items(B, S, N, H, D):
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=7 * S + N)
     got = run_layer(q, k, v, mask, bias, d_o)
     ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
     assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
