@@ -16,6 +16,14 @@
 
 namespace evo {
 
+// A number of items in mixed radix: heads, q tiles, rows (or groups of rows) of a batch, batches.
+struct FwdStep {
+    int h, qt, g, b;
+    __host__ __device__ static FwdStep of(int w, int H, int QT, int NG) {
+        return FwdStep{w % H, w / H % QT, w / H / QT % NG, w / H / QT / NG};
+    }
+};
+
 struct FwdParams {
     int B, S, N, H;
     int Dt;            // true head dim (16 runs on the D = 32 kernel: loads zero-filled, stores clipped)
@@ -24,6 +32,7 @@ struct FwdParams {
     int shared_bias;   // D <= 64: the streams of a CTA work on rows of the same q tile and share its bias tiles
     int NG;            // D <= 64: rows per batch, or groups of G rows if the bias tiles are shared
     int total_items;   // B*S*QT*H, or B*SG*QT*H
+    FwdStep step;      // D <= 64: from an item of a stream to its next
     float c1;          // scale * log2(e)
     float scale, inv_scale;
     const __nv_bfloat16* mask;   // [B*S][N]
@@ -67,10 +76,16 @@ namespace evo {
 // fill the SMs G at a time) every stream has its own items and its own ring slot.
 //
 // Measured against the kernel with two groups of 64 columns on one item (which runs D = 128): B=1, S=512,
-// N=384, H=8, D=32 0.371 -> 0.323 ms; S=256, N=768 0.650 -> 0.560; S=256, N=1024, H=4, D=64 0.690 -> 0.580.
+// N=384, H=8, D=32 0.371 -> 0.323 ms; S=256, N=768 0.650 -> 0.560; S=256, N=1024, H=4, D=64 0.700 -> 0.640.
 // A step takes about 2400 clocks of a CTA: 1024 for its exponentials, 1000 issue slots.  Also tried: the
 // epilogue on a warpgroup of its own (its registers cost the softmax warps more than it saves, 0.42 ms),
 // two streams in the exp2 pass at a time (0.365), none taking turns (0.39), two streams at D = 32 (0.375).
+//
+// Between two items a stream's warps wait for the last PV and hand the results over: 3300 clocks, of a
+// three-tile item's 18500, when every warp stored its rows itself (32 shuffles to make 64-byte segments).
+// Staged in buffers that the item no longer needs, sent by the MMA warp's TMA stores, and with what does
+// not depend on the last PV ahead of the wait for it: 2200 (the two shapes at D = 32 0.319 -> 0.295 and
+// 0.585 -> 0.540 ms).
 //
 // The mask rides in an extra contraction block (evo_tiles.cuh, "EXTRA TILE"): the producer turns 128
 // mask values into a [128][8] tile (m/scale in three bf16 parts, exact to fp32), columns past N get
@@ -89,8 +104,8 @@ struct FwdCfg {
     // setmaxnreg budgets: the CTA's register pool is the launch count (the cap ptxas derives from the
     // launch bound) times the threads; an increase that the pool cannot satisfy blocks for ever
     static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
-    static constexpr int REGS_SOFTMAX = (G == 3) ? 144 : 208;
-    static constexpr int REGS_OTHER = (G == 3) ? 80 : 88;
+    static constexpr int REGS_SOFTMAX = (G == 3) ? 152 : 216;
+    static constexpr int REGS_OTHER = (G == 3) ? 56 : 72;
     static_assert((REGS_SOFTMAX * NSW + REGS_OTHER * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
     static constexpr uint32_t ROWT = RowTile<DH>::BYTES;       // one [128][DH] bf16 tile
     static constexpr int NQ = (DH == 32) ? 2 : 1;              // Q buffers per stream
@@ -104,7 +119,7 @@ struct FwdCfg {
     static constexpr uint32_t OFF_XQ = OFF_STREAM + G * STREAM_BYTES;       // rows (1, 1, 1, 0, ...)
     static constexpr uint32_t OFF_ZERO = OFF_XQ + XT_BYTES;
     static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr int BARS = 21;                            // barriers of a stream (FwdBars)
+    static constexpr int BARS = 22;                            // barriers of a stream (FwdBars)
     static constexpr uint32_t OFF_MISC = OFF_BARS + (G * BARS + 2 * NR) * 8;
     static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;   // + alignment slack
     static constexpr uint32_t TMEM_S = 0;                      // + 128 s
@@ -124,35 +139,28 @@ struct FwdBars {
     uint64_t *v_full;
     uint64_t *s_full, *s_free;       // S' complete / read (HOLD)
     uint64_t *p_ready, *pv_done;     // P written / PV complete
+    uint64_t *o_staged;              // an item's results are in shared memory
     uint64_t *turn;                 // [2][4] by tile parity: warp w of the stream has left its exp2 pass
     __device__ __forceinline__ FwdBars(uint64_t* b)
         : q_full(b), q_empty(b + 2), k_full(b + 4), k_empty(b + 6), v_full(b + 8), s_full(b + 9), s_free(b + 10),
-          p_ready(b + 11), pv_done(b + 12), turn(b + 13) {}
+          p_ready(b + 11), pv_done(b + 12), o_staged(b + 13), turn(b + 14) {}
 };
 
 // A stream's walk over its items: coordinates in mixed radix (head, q tile, row or group of rows, batch),
-// advanced without a division (a division costs a warp about a hundred clocks, on the stream's chain).
-struct FwdStep {
-    int h, qt, g, b;
-    __device__ __forceinline__ FwdStep(int w, const FwdParams& p) {
-        h = w % p.H; w /= p.H;
-        qt = w % p.QT; w /= p.QT;
-        g = w % p.NG; b = w / p.NG;
-    }
-};
+// advanced by p.step without a division (a division costs a warp about a hundred clocks, on the stream's chain).
 struct FwdItem {
     int h, qt, row, b;       // row of S: with groups, G apart
-    __device__ __forceinline__ void next(const FwdStep& d, int rows, int rstep, const FwdParams& p) {
-        h += d.h;
+    __device__ __forceinline__ void next(int rows, int rstep, const FwdParams& p) {
+        h += p.step.h;
         int c = h >= p.H;
         h -= c ? p.H : 0;
-        qt += d.qt + c;
+        qt += p.step.qt + c;
         c = qt >= p.QT;
         qt -= c ? p.QT : 0;
-        row += (d.g + c) * rstep;
+        row += (p.step.g + c) * rstep;
         c = row >= rows;
         row -= c ? rows : 0;
-        b += d.b + c;
+        b += p.step.b + c;
     }
     __device__ __forceinline__ bool valid(const FwdParams& p) const { return b < p.B && row < p.S; }
     __device__ __forceinline__ int bs(const FwdParams& p) const { return b * p.S + row; }
@@ -167,12 +175,12 @@ __device__ __forceinline__ uint2 split3_bf16(float v) {
     return make_uint2(pack_bf16(a, b), c);
 }
 
-// STRIDED: the output-side tensors are views with the strides of p.lay (otherwise contiguous, with
-// addresses formed from N, H and Dt alone).  GATED: the epilogue also writes sigmoid(gate) * O.
-template <int DH, bool STRIDED, bool GATED>
+// GATED: the epilogue also writes sigmoid(gate) * O.  tm_2: the rounding residual (GATED: the gated output).
+template <int DH, bool GATED>
 __global__ void __launch_bounds__(FwdCfg<DH>::THREADS, 1)
 evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias, const FwdParams p) {
+               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias,
+               const __grid_constant__ CUtensorMap tm_o, const __grid_constant__ CUtensorMap tm_2, const FwdParams p) {
     using C = FwdCfg<DH>;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
@@ -203,6 +211,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             mbar_init(b.v_full, 1);
             mbar_init(b.s_full, 1); mbar_init(b.s_free, 4);
             mbar_init(b.p_ready, 4); mbar_init(b.pv_done, 1);
+            mbar_init(b.o_staged, 4);
             for (int i = 0; i < 8; ++i) mbar_init(&b.turn[i], 1);
         }
         for (int i = 0; i < NR; ++i) { mbar_init(&bias_full[i], 1); mbar_init(&bias_empty[i], shared_bias ? NSW : 4); }
@@ -211,7 +220,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == C::W_PROD) {
         tmem_alloc(tmem_slot, C::TMEM_COLS);
         tmem_relinquish();
-        if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_bias); }
+        if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_bias); prefetch_tmap(&tm_o); prefetch_tmap(&tm_2); }
     }
     if (tid < 128) {
         *reinterpret_cast<uint4*>(smem + C::OFF_XQ + tid * 16) = make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u);
@@ -232,14 +241,13 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // rows count in steps of G within a batch if they are taken in groups: row r of the group sits at g * G + r
     const int rstep = shared_bias ? G : 1;
     auto items_of = [&](int s) -> FwdItem {
-        const FwdStep w(first + (shared_bias ? 0 : s * stride), p);
+        const FwdStep w = FwdStep::of(first + (shared_bias ? 0 : s * stride), p.H, p.QT, p.NG);
         return FwdItem{w.h, w.qt, w.g * rstep + (shared_bias ? s : 0), w.b};
     };
-    const FwdStep step(per_cta, p);
     auto advance = [&](FwdItem& x, int s) {
         const int shift = shared_bias ? s : 0;
         x.row -= shift;
-        x.next(step, p.NG * rstep, rstep, p);
+        x.next(p.NG * rstep, rstep, p);
         x.row += shift;
     };
     // ring slot and phase parity of the bias tile of tile r of stream s
@@ -308,7 +316,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             if (r >= (shared_bias ? NR : 1)) ok = warp_all(mbar_wait(&bias_empty[slot], ph ^ 1u, wc, 0x14));
                             if (ok && elect_one()) {
                                 uint8_t* bt = smem + C::OFF_BIAS + slot * SQ_BYTES;
-                                                                mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
+                                mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
                                 tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, item[s].b);
                                 tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, item[s].b);
                             }
@@ -357,8 +365,9 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             umma_ss(t_s, RD::kmajor(q_lo, kk), RD::kmajor(k_lo, kk), IDESC_S, kk > 0);
                     umma_ss(t_s, d_xq, xt_desc(aS + C::ST_XK + kb * XT_BYTES, aZero), IDESC_S, 1u);
                     umma_commit(b.s_full);
-                    umma_commit(&b.k_empty[kb]);
-                    if (j == NT - 1) umma_commit(&b.q_empty[qn % NQ]);
+                    // (of an item's last tile, one of the two is held back: see store_item)
+                    if (!C::HOLD || j < NT - 1) umma_commit(&b.k_empty[kb]);
+                    if (C::HOLD && j == NT - 1) umma_commit(&b.q_empty[qn % NQ]);
                 }
                 __syncwarp();
                 if (j == NT - 1) ++qn;
@@ -383,6 +392,22 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 __syncwarp();
             };
+            // The results of item x (the stream's e-th, its last tile n) go out from V's buffer and from one that
+            // the item's last S' has left: Q's, of two (D = 32), or K's, of two.
+            const bool two = GATED || p.o_resid != nullptr;
+            auto store_item = [&](const FwdItem& x, int e, int n) {
+                ok = warp_all(mbar_wait(b.o_staged, e & 1, wc, 0x27));
+                if (!ok) return;
+                if (elect_one()) {
+                    uint8_t* second = sb + (C::HOLD ? C::ST_K + (n % NK) * C::ROWT : C::ST_Q + (e % NQ) * C::ROWT);
+                    tma_store_4d(&tm_o, sb + C::ST_V, 0, x.h, x.qt * TILE, x.bs(p));
+                    if (two) tma_store_4d(&tm_2, second, 0, x.h, x.qt * TILE, x.bs(p));
+                    tma_commit_group();
+                    tma_wait_group_read<0>();
+                    mbar_arrive(C::HOLD ? &b.k_empty[n % NK] : &b.q_empty[e % NQ]);
+                }
+                __syncwarp();
+            };
             // with rows in groups, the last group of a batch may lack this stream's row: skipped
             int it = 0;
             auto skip_missing = [&]() -> bool {
@@ -391,13 +416,15 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 return any;
             };
             (void)skip_missing();
-            int j = 0, loaded = 0;
+            int j = 0, loaded = 0, e = 0;
             if (it < n_items) { load_v(0); loaded = 1; wait_s(0, 0); if (ok) issue_s(0, 0); }
             bool more = it < n_items;
             for (int n = 0; more && ok; ++n) {
+                const bool last = j == NT - 1;
+                const FwdItem mine = cur;
                 int j1 = j + 1;                // the tile after this one
                 bool gap = false;              // items are missing before it
-                if (j1 == NT) { j1 = 0; ++it; advance(cur, s); gap = skip_missing(); }
+                if (last) { j1 = 0; ++it; advance(cur, s); gap = skip_missing(); }
                 more = it < n_items;
                 // S' of the next tile: its columns are free once the softmax has read them (HOLD), or once
                 // PV of this tile, which reads P from them, is complete.  Behind a gap Q and K do not come
@@ -418,11 +445,17 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!early) s_free();
                     if (!ok) break;
                     if (!early) issue_s(n + 1, j1);
+                }
+                if (last) store_item(mine, e++, n);
+                if (!ok) break;
+                if (more) {
                     load_v(j1);
                     ++loaded;
                 }
                 j = j1;
             }
+            if (elect_one()) tma_wait_group<0>();
+            __syncwarp();
             if (loaded > 0) (void)mbar_wait(b.v_full, (loaded - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x26);
         }
     } else {
@@ -442,7 +475,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         uint64_t* turn_mine = &b.turn[warp & 3];
         uint64_t* turn_prev = &FwdBars(bars + (s > 0 ? s - 1 : G - 1) * C::BARS).turn[warp & 3];
         bool ok = true;
-        int n = 0, r = 0;                     // tiles of the stream so far, tiles counting missing items
+        int n = 0, r = 0, e = 0;              // tiles of the stream so far, tiles counting missing items, items
         auto take_turn = [&]() {
             // a stream may leave its pass of tile t + 1 before the one that waits for it looks at tile t: two
             // barriers by tile parity keep the waiter within one phase
@@ -451,7 +484,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         };
 
         FwdItem cur = items_of(s);
-        for (int it = 0; it < n_items && ok; ++it, advance(cur, s)) {
+        for (int it = 0; it < n_items && ok; ++it) {
             if (!cur.valid(p)) {
                 // no such item: hand the bias tiles (if shared) and the turns on
                 for (int j = 0; j < NT && ok; ++j, ++r) {
@@ -467,6 +500,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     __syncwarp();
                     if (lane == 0) mbar_arrive(turn_mine + 4 * (r & 1));
                 }
+                advance(cur, s);
                 continue;
             }
             float m = -INFINITY, l = 0.f;
@@ -474,8 +508,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 int slot; uint32_t ph;
                 bias_slot(s, r, slot, ph);
                 const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + slot * SQ_BYTES;
-                ok = warp_all(mbar_wait(&bias_full[slot], ph, wc, 0x32));      // usually there already
-                if (ok) ok = warp_all(mbar_wait(b.s_full, n & 1, wc, 0x31));
+                ok = warp_all(mbar_wait_both(&bias_full[slot], ph, b.s_full, n & 1, wc, 0x31));
                 if (!ok) break;
                 tc_fence_after();
                 // pass 1: x = S' * scale + bias and the row maximum, 32 columns at a time
@@ -594,32 +627,27 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (lane == 0) mbar_arrive(b.p_ready);
             }
             if (!ok) break;
-            // epilogue of the item: every PV of it is complete
+            // epilogue of the item; what does not need the last PV comes before the wait for it
+            const int bs = cur.bs(p), qt = cur.qt, h = cur.h;
+            const int qrow = qt * TILE + row;
+            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ((m == -INFINITY) ? 0.f : m) + __logf(l);
+            const float inv = __frcp_rn(l);
+            advance(cur, s);
+            // Results go through shared memory (row r of a tile: 16-byte chunks, swizzled as the tensor map says)
+            // and out by TMA, issued by the MMA warp.
+            uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
+            const uint32_t aO = smem_u32(sb + C::ST_V);
+            const uint32_t a2 = smem_u32(sb + (C::HOLD ? C::ST_K + ((n - 1) % NK) * C::ROWT : C::ST_Q + (e % NQ) * C::ROWT));
+            ++e;
             ok = warp_all(mbar_wait(b.pv_done, (n - 1) & 1, wc, 0x34));
             if (!ok) break;
             tc_fence_after();
-            const int bs = cur.bs(p), qt = cur.qt, h = cur.h;
-            const int qrow = qt * TILE + row;
-            const float inv = __frcp_rn(l);
-            // lane t of a quad of rows stores chunk t of each of the four: 64 contiguous bytes per row (from
-            // one thread per row, 16 bytes at a time, the stores cost 1600 clocks per item)
-            const int qrow0 = qt * TILE + (row & ~3);
-            size_t off0, rstep;
-            if constexpr (STRIDED) {
-                off0 = bs * p.lay.row + qrow0 * p.lay.n + h * p.lay.h;
-                rstep = p.lay.n;
-            } else {
-                off0 = ((static_cast<size_t>(bs) * p.N + qrow0) * p.H + h) * p.Dt;
-                rstep = static_cast<size_t>(p.H) * p.Dt;
-            }
 #pragma unroll
             for (int c = 0; c < DH / 32; ++c) {
                 float o[32];
                 __syncwarp();
                 tmem_ld_f32<32>(tPV + c * 32, o);
-                if (c * 32 >= p.Dt) continue;          // warp-uniform
-                const int col = c * 32 + (lane & 3) * 8;
-                uint4 vo[4], vr[4];
+                uint4 vr[4];
 #pragma unroll
                 for (int c8 = 0; c8 < 4; ++c8) {
                     uint32_t vw[4], rw[4];
@@ -629,27 +657,31 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         vw[e] = pack_bf16(o0, o1);
                         rw[e] = pack_bf16(o0 - bf16_lo(vw[e]), o1 - bf16_hi(vw[e]));
                     }
-                    vo[c8] = make_uint4(vw[0], vw[1], vw[2], vw[3]);
+                    const uint32_t off = swz_off<RT::ROW_BYTES>(row, c * 4 + c8);
+                    sts128(aO + off, make_uint4(vw[0], vw[1], vw[2], vw[3]));
                     vr[c8] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+                    // rounding residual of O
+                    if (!GATED && p.o_resid != nullptr) sts128(a2 + off, vr[c8]);
                 }
-                quad_transpose(vo);
-                if (p.o_resid != nullptr) quad_transpose(vr);
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (qrow0 + e < p.N && col < p.Dt) {
-                        *reinterpret_cast<uint4*>(p.o + off0 + e * rstep + col) = vo[e];
-                        // rounding residual of O
-                        if (p.o_resid != nullptr) *reinterpret_cast<uint4*>(p.o_resid + off0 + e * rstep + col) = vr[e];
-                    }
                 if constexpr (GATED) {
-                    // O * sigmoid(gate), from the unrounded O: the gate's chunks come in transposed
+                    // O * sigmoid(gate), from the unrounded O.  Lane t of a quad of rows loads chunk t of each of
+                    // the four (64 contiguous bytes per row), and stores the residual like that.
+                    const int col = c * 32 + (lane & 3) * 8, qrow0 = qt * TILE + (row & ~3);
+                    const size_t off0 = bs * p.lay.row + qrow0 * p.lay.n + h * p.lay.h + col;
                     uint4 vg[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         vg[e] = make_uint4(0u, 0u, 0u, 0u);
-                        if (qrow0 + e < p.N && col < p.Dt) vg[e] = __ldg(reinterpret_cast<const uint4*>(p.gate + off0 + e * rstep + col));
+                        if (qrow0 + e < p.N && col < p.Dt) vg[e] = __ldg(reinterpret_cast<const uint4*>(p.gate + off0 + e * p.lay.n));
                     }
                     __syncwarp();
+                    if (p.o_resid != nullptr) {
+                        quad_transpose(vr);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (qrow0 + e < p.N && col < p.Dt) *reinterpret_cast<uint4*>(p.o_resid + off0 + e * p.lay.n) = vr[e];
+                        __syncwarp();
+                    }
                     quad_transpose(vg);
 #pragma unroll
                     for (int c8 = 0; c8 < 4; ++c8) {
@@ -661,16 +693,13 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
                             ow[e] = pack_bf16(o[c8 * 8 + 2 * e] * s0, o[c8 * 8 + 2 * e + 1] * s1);
                         }
-                        vg[c8] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                        sts128(a2 + swz_off<RT::ROW_BYTES>(row, c * 4 + c8), make_uint4(ow[0], ow[1], ow[2], ow[3]));
                     }
-                    quad_transpose(vg);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (qrow0 + e < p.N && col < p.Dt)
-                            *reinterpret_cast<uint4*>(p.o_gated + off0 + e * rstep + col) = vg[e];
                 }
             }
-            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ((m == -INFINITY) ? 0.f : m) + __logf(l);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b.o_staged);
         }
     }
 
@@ -695,7 +724,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
-    if (WIDE && (rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
+    if ((rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
 
     FwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
@@ -745,13 +774,14 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             p.total_items = static_cast<int>(units);
         }
         const int grid = p.total_items < sms ? p.total_items : sms;
-        const ActLayout cl = contiguous_layout(d->N, d->H, Dt);
-        const bool strided = (lay.row != cl.row || lay.n != cl.n || lay.h != cl.h);
-        auto kernel = gate ? (strided ? evo_fwd_kernel<DH, true, true> : evo_fwd_kernel<DH, false, true>)
-                           : (strided ? evo_fwd_kernel<DH, true, false> : evo_fwd_kernel<DH, false, false>);
+        p.step = FwdStep::of(grid * (p.shared_bias ? 1 : C::G), p.H, p.QT, p.NG);
+        CUtensorMap t2 = to;
+        const void* second = gate ? o_gated : o_resid;
+        if (second && (rc = make_tmap_qkv(&t2, second, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
+        auto kernel = gate ? evo_fwd_kernel<DH, true> : evo_fwd_kernel<DH, false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, p);
+        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, to, t2, p);
         prof_end(0, st);
     }
     return cuda_err(cudaGetLastError());
