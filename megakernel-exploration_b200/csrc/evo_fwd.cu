@@ -28,15 +28,13 @@ struct FwdParams {
     int B, S, N, H;
     int Dt;            // true head dim (16 runs on the D = 32 kernel: loads zero-filled, stores clipped)
     int KB;            // contraction blocks of 16 head-dim columns that hold data: ceil(Dt / 16)
-    int QT;            // q tiles (= kv tiles) per row: ceil(N / 128)
+    int QT;            // q tiles (= kv tiles) per row: ceil(N / 128) (D > 64: pairs of them)
     int shared_bias;   // D <= 64: the streams of a CTA work on rows of the same q tile and share its bias tiles
     int NG;            // D <= 64: rows per batch, or groups of G rows if the bias tiles are shared
     int total_items;   // B*S*QT*H, or B*SG*QT*H
-    FwdStep step;      // D <= 64: from an item of a stream to its next
-    float c1;          // scale * log2(e)
+    FwdStep step;      // from an item of a stream to its next
     float scale, inv_scale;
     const __nv_bfloat16* mask;   // [B*S][N]
-    const __nv_bfloat16* bias;   // [B][H][N][N] (read directly when the bias tile is not staged)
     float* lse;                  // [B*S][H][N]
     __nv_bfloat16* o;            // activation layout `lay`
     __nv_bfloat16* o_resid;      // activation layout `lay`, or nullptr
@@ -45,10 +43,6 @@ struct FwdParams {
     ActLayout lay;               // element strides of the activation tensors
     unsigned int* status;
 };
-
-}  // namespace evo
-#include "evo_fwd_wide.cuh"
-namespace evo {
 
 // ---------------------------------------------------------------------------
 // D <= 64: independent item streams.
@@ -708,6 +702,10 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == C::W_PROD) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
+}  // namespace evo
+#include "evo_fwd_wide.cuh"
+namespace evo {
+
 // lay_in: q, k, v; lay: the output side (o, o_resid, gate, o_gated)
 template <int DH>
 static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout& lay, const void* q, const void* k, const void* v,
@@ -717,14 +715,13 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const int BS = d->B * d->S;
     const int QT = (d->N + TILE - 1) / TILE;
 
-    CUtensorMap tq, tk, tv, tb, to;
+    CUtensorMap tq, tk, tv, tb;
     int rc;
     const int Dt = d->D;          // 16 on the D = 32 kernel: boxes of 32 columns over tensors of 16
     if ((rc = make_tmap_qkv(&tq, q, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
-    if ((rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
 
     FwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
@@ -734,9 +731,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.total_items = BS * QT * d->H;
     p.scale = (scale > 0.f) ? scale : 1.0f / sqrtf(static_cast<float>(Dt));
     p.inv_scale = 1.0f / p.scale;
-    p.c1 = p.scale * LOG2E;
     p.mask = static_cast<const __nv_bfloat16*>(mask);
-    p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.lse = lse;
     p.o = static_cast<__nv_bfloat16*>(o);
     p.o_resid = static_cast<__nv_bfloat16*>(o_resid);
@@ -749,15 +744,17 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     int sms = 0;
     if ((rc = sm_count(&sms))) return rc;
     if constexpr (WIDE) {
+        using C = FwdWideCfg;
+        // pairs of q tiles; with one q tile per row, items dealt to the two streams of a CTA in turn
+        p.NG = d->S;
+        p.QT = (QT + 1) / 2;
+        p.total_items = BS * p.QT * d->H;
         const int grid = p.total_items < sms ? p.total_items : sms;
-        using C = FwdWideCfg<DH, 2>;
-        const ActLayout cl = contiguous_layout(d->N, d->H, DH);
-        const bool strided = (lay.row != cl.row || lay.n != cl.n || lay.h != cl.h);
-        auto kernel = gate ? (strided ? evo_fwd_wide_kernel<DH, true, 2, true> : evo_fwd_wide_kernel<DH, false, 2, true>)
-                           : (strided ? evo_fwd_wide_kernel<DH, true, 2, false> : evo_fwd_wide_kernel<DH, false, 2, false>);
+        p.step = FwdStep::of(grid * (QT == 1 ? 2 : 1), p.H, p.QT, p.NG);
+        auto kernel = gate ? evo_fwd_wide_kernel<true> : evo_fwd_wide_kernel<false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, to, p);
+        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, p);
         prof_end(0, st);
     } else {
         using C = FwdCfg<DH>;
@@ -775,7 +772,9 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         }
         const int grid = p.total_items < sms ? p.total_items : sms;
         p.step = FwdStep::of(grid * (p.shared_bias ? 1 : C::G), p.H, p.QT, p.NG);
-        CUtensorMap t2 = to;
+        CUtensorMap to, t2;
+        if ((rc = make_tmap_qkv(&to, o, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
+        t2 = to;
         const void* second = gate ? o_gated : o_resid;
         if (second && (rc = make_tmap_qkv(&t2, second, BS, d->N, d->H, Dt, TILE, lay, RowTile<DH>::BOX_D))) return rc;
         auto kernel = gate ? evo_fwd_kernel<DH, true> : evo_fwd_kernel<DH, false>;

@@ -24,6 +24,20 @@ def test_forward_streams(B, S, N, H, D):
     assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
 
 
+# D = 96 and 128: pairs of q tiles, or (one tile per row) items dealt to two streams
+@pytest.mark.parametrize("B,S,N,H,D", [
+    (1, 37, 392, 5, 128),    # four tiles, several pairs per CTA
+    (2, 25, 264, 3, 96),     # three tiles: every second pair lacks its second
+    (1, 101, 128, 3, 128),   # 303 items for 296 streams: some without a second
+    (2, 1, 8, 3, 96),        # fewer items than SMs
+])
+def test_forward_wide(B, S, N, H, D):
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=3 * S + N)
+    got = run_layer(q, k, v, mask, bias, d_o)
+    ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
+    assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
+
+
 # dQ/dK/dV kernel: whole items (every kv tile of a row and head in one CTA) where (rows x heads) fill the 148
 # SMs, single segments where they do not; one and two tiles keep dQ in tensor memory, more go through scratch
 @pytest.mark.parametrize("B,S,N,H,D", [
