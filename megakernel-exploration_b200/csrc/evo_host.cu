@@ -38,8 +38,9 @@ EncodeTiledFn encode_tiled_fn() {
 namespace {
 // Encoded tensor maps keyed on everything the encoder sees.  A training loop calls with the same few
 // (pointer, shape, strides) combinations step after step; encoding costs microseconds per map on the
-// host, a dozen maps per step.  Direct-mapped by a hash of the key and one table per thread: a lookup
-// is one comparison without a lock (a scan of 256 entries under a mutex cost a step up to 20 us).
+// host, a dozen maps per step.  Sets of four by a hash of the key and one table per thread: a lookup is
+// a few comparisons without a lock (a scan of 256 entries under a mutex cost a step up to 20 us; in sets
+// of one, two of a step's dozen maps shared a set, and were encoded anew every step, for one layout of pointers in six).
 struct TmapKey {
     const void* base;
     int dt, rank, swz;
@@ -61,8 +62,12 @@ struct TmapEntry {
     TmapKey key;             // rank 0: empty
     CUtensorMap map;
 };
-constexpr size_t TMAP_CACHE = 256;
-thread_local std::unique_ptr<TmapEntry[]> t_tmap_cache;
+struct TmapSet {
+    TmapEntry way[4];
+    unsigned next;           // the way to give up next
+};
+constexpr size_t TMAP_SETS = 64;
+thread_local std::unique_ptr<TmapSet[]> t_tmap_cache;
 }  // namespace
 
 static int encode_tmap(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int rank,
@@ -102,18 +107,22 @@ int make_tmap(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int ra
         key.stride[i] = i > 0 ? dims[i].stride_bytes : 0;
         key.box[i] = dims[i].box;
     }
-    if (!t_tmap_cache) t_tmap_cache.reset(new TmapEntry[TMAP_CACHE]());
-    TmapEntry& e = t_tmap_cache[key.hash() % TMAP_CACHE];
+    if (!t_tmap_cache) t_tmap_cache.reset(new TmapSet[TMAP_SETS]());
+    TmapSet& set = t_tmap_cache[key.hash() % TMAP_SETS];
+    for (const TmapEntry& w : set.way)
+        if (w.key == key) {
+            *out = w.map;
+            return EVO_OK;
+        }
     // A tensor map holds a virtual address and a shape, nothing device-specific: an entry encoded
     // while one device was current is valid for the same pointer under any other.
-    if (!(e.key == key)) {
-        const int rc = encode_tmap(&e.map, base, dt, rank, dims, swz);
-        if (rc) {
-            e.key = TmapKey{};
-            return rc;
-        }
-        e.key = key;
+    TmapEntry& e = set.way[set.next++ % 4];
+    const int rc = encode_tmap(&e.map, base, dt, rank, dims, swz);
+    if (rc) {
+        e.key = TmapKey{};
+        return rc;
     }
+    e.key = key;
     *out = e.map;
     return EVO_OK;
 }
@@ -129,23 +138,6 @@ int make_tmap_qkv(CUtensorMap* out, const void* base, int BS, int N, int H, int 
         {static_cast<uint64_t>(BS), static_cast<uint64_t>(lay.row) * e, 1},
     };
     return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, d, row_swizzle(box_d));
-}
-
-int make_tmap_qkv_cols(CUtensorMap* out, const void* base, int BS, int N, int H, int D, int rows, int cols,
-                       const ActLayout& lay) {
-    const uint64_t e = 2;
-    const int rb = cols * 2;
-    if (rb != 16 && rb != 32 && rb != 64 && rb != 128) return EVO_ERR_TENSOR_MAP;
-    TmapDim d[4] = {
-        {static_cast<uint64_t>(D), 0, static_cast<uint32_t>(cols)},
-        {static_cast<uint64_t>(H), static_cast<uint64_t>(lay.h) * e, 1},
-        {static_cast<uint64_t>(N), static_cast<uint64_t>(lay.n) * e, static_cast<uint32_t>(rows)},
-        {static_cast<uint64_t>(BS), static_cast<uint64_t>(lay.row) * e, 1},
-    };
-    const CUtensorMapSwizzle sw = rb == 16 ? CU_TENSOR_MAP_SWIZZLE_NONE
-                                : (rb == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
-                                : (rb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B));
-    return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, d, sw);
 }
 
 int layout_from_strides(const EvoDims* d, const EvoStrides* s, ActLayout* out) {
@@ -194,19 +186,6 @@ int make_tmap_rows_box(CUtensorMap* out, const void* base, int elem_bytes, int B
     };
     return make_tmap(out, base, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                      4, d, swizzle_for(rb));
-}
-
-int make_tmap_dbias_box(CUtensorMap* out, const void* base, int B, int H, int N, int box_cols, int rows) {
-    const uint64_t e = 4;
-    const int rb = box_cols * 4;
-    if (rb != 32 && rb != 64 && rb != 128) return EVO_ERR_TENSOR_MAP;
-    TmapDim d[4] = {
-        {static_cast<uint64_t>(N), 0, static_cast<uint32_t>(box_cols)},
-        {static_cast<uint64_t>(N), N * e, static_cast<uint32_t>(rows)},
-        {static_cast<uint64_t>(H), static_cast<uint64_t>(N) * N * e, 1},
-        {static_cast<uint64_t>(B), static_cast<uint64_t>(H) * N * N * e, 1},
-    };
-    return make_tmap(out, base, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d, swizzle_for(rb));
 }
 
 // Binds the device's primary context to the calling thread.  The tensor-map

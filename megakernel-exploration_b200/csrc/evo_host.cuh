@@ -49,15 +49,10 @@ int layout_from_strides(const EvoDims* d, const EvoStrides* s, ActLayout* out);
 // read by the D = 32 kernels) is zero-filled past D on loads and clipped on stores.
 int make_tmap_qkv(CUtensorMap* out, const void* base, int BS, int N, int H, int D, int rows,
                   const ActLayout& lay, int box_d = 0);
-// The same view with a box of [rows x cols] head-dim columns (cols * 2 bytes = 32, 64 or 128), swizzled by box row.
-int make_tmap_qkv_cols(CUtensorMap* out, const void* base, int BS, int N, int H, int D, int rows, int cols,
-                       const ActLayout& lay);
 // [BS][N][H][D] of `elem_bytes`-wide elements (2: bf16, 4: fp32) with a box of
 // [rows x box_cols]; the swizzle matches the box row (32, 64 or 128 bytes).
 int make_tmap_rows_box(CUtensorMap* out, const void* base, int elem_bytes, int BS, int N, int H, int D,
                        int box_cols, int rows);
-// fp32 [B][H][N][N] with a box of [rows x box_cols], swizzle by box row bytes.
-int make_tmap_dbias_box(CUtensorMap* out, const void* base, int B, int H, int N, int box_cols, int rows);
 // bf16 [B][H][N][N] viewed as (N, N, H, B); box [rows x 64 cols], 128B swizzle.
 int make_tmap_bias(CUtensorMap* out, const void* base, int B, int H, int N, int rows = 128);
 
