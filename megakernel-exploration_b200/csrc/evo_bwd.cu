@@ -23,6 +23,7 @@
 #include "evo_ptx.cuh"
 #include "evo_tiles.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -37,16 +38,19 @@ struct BwdParams {
     int KB;          // contraction blocks of 16 head-dim columns that hold data: ceil(Dt / 16)
     int NT;          // tiles per row: ceil(N / 128)
     int NTP;         // NT * 128
-    int total_items; // B * S * H, or B * S * H * NT segments
+    int pairs;       // B * S * H
+    int n_whole;     // pairs taken whole; the others are dealt by segments
     float scale;     // softmax scale
     float c1;        // scale * log2(e)
     const __nv_bfloat16* xq;   // [B*S][H][NTP][8] extra tiles of the q rows  (bwd_prep_kernel)
     const __nv_bfloat16* xk;   // [B*S][NTP][8]    extra tiles of the kv rows
     const __nv_bfloat16* bias; // [B][H][N][N]
     void* dbias;               // [B][H][N][N], fp32 or bf16 (written by this kernel only when S = 1)
-    float* dq_scratch;         // WHOLE: per CTA scratch_stride 16-byte words, partial sums of dQ
+    float* dq_scratch;         // whole pairs: per CTA scratch_stride 16-byte words, partial sums of dQ
     size_t scratch_stride;
-    __nv_bfloat16* dq;    // activation layout `lay` (dq: written by this kernel only when WHOLE)
+    float* dq_acc;             // the others: [B*S - acc_row0][N][H][DH], zeroed before the launch
+    int acc_row0;              // their first S row
+    __nv_bfloat16* dq;    // activation layout `lay` (dq: of the whole pairs only)
     __nv_bfloat16* dk;
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
@@ -58,7 +62,36 @@ struct BwdParams {
 // per item) is not launched.
 enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2 };
 
-
+// What a CTA of the dQ/dK/dV kernels walks: the segments (kv tiles) of whole pairs (S row, head) one after another,
+// single segments, or the one and then the other.  A template parameter: chosen at run time it costs the drain warps,
+// and all of a D = 128 step, 5 %.
+enum Walk { WALK_SEGMENTS, WALK_WHOLE, WALK_BOTH };
+template <int WALK>
+struct Segments {
+    int first, stride, NT, H, n_whole, n_ws, n;     // n_ws: segments of whole pairs; n: all
+    __device__ __forceinline__ explicit Segments(const BwdParams& p)
+        : first(blockIdx.x), stride(gridDim.x), NT(p.NT), H(p.H), n_whole(WALK == WALK_SEGMENTS ? 0 : p.n_whole) {
+        auto share = [&](int total) { return total > first ? (total - first + stride - 1) / stride : 0; };
+        n_ws = WALK == WALK_SEGMENTS ? 0 : share(n_whole) * NT;
+        n = WALK == WALK_WHOLE ? n_ws : n_ws + share((p.pairs - n_whole) * NT);
+    }
+    __device__ __forceinline__ bool whole(int sg) const {
+        return WALK == WALK_WHOLE || (WALK == WALK_BOTH && sg < n_ws);
+    }
+    __device__ __forceinline__ void decode(int sg, int& bs, int& h, int& j) const {
+        int pair;
+        if (whole(sg)) {
+            j = sg % NT;
+            pair = first + sg / NT * stride;
+        } else {
+            const int w = first + (sg - n_ws) * stride;
+            j = w % NT;
+            pair = n_whole + w / NT;
+        }
+        h = pair % H;
+        bs = pair / H;
+    }
+};
 
 }  // namespace evo
 #include "evo_bwd_wide.cuh"
@@ -96,19 +129,21 @@ namespace evo {
 //                         segment K, V and the extra tile of the kv rows
 //   warps 21, 22, 23      MMA issuers, one chain family each: S'^T and dP'^T; dV and dK; dQ
 //
-// dQ is a sum over kv tiles.  WHOLE: an item is all NT segments of a (row, head), so one CTA sees the
-// whole sum.  With one or two tiles it stays in tensor memory until the last segment; otherwise the drain
+// dQ is a sum over kv tiles.  A CTA takes all NT segments of a pair (S row, head) where it can, and so sees
+// the whole sum.  With one or two tiles it stays in tensor memory until the last segment; otherwise the drain
 // warps keep partial sums in a scratch area of the CTA, in L2 (written and added to by bulk copies: loads
 // and stores of their own held up the compute warps' shared-memory accesses), and the last segment's go out
-// as bf16.  Where there are too few items for that, an item is one segment, and the partial sums meet in an
-// fp32 accumulator in memory (TMA reduce-add), which costs a pass to zero it and a pass to convert it.
+// as bf16.  Whole pairs fill whole rounds of the SMs; the pairs that are left over are dealt by segments, and
+// their partial sums meet in an fp32 accumulator in memory (TMA reduce-add), which costs a pass to zero it and
+// a pass to convert it, of those pairs only (against all pairs whole, or none, the kernel alone: S=384, N=384, H=4,
+// D=32 182 -> 176 us; S=200, N=200, H=4 47 -> 44; S=1024, N=768, H=8 3333 -> 3255).
 //
 // Measured against one kernel with P and dS in shared memory and two compute groups (whole backward):
 // B=1, S=512, N=384, H=8, D=32 0.81 -> 0.71 ms; S=256, N=768 1.40 -> 1.28; S=256, N=1024, H=4, D=64 1.93 ->
 // 1.59; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
 // D = 128: evo_bwd_wide.cuh.
 // ---------------------------------------------------------------------------
-template <int DH, bool WHOLE>
+template <int DH>
 struct BwdCfg {
     static constexpr bool ALIAS = (DH == 64);
     static constexpr bool TWO_PHASE = (DH == 64);
@@ -155,13 +190,14 @@ struct BwdCfg {
     static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
 };
 
-template <int DH, bool WHOLE, int DBIAS_HERE>
-__global__ void __launch_bounds__((BwdCfg<DH, WHOLE>::THREADS), 1)
+template <int DH, int WALK, int DBIAS_HERE>
+__global__ void __launch_bounds__(BwdCfg<DH>::THREADS, 1)
 evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_dq,
-               const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
-    using C = BwdCfg<DH, WHOLE>;
+               const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
+               const __grid_constant__ CUtensorMap tm_acc, const BwdParams p) {
+    using C = BwdCfg<DH>;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
     constexpr int QS = C::QS, NKV = C::NKV, NB = C::NB, DQB = C::DQ_BUFS;
@@ -215,6 +251,7 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == C::W_PROD && lane == 0) {
         prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do);
         prefetch_tmap(&tm_bias); prefetch_tmap(&tm_dq); prefetch_tmap(&tm_dk); prefetch_tmap(&tm_dv);
+        prefetch_tmap(&tm_acc);
     }
     // constant extra tiles: row n of the -delta selector is (0,0,0,0,1,1,0,0); the zero tile
     if (tid < 128) {
@@ -227,22 +264,12 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // Segments of this CTA: segment sg is kv tile sg % NT of item sg / NT (WHOLE), or an item of its own.
-    // Item index -> (batch * S + row, head[, kv tile]), the last one fastest.
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int n_items = (p.total_items > first) ? (p.total_items - first + stride - 1) / stride : 0;
-    const int n_segs = WHOLE ? n_items * NT : n_items;
-    const bool resident = WHOLE && NT <= DQB;      // dQ stays in tensor memory for the item
-    auto decode = [&](int sg, int& bs, int& h, int& j) {
-        int w = first + (WHOLE ? sg / NT : sg) * stride;
-        if (WHOLE) {
-            j = sg % NT;
-        } else {
-            j = w % NT;
-            w /= NT;
-        }
-        h = w % p.H;
-        bs = w / p.H;
+    const Segments<WALK> seg(p);
+    const int n_segs = seg.n;
+    const bool res_ok = NT <= DQB;       // dQ of a whole pair stays in tensor memory
+    // dQ accumulators in order of use: one per step, or (resident) one per q tile of a pair
+    auto dq_event = [&](bool resident, int sg, int j, int i) {
+        return resident ? (sg - j) + i : sg * NT + i - (res_ok ? seg.n_ws * (NT - 1) : 0);
     };
 
     if (warp == C::W_PROD) {
@@ -251,7 +278,7 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         int gs = 0, n_st = 0, n_bias = 0, n_kv = 0;      // steps; loads issued
         for (int sg = 0; sg < n_segs && ok; ++sg) {
             int bs, h, j;
-            decode(sg, bs, h, j);
+            seg.decode(sg, bs, h, j);
             const int b = bs / p.S;
             const __nv_bfloat16* xq = p.xq + (static_cast<size_t>(bs) * p.H + h) * p.NTP * 8;
             {
@@ -395,9 +422,8 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                     __syncwarp();
                 } else {
-                    // accumulators: one per step, or (resident) one per q tile of the item
-                    const int j = WHOLE ? sg % NT : 0;
-                    const int ev = resident ? (sg - j) + i : gs;
+                    const bool whole = seg.whole(sg), resident = whole && res_ok;
+                    const int j = whole ? sg % NT : 0, ev = dq_event(resident, sg, j, i);
                     if (ev >= DQB && !(resident && j > 0)) ok = warp_all(mbar_wait(&dq_free[ev % DQB], ((ev / DQB) - 1) & 1, wc, 0x54));
                     if (ok) ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5b));
                     if (!ok) break;
@@ -456,99 +482,104 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 u[c8] = make_uint4(pack_bf16(v[c8 * 8 + 0] * sc, v[c8 * 8 + 1] * sc), pack_bf16(v[c8 * 8 + 2] * sc, v[c8 * 8 + 3] * sc),
                                    pack_bf16(v[c8 * 8 + 4] * sc, v[c8 * 8 + 5] * sc), pack_bf16(v[c8 * 8 + 6] * sc, v[c8 * 8 + 7] * sc));
         };
-        // WHOLE: the partial sums of this CTA, in units of 4 KB: 32 rows x 32 columns as [16-byte word][row]
+        // whole pairs: the partial sums of this CTA, in units of 4 KB: 32 rows x 32 columns as [16-byte word][row]
         float4* part = reinterpret_cast<float4*>(p.dq_scratch) + static_cast<size_t>(blockIdx.x) * p.scratch_stride;
         bool ok = true;
-        int gs = 0;
-        for (int sg = 0; sg < n_segs && ok; ++sg) {
-            int bs, h, j;
-            decode(sg, bs, h, j);
-            for (int i = 0; i < NT && ok; ++i, ++gs) {
-                if (resident && j < NT - 1) continue;          // dQ is still being summed
-                const int ev = resident ? (sg - j) + i : gs, b = ev % DQB;
-                const bool rows = i * TILE + wrow0 < p.N;     // warp-uniform: some row of this warp exists
-                const bool final_sum = WHOLE && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
-                float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
-                float4 old[8];
-                // The bulk copy that last wrote this part of the scratch area, NT >= 3 steps ago, is complete
-                // before the sum is added to or read: at least two were issued after it.
-                if (WHOLE && j > 0 && !resident) {
-                    if (lane == 0) tma_wait_group<2>();
-                    if (add) fence_async_all();
-                    __syncwarp();
+        auto drain = [&](auto whole_c, int sg0, int sg1) {
+            constexpr bool whole = decltype(whole_c)::value;
+            for (int sg = sg0; sg < sg1 && ok; ++sg) {
+                int bs, h, j;
+                seg.decode(sg, bs, h, j);
+                const bool resident = whole && res_ok;
+                for (int i = 0; i < NT && ok; ++i) {
+                    if (resident && j < NT - 1) continue;          // dQ is still being summed
+                    const int ev = dq_event(resident, sg, j, i), b = ev % DQB;
+                    const bool rows = i * TILE + wrow0 < p.N;     // warp-uniform: some row of this warp exists
+                    const bool final_sum = whole && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
+                    float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
+                    float4 old[8];
+                    // The bulk copy that last wrote this part of the scratch area, NT >= 3 steps ago, is complete
+                    // before the sum is added to or read: at least two were issued after it.
+                    if (whole && j > 0 && !resident) {
+                        if (lane == 0) tma_wait_group<2>();
+                        if (add) fence_async_all();
+                        __syncwarp();
+                    }
+                    ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
+                    if (!ok) break;
+                    tc_fence_after();
+    #pragma unroll
+                    for (int rd = 0; rd < DH / 32; ++rd) {
+                        float dqv[32];
+                        tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
+                        if (rd == DH / 32 - 1) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&dq_free[b]);
+                        }
+                        if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
+                        if (final_sum) {
+                            if (add) {
+    #pragma unroll
+                                for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + (rd * 8 + c) * 32 + lane);
+    #pragma unroll
+                                for (int c = 0; c < 8; ++c) {
+                                    dqv[4 * c] += old[c].x; dqv[4 * c + 1] += old[c].y;
+                                    dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
+                                }
+                            }
+                            uint4 u[4];
+                            pack_rows(u, dqv, p.scale);
+                            store_rows(&tm_dq, u, h, i * TILE + wrow0, rd * 32, bs);
+                            continue;
+                        }
+                        uint8_t* wq = next_slot(false);
+                        const float sc = whole ? 1.0f : p.scale;
+    #pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            *reinterpret_cast<float4*>(wq + (whole ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
+                                make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
+                        fence_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (!whole)
+                                tma_reduce_add_4d(&tm_acc, wq, rd * 32, h, i * TILE + wrow0, bs - p.acc_row0);
+                            else if (j == 0)
+                                bulk_store(ps + rd * 8 * 32, wq, C::WQ_BYTES);
+                            else
+                                bulk_reduce_add_f32(ps + rd * 8 * 32, wq, C::WQ_BYTES);
+                            tma_commit_group();
+                        }
+                    }
                 }
-                ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
+                if (!ok) break;
+                ok = warp_all(mbar_wait(dkv_full, sg & 1, wc, 0x69));
                 if (!ok) break;
                 tc_fence_after();
-#pragma unroll
-                for (int rd = 0; rd < DH / 32; ++rd) {
-                    float dqv[32];
-                    tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
-                    if (rd == DH / 32 - 1) {
+                const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
+    #pragma unroll
+                for (int t = 0; t < 2; ++t) {                   // dK, then dV
+                    uint4 u[DH / 32][4];
+    #pragma unroll
+                    for (int c = 0; c < DH / 32; ++c) {
+                        float v[32];
+                        __syncwarp();
+                        tmem_ld_f32<32>(lane_base + (t ? C::TMEM_DV : C::TMEM_DK) + c * 32, v);
+                        pack_rows(u[c], v, t ? 1.0f : p.scale);
+                    }
+                    if (t == 1) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&dq_free[b]);
+                        if (lane == 0) mbar_arrive(dkv_free);
                     }
-                    if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
-                    if (final_sum) {
-                        if (add) {
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + (rd * 8 + c) * 32 + lane);
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) {
-                                dqv[4 * c] += old[c].x; dqv[4 * c + 1] += old[c].y;
-                                dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
-                            }
-                        }
-                        uint4 u[4];
-                        pack_rows(u, dqv, p.scale);
-                        store_rows(&tm_dq, u, h, i * TILE + wrow0, rd * 32, bs);
-                        continue;
-                    }
-                    uint8_t* wq = next_slot(false);
-                    const float sc = WHOLE ? 1.0f : p.scale;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c)
-                        *reinterpret_cast<float4*>(wq + (WHOLE ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
-                            make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (!WHOLE)
-                            tma_reduce_add_4d(&tm_dq, wq, rd * 32, h, i * TILE + wrow0, bs);
-                        else if (j == 0)
-                            bulk_store(ps + rd * 8 * 32, wq, C::WQ_BYTES);
-                        else
-                            bulk_reduce_add_f32(ps + rd * 8 * 32, wq, C::WQ_BYTES);
-                        tma_commit_group();
-                    }
+    #pragma unroll
+                    for (int c = 0; c < DH / 32; ++c)
+                        if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[c], h, j * TILE + wrow0, c * 32, bs);
                 }
             }
-            if (!ok) break;
-            ok = warp_all(mbar_wait(dkv_full, sg & 1, wc, 0x69));
-            if (!ok) break;
-            tc_fence_after();
-            const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {                   // dK, then dV
-                uint4 u[DH / 32][4];
-#pragma unroll
-                for (int c = 0; c < DH / 32; ++c) {
-                    float v[32];
-                    __syncwarp();
-                    tmem_ld_f32<32>(lane_base + (t ? C::TMEM_DV : C::TMEM_DK) + c * 32, v);
-                    pack_rows(u[c], v, t ? 1.0f : p.scale);
-                }
-                if (t == 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(dkv_free);
-                }
-#pragma unroll
-                for (int c = 0; c < DH / 32; ++c)
-                    if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[c], h, j * TILE + wrow0, c * 32, bs);
-            }
-        }
+        };
+        if (WALK != WALK_SEGMENTS) drain(std::true_type{}, 0, seg.n_ws);
+        if (WALK != WALK_WHOLE) drain(std::false_type{}, seg.n_ws, n_segs);
         if (lane == 0) tma_wait_group<0>();
     } else {
         // ------------------------------ compute groups ------------------------------
@@ -596,7 +627,7 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
         for (int sg = 0; sg < n_segs && ok; ++sg) {
             int bs = 0, h = 0, j = 0;
-            if constexpr (DBIAS_HERE != DBIAS_NO) decode(sg, bs, h, j);
+            if constexpr (DBIAS_HERE != DBIAS_NO) seg.decode(sg, bs, h, j);
             for (int i = 0; i < NT && ok; ++i, ++gs) {
                 const int bb = gs % NB;
                 if constexpr (C::TWO_PHASE) {
@@ -891,12 +922,14 @@ __global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const P
         for (size_t i = t0; i < p.n_zero[z]; i += gstride) p.zero[z][i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// The results that were accumulated in fp32, in their final type: dQ ([B*S][N][H][DH] contiguous) -> bf16 in
-// the activation layout, and dBias -> bf16 if the caller wants it so.  Eight elements per thread.
+// The results that were accumulated in fp32, in their final type: dQ of the pairs from pair0 on, which lie
+// in rows row0 and up ([row][N][H][DH]) -> bf16 in the activation layout; and dBias -> bf16 if the caller wants it so.
+// Eight elements per thread.
 struct FinishParams {
     const float* dq_acc;
     __nv_bfloat16* dq;
     size_t n8;                 // groups of eight of dq_acc
+    int pair0, row0;
     int N, H, Dt;
     ActLayout lay;
     const float* dbias_acc;    // nullptr: dBias is final already
@@ -912,10 +945,8 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     for (size_t i = t0; i < p.n8; i += gstride) {
-        const size_t rowi = i / (DH / 8);                 // (bs, n, h) of this group of eight
+        const size_t rowi = i / (DH / 8);                 // (row, n, h) of this group of eight
         const int d8 = static_cast<int>(i % (DH / 8));
-        if (d8 * 8 >= p.Dt) continue;
-        const uint4 u = cvt8(p.dq_acc + 8 * i);
         size_t bs, n, h;
         if (p.n8 < 0x80000000ull) {
             const uint32_t r32 = static_cast<uint32_t>(rowi), b32 = r32 / p.H, s32 = b32 / p.N;
@@ -928,6 +959,9 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
             bs = bn / p.N;
             n = bn - bs * p.N;
         }
+        bs += p.row0;
+        if (d8 * 8 >= p.Dt || bs * p.H + h < static_cast<size_t>(p.pair0)) continue;
+        const uint4 u = cvt8(p.dq_acc + 8 * i);
         *reinterpret_cast<uint4*>(p.dq + bs * p.lay.row + n * p.lay.n + h * p.lay.h + d8 * 8) = u;
     }
     if (p.dbias_acc)
@@ -970,9 +1004,9 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const ActLayout lay_do = gate ? contiguous_layout(d->N, d->H, d->D) : lay_out;
     uint4* xq = reinterpret_cast<uint4*>(ws + w.off_xq);
     uint4* xk = reinterpret_cast<uint4*>(ws + w.off_xk);
-    float* dq_acc = reinterpret_cast<float*>(ws + w.off_dq);
+    float* dq_ws = reinterpret_cast<float*>(ws + w.off_dq);
 
-    CUtensorMap tq, tk, tv, tdo, tb, tdq, tdk, tdv;
+    CUtensorMap tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc;
     int rc;
     const int Dt = d->D;          // 16 on the D = 32 kernel: boxes of 32 columns over tensors of 16
     if ((rc = make_tmap_qkv(&tq, q, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
@@ -1003,25 +1037,45 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     // SMs left to other work (a collective on another stream) while the dQ/dK/dV kernel runs
     int use_sms = sms - (reserved_sms > 0 ? reserved_sms : 0);
     if (use_sms < 1) use_sms = 1;
-    // Whole items (all kv tiles of a row and head) where that costs no more time than single segments: the
-    // rounds of the fullest SM, against those of segments plus the two passes over the fp32 accumulator
-    // (about 1 / (2 NT) of the kernel).
-    const long pairs = static_cast<long>(BS) * d->H;
-    const long t_whole = (pairs + use_sms - 1) / use_sms * NT, t_seg = (pairs * NT + use_sms - 1) / use_sms;
-    const bool whole = NT == 1 || t_whole * 2 * NT <= t_seg * (2 * NT + 1);
-    p.total_items = static_cast<int>(whole ? pairs : pairs * NT);
-    p.dq_scratch = dq_acc;
-    if constexpr (DH <= 64) {
-        // what the drain warps write: boxes of 32 rows x 32 columns (dQ: bf16, or the fp32 accumulator)
-        if (whole) rc = make_tmap_qkv(&tdq, dq, BS, d->N, d->H, Dt, 32, lay_grad, 32);
-        else rc = make_tmap_rows_box(&tdq, dq_acc, 4, BS, d->N, d->H, DH, 32, 32);
-        if (rc || (rc = make_tmap_qkv(&tdk, dk, BS, d->N, d->H, Dt, 32, lay_grad, 32)) ||
-            (rc = make_tmap_qkv(&tdv, dv, BS, d->N, d->H, Dt, 32, lay_grad, 32)))
-            return rc;
+    // D <= 64: pairs (S row, head) are taken whole as far as they fill whole rounds of the SMs, and so are those left
+    // over if single segments of them would not end a round sooner.  (Rounds are the same as with segments alone,
+    // the accumulator and its passes are those of less than one round of pairs.)
+    // D = 128: all or none, whole where that costs no more time than segments: the rounds of the fullest SM, against
+    // those of segments plus the two passes over the accumulator (about 1 / (2 NT) of the kernel).  Most of the pairs
+    // whole is no gain there: 148 pairs' operands and partial sums at a time outgrow the L2, and the kernel has one
+    // load stage (B=1, S=40, N=768, H=4: 193 -> 214 us, passes 42 -> 25).
+    const int pairs = BS * d->H;
+    const size_t n32 = static_cast<size_t>((d->N + 31) / 32) * 32;
+    const long t_seg = (static_cast<long>(pairs) * NT + use_sms - 1) / use_sms;
+    if constexpr (DH == 128) {
+        const long t_whole = static_cast<long>((pairs + use_sms - 1) / use_sms) * NT;
+        p.n_whole = (NT == 1 || t_whole * 2 * NT <= t_seg * (2 * NT + 1)) ? pairs : 0;
+    } else {
+        const int left = pairs % use_sms, full = pairs - left;
+        p.n_whole = (left && t_seg < static_cast<long>(full / use_sms + 1) * NT) ? full : pairs;
+        // the workspace holds the partial sums of every CTA and the accumulator from the row on that pair `full` is in
+        const size_t acc_n = static_cast<size_t>(pairs - full / d->H * d->H) * d->N;
+        if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > pairs * n32) p.n_whole = 0;
     }
-    p.scratch_stride = static_cast<size_t>((d->N + 31) / 32) * 32 * DH / 4;
+    p.pairs = pairs;
+    p.acc_row0 = p.n_whole / d->H;
+    const int rest_rows = p.n_whole < pairs ? BS - p.acc_row0 : 0;
+    const int grid = static_cast<int>(std::min<long>(p.n_whole ? pairs : static_cast<long>(pairs) * NT, use_sms));
+    // workspace: the partial sums of every CTA with whole pairs, then the accumulator of the rest
+    p.scratch_stride = n32 * DH / 4;
+    p.dq_scratch = dq_ws;
+    p.dq_acc = dq_ws + (p.n_whole ? grid : 0) * p.scratch_stride * 4;
+    if constexpr (DH <= 64) {
+        // what the drain warps write: boxes of 32 rows x 32 columns
+        if ((rc = make_tmap_qkv(&tdq, dq, BS, d->N, d->H, Dt, 32, lay_grad, 32)) ||
+            (rc = make_tmap_qkv(&tdk, dk, BS, d->N, d->H, Dt, 32, lay_grad, 32)) ||
+            (rc = make_tmap_qkv(&tdv, dv, BS, d->N, d->H, Dt, 32, lay_grad, 32)) ||
+            (rc = rest_rows ? make_tmap_rows_box(&tacc, p.dq_acc, 4, rest_rows, d->N, d->H, DH, 32, 32) : 0))
+            return rc;
+        if (!rest_rows) tacc = tdq;
+    }
 
-    const size_t dq_bytes = static_cast<size_t>(BS) * d->N * d->H * DH * 4;
+    const size_t acc_bytes = static_cast<size_t>(rest_rows) * d->N * d->H * DH * 4;
     const size_t db_elems = static_cast<size_t>(d->B) * d->H * d->N * d->N;
 
     // one S row and the whole backward in this call: the dQ/dK/dV kernel writes dBias (= dS) itself
@@ -1046,8 +1100,8 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         r.d_gate = static_cast<__nv_bfloat16*>(d_gate);
         r.zero[0] = reinterpret_cast<uint4*>(dbias_acc);
         r.n_zero[0] = (!dbias_here && slices > 1) ? db_elems / 4 : 0;
-        r.zero[1] = reinterpret_cast<uint4*>(dq_acc);
-        r.n_zero[1] = (both && !whole) ? dq_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
+        r.zero[1] = reinterpret_cast<uint4*>(p.dq_acc);
+        r.n_zero[1] = both ? acc_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
         r.inv_scale = 1.0f / p.scale;
         r.BS = BS; r.N = d->N; r.H = d->H; r.NTP = p.NTP; r.Dt = Dt;
         r.lay = lay_out;
@@ -1071,8 +1125,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
 
-    if (!both && !whole && (rc = cuda_err(cudaMemsetAsync(dq_acc, 0, dq_bytes, st)))) return rc;
-    const int grid = p.total_items < use_sms ? p.total_items : use_sms;
+    if (!both && rest_rows && (rc = cuda_err(cudaMemsetAsync(p.dq_acc, 0, acc_bytes, st)))) return rc;
     const int mode = !dbias_here ? DBIAS_NO : (dbias_bf16 ? DBIAS_BF16 : DBIAS_F32);
     auto run = [&](auto kernel, int threads, uint32_t smem, auto... maps) -> int {
         const int e = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
@@ -1082,27 +1135,31 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         prof_end(1, st);
         return cuda_err(cudaGetLastError());
     };
-    auto launch = [&](auto whole_c) -> int {
-        constexpr bool W = decltype(whole_c)::value;
+    auto launch = [&](auto walk_c) -> int {
+        constexpr int W = decltype(walk_c)::value;
         if constexpr (DH == 128) {
-            using C = BwdWideCfg<DH, W>;
+            using C = BwdWideCfg<DH>;
             auto kernel = mode == DBIAS_NO ? evo_bwd_wide_kernel<DH, W, DBIAS_NO>
                                            : (mode == DBIAS_BF16 ? evo_bwd_wide_kernel<DH, W, DBIAS_BF16> : evo_bwd_wide_kernel<DH, W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
         } else {
-            using C = BwdCfg<DH, W>;
+            using C = BwdCfg<DH>;
             auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<DH, W, DBIAS_NO>
                                            : (mode == DBIAS_BF16 ? evo_bwd_kernel<DH, W, DBIAS_BF16> : evo_bwd_kernel<DH, W, DBIAS_F32>);
-            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv);
+            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         }
     };
-    rc = whole ? launch(std::true_type{}) : launch(std::false_type{});
-    if (rc || (whole && !convert_dbias)) return rc;
+    if (p.n_whole == pairs) rc = launch(std::integral_constant<int, WALK_WHOLE>{});
+    else if (p.n_whole == 0) rc = launch(std::integral_constant<int, WALK_SEGMENTS>{});
+    else if constexpr (DH != 128) rc = launch(std::integral_constant<int, WALK_BOTH>{});
+    if (rc || (!rest_rows && !convert_dbias)) return rc;
 
     FinishParams f;
-    f.dq_acc = dq_acc;
+    f.dq_acc = p.dq_acc;
     f.dq = static_cast<__nv_bfloat16*>(dq);
-    f.n8 = whole ? 0 : dq_bytes / 32;
+    f.n8 = acc_bytes / 32;
+    f.pair0 = p.n_whole;
+    f.row0 = p.acc_row0;
     f.N = d->N; f.H = d->H; f.Dt = Dt;
     f.lay = lay_grad;
     f.dbias_acc = convert_dbias ? dbias_acc : nullptr;

@@ -1,5 +1,5 @@
 // dQ, dK, dV at D = 96 and 128 (evo_bwd.cu has the interface, the D <= 64 kernel and what the two share:
-// transposed products, WHOLE items or single segments).  Tensor memory holds S', dP', dK and dV and
+// transposed products, whole pairs or single segments).  Tensor memory holds S', dP', dK and dV and
 // nothing else: P^T and dS^T overwrite the columns they were computed from, and dQ takes the columns of S'
 // once dV, which reads P^T from them, is complete.  A step is then one chain
 //
@@ -17,7 +17,7 @@
 
 namespace evo {
 
-template <int DH, bool WHOLE>
+template <int DH>
 struct BwdWideCfg {
     static_assert(DH == 128, "the D <= 64 kernel is in evo_bwd.cu");
     static constexpr int NG = 4;                       // compute groups
@@ -48,12 +48,12 @@ struct BwdWideCfg {
     static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0, "tile alignment");
 };
 
-template <int DH, bool WHOLE, int DBIAS_HERE>
-__global__ void __launch_bounds__((BwdWideCfg<DH, WHOLE>::THREADS), 1)
+template <int DH, int WALK, int DBIAS_HERE>
+__global__ void __launch_bounds__(BwdWideCfg<DH>::THREADS, 1)
 evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_bias, const BwdParams p) {
-    using C = BwdWideCfg<DH, WHOLE>;
+    using C = BwdWideCfg<DH>;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
 
@@ -111,22 +111,9 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // Segments of this CTA: segment sg is kv tile sg % NT of item sg / NT (WHOLE), or an item of its own.
-    // Item index -> (batch * S + row, head[, kv tile]), the last one fastest.
-    const int first = blockIdx.x, stride = gridDim.x;
-    const int n_items = (p.total_items > first) ? (p.total_items - first + stride - 1) / stride : 0;
-    const int n_segs = WHOLE ? n_items * NT : n_items;
-    auto decode = [&](int sg, int& bs, int& h, int& j) {
-        int w = first + (WHOLE ? sg / NT : sg) * stride;
-        if (WHOLE) {
-            j = sg % NT;
-        } else {
-            j = w % NT;
-            w /= NT;
-        }
-        h = w % p.H;
-        bs = w / p.H;
-    };
+    static_assert(WALK != WALK_BOTH, "all pairs whole, or none");
+    const Segments<WALK> seg(p);
+    const int n_segs = seg.n;
 
     if (warp == C::W_PROD) {
         // ------------------------------ producer ------------------------------
@@ -134,7 +121,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         int gs = 0, n_do = 0, n_q = 0, n_bias = 0, n_kv = 0;      // steps; loads issued
         for (int sg = 0; sg < n_segs && ok; ++sg) {
             int bs, h, j;
-            decode(sg, bs, h, j);
+            seg.decode(sg, bs, h, j);
             const int b = bs / p.S;
             const __nv_bfloat16* xq = p.xq + (static_cast<size_t>(bs) * p.H + h) * p.NTP * 8;
             if (sg > 0) ok = warp_all(mbar_wait(kv_empty, (sg - 1) & 1, wc, 0x40));
@@ -289,7 +276,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + (row >> 6) * SQ_SUB_BYTES + 32 * g * 128 + (row & 7) * 2;
         const uint32_t bchunk = (row & 63) >> 3;
         const uint32_t scratch_w = smem_u32(tmem_slot + 2);       // a word nobody reads
-        // WHOLE: this thread's 16-byte words of the partial sums of dQ, 32 lanes side by side
+        // whole pairs: this thread's 16-byte words of the partial sums of dQ, 32 lanes side by side
         float4* part = reinterpret_cast<float4*>(p.dq_scratch) + static_cast<size_t>(blockIdx.x) * p.scratch_stride + lane;
         const int w4 = warp & 3, wrow0 = 32 * w4;
         const bool has_cols = 32 * g < p.Dt;      // warp-uniform: head-dim columns of this group that exist
@@ -308,13 +295,14 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 if (r0 + e < p.N) *reinterpret_cast<uint4*>(out + (r0 + e) * p.lay.n + col) = u[e];
             __syncwarp();
         };
+        constexpr bool whole = WALK == WALK_WHOLE;
         bool ok = true;
         int gs = 0;
         const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
 
         for (int sg = 0; sg < n_segs && ok; ++sg) {
             int bs, h, j;
-            decode(sg, bs, h, j);
+            seg.decode(sg, bs, h, j);
             const size_t head = bs * p.lay.row + h * p.lay.h;
             for (int i = 0; i < NT && ok; ++i, ++gs) {
                 ok = warp_all(mbar_wait(sdp_full, gs & 1, wc, 0x63));
@@ -391,7 +379,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const bool rows = has_cols && i * TILE + wrow0 < p.N;      // warp-uniform
                 float4* ps = part + static_cast<size_t>((i * 4 + w4) * (DH / 4) + 8 * g) * 32;
                 float4 old[8];
-                if (WHOLE && j > 0 && rows) {                  // requested before the wait
+                if (whole && j > 0 && j == NT - 1 && rows) {   // requested before the wait
 #pragma unroll
                     for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + c * 32);
                 }
@@ -404,7 +392,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dq_free);
                 if (rows) {
-                    if constexpr (WHOLE) {
+                    if (whole && j == NT - 1) {
                         if (j > 0) {
 #pragma unroll
                             for (int c = 0; c < 8; ++c) {
@@ -412,17 +400,21 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                                 dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
                             }
                         }
-                        if (j < NT - 1) {
+                        store_rows(p.dq + head, dqv, p.scale, i * TILE + wrow0);
+                    } else if (whole && j == 0) {
 #pragma unroll
-                            for (int c = 0; c < 8; ++c)
-                                __stcg(ps + c * 32, make_float4(dqv[4 * c], dqv[4 * c + 1], dqv[4 * c + 2], dqv[4 * c + 3]));
-                        } else {
-                            store_rows(p.dq + head, dqv, p.scale, i * TILE + wrow0);
-                        }
+                        for (int c = 0; c < 8; ++c)
+                            __stcg(ps + c * 32, make_float4(dqv[4 * c], dqv[4 * c + 1], dqv[4 * c + 2], dqv[4 * c + 3]));
+                    } else if (whole) {
+                        // added in L2, nothing to wait for here; the thread that reads the sum in the last segment is
+                        // the same (loaded, added and stored by each segment instead: S=37, N=768, H=4 186 -> 194 us)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            red_add_v4(reinterpret_cast<float*>(ps + c * 32), dqv[4 * c], dqv[4 * c + 1], dqv[4 * c + 2], dqv[4 * c + 3]);
                     } else {
                         // fp32 accumulator [B*S][N][H][DH]: lane t of a quad adds chunks t and 4 + t of four rows
                         const int r0 = i * TILE + wrow0 + (lane & ~3);
-                        float* acc = p.dq_scratch + ((static_cast<size_t>(bs) * p.N + r0) * p.H + h) * DH + 32 * g + 4 * (lane & 3);
+                        float* acc = p.dq_acc + ((static_cast<size_t>(bs) * p.N + r0) * p.H + h) * DH + 32 * g + 4 * (lane & 3);
 #pragma unroll
                         for (int hf = 0; hf < 2; ++hf) {
                             uint4 u[4];
@@ -434,10 +426,8 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 #pragma unroll
                             for (int e = 0; e < 4; ++e)
                                 if (r0 + e < p.N)
-                                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                                                 ::"l"(acc + static_cast<size_t>(e) * p.H * DH + 16 * hf), "f"(__uint_as_float(u[e].x)),
-                                                   "f"(__uint_as_float(u[e].y)), "f"(__uint_as_float(u[e].z)), "f"(__uint_as_float(u[e].w))
-                                                 : "memory");
+                                    red_add_v4(acc + static_cast<size_t>(e) * p.H * DH + 16 * hf, __uint_as_float(u[e].x),
+                                               __uint_as_float(u[e].y), __uint_as_float(u[e].z), __uint_as_float(u[e].w));
                         }
                         __syncwarp();
                     }

@@ -61,3 +61,22 @@ def test_backward_items(B, S, N, H, D):
     got = run_layer(q, k, v, mask, bias, d_o)
     ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
     assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
+
+
+# ... and pairs of a row and a head past the last full round of the 148 SMs, dealt by segments after the whole ones
+@pytest.mark.parametrize("B,S,N,H,D", [
+    (1, 50, 200, 3, 32),     # 148 + 2; dQ of the whole ones stays in tensor memory
+    (1, 101, 136, 3, 64),    # 296 + 7
+    (1, 50, 264, 3, 32),     # 148 + 2, dQ of the whole ones goes through scratch
+    (1, 50, 392, 3, 64),
+    (2, 38, 520, 4, 16),     # 296 + 8
+    (1, 20, 200, 16, 32),    # 296 + 24: the first of the rest lies in the middle of a row
+    (1, 19, 264, 8, 64),     # 152: the accumulator of whole rows does not fit, so all by segments
+    (1, 38, 264, 4, 128),    # D = 128: all of them by segments
+    (150, 1, 200, 1, 64),    # one row: the same kernel also writes dBias
+])
+def test_backward_rest(B, S, N, H, D):
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=7 * S + N)
+    got = run_layer(q, k, v, mask, bias, d_o)
+    ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
+    assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
