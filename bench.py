@@ -40,7 +40,7 @@ import evo_workloads as wl  # noqa: E402
 
 # DRAM bytes per S row of one evo_bwd_kernel launch, from the ncu capture summarised under profiles/
 # (160.77 MB read + 53.59 MB written at 128 rows of cfg2).
-NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (160.77e6 + 53.59e6) / 128}
+NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.18e6 + 46.15e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"
 UNIT = "TFLOP/s"
@@ -444,7 +444,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "bytes_are": "per rank (the value is the whole job)",
                     "ms_per_step": ms_e2e / e2e_steps, "steps": e2e_steps},
-            "gpu_launches": 5 * args.steps,   # forward; backward: prep, dBias, dQ/dK/dV, dQ conversion
+            "gpu_launches": 5 * args.steps,   # forward; backward: prep, dBias, dQ/dK/dV, conversion of fp32 sums
             "graph_replay": bool(args.graph),
             "roofline": roofline,
         }
