@@ -22,6 +22,7 @@
 // S=300, N=600, H=8, D=96 1.11 -> 0.92.  Without turns on the exp2 pass the streams fall into step and queue
 // for the tensor core together (0.272); handing the turn on halfway through the pass 0.279.
 #pragma once
+#include "evo_bias_ring.cuh"
 
 namespace evo {
 
@@ -35,14 +36,15 @@ struct FwdWideCfg {
     static constexpr int REGS_SOFTMAX = 216, REGS_OTHER = 72;
     static_assert((REGS_SOFTMAX * NSW + REGS_OTHER * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
     static constexpr uint32_t ROWT = RowTile<DH>::BYTES;       // one [128][128] bf16 tile
-    static constexpr int NK = 2, NR = 3;                       // K buffers, half tiles of bias
+    static constexpr int NK = 2;                               // K buffers
+    static constexpr int NR = WideBiasRing::SLOTS, NF = WideBiasRing::PER_ROUND;   // half tiles of bias, their "full" barriers
     static constexpr uint32_t OFF_Q = 0, OFF_K = 2 * ROWT, OFF_V = OFF_K + NK * ROWT, OFF_BIAS = OFF_V + ROWT;
     static constexpr uint32_t OFF_XK = OFF_BIAS + NR * SQ_SUB_BYTES;
     // constant extra tiles, above every tile that refers to the zero tile
     static constexpr uint32_t OFF_XQ = OFF_XK + NK * XT_BYTES; // rows (1, 1, 1, 0, ...)
     static constexpr uint32_t OFF_ZERO = OFF_XQ + XT_BYTES;
     static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr int BARS = 3 * 2 + 1 + 2 * NK + 3 * 2 + 2 * NR + 16;
+    static constexpr int BARS = 3 * 2 + 1 + 2 * NK + 3 * 2 + NF + NR + 16;
     static constexpr uint32_t OFF_MISC = OFF_BARS + BARS * 8;
     static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;   // + alignment slack
     static constexpr uint32_t TMEM_S = 0, TMEM_PV = 256;       // + 128 s; P: 64 columns over S
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(FwdWideCfg::THREADS, 1)
 evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias, const FwdParams p) {
     using C = FwdWideCfg;
-    constexpr int DH = C::DH, NK = C::NK, NR = C::NR;
+    constexpr int DH = C::DH, NK = C::NK, NR = C::NR, NF = C::NF;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
 
@@ -72,8 +74,8 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     uint64_t* s_full = k_empty + NK;         // [stream]
     uint64_t* p_ready = s_full + 2;          // [stream]
     uint64_t* pv_done = p_ready + 2;         // [stream]
-    uint64_t* bias_full = pv_done + 2;       // [NR]
-    uint64_t* bias_empty = bias_full + NR;   // [NR]
+    uint64_t* bias_full = pv_done + 2;       // [NF]: half tile of the round (evo_bias_ring.cuh)
+    uint64_t* bias_empty = bias_full + NF;   // [NR]: slot
     uint64_t* turn = bias_empty + NR;        // [stream][tile parity][warp]: the warp has left its exp2 pass
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
     volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -95,7 +97,8 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         }
         mbar_init(v_empty, 2);
         for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], own ? 1 : 2); }
-        for (int i = 0; i < NR; ++i) { mbar_init(&bias_full[i], 1); mbar_init(&bias_empty[i], 4); }
+        for (int i = 0; i < NF; ++i) mbar_init(&bias_full[i], 1);
+        for (int i = 0; i < NR; ++i) mbar_init(&bias_empty[i], 4);
         for (int i = 0; i < 16; ++i) mbar_init(&turn[i], 1);
         fence_mbar_init();
     }
@@ -220,32 +223,33 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             // ------------------------------ bias ------------------------------
             FwdItem cur0 = items_of(0), cur1 = items_of(1);
             bool ok = true;
-            int slot = 0, use = 0;             // of half tile 4 r + 2 s + half
+            WideBiasRing ring = WideBiasRing::at(0);
             int n_loads = 0;
             for (int it = 0; it < n_items && ok; ++it) {
                 const FwdItem x0 = tile_of(cur0, 0), x1 = tile_of(own ? cur1 : cur0, 1);
                 for (int j = 0; j < NT && ok; ++j) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        if (ok && use > 0) ok = warp_all(mbar_wait(&bias_empty[slot], (use - 1) & 1, wc, 0x16));
+                        if (ok && ring.use > 0) ok = warp_all(mbar_wait(&bias_empty[ring.slot], ring.empty_parity(), wc, 0x16));
                         if (!ok) break;
                         const FwdItem& x = i < 2 ? x0 : x1;
+                        uint64_t* full = &bias_full[WideBiasRing::full_bar(i >> 1, i & 1)];
                         if (elect_one()) {
-                            mbar_arrive_expect_tx(&bias_full[slot], SQ_SUB_BYTES);
-                            tma_load_4d(smem + C::OFF_BIAS + slot * SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64 * (i & 1),
+                            mbar_arrive_expect_tx(full, SQ_SUB_BYTES);
+                            tma_load_4d(smem + C::OFF_BIAS + ring.slot * SQ_SUB_BYTES, &tm_bias, full, j * TILE + 64 * (i & 1),
                                         x.qt * TILE, x.h, x.b);
                         }
                         __syncwarp();
                         ++n_loads;
-                        if (++slot == NR) { slot = 0; ++use; }
+                        ring.advance(1);
                     }
                 }
                 advance(cur0);
                 advance(cur1);
             }
             const WaitCtx dc{tmem_slot + 3, p.status};
-            for (int i = (n_loads > NR ? n_loads - NR : 0); i < n_loads; ++i)
-                (void)mbar_wait(&bias_full[i % NR], (i / NR) & 1, dc, 0x17);
+            for (int i = (n_loads > NF ? n_loads - NF : 0); i < n_loads; ++i)
+                (void)mbar_wait(&bias_full[i % NF], WideBiasRing::full_parity(i / NF), dc, 0x17);
         } else {
             // ------------------------------ MMA warp of one stream ------------------------------
             const int s = warp - C::W_MMA;
@@ -322,13 +326,12 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const float2 sc2 = make_float2(p.scale, p.scale), l2e2 = make_float2(LOG2E, LOG2E);
         bool ok = true;
         int n = 0;
-        int slot = (2 * s) % NR;             // of half tile 4 n + 2 s, and how often the ring has come round
-        uint32_t use = 0;
+        WideBiasRing ring = WideBiasRing::at(2 * s);
         FwdItem cur = items_of(s);
         for (int it = 0; it < n_items && ok; ++it) {
             float m = -INFINITY, l = 0.f;
             for (int j = 0; j < NT; ++j, ++n) {
-                ok = warp_all(mbar_wait_both(&bias_full[slot], use & 1u, &s_full[s], n & 1, wc, 0x31));
+                ok = warp_all(mbar_wait_both(&bias_full[WideBiasRing::full_bar(s, 0)], WideBiasRing::full_parity(n), &s_full[s], n & 1, wc, 0x31));
                 if (!ok) break;
                 tc_fence_after();
                 // pass 1: x = S' * scale + bias and the row maximum, 32 columns at a time
@@ -340,12 +343,12 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 for (int ch = 0; ch < 4; ++ch) {
                     uint32_t (&cv)[32] = sv[ch & 1];
                     if (ch == 2) {
-                        ok = warp_all(mbar_wait(&bias_full[slot], use & 1u, wc, 0x32));
+                        ok = warp_all(mbar_wait(&bias_full[WideBiasRing::full_bar(s, 1)], WideBiasRing::full_parity(n), wc, 0x32));
                         if (!ok) break;
                     }
                     uint4 bv[4];
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) bv[q4] = lds128(aBias + slot * SQ_SUB_BYTES + sq_chunk_off(row, (ch & 1) * 4 + q4));
+                    for (int q4 = 0; q4 < 4; ++q4) bv[q4] = lds128(aBias + ring.slot * SQ_SUB_BYTES + sq_chunk_off(row, (ch & 1) * 4 + q4));
                     tmem_wait_ld();
                     if (ch < 3) tmem_ld32(tS + 32 * (ch + 1), sv[(ch + 1) & 1]);
 #pragma unroll
@@ -362,10 +365,8 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     if (ch & 1) {
                         // the maximum depends on every bias value read: the half tile may be refilled
                         const float dep = fmaxf(fmaxf(tmx[0], tmx[1]), fmaxf(tmx[2], tmx[3]));
-                        mbar_release_after_loads(&bias_empty[slot], __float_as_uint(dep), scratch_w);
-                        const int step = ch == 1 ? 1 : 3;          // to the other half, or past the other stream's two
-                        slot += step;
-                        if (slot >= NR) { slot -= NR; ++use; }
+                        mbar_release_after_loads(&bias_empty[ring.slot], __float_as_uint(dep), scratch_w);
+                        ring.advance(ch == 1 ? 1 : 3);             // to the other half, or past the other stream's two
                     }
                 }
                 if (!ok) break;
