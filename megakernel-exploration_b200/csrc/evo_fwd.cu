@@ -169,6 +169,11 @@ __device__ __forceinline__ uint2 split3_bf16(float v) {
     return make_uint2(pack_bf16(a, b), c);
 }
 
+// Largest |m| of a row for which exponentials take x log2e - m log2e as one multiply-add: m log2e, rounded, is then off
+// by less than 2^-12.  Larger are a row, or the tiles of it so far, all masked by additive terms like -1e9 or -1e30
+// (there the rounding alone would be 64, or more than any exponent).
+constexpr float FWD_FAR = 4096.f;
+
 // GATED: the epilogue also writes sigmoid(gate) * O.  tm_2: the rounding residual (GATED: the gated output).
 template <int DH, bool GATED>
 __global__ void __launch_bounds__(FwdCfg<DH>::THREADS, 1)
@@ -552,7 +557,10 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const float m_old = m;
                 m = m_new;
                 const float ms = (m == -INFINITY) ? 0.f : m;
-                const float nm = -ms * LOG2E;
+                // Exponentials are of x log2e - m log2e, or, with an m so far out that the rounding of m log2e would
+                // show (1e-3 and up), of (x - m) log2e.
+                const float sub = fabsf(ms) > FWD_FAR ? ms : 0.f;
+                const float nm = sub != 0.f ? 0.f : -ms * LOG2E;
                 if constexpr (C::HOLD) {
                     // P's columns are free and the accumulator is at rest once the previous PV is complete
                     if (n > 0) {
@@ -562,7 +570,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                 }
                 if (__any_sync(0xffffffffu, need)) {
-                    const float alpha = need ? ex2(fmaf(m_old, LOG2E, nm)) : 1.0f;
+                    const float alpha = need ? ex2(fmaf(m_old - sub, LOG2E, nm)) : 1.0f;
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
@@ -578,6 +586,27 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         tmem_st32(tPV + c * 32, r);
                     }
                     l *= alpha;
+                }
+                if (__any_sync(0xffffffffu, sub != 0.f)) {
+                    const float2 sub2 = make_float2(-sub, -sub);
+                    if constexpr (C::HOLD) {
+#pragma unroll
+                        for (int i = 0; i < 64; ++i) xh[i] = fadd2(xh[i], sub2);
+                    } else {
+                        tmem_wait_st();                 // x is written
+#pragma unroll 1
+                        for (int c = 0; c < 4; ++c) {
+                            tmem_ld32(tS + c * 32, sv[0]);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; i += 2) {
+                                const float2 v2 = fadd2(u2f2(sv[0][i], sv[0][i + 1]), sub2);
+                                sv[0][i] = __float_as_uint(v2.x);
+                                sv[0][i + 1] = __float_as_uint(v2.y);
+                            }
+                            tmem_st32(tS + c * 32, sv[0]);
+                        }
+                    }
                 }
                 take_turn();
                 if (!ok) break;

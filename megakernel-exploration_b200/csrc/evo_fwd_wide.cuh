@@ -378,10 +378,13 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const float m_old = m;
                 m = m_new;
                 const float ms = (m == -INFINITY) ? 0.f : m;
-                const float nm = -ms * LOG2E;
+                // Exponentials are of x log2e - m log2e, or, with an m so far out that the rounding of m log2e would
+                // show (1e-3 and up), of (x - m) log2e.
+                const float sub = fabsf(ms) > FWD_FAR ? ms : 0.f;
+                const float nm = sub != 0.f ? 0.f : -ms * LOG2E;
                 if (__any_sync(0xffffffffu, need)) {
                     // (the accumulator is at rest: S' of this tile followed PV of the one before)
-                    const float alpha = need ? ex2(fmaf(m_old, LOG2E, nm)) : 1.0f;
+                    const float alpha = need ? ex2(fmaf(m_old - sub, LOG2E, nm)) : 1.0f;
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
@@ -397,6 +400,11 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                         tmem_st32(tPV + c * 32, r);
                     }
                     l *= alpha;
+                }
+                if (__any_sync(0xffffffffu, sub != 0.f)) {
+                    const float2 sub2 = make_float2(-sub, -sub);
+#pragma unroll
+                    for (int i = 0; i < 64; ++i) xh[i] = fadd2(xh[i], sub2);
                 }
                 // The streams take turns on the exp2 pass, scheduler by scheduler, so that one is in it while the
                 // other is in its products and sums: stream 1 after stream 0's pass of this tile, stream 0 after

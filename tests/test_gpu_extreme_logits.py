@@ -1,0 +1,57 @@
+"""Logits at the ends of their range: rows, or leading tiles of rows, masked by large finite terms, by the type's lowest
+value and by -inf; NaN and +inf in one place.  What is expected is the softmax in 64 bits on the rounded inputs."""
+import pytest
+import torch
+
+from oracle import evo_ref
+from _util import bf16_round
+
+pytestmark = pytest.mark.gpu
+
+# head dims of the three forward kernels; one tile, a ragged second one, three
+SHAPES = [(N, D) for D in (16, 32, 64, 96, 128) for N in (64, 136, 264)]
+B, S, H = 1, 4, 3
+
+
+def _inputs(N, D):
+    q, k, v, _, bias, _ = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "valid", seed=N + D)
+    return bf16_round(q, k, v, torch.zeros(B, S, 1, 1, N), bias)
+
+
+def _out(q, k, v, mask, bias):
+    from tk_evo_attention_layer import TKEvoAttention
+    import _evoattn
+    c = lambda t: t.cuda().to(torch.bfloat16)
+    o = TKEvoAttention.apply(c(q), c(k), c(v), c(mask), c(bias)).float().cpu()
+    _evoattn.device_status()
+    return o
+
+
+def _ref(q, k, v, mask, bias):
+    # sums in fp32, where a term of -1e30 absorbs the logit it is added to, then 64 bits
+    return evo_ref.evo_attention_ref(q, k, v, mask, bias).double()
+
+
+def _close(o, ref):
+    # a bf16 output with bf16 P against values of order one: two bf16 steps of the largest
+    assert torch.isfinite(o).all()
+    assert (o.double() - ref).abs().max() <= 2.0 ** -7 * max(1.0, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("N,D", SHAPES)
+@pytest.mark.parametrize("low", [-1e10, -1e30, -1e36])
+def test_masked_by_large_terms(N, D, low):
+    """Every residue of a row masked: the mean of V; the first tile masked: the softmax over the rest.  Through the mask and
+    through the pair bias."""
+    q, k, v, mask, bias = _inputs(N, D)
+    low = torch.tensor(low).to(torch.bfloat16).float().item()
+    m = mask.clone()
+    m[:, 0] = low                           # row 0: nothing left
+    m[:, 1, ..., :min(N - 8, 128)] = low    # row 1: the first tile (or all but eight residues) masked
+    o = _out(q, k, v, m, bias)
+    _close(o, _ref(q, k, v, m, bias))
+    b = bias.clone()
+    b[..., 3, :] = low                      # query 3: nothing left
+    b[..., 5, :min(N - 8, 128)] = low
+    o = _out(q, k, v, mask, b)
+    _close(o, _ref(q, k, v, mask, b))
