@@ -83,7 +83,7 @@ struct FwdParams {
 //
 // The mask rides in an extra contraction block (evo_tiles.cuh, "EXTRA TILE"): the producer turns 128
 // mask values into a [128][8] tile (m/scale in three bf16 parts, exact to fp32), columns past N get
-// -1e38.  The base of the exponentials: x in natural units, P = exp2(x log2e - m log2e).
+// -inf.  The base of the exponentials: x in natural units, P = exp2(x log2e - m log2e).
 // ---------------------------------------------------------------------------
 template <int DH>
 struct FwdCfg {
@@ -160,12 +160,16 @@ struct FwdItem {
     __device__ __forceinline__ int bs(const FwdParams& p) const { return b * p.S + row; }
 };
 
-// v as three bf16 parts (24 significant bits), in the layout of words 0 and 1 of an extra-tile row
-__device__ __forceinline__ uint2 split3_bf16(float v) {
-    v = fminf(fmaxf(v, -1e38f), 1e38f);
+// Mask value m, divided by the scale, as three bf16 parts (24 significant bits), in the layout of words 0 and 1 of an
+// extra-tile row.  A finite one stays finite, so that every mask that a type can hold ranks above the -inf of the columns
+// past N (a row of which nothing else is left is then the mean of its N values); infinities and NaN go through.
+__device__ __forceinline__ uint2 mask_term(float m, float inv_scale) {
+    const bool finite = fabsf(m) < INFINITY;
+    const float v = finite ? fminf(fmaxf(m * inv_scale, -3e38f), 3e38f) : m;
     const float a = __bfloat162float(__float2bfloat16_rn(v));
-    const float b = __bfloat162float(__float2bfloat16_rn(v - a));
-    const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn((v - a) - b));
+    const float r = finite ? v - a : 0.f;
+    const float b = __bfloat162float(__float2bfloat16_rn(r));
+    const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn(r - b));
     return make_uint2(pack_bf16(a, b), c);
 }
 
@@ -301,7 +305,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         const float mv[4] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y)};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
-                            const uint2 w = split3_bf16(c < p.N ? mv[e] * p.inv_scale : -1e38f);
+                            const uint2 w = mask_term(c < p.N ? mv[e] : -INFINITY, p.inv_scale);
                             *reinterpret_cast<uint4*>(sb + C::ST_XK + kb * XT_BYTES + (4 * lane + e) * 16) = make_uint4(w.x, w.y, 0u, 0u);
                         }
                         fence_async_smem();
@@ -653,8 +657,9 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // epilogue of the item; what does not need the last PV comes before the wait for it
             const int bs = cur.bs(p), qt = cur.qt, h = cur.h;
             const int qrow = qt * TILE + row;
-            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ((m == -INFINITY) ? 0.f : m) + __logf(l);
-            const float inv = __frcp_rn(l);
+            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = (m == -INFINITY) ? m : m + __logf(l);
+            // (a row of which every logit is -inf has no softmax: NaN, and a log-sum-exp of -inf)
+            const float inv = (m == -INFINITY) ? __int_as_float(0x7fffffff) : __frcp_rn(l);
             advance(cur, s);
             // Results go through shared memory (row r of a tile: 16-byte chunks, swizzled as the tensor map says)
             // and out by TMA, issued by the MMA warp.

@@ -167,7 +167,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const float mv[4] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y)};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const uint2 w = split3_bf16(c < p.N ? mv[e] * p.inv_scale : -1e38f);
+                    const uint2 w = mask_term(c < p.N ? mv[e] : -INFINITY, p.inv_scale);
                     *reinterpret_cast<uint4*>(smem + C::OFF_XK + kb * XT_BYTES + (4 * lane + e) * 16) = make_uint4(w.x, w.y, 0u, 0u);
                 }
                 fence_async_smem();
@@ -445,8 +445,8 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             // epilogue of the item; what does not need the last PV comes before the wait for it
             const FwdItem x = tile_of(cur, s);
             const int bs = x.bs(p), h = x.h, qrow = x.qt * TILE + row;
-            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = ((m == -INFINITY) ? 0.f : m) + __logf(l);
-            const float inv = __frcp_rn(l);
+            if (qrow < p.N) p.lse[(static_cast<size_t>(bs) * p.H + h) * p.N + qrow] = (m == -INFINITY) ? m : m + __logf(l);
+            const float inv = (m == -INFINITY) ? __int_as_float(0x7fffffff) : __frcp_rn(l);     // no logit above -inf: NaN
             advance(cur);
             // lane t of a quad of rows stores chunk t of each of the four: 64 contiguous bytes per row
             const int qrow0 = x.qt * TILE + (row & ~3);

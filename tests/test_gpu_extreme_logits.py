@@ -55,3 +55,34 @@ def test_masked_by_large_terms(N, D, low):
     b[..., 5, :min(N - 8, 128)] = low
     o = _out(q, k, v, mask, b)
     _close(o, _ref(q, k, v, mask, b))
+
+
+@pytest.mark.parametrize("N,D", SHAPES)
+@pytest.mark.parametrize("low", [-1e38, -2e38, torch.finfo(torch.bfloat16).min])
+def test_masked_by_lowest(N, D, low):
+    """The padding of a ragged tile ranks below every finite mask: a row masked as far as bf16 goes is the mean of its N values."""
+    q, k, v, mask, bias = _inputs(N, D)
+    m = mask.clone()
+    m[:, 0] = torch.tensor(low).to(torch.bfloat16).float()
+    o = _out(q, k, v, m, torch.zeros_like(bias))
+    _close(o[:, 0], v[:, 0].double().mean(1, keepdim=True).expand(B, N, H, D))
+    _close(o[:, 1:], _ref(q, k, v, mask, torch.zeros_like(bias))[:, 1:])
+
+
+@pytest.mark.parametrize("N,D", SHAPES)
+def test_masked_by_infinity(N, D):
+    """-inf in the mask or the pair bias: excluded; a row or query with nothing else has no softmax and is NaN, no other is."""
+    q, k, v, mask, bias = _inputs(N, D)
+    ninf = float("-inf")
+    m = mask.clone()
+    m[:, 0] = ninf
+    m[:, 1, ..., :min(N - 8, 128)] = ninf
+    b = bias.clone()
+    b[..., 3, :] = ninf
+    b[..., 5, :min(N - 8, 128)] = ninf
+    ref = _ref(q, k, v, m, b)
+    gone = ref.isnan()
+    assert gone[:, 0].all() and gone[:, :, 3].all() and not gone[:, 1:, 5].any()
+    o = _out(q, k, v, m, b)
+    assert torch.equal(o.isnan(), gone)
+    _close(o[~gone], ref[~gone])
