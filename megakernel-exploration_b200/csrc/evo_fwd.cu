@@ -164,19 +164,20 @@ struct FwdItem {
 // extra-tile row.  A finite one stays finite, so that every mask that a type can hold ranks above the -inf of the columns
 // past N (a row of which nothing else is left is then the mean of its N values); infinities and NaN go through.
 __device__ __forceinline__ uint2 mask_term(float m, float inv_scale) {
-    const bool finite = fabsf(m) < INFINITY;
-    const float v = finite ? fminf(fmaxf(m * inv_scale, -3e38f), 3e38f) : m;
+    const float v = fmaxf(m * inv_scale, -3e38f);
     const float a = __bfloat162float(__float2bfloat16_rn(v));
-    const float r = finite ? v - a : 0.f;
-    const float b = __bfloat162float(__float2bfloat16_rn(r));
-    const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn(r - b));
+    const float b = __bfloat162float(__float2bfloat16_rn(v - a));
+    // (2^-60 m is nothing beside the third part of a finite m, and all of an infinite one)
+    const uint32_t c = __bfloat16_as_ushort(__float2bfloat16_rn(fmaf(m, 8.67361738e-19f, (v - a) - b)));
     return make_uint2(pack_bf16(a, b), c);
 }
 
-// Largest |m| of a row for which exponentials take x log2e - m log2e as one multiply-add: m log2e, rounded, is then off
-// by less than 2^-12.  Larger are a row, or the tiles of it so far, all masked by additive terms like -1e9 or -1e30
-// (there the rounding alone would be 64, or more than any exponent).
-constexpr float FWD_FAR = 4096.f;
+// From this |m| of a row on (one, or the tiles of it so far, all masked by terms like -1e9 or -1e30) m log2e, rounded, is
+// off by 32 and more, and 2^(x log2e - m log2e) no exponential of x - m any longer.  But there the logits are multiples
+// of 32, so that all below m get nothing, whatever the base: with 2 instead of e, x - m is exact.
+// (Kernel alone, without any of it / this / x - m formed first in a branch for such rows: B=1, S=256, N=1024, H=4, D=64
+// 0.587 / 0.593 / 0.688 ms; S=512, N=384, H=8, D=32 0.288 / 0.291 / 0.299.)
+constexpr float FWD_FAR = 536870912.f;         // 2^29
 
 // GATED: the epilogue also writes sigmoid(gate) * O.  tm_2: the rounding residual (GATED: the gated output).
 template <int DH, bool GATED>
@@ -470,7 +471,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
         const uint32_t tS = lane_base + C::TMEM_S + 128 * s, tPV = lane_base + C::TMEM_PV + DH * s, tP = lane_base + C::p_col(s);
         const uint32_t scratch_w = smem_u32(tmem_slot + 2);           // a word nobody reads
-        const float2 sc2 = make_float2(p.scale, p.scale), l2e2 = make_float2(LOG2E, LOG2E);
+        const float2 sc2 = make_float2(p.scale, p.scale);
         // The exp2 pass loads the special-function unit, the passes around it the other pipes.  Left alone
         // the warps of a scheduler fall into step, all in the same pass at the same time; so the streams
         // take turns on it, scheduler by scheduler, and a warp hands its turn on halfway through the pass (a
@@ -561,10 +562,10 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const float m_old = m;
                 m = m_new;
                 const float ms = (m == -INFINITY) ? 0.f : m;
-                // Exponentials are of x log2e - m log2e, or, with an m so far out that the rounding of m log2e would
-                // show (1e-3 and up), of (x - m) log2e.
-                const float sub = fabsf(ms) > FWD_FAR ? ms : 0.f;
-                const float nm = sub != 0.f ? 0.f : -ms * LOG2E;
+                // Exponentials are 2^(x le - m le), one multiply-add each.  le is log2e, or 1 where |m| is so large that the
+                // logits lie 32 and more apart (FWD_FAR).
+                const float le = fabsf(m) < FWD_FAR ? LOG2E : 1.f;
+                const float nm = -ms * le;
                 if constexpr (C::HOLD) {
                     // P's columns are free and the accumulator is at rest once the previous PV is complete
                     if (n > 0) {
@@ -574,7 +575,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                 }
                 if (__any_sync(0xffffffffu, need)) {
-                    const float alpha = need ? ex2(fmaf(m_old - sub, LOG2E, nm)) : 1.0f;
+                    const float alpha = need ? ex2(fmaf(m_old, le, nm)) : 1.0f;
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
@@ -591,31 +592,10 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                     l *= alpha;
                 }
-                if (__any_sync(0xffffffffu, sub != 0.f)) {
-                    const float2 sub2 = make_float2(-sub, -sub);
-                    if constexpr (C::HOLD) {
-#pragma unroll
-                        for (int i = 0; i < 64; ++i) xh[i] = fadd2(xh[i], sub2);
-                    } else {
-                        tmem_wait_st();                 // x is written
-#pragma unroll 1
-                        for (int c = 0; c < 4; ++c) {
-                            tmem_ld32(tS + c * 32, sv[0]);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const float2 v2 = fadd2(u2f2(sv[0][i], sv[0][i + 1]), sub2);
-                                sv[0][i] = __float_as_uint(v2.x);
-                                sv[0][i + 1] = __float_as_uint(v2.y);
-                            }
-                            tmem_st32(tS + c * 32, sv[0]);
-                        }
-                    }
-                }
                 take_turn();
                 if (!ok) break;
                 // pass 2: P = exp2(x log2e - m log2e), row sum, bf16 pairs into tensor memory
-                const float2 nm2 = make_float2(nm, nm);
+                const float2 nm2 = make_float2(nm, nm), le2 = make_float2(le, le);
                 float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
                 if constexpr (!C::HOLD) {
                     tmem_wait_st();                     // x is written
@@ -632,7 +612,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     for (int k = 0; k < 16; ++k) {
                         const float2 x = C::HOLD ? xh[C::HOLD ? ch * 16 + k : 0]
                                                  : u2f2(sv[ch & 1][2 * k], sv[ch & 1][2 * k + 1]);
-                        const float2 d2 = ffma2(x, l2e2, nm2);
+                        const float2 d2 = ffma2(x, le2, nm2);
                         const float2 p2 = use_poly<C::POLY_EVERY>(k) ? ex2_poly2<5>(d2) : make_float2(ex2(d2.x), ex2(d2.y));
                         rs[k & 1] = fadd2(rs[k & 1], p2);
                         pk[k] = pack_bf16(p2.x, p2.y);

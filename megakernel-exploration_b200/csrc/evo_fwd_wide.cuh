@@ -323,7 +323,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         const uint32_t tS = lane_base + C::TMEM_S + 128 * s, tPV = lane_base + C::TMEM_PV + DH * s;
         const uint32_t scratch_w = smem_u32(tmem_slot + 2);           // a word nobody reads
         const uint32_t aBias = smem_u32(smem + C::OFF_BIAS);
-        const float2 sc2 = make_float2(p.scale, p.scale), l2e2 = make_float2(LOG2E, LOG2E);
+        const float2 sc2 = make_float2(p.scale, p.scale);
         bool ok = true;
         int n = 0;
         WideBiasRing ring = WideBiasRing::at(2 * s);
@@ -378,13 +378,13 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 const float m_old = m;
                 m = m_new;
                 const float ms = (m == -INFINITY) ? 0.f : m;
-                // Exponentials are of x log2e - m log2e, or, with an m so far out that the rounding of m log2e would
-                // show (1e-3 and up), of (x - m) log2e.
-                const float sub = fabsf(ms) > FWD_FAR ? ms : 0.f;
-                const float nm = sub != 0.f ? 0.f : -ms * LOG2E;
+                // Exponentials are 2^(x le - m le), one multiply-add each.  le is log2e, or 1 where |m| is so large that the
+                // logits lie 32 and more apart (FWD_FAR).
+                const float le = fabsf(m) < FWD_FAR ? LOG2E : 1.f;
+                const float nm = -ms * le;
                 if (__any_sync(0xffffffffu, need)) {
                     // (the accumulator is at rest: S' of this tile followed PV of the one before)
-                    const float alpha = need ? ex2(fmaf(m_old - sub, LOG2E, nm)) : 1.0f;
+                    const float alpha = need ? ex2(fmaf(m_old, le, nm)) : 1.0f;
                     const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
@@ -401,11 +401,6 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     }
                     l *= alpha;
                 }
-                if (__any_sync(0xffffffffu, sub != 0.f)) {
-                    const float2 sub2 = make_float2(-sub, -sub);
-#pragma unroll
-                    for (int i = 0; i < 64; ++i) xh[i] = fadd2(xh[i], sub2);
-                }
                 // The streams take turns on the exp2 pass, scheduler by scheduler, so that one is in it while the
                 // other is in its products and sums: stream 1 after stream 0's pass of this tile, stream 0 after
                 // stream 1's of the one before.
@@ -413,14 +408,14 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 if (t >= 0) ok = warp_all(mbar_wait(&turn[8 * (s ^ 1) + 4 * (t & 1) + (warp & 3)], (t >> 1) & 1, wc, 0x38));
                 if (!ok) break;
                 // pass 2: P = exp2(x log2e - m log2e), row sum, bf16 pairs over the S columns
-                const float2 nm2 = make_float2(nm, nm);
+                const float2 nm2 = make_float2(nm, nm), le2 = make_float2(le, le);
                 float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch) {
                     uint32_t pk[16];
 #pragma unroll
                     for (int k = 0; k < 16; ++k) {
-                        const float2 d2 = ffma2(xh[ch * 16 + k], l2e2, nm2);
+                        const float2 d2 = ffma2(xh[ch * 16 + k], le2, nm2);
                         const float2 p2 = make_float2(ex2(d2.x), ex2(d2.y));
                         rs[k & 1] = fadd2(rs[k & 1], p2);
                         pk[k] = pack_bf16(p2.x, p2.y);
