@@ -535,7 +535,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         for (int e = 0; e < 4; ++e) {
                             const int k = q4 * 4 + e;
                             const float2 x = ffma2(u2f2(cv[2 * k], cv[2 * k + 1]), sc2, bf16x2_f2(bw[e]));
-                            tmx[e] = fmax3(tmx[e], x.x, x.y);
+                            tmx[e] = fmax3_nan(tmx[e], x.x, x.y);
                             if constexpr (C::HOLD) {
                                 xh[ch * 16 + k] = x;
                             } else {
@@ -546,7 +546,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                     if constexpr (!C::HOLD) tmem_st32(tS + 32 * ch, cv);
                 }
-                const float tmax = fmaxf(fmaxf(tmx[0], tmx[1]), fmaxf(tmx[2], tmx[3]));
+                const float tmax = fmax_nan(fmax3_nan(tmx[0], tmx[1], tmx[2]), tmx[3]);
                 if constexpr (C::HOLD) {
                     tc_fence_before();
                     __syncwarp();
@@ -557,14 +557,16 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
                 // the exact online softmax: the largest P of a row is exp2(0) = 1, which bf16 represents
                 // exactly.  When the maximum rises, accumulator and row sum are rescaled.
-                const float m_new = fmaxf(m, tmax);
+                const float m_new = fmax_nan(m, tmax);
                 const bool need = (j > 0) && (m_new > m);
                 const float m_old = m;
                 m = m_new;
                 const float ms = (m == -INFINITY) ? 0.f : m;
                 // Exponentials are 2^(x le - m le), one multiply-add each.  le is log2e, or 1 where |m| is so large that the
                 // logits lie 32 and more apart (FWD_FAR).
-                const float le = fabsf(m) < FWD_FAR ? LOG2E : 1.f;
+                // (NaN or +inf among the logits makes m so, and with le = 0 all exponentials NaN, whichever columns they are in: those
+                // that the polynomial takes would drop a NaN of their own)
+                const float le = fabsf(m) < FWD_FAR ? LOG2E : (C::POLY_EVERY == 0 || m < INFINITY ? 1.f : 0.f);
                 const float nm = -ms * le;
                 if constexpr (C::HOLD) {
                     // P's columns are free and the accumulator is at rest once the previous PV is complete

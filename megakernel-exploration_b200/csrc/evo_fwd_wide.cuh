@@ -358,22 +358,22 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                         for (int e = 0; e < 4; ++e) {
                             const int k = q4 * 4 + e;
                             const float2 x = ffma2(u2f2(cv[2 * k], cv[2 * k + 1]), sc2, bf16x2_f2(bw[e]));
-                            tmx[e] = fmax3(tmx[e], x.x, x.y);
+                            tmx[e] = fmax3_nan(tmx[e], x.x, x.y);
                             xh[ch * 16 + k] = x;
                         }
                     }
                     if (ch & 1) {
                         // the maximum depends on every bias value read: the half tile may be refilled
-                        const float dep = fmaxf(fmaxf(tmx[0], tmx[1]), fmaxf(tmx[2], tmx[3]));
+                        const float dep = fmax_nan(fmax3_nan(tmx[0], tmx[1], tmx[2]), tmx[3]);
                         mbar_release_after_loads(&bias_empty[ring.slot], __float_as_uint(dep), scratch_w);
                         ring.advance(ch == 1 ? 1 : 3);             // to the other half, or past the other stream's two
                     }
                 }
                 if (!ok) break;
-                const float tmax = fmaxf(fmaxf(tmx[0], tmx[1]), fmaxf(tmx[2], tmx[3]));
+                const float tmax = fmax_nan(fmax3_nan(tmx[0], tmx[1], tmx[2]), tmx[3]);
                 // the exact online softmax: the largest P of a row is exp2(0) = 1, which bf16 represents
                 // exactly.  When the maximum rises, accumulator and row sum are rescaled.
-                const float m_new = fmaxf(m, tmax);
+                const float m_new = fmax_nan(m, tmax);
                 const bool need = (j > 0) && (m_new > m);
                 const float m_old = m;
                 m = m_new;

@@ -554,7 +554,7 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 2^x for x <= 0 (any magnitude, -inf included) on the fused-multiply-add pipe instead of
+// 2^x for x <= 0 (any magnitude, -inf included; NaN, which the lower bound drops, is the caller's business) on the fused-multiply-add pipe instead of
 // the special-function unit, two values at a time: x = n + f with n = round(x), f in
 // [-0.5, 0.5]; 2^f by a polynomial that minimises the largest relative error (least squares on
 // Chebyshev nodes, reweighted): degree 3 7.5e-5, far below a bf16 rounding; degree 5 2.3e-7, what
@@ -601,13 +601,18 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
-// Packed fp32 pairs (one instruction, two lanes of work) and the three-input maximum.
+// Packed fp32 pairs (one instruction, two lanes of work) and maxima that are NaN if an input is.
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
+__device__ __forceinline__ float fmax3_nan(float a, float b, float c) {
     float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float fmax_nan(float a, float b) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
     return d;
 }
 __device__ __forceinline__ float2 bf16x2_f2(uint32_t w) { return make_float2(bf16_lo(w), bf16_hi(w)); }

@@ -86,3 +86,29 @@ def test_masked_by_infinity(N, D):
     o = _out(q, k, v, m, b)
     assert torch.equal(o.isnan(), gone)
     _close(o[~gone], ref[~gone])
+
+
+@pytest.mark.parametrize("N,D", SHAPES)
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nan_and_inf_show(N, D, bad):
+    """One NaN or +inf in the pair bias (any column residue mod 8, as pairs of columns take different routes through the exponential),
+    in the mask or in K makes NaN of the queries that see it, and of no other."""
+    q, k, v, mask, bias = _inputs(N, D)
+    b = bias.clone()
+    for c in range(8):
+        b[:, :, :, 2 * c, N - 8 + c] = bad      # query 2 c, in the last tile
+        b[:, :, :, 2 * c + 17, c] = bad         # ... in the first
+    o = _out(q, k, v, mask, b)
+    hit = sorted([2 * c for c in range(8)] + [2 * c + 17 for c in range(8)])
+    assert o[:, :, hit].isnan().all()
+    rest = [i for i in range(N) if i not in hit]
+    _close(o[:, :, rest], _ref(q, k, v, mask, bias)[:, :, rest])
+    for c in (0, 6):
+        m = mask.clone()
+        m[:, 2, ..., N - 8 + c] = bad
+        o = _out(q, k, v, m, bias)
+        assert o[:, 2].isnan().all() and torch.isfinite(o[:, :2]).all() and torch.isfinite(o[:, 3:]).all()
+    k2 = k.clone()
+    k2[:, 1, 7, 1, 3] = float("nan")
+    o = _out(q, k2, v, mask, bias)
+    assert o[:, 1, :, 1].isnan().all() and torch.isfinite(o[:, 0]).all() and torch.isfinite(o[:, 1, :, 0]).all()
