@@ -194,9 +194,8 @@ struct EvoBackward : public torch::autograd::Node {
     }
 };
 
-// bias16: pair_bias itself if it is bf16, else its bf16 copy (the caller casts once per version of the tensor).
 std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& res_mask, const Tensor& pair_bias,
-                            const Tensor& bias16, const std::optional<Tensor>& gate) {
+                            const std::optional<Tensor>& gate) {
     if (Q.dim() != 5 || !Q.is_cuda()) return std::nullopt;
     const auto sz = Q.sizes();
     const int64_t B = sz[0], S = sz[1], N = sz[2], H = sz[3], D = sz[4];
@@ -204,8 +203,7 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
     if (res_mask.sizes() != at::IntArrayRef({B, S, 1, 1, N}) || pair_bias.sizes() != at::IntArrayRef({B, 1, H, N, N})) return std::nullopt;
     if (gate && gate->sizes() != sz) return std::nullopt;
     const auto dev = Q.device();
-    if (K.device() != dev || V.device() != dev || res_mask.device() != dev || pair_bias.device() != dev || bias16.device() != dev)
-        return std::nullopt;
+    if (K.device() != dev || V.device() != dev || res_mask.device() != dev || pair_bias.device() != dev) return std::nullopt;
     if (gate && gate->device() != dev) return std::nullopt;
     if (B > INT32_MAX || S > INT32_MAX || N > INT32_MAX || H > INT32_MAX) return std::nullopt;
 
@@ -223,7 +221,7 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
             c.k = bf16_contiguous(K);
             c.v = bf16_contiguous(V);
         }
-        c.bias = bf16_contiguous(bias16);      // the caller's cast of an fp32 bias, or the bf16 bias itself
+        c.bias = bf16_contiguous(pair_bias);
         c.mask = bf16_contiguous(res_mask);
         if (!aligned(c.q) || !aligned(c.k) || !aligned(c.v) || !aligned(c.bias) || !aligned(c.mask)) return std::nullopt;
         if (gate) c.gate = as_output(*gate, c.q, c.lay);

@@ -99,22 +99,22 @@ def _bf16c(x: torch.Tensor) -> torch.Tensor:
     return x.contiguous()
 
 
-# bf16 copies of fp32 pair-bias tensors: a model calls the layer with the same pair bias for every
-# block of a stack and, in evaluation, for every step, and the fp32 -> bf16 cast is the single largest
-# cost the reference measured around its forward (evo_h100/README.md:655-669).  An entry is served only
-# to the very tensor object it was made from (held by weak reference, so a new tensor that happens to
-# reuse the address of a freed one never matches) and only while its version counter, which every
-# in-place write bumps, is unchanged.
+# bf16 copies of fp32 pair-bias tensors in host memory.  An entry is served only to the very tensor object it was made
+# from (held by weak reference, so a new tensor that happens to reuse the address of a freed one never
+# matches) and only while its version counter, which every in-place write bumps, is unchanged.  On a GPU every call
+# casts: a kept copy would be read on streams that do not wait for the one that wrote it, would be missing from (or,
+# made during its capture, filled only by) a CUDA graph, and would miss writes through .data and by other libraries'
+# kernels, which leave the version counter alone.  A caller that uses one fp32 bias many times casts it once itself.
 _BIAS_CACHE: "dict[int, tuple]" = {}
 _BIAS_CACHE_MAX = 8
 
 
 def _bias_bf16(pair_bias: torch.Tensor, B: int, H: int, N: int) -> torch.Tensor:
-    """pair_bias (B, 1, H, N, N) as a contiguous bf16 (B, H, N, N) tensor, cast at most once per version."""
+    """pair_bias (B, 1, H, N, N) as a contiguous bf16 (B, H, N, N) tensor; in host memory cast at most once per version."""
     import weakref
     pb = pair_bias.reshape(B, H, N, N)
-    if pb.dtype == torch.bfloat16:
-        return pb.contiguous()
+    if pb.dtype == torch.bfloat16 or pair_bias.is_cuda or pair_bias.is_inference():     # (no version counter in inference mode)
+        return _bf16c(pb)
     key = id(pair_bias)
     hit = _BIAS_CACHE.get(key)
     if hit is not None and hit[0]() is pair_bias and hit[1] == pair_bias._version:
@@ -222,14 +222,9 @@ class TKEvoAttention(torch.autograd.Function):
     def apply(cls, *args):
         if (5 <= len(args) <= 7 and (len(args) == 5 or args[5] is None)
                 and isinstance(args[0], torch.Tensor) and args[0].is_cuda):
-            Q, K, V, res_mask, pair_bias = args[:5]
-            if Q.dim() == 5 and pair_bias.dim() == 5:
-                bias = _bias_bf16(pair_bias, Q.shape[0], Q.shape[3], Q.shape[2]) \
-                    if pair_bias.dtype != torch.bfloat16 and pair_bias.shape == (Q.shape[0], 1, Q.shape[3], Q.shape[2], Q.shape[2]) \
-                    else pair_bias
-                out = _native()(Q, K, V, res_mask, pair_bias, bias, args[6] if len(args) == 7 else None)
-                if out is not None:
-                    return out
+            out = _native()(*args[:5], args[6] if len(args) == 7 else None)
+            if out is not None:
+                return out
         return super().apply(*args)
 
     @staticmethod

@@ -1,0 +1,57 @@
+"""What the operator shares with other torch operators besides its values: fresh inputs, autograd's edges, other modes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+B, S, N, H, D = 1, 4, 64, 2, 32
+# the second head dim is padded by the layer and takes the Python host path
+HEAD_DIMS = (32, 24)
+
+
+def _inputs(d=D, seed=3):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)
+    return r(B, S, N, H, d), r(B, S, N, H, d), r(B, S, N, H, d), torch.zeros(B, S, 1, 1, N, device="cuda"), r(B, 1, H, N, N)
+
+
+def _apply(*a):
+    from tk_evo_attention_layer import TKEvoAttention
+    return TKEvoAttention.apply(*a)
+
+
+@pytest.mark.parametrize("d", HEAD_DIMS)
+def test_fp32_bias_is_read_anew(d):
+    """A pair bias of another type is cast on every call: after a write that bumps no version counter, in inference mode, on
+    another stream than that of an earlier call, and in a CUDA graph."""
+    q, k, v, m, b = _inputs(d)
+    b2 = _inputs(d, seed=4)[4]
+    want, want2 = _apply(q, k, v, m, b), _apply(q, k, v, m, b2)
+    assert not torch.equal(want, want2)
+    f = b.float()
+    assert torch.equal(_apply(q, k, v, m, f), want)
+    f.data.copy_(b2)
+    assert torch.equal(_apply(q, k, v, m, f), want2)
+    with torch.inference_mode():
+        assert torch.equal(_apply(q, k, v, m, b.float()), want)
+    # the copy of the first call is still in the making when the second stream reads the same tensor
+    f.copy_(b)
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(20_000_000)
+        o1 = _apply(q, k, v, m, f)
+    with torch.cuda.stream(two):
+        o2 = _apply(q, k, v, m, f)
+    torch.cuda.synchronize()
+    assert torch.equal(o1, want) and torch.equal(o2, want)
+    # captured: a replay reads the bias that is there then, and an eager call after the capture does not read the graph's
+    g = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(g):
+        o = _apply(q, k, v, m, f)
+    assert torch.equal(_apply(q, k, v, m, f), want)
+    f.copy_(b2)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(o, want2)
+    del g

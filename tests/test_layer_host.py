@@ -104,3 +104,12 @@ def test_views_with_holes_are_read_in_place():
     assert L._inplace_view_strides(odd, odd, odd) is None
     ov = torch.zeros((N + 4, H, D), dtype=bf).as_strided((1, 1, N, H, D), (0, 0, D, D, 1))   # rows overlap heads
     assert L._inplace_view_strides(ov, ov, ov) is None
+
+
+def test_bias_cast_in_inference_mode():
+    """An fp32 pair bias made in inference mode has no version counter: it is cast like any other."""
+    import tk_evo_attention_layer as L
+    with torch.inference_mode():
+        pb = torch.randn((1, 1, 2, 16, 16))
+        out = L._bias_bf16(pb, 1, 2, 16)
+    assert torch.equal(out, pb.reshape(1, 2, 16, 16).to(torch.bfloat16))
