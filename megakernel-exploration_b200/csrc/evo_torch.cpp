@@ -132,8 +132,9 @@ Forward run_forward(const Call& c, bool need_grad) {
     return f;
 }
 
-// The backward's autograd node.  Edges: q, k, v, pair_bias, gate (the bf16, laid-out forms of them that
-// the kernels read are what is saved).
+// The backward's autograd node.  Its edges are the operator's arguments in their order: q, k, v, res_mask (which gets no
+// gradient), pair_bias and, with a gate, the place of process_group and the gate.  What is saved are the bf16, laid-out
+// forms that the kernels read.
 struct EvoBackward : public torch::autograd::Node {
     SavedVariable q, k, v, bias, mask, gate, o, o_resid, lse;
     bool gated = false;
@@ -190,7 +191,8 @@ struct EvoBackward : public torch::autograd::Node {
         a.stream = c10::cuda::getCurrentCUDAStream().stream();
         check(evo_bwd_ex(&a), "evo_bwd_ex");
         if (!bf && bias_type != at::kFloat) dbias = dbias.to(bias_type);
-        return {dq, dk, dv, dbias, d_gate};
+        if (gated) return {dq, dk, dv, Tensor(), dbias, Tensor(), d_gate};
+        return {dq, dk, dv, Tensor(), dbias};
     }
 };
 
@@ -208,8 +210,8 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
     if (B > INT32_MAX || S > INT32_MAX || N > INT32_MAX || H > INT32_MAX) return std::nullopt;
 
     const bool need_grad = at::GradMode::is_enabled() &&
-                           (Q.requires_grad() || K.requires_grad() || V.requires_grad() || pair_bias.requires_grad() ||
-                            (gate && gate->requires_grad()));
+                           (Q.requires_grad() || K.requires_grad() || V.requires_grad() || res_mask.requires_grad() ||
+                            pair_bias.requires_grad() || (gate && gate->requires_grad()));
     Call c;
     {
         const at::NoGradGuard no_grad;
@@ -237,7 +239,9 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
         f = run_forward(c, true);
     }
     const std::shared_ptr<EvoBackward> node(new EvoBackward(), torch::autograd::deleteNode);
-    node->set_next_edges(torch::autograd::collect_next_edges(Q, K, V, pair_bias, gate ? *gate : Tensor()));
+    variable_list inputs{Q, K, V, res_mask, pair_bias};
+    if (gate) inputs.insert(inputs.end(), {Tensor(), *gate});
+    node->set_next_edges(torch::autograd::collect_next_edges(inputs));
     node->q = SavedVariable(c.q, false);
     node->k = SavedVariable(c.k, false);
     node->v = SavedVariable(c.v, false);

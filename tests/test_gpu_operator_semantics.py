@@ -55,3 +55,27 @@ def test_fp32_bias_is_read_anew(d):
     torch.cuda.synchronize()
     assert torch.equal(o, want2)
     del g
+
+
+@pytest.mark.parametrize("d", HEAD_DIMS)
+@pytest.mark.parametrize("which", range(5))
+def test_one_input_requires_grad(d, which):
+    """Any one input that requires a gradient puts the output on the graph, with an edge per argument in the arguments'
+    order; the mask's gets nothing."""
+    x = list(_inputs(d))
+    x[which] = x[which].requires_grad_(True)
+    o = _apply(*x)
+    assert o.requires_grad
+    edges = [f is not None for f, _ in o.grad_fn.next_functions]
+    assert edges == [i == which for i in range(5)]
+    o.float().sum().backward()
+    assert (x[which].grad is None) == (which == 3)
+
+
+def test_gate_edge():
+    x = list(_inputs())
+    gate = torch.randn_like(x[0]).requires_grad_(True)
+    o = _apply(*x, None, gate)
+    assert [f is not None for f, _ in o.grad_fn.next_functions] == [False] * 6 + [True]
+    o.float().sum().backward()
+    assert gate.grad.shape == gate.shape
