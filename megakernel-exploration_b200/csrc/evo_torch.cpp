@@ -207,6 +207,9 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
     const auto dev = Q.device();
     if (K.device() != dev || V.device() != dev || res_mask.device() != dev || pair_bias.device() != dev) return std::nullopt;
     if (gate && gate->device() != dev) return std::nullopt;
+    // no forward-mode derivative: the Python operator says so
+    for (const Tensor* t : {&Q, &K, &V, &res_mask, &pair_bias, gate ? &*gate : &Q})
+        if (t->_fw_grad(0).defined()) return std::nullopt;
     if (B > INT32_MAX || S > INT32_MAX || N > INT32_MAX || H > INT32_MAX) return std::nullopt;
 
     const bool need_grad = at::GradMode::is_enabled() &&

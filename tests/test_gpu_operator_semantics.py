@@ -79,3 +79,15 @@ def test_gate_edge():
     assert [f is not None for f, _ in o.grad_fn.next_functions] == [False] * 6 + [True]
     o.float().sum().backward()
     assert gate.grad.shape == gate.shape
+
+
+@pytest.mark.parametrize("d", HEAD_DIMS)
+@pytest.mark.parametrize("which", range(5))
+def test_forward_mode_is_refused(d, which):
+    """There is no forward-mode derivative: a tangent is an error, not dropped."""
+    import torch.autograd.forward_ad as fwad
+    x = list(_inputs(d))
+    with fwad.dual_level():
+        x[which] = fwad.make_dual(x[which], torch.ones_like(x[which]))
+        with pytest.raises(NotImplementedError):
+            _apply(*x)
