@@ -12,11 +12,13 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/evoattn.h"
 
@@ -198,6 +200,9 @@ struct EvoBackward : public torch::autograd::Node {
 
 std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& res_mask, const Tensor& pair_bias,
                             const std::optional<Tensor>& gate) {
+    // A trace has to record the operator, and function transforms have to refuse it: both as the Python one does.
+    if (torch::jit::tracer::isTracing() ||
+        c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode)) return std::nullopt;
     if (Q.dim() != 5 || !Q.is_cuda()) return std::nullopt;
     const auto sz = Q.sizes();
     const int64_t B = sz[0], S = sz[1], N = sz[2], H = sz[3], D = sz[4];

@@ -91,3 +91,30 @@ def test_forward_mode_is_refused(d, which):
         x[which] = fwad.make_dual(x[which], torch.ones_like(x[which]))
         with pytest.raises(NotImplementedError):
             _apply(*x)
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("d", HEAD_DIMS)
+def test_jit_trace_records_the_operator(d):
+    """A traced function computes on its own inputs, gradients included, not on those it was traced with."""
+    q, k, v, m, b = _inputs(d)
+    f = lambda *x: _apply(*x) * 1.0
+    q1, q2 = q.clone().requires_grad_(True), (2 * q).requires_grad_(True)
+    traced = torch.jit.trace(f, (q1, k, v, m, b), check_trace=False)
+    o, want = traced(q2, k, v, m, b), f(q2, k, v, m, b)
+    assert torch.equal(o, want)
+    d_o = torch.randn_like(o)
+    assert torch.equal(torch.autograd.grad(o, q2, d_o)[0], torch.autograd.grad(want, q2, d_o)[0])
+
+
+@pytest.mark.parametrize("d", HEAD_DIMS)
+def test_function_transforms_are_refused(d):
+    """vmap and grad of torch.func are errors, whether or not they are over one of the operator's inputs."""
+    q, k, v, m, b = _inputs(d)
+    two = torch.stack([q, q])
+    for call in (lambda: torch.func.vmap(lambda x: _apply(x, k, v, m, b))(two),
+                 lambda: torch.func.vmap(lambda x: _apply(q, k, v, m, b) + x)(two),
+                 lambda: torch.func.grad(lambda x: _apply(x, k, v, m, b).float().sum())(q),
+                 lambda: torch.func.grad(lambda x: (_apply(q, k, v, m, b) * x).float().sum())(q)):
+        with pytest.raises(RuntimeError, match="setup_context"):
+            call()
