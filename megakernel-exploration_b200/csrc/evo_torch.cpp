@@ -103,6 +103,17 @@ Tensor as_output(const Tensor& t, const Tensor& q, const Layout& l) {
     return c;
 }
 
+// `t` contiguous, 16-byte aligned and of the given type, copied only if it is not.
+Tensor plain(const Tensor& t, at::ScalarType type) {
+    Tensor c = (t.scalar_type() == type ? t : t.to(type)).contiguous();
+    return aligned(c) ? c : c.clone();
+}
+
+// Can q, k or v be read through the strides of `l`?
+bool lies_as_input(const Tensor& t, const Layout& l) {
+    return t.scalar_type() == at::kBFloat16 && t.strides() == at::IntArrayRef(l.strides, 5) && aligned(t);
+}
+
 struct Call {
     Tensor q, k, v, bias, mask, gate;      // gate: undefined without one
     Layout lay;
@@ -142,6 +153,7 @@ struct EvoBackward : public torch::autograd::Node {
     bool gated = false;
     Layout lay;
     EvoDims dims{};
+    c10::Device device = c10::Device(c10::DeviceType::CUDA, 0);
     float scale = 0.f;
     at::ScalarType bias_type = at::kBFloat16;
 
@@ -156,9 +168,27 @@ struct EvoBackward : public torch::autograd::Node {
         const std::lock_guard<std::mutex> lock(mutex_);
         const at::NoGradGuard no_grad;
         const auto self = getptr();
-        const Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack(), mask_ = mask.unpack();
-        const Tensor o_ = o.unpack(self), resid_ = o_resid.unpack(), lse_ = lse.unpack(), gate_ = gated ? gate.unpack() : Tensor();
-        const c10::cuda::CUDAGuard guard(q_.device());
+        // What a saved-tensor hook hands back has the values that were saved, but need not lie where they lay: a view may
+        // come back contiguous, or off its alignment.
+        auto whole = [&](const Tensor& t, int64_t numel) -> const Tensor& {
+            TORCH_CHECK(t.device() == device && t.numel() == numel,
+                        "TKEvoAttention: a saved tensor came back on another device or with another size than it had");
+            return t;
+        };
+        const int64_t rows = int64_t{dims.B} * dims.S * dims.N, acts = rows * dims.H * dims.D;
+        const c10::cuda::CUDAGuard guard(device);
+        Tensor q_ = whole(q.unpack(), acts), k_ = whole(k.unpack(), acts), v_ = whole(v.unpack(), acts);
+        const bool in_view = lay.in_view && lies_as_input(q_, lay) && lies_as_input(k_, lay) && lies_as_input(v_, lay);
+        if (!in_view) {
+            q_ = plain(q_, at::kBFloat16);
+            k_ = plain(k_, at::kBFloat16);
+            v_ = plain(v_, at::kBFloat16);
+        }
+        const Tensor bias_ = plain(whole(bias.unpack(), int64_t{dims.B} * dims.H * dims.N * dims.N), at::kBFloat16);
+        const Tensor mask_ = plain(whole(mask.unpack(), rows), at::kBFloat16);
+        const Tensor lse_ = plain(whole(lse.unpack(), rows * dims.H), at::kFloat);
+        const Tensor o_ = as_output(whole(o.unpack(self), acts), q_, lay), resid_ = as_output(whole(o_resid.unpack(), acts), q_, lay);
+        const Tensor gate_ = gated ? as_output(whole(gate.unpack(), acts), q_, lay) : Tensor();
         const Tensor d_out = grads[0].defined() ? as_output(grads[0], q_, lay) : empty_like_act(q_, lay).zero_();
         Tensor dq = empty_like_act(q_, lay), dk = empty_like_act(q_, lay), dv = empty_like_act(q_, lay), d_gate;
         if (gated) d_gate = empty_like_act(q_, lay);
@@ -167,7 +197,7 @@ struct EvoBackward : public torch::autograd::Node {
                                               std::nullopt);
         EvoBwdArgs a{};
         a.dims = dims;
-        a.s_qkv = lay.in_view ? &lay.in : nullptr;
+        a.s_qkv = in_view ? &lay.in : nullptr;
         a.s_out = a.s_grad = lay.out_view ? &lay.in : nullptr;
         a.q = q_.const_data_ptr();
         a.k = k_.const_data_ptr();
@@ -261,6 +291,7 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
     node->lse = SavedVariable(f.lse, false);
     node->lay = c.lay;
     node->dims = c.dims;
+    node->device = dev;
     node->scale = c.scale;
     node->bias_type = c.bias_type;
     torch::autograd::set_history(f.out, node);

@@ -184,6 +184,19 @@ def _inplace_view_strides(Q, K, V):
     return tuple(st)
 
 
+def _laid_out(t, dtype, device, strides):
+    """`t` with the given strides (None: contiguous), 16-byte aligned and of the given type; copied only if it is not.  A saved
+    tensor that went through a hook has its values but need not lie where it lay."""
+    if t.device != device:
+        raise RuntimeError("TKEvoAttention: a saved tensor came back on another device than it had")
+    fits = t.is_contiguous() if strides is None else tuple(t.stride()) == tuple(strides)
+    if fits and t.dtype == dtype and t.data_ptr() % 16 == 0:
+        return t
+    out = torch.empty(t.shape, dtype=dtype, device=device) if strides is None \
+        else torch.empty_strided(t.shape, strides, dtype=dtype, device=device)
+    return out.copy_(t)
+
+
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
@@ -324,7 +337,14 @@ class TKEvoAttention(torch.autograd.Function):
         B, N_SEQ, N_CTX, H = ctx.dims
         D, padded_D = ctx.true_D, ctx.padded_D
 
-        strides = ctx.strides
+        strides, in_strides = ctx.strides, ctx.in_strides
+        if in_strides is not None and not all(t.dtype == torch.bfloat16 and tuple(t.stride()) == in_strides
+                                              and t.data_ptr() % 16 == 0 for t in (q, k, v)):
+            in_strides = strides
+        q, k, v = (_laid_out(t, torch.bfloat16, dO.device, in_strides) for t in (q, k, v))
+        o, o_resid, g = (t if t is None else _laid_out(t, torch.bfloat16, dO.device, strides) for t in (o, o_resid, g))
+        bias, mask = (_laid_out(t, torch.bfloat16, dO.device, None) for t in (bias, mask))
+        lse = _laid_out(lse, torch.float32, dO.device, None)
         if strides is not None:
             like = lambda: torch.empty_strided(q.shape, strides, dtype=q.dtype, device=q.device)
             if dO.dtype == torch.bfloat16 and tuple(dO.stride()) == strides and dO.data_ptr() % 16 == 0:
@@ -347,10 +367,10 @@ class TKEvoAttention(torch.autograd.Function):
         st_ = _evoattn.EvoStrides(*strides[:4]) if strides is not None else None
         args = (dims, st_, q, k, v, bias, mask, o, o_resid, lse, d_o, dq, dk, dv, dbias, ws, ctx.softmax_scale)
         with _device_ctx(q):
-            if ctx.in_strides != strides:
+            if in_strides != strides:
                 # q, k, v read through their own view; everything else in the layout of `strides`
                 import torch.distributed as dist
-                vargs = (dims, _evoattn.EvoStrides(*ctx.in_strides[:4]), st_, st_, q, k, v, bias, mask, g, o, o_resid,
+                vargs = (dims, _evoattn.EvoStrides(*in_strides[:4]), st_, st_, q, k, v, bias, mask, g, o, o_resid,
                          lse, d_o, dq, dk, dv, d_gate, dbias, ws, ctx.softmax_scale)
                 if ctx.process_group is None:
                     _evoattn.bwd_views(*vargs, _evoattn.BWD_PHASE_DBIAS | _evoattn.BWD_PHASE_DQKV, 0, _stream())

@@ -118,3 +118,50 @@ def test_function_transforms_are_refused(d):
                  lambda: torch.func.grad(lambda x: (_apply(q, k, v, m, b) * x).float().sum())(q)):
         with pytest.raises(RuntimeError, match="setup_context"):
             call()
+
+
+def _off_by_one(t):
+    """The same values two (or four) bytes off the alignment."""
+    room = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+    return room[1:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("route", ["native", "python"])
+@pytest.mark.parametrize("view", ["plain", "ending", "fused"])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("back", [lambda t: t.cuda(), _off_by_one])
+def test_saved_tensor_hooks(route, view, gated, back):
+    """Saved tensors that come back from a hook contiguous where they were views, or misaligned, give the same gradients."""
+    from tk_evo_attention_layer import TKEvoAttention
+    q, k, v, m, b = _inputs()
+    if view == "fused":
+        q, k, v = torch.stack([q, k, v], 3).unbind(3)
+    elif view == "ending":
+        q, k, v = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v))
+    x = [t.detach().requires_grad_(True) for t in (q, k, v, b)]
+    gate = (q * 2).detach().requires_grad_(True) if gated else None
+    d_o = torch.randn(q.shape, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda").to(torch.bfloat16)
+    call = TKEvoAttention.apply if route == "native" else super(TKEvoAttention, TKEvoAttention).apply
+
+    def grads():
+        o = call(x[0], x[1], x[2], m, x[3], None, gate) if gated else call(x[0], x[1], x[2], m, x[3])
+        return o, torch.autograd.grad(o, x + ([gate] if gated else []), d_o)
+
+    o, want = grads()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu().contiguous(), back):
+        o2, got = grads()
+    assert torch.equal(o, o2)
+    for i, (a, c) in enumerate(zip(want, got)):
+        if i == 3:      # sums over slices of S meet in any order
+            assert (a.float() - c.float()).abs().max() <= 2.0 ** -7 * a.float().abs().max()
+        else:
+            assert torch.equal(a, c), i
+
+
+def test_saved_tensor_of_another_size_is_an_error():
+    q, k, v, m, b = _inputs()
+    q.requires_grad_(True)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t[..., :8] if t.dim() == 5 else t):
+        o = _apply(q, k, v, m, b)
+    with pytest.raises(RuntimeError, match="another"):
+        o.sum().backward()
