@@ -110,8 +110,9 @@ int evo_bwd_phased(const EvoDims* dims, const EvoStrides* strides, const void* q
                    float* dbias, void* workspace, size_t workspace_bytes, float scale, unsigned phases,
                    int reserved_sms, void* stream);
 
-/* Bytes of scratch evo_bwd needs for these dims (per-row and per-column extra tiles of the
- * logits + fp32 dQ accumulator). */
+/* Bytes of scratch evo_bwd wants for these dims (per-row and per-column extra tiles of the
+ * logits + fp32 partial sums of dQ).  A workspace that holds N instead of N rounded up to 32
+ * rows of dQ per (row of S, head) is accepted as well, and may cost time. */
 size_t evo_bwd_workspace_bytes(const EvoDims* dims);
 
 /* Backward.  Replaces evoattention_backward (tk_evoattention.cu:1051-1197):
@@ -138,8 +139,8 @@ int evo_bwd(const EvoDims* dims, const void* q, const void* k, const void* v,
  * already owns the whole GPU, a plugin loaded into such a process, or code that
  * runs where an allocation would stall or fail (for example inside a section
  * the host has frozen against allocator calls).
- *   - Problems whose evo_bwd_workspace_bytes(dims) exceeds the capacity are
- *     refused with EVO_ERR_TOO_LARGE; nothing is launched.
+ *   - Problems whose smallest workspace (evo_bwd_workspace_bytes) exceeds the
+ *     capacity are refused with EVO_ERR_TOO_LARGE; nothing is launched.
  *   - The first call on each device looks up the array's device address (once,
  *     with that device current).  Make that first call before any stream
  *     capture begins on the device.

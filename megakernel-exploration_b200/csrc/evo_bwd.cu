@@ -969,9 +969,11 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
 }
 
 struct BwdWorkspace {
-    size_t off_xq, off_xk, off_dq, off_do, off_db, total;
+    size_t off_xq, off_xk, off_do, off_db, off_dq, least, total;
 };
 
+// The fp32 dQ area, kernel width, comes last: the accumulator of B * S * H pairs takes N rows of each (`least`), the
+// scratch of as many CTAs that take pairs whole N rounded up to 32 (`total`, what the entry points ask for).
 static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false, bool dbias_bf16 = false) {
     const size_t BS = static_cast<size_t>(d->B) * d->S;
     const size_t NTP = static_cast<size_t>((d->N + TILE - 1) / TILE) * TILE;
@@ -979,13 +981,13 @@ static BwdWorkspace bwd_workspace(const EvoDims* d, bool gated = false, bool dbi
     BwdWorkspace w;
     w.off_xq = 0;
     w.off_xk = up(w.off_xq + BS * d->H * NTP * 16);
-    w.off_dq = up(w.off_xk + BS * NTP * 16);
-    const size_t dh = d->D <= 32 ? 32 : (d->D <= 64 ? 64 : 128);
-    // fp32 dQ, kernel width: the accumulator, or the scratch of at most B * S * H CTAs
-    w.off_do = up(w.off_dq + BS * d->H * ((d->N + 31) / 32 * 32) * dh * 4);
+    w.off_do = up(w.off_xk + BS * NTP * 16);
     w.off_db = gated ? up(w.off_do + BS * d->N * d->H * d->D * 2) : w.off_do;    // bf16 d_out * sigmoid(gate)
     // fp32 dBias of a caller that wants bf16 (one S row needs none: dBias is not a sum)
-    w.total = (dbias_bf16 && d->S > 1) ? up(w.off_db + static_cast<size_t>(d->B) * d->H * d->N * d->N * 4) : w.off_db;
+    w.off_dq = (dbias_bf16 && d->S > 1) ? up(w.off_db + static_cast<size_t>(d->B) * d->H * d->N * d->N * 4) : w.off_db;
+    const size_t dh = d->D <= 32 ? 32 : (d->D <= 64 ? 64 : 128);
+    w.least = up(w.off_dq + BS * d->H * d->N * dh * 4);
+    w.total = up(w.off_dq + BS * d->H * ((d->N + 31) / 32 * 32) * dh * 4);
     return w;
 }
 
@@ -994,8 +996,8 @@ template <int DH>
 static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout& lay_out, const ActLayout& lay_grad,
                       const void* q, const void* k, const void* v, const void* bias,
                       const void* mask, const void* o, const void* o_resid, const float* lse, const void* d_o_in,
-                      void* dq, void* dk, void* dv, void* dbias_out, bool dbias_bf16, uint8_t* ws, float scale, unsigned phases,
-                      int reserved_sms, cudaStream_t st, const void* gate, void* d_gate) {
+                      void* dq, void* dk, void* dv, void* dbias_out, bool dbias_bf16, uint8_t* ws, size_t ws_bytes, float scale,
+                      unsigned phases, int reserved_sms, cudaStream_t st, const void* gate, void* d_gate) {
     const int BS = d->B * d->S;
     const int NT = (d->N + TILE - 1) / TILE;
     const BwdWorkspace w = bwd_workspace(d, gate != nullptr, dbias_bf16);
@@ -1046,6 +1048,8 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     // load stage (B=1, S=40, N=768, H=4: 193 -> 214 us, passes 42 -> 25).
     const int pairs = BS * d->H;
     const size_t n32 = static_cast<size_t>((d->N + 31) / 32) * 32;
+    // rows of the dQ area; a caller with less than the entry points ask for gets fewer whole pairs
+    const size_t room = static_cast<size_t>(pairs) * (ws_bytes >= w.total ? n32 : static_cast<size_t>(d->N));
     const long t_seg = (static_cast<long>(pairs) * NT + use_sms - 1) / use_sms;
     if constexpr (DH == 128) {
         const long t_whole = static_cast<long>((pairs + use_sms - 1) / use_sms) * NT;
@@ -1055,8 +1059,10 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         p.n_whole = (left && t_seg < static_cast<long>(full / use_sms + 1) * NT) ? full : pairs;
         // the workspace holds the partial sums of every CTA and the accumulator from the row on that pair `full` is in
         const size_t acc_n = static_cast<size_t>(pairs - full / d->H * d->H) * d->N;
-        if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > pairs * n32) p.n_whole = 0;
+        if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > room) p.n_whole = 0;
     }
+    // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; two at D <= 64)
+    if (p.n_whole == pairs && NT > (DH == 128 ? 1 : 2) && std::min(pairs, use_sms) * n32 > room) p.n_whole = 0;
     p.pairs = pairs;
     p.acc_row0 = p.n_whole / d->H;
     const int rest_rows = p.n_whole < pairs ? BS - p.acc_row0 : 0;
@@ -1210,7 +1216,7 @@ extern "C" int evo_bwd_static_scratch(const EvoDims* dims, const void* q, const 
                                       void* dv, float* dbias, float scale, void* stream) {
     int rc = evo::check_dims(dims);
     if (rc) return rc;
-    if (evo::bwd_workspace(dims).total > EVO_STATIC_SCRATCH_BYTES) return EVO_ERR_TOO_LARGE;
+    if (evo::bwd_workspace(dims).least > EVO_STATIC_SCRATCH_BYTES) return EVO_ERR_TOO_LARGE;
     if ((rc = evo::ensure_context())) return rc;
     uint8_t* scratch = nullptr;
     if ((rc = evo::static_scratch(&scratch))) return rc;
@@ -1302,11 +1308,11 @@ extern "C" int evo_bwd_ex(const EvoBwdArgs* a) {
     if ((a->gate == nullptr) != (a->d_gate == nullptr)) return EVO_ERR_NULL_PTR;
     if (all & 15u) return EVO_ERR_ALIGNMENT;
     if ((reinterpret_cast<uintptr_t>(a->workspace) & 255u) ||
-        a->workspace_bytes < evo::bwd_workspace(dims, a->gate != nullptr, a->dbias_bf16 != 0).total)
+        a->workspace_bytes < evo::bwd_workspace(dims, a->gate != nullptr, a->dbias_bf16 != 0).least)
         return EVO_ERR_WORKSPACE;
     if ((rc = evo::ensure_context())) return rc;
     auto launch = dims->D <= 32 ? evo::launch_bwd<32> : (dims->D <= 64 ? evo::launch_bwd<64> : evo::launch_bwd<128>);
     return launch(dims, lay, lay_out, lay_grad, a->q, a->k, a->v, a->pair_bias, a->res_mask, a->o, a->o_resid, a->lse,
-                  a->d_out, a->dq, a->dk, a->dv, a->dbias, a->dbias_bf16 != 0, static_cast<uint8_t*>(a->workspace), a->scale,
+                  a->d_out, a->dq, a->dk, a->dv, a->dbias, a->dbias_bf16 != 0, static_cast<uint8_t*>(a->workspace), a->workspace_bytes, a->scale,
                   a->phases, a->reserved_sms, static_cast<cudaStream_t>(a->stream), a->gate, a->d_gate);
 }

@@ -60,3 +60,26 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_evoattn, "LIB_PATH", "/nonexistent/libevoattn.so")
     with pytest.raises(ImportError):
         _evoattn.lib()
+
+
+def _bytes_of_n_rows(d):
+    """Workspace whose fp32 dQ area holds N rows per (row of S, head), without rounding N up."""
+    up = lambda x: -(-x // 256) * 256
+    bs, ntp, dh = d.B * d.S, -(-d.N // 128) * 128, 32 if d.D <= 32 else 64 if d.D <= 64 else 128
+    return up(up(up(bs * d.H * ntp * 16) + bs * ntp * 16) + bs * d.N * d.H * dh * 4)
+
+
+def test_static_scratch_takes_what_fits_without_rounding():
+    """The rounding of N in evo_bwd_workspace_bytes does not shrink what the fixed scratch array takes."""
+    import _evoattn
+    lib = _evoattn.lib()
+    cap = lib.evo_bwd_static_scratch_capacity()
+    for n, d in ((40, 32), (136, 64), (264, 128)):
+        h = 4
+        s = max(s for s in range(1, 4096) if _bytes_of_n_rows(_evoattn.EvoDims(1, s, n, h, d)) <= cap)
+        dims = _evoattn.EvoDims(1, s, n, h, d)
+        assert lib.evo_bwd_workspace_bytes(C.byref(dims)) > cap
+        nulls = [None] * 13
+        assert lib.evo_bwd_static_scratch(C.byref(dims), *nulls, 0.0, None) != -9      # (a null pointer, or no device)
+        dims = _evoattn.EvoDims(1, s + 1, n, h, d)
+        assert lib.evo_bwd_static_scratch(C.byref(dims), *nulls, 0.0, None) == -9

@@ -2,6 +2,7 @@
 cut short at the end of a batch; separate items per stream, with streams that run out; ragged last tiles.
 Tolerance: the operator's parity bar (tests/_util.py)."""
 import pytest
+import torch
 
 from oracle import evo_ref
 from _util import assert_parity, oracle_on_rounded, run_layer
@@ -80,3 +81,51 @@ def test_backward_rest(B, S, N, H, D):
     got = run_layer(q, k, v, mask, bias, d_o)
     ref = oracle_on_rounded(q, k, v, mask, bias, d_o)
     assert_parity(ref, got, tag=f"B={B} S={S} H={H} N={N} D={D}")
+
+
+# ... in the smallest workspace that is accepted, whose dQ area has no room for N rounded up to 32 rows per pair
+@pytest.mark.parametrize("B,S,N,H,D", [
+    (1, 5, 264, 3, 32),      # fewer pairs than SMs: scratch of all does not fit, so segments
+    (1, 5, 200, 3, 64),      # two tiles need no scratch
+    (1, 50, 264, 6, 32),     # 296 + 4
+    (1, 75, 264, 4, 64),     # 300 pairs
+    (1, 37, 264, 4, 128),    # D = 128, three tiles: 148 pairs
+    (1, 37, 104, 4, 96),     # ... one
+])
+@pytest.mark.parametrize("gated", [False, True])
+def test_backward_smallest_workspace(B, S, N, H, D, gated):
+    import _evoattn
+    inputs = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=S + N)
+    q, k, v, mask, bias, d_o = (t.cuda().to(torch.bfloat16) for t in inputs)
+    dims, st = _evoattn.EvoDims(B, S, N, H, D), torch.cuda.current_stream().cuda_stream
+    o, og, resid = (torch.empty_like(q) for _ in range(3))
+    lse = torch.empty((B, S, H, N), device="cuda")
+    gate = torch.randn_like(q) if gated else None
+    _evoattn.fwd_gated(dims, None, q, k, v, bias, mask, gate, o, og if gated else None, resid, lse, 0.0, st)
+    full = _evoattn.bwd_gated_workspace_bytes(dims) if gated else _evoattn.bwd_workspace_bytes(dims)
+    dh = 32 if D <= 32 else 64 if D <= 64 else 128
+    least = full - (-N % 32) * B * S * H * dh * 4 // 256 * 256
+    both = _evoattn.BWD_PHASE_DBIAS | _evoattn.BWD_PHASE_DQKV
+
+    def run(size, *phases):
+        out = [torch.full_like(q, float("nan")) for _ in range(3)]
+        d_gate = torch.full_like(q, float("nan")) if gated else None
+        dbias = torch.full((B, H, N, N), float("nan"), device="cuda")
+        ws = torch.full((size + 4096,), 0x7f, dtype=torch.uint8, device="cuda")
+        for ph in phases:
+            _evoattn.bwd_gated(dims, None, q, k, v, bias, mask, gate, o, resid, lse, d_o, *out, d_gate, dbias, ws[:size], 0.0,
+                               ph, 0, st)
+        _evoattn.device_status()
+        assert (ws[size:] == 0x7f).all()          # nothing past the end
+        return out + [dbias] + ([d_gate] if gated else [])
+
+    ref = run(full, both)
+    for phases in ((both,), (_evoattn.BWD_PHASE_DBIAS, _evoattn.BWD_PHASE_DQKV)):
+        got = run(least, *phases)
+        for name, a, b in zip(("dq", "dk", "dv", "dbias", "dgate"), ref, got):
+            # dQ: the same fp32 partial sums in another order, then bf16; dBias: fp32 sums over slices in any order
+            tol = {"dq": 2.0 ** -7, "dbias": 1e-5}.get(name, 0.0) * a.float().abs().max().item()
+            assert (a.float() - b.float()).abs().max().item() <= tol, name
+    with pytest.raises(_evoattn.EvoAttnError) as e:
+        run(least - 256, both)
+    assert e.value.code == -4
