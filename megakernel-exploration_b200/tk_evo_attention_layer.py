@@ -42,6 +42,7 @@ from __future__ import annotations
 
 import os
 import sys
+import warnings
 
 import torch
 import torch.nn.functional as F
@@ -214,12 +215,20 @@ _native_apply = None
 
 
 def _native():
-    """apply() of _evo_torch.so, the operator's host path in native code (csrc/evo_torch.cpp)."""
+    """apply() of _evo_torch.so, the operator's host path in native code (csrc/evo_torch.cpp).  Where only libevoattn.so is
+    there, built without torch's headers or for another torch, the Python body below serves every call on
+    the same kernels, and a warning says what that costs."""
     global _native_apply
     if _native_apply is None:
         _evoattn.lib()                      # the kernels' library, with its own check and error message
-        import _evo_torch
-        _native_apply = _evo_torch.apply
+        try:
+            import _evo_torch
+        except ImportError as e:
+            warnings.warn(f"_evo_torch.so did not load ({e}): calls take the Python host path, about 0.1 ms more per step. "
+                          f"Build it with `python {os.path.join(HERE, 'build.py')}`.", RuntimeWarning, stacklevel=3)
+            _native_apply = lambda *args: None
+        else:
+            _native_apply = _evo_torch.apply
     return _native_apply
 
 

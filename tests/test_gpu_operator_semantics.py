@@ -165,3 +165,14 @@ def test_saved_tensor_of_another_size_is_an_error():
         o = _apply(q, k, v, m, b)
     with pytest.raises(RuntimeError, match="another"):
         o.sum().backward()
+
+
+def test_without_the_native_host_path(monkeypatch):
+    import sys
+    import tk_evo_attention_layer as L
+    x = _inputs()
+    want = _apply(*x)
+    monkeypatch.setattr(L, "_native_apply", None)
+    monkeypatch.setitem(sys.modules, "_evo_torch", None)
+    with pytest.warns(RuntimeWarning, match="build.py"):
+        assert torch.equal(_apply(*x), want)

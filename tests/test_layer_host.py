@@ -113,3 +113,14 @@ def test_bias_cast_in_inference_mode():
         pb = torch.randn((1, 1, 2, 16, 16))
         out = L._bias_bf16(pb, 1, 2, 16)
     assert torch.equal(out, pb.reshape(1, 2, 16, 16).to(torch.bfloat16))
+
+
+def test_without_the_native_host_path(monkeypatch):
+    """Without _evo_torch.so a call goes to the Python body, which needs libevoattn.so alone; once, a warning says how to build it."""
+    import sys
+    import tk_evo_attention_layer as L
+    monkeypatch.setattr(L, "_native_apply", None)
+    monkeypatch.setitem(sys.modules, "_evo_torch", None)          # import raises ImportError
+    with pytest.warns(RuntimeWarning, match="build.py"):
+        assert L._native()(*_inputs(), None) is None
+    assert L._native()(*_inputs(), None) is None
