@@ -57,7 +57,9 @@ enum {
     EVO_ERR_TOO_LARGE = -9      /* problem exceeds a fixed-capacity entry point   */
 };
 
-/* Library ABI version (major*100 + minor). */
+/* Library ABI version (major*100 + minor).  Minor 4 added evo_bwd_ex and
+ * evo_bwd_ex_workspace_bytes. */
+#define EVO_ABI_VERSION 104
 int evo_version(void);
 const char* evo_strerror(int code);
 /* cudaError_t of the most recent failing runtime call on this thread (0 if none). */

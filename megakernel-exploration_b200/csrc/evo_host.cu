@@ -314,7 +314,7 @@ int check_dims(const EvoDims* d) {
 
 extern "C" {
 
-int evo_version(void) { return 103; }
+int evo_version(void) { return EVO_ABI_VERSION; }
 
 int evo_last_cuda_error(void) { return evo::t_last_cuda_error; }
 

@@ -26,6 +26,15 @@ def test_header_symbols_exported():
     assert sorted(_evoattn.SYMBOLS) == names
 
 
+def test_version_is_the_header_s():
+    import _evoattn
+    src = open(os.path.join(ROOT, "include", "evoattn.h")).read()
+    declared = int(re.search(r"#define EVO_ABI_VERSION (\d+)", src).group(1))
+    assert _evoattn.lib().evo_version() == declared == _evoattn.ABI_VERSION
+    # what each minor version added since 103
+    assert declared >= 104 and "evo_bwd_ex" in _declared_symbols()
+
+
 def test_version_and_strerror():
     import _evoattn
     lib = _evoattn.lib()
