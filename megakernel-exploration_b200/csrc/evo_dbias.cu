@@ -137,12 +137,10 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         *reinterpret_cast<uint4*>(smem + C::OFF_ZERO + r * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     fence_async_smem();
-    EVO_TRACE_INIT();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    EVO_TS(t_kernel);
 
     const int first = blockIdx.x;
     const int stride = gridDim.x;
@@ -309,7 +307,6 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 const int buf = gs & 1;
                 ok = warp_all(mbar_wait(&sdp_full[buf], (gs >> 1) & 1, wc, 0xa0));
                 if (!ok) break;
-                EVO_TS(t_math);
                 tc_fence_after();
                 // Chunks of 16 columns.  The tensor-memory loads of chunk ch+1 are in flight
                 // during the arithmetic of chunk ch.  Per element: x = S' c1 + bias log2e (S'
@@ -340,7 +337,6 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     for (int k = 0; k < 8; ++k)
                         acc[ch * 8 + k] = ffma2(p2[k], u2f2(dv[cb][2 * k], dv[cb][2 * k + 1]), acc[ch * 8 + k]);
                 }
-                EVO_TE(t_math, p.status, 0xa8);
             }
             if (!ok) break;
 
@@ -374,10 +370,8 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
     }
 
-    if (tid == 0) EVO_TE(t_kernel, p.status, 0xaf);
     tc_fence_before();
     __syncthreads();
-    EVO_TRACE_FLUSH(p.status);
     if (warp == NCW + 1) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 

@@ -38,7 +38,6 @@ struct WaitCtx {
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred = 0;
@@ -93,78 +92,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Non-blocking probe of phase `parity`.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred P;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, P;\n\t"
-        "}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Optional cycle accounting (builds with -DEVO_TRACE only): per wait site / code
-// region, summed over warps and CTAs, in the words that follow the status word.
-#if defined(EVO_TRACE) && defined(EVO_TL_ONLY)
-__device__ __forceinline__ void trace_add(unsigned int*, uint32_t, long long) {}
-__device__ __forceinline__ void trace_init() {}
-__device__ __forceinline__ void trace_flush(unsigned int*) {}
-#elif defined(EVO_TRACE)
-// accumulators live in shared memory during the kernel and are added to the global
-// words once at the end, so that tracing perturbs the timing as little as possible
-__device__ __forceinline__ unsigned long long* trace_smem() {
-    __shared__ unsigned long long t[512];
-    return t;
-}
-__device__ __forceinline__ void trace_add(unsigned int*, uint32_t site, long long dt) {
-    if ((threadIdx.x & 31u) == 0u) {
-        unsigned long long* t = trace_smem();
-        atomicAdd(&t[(site & 255u) * 2], static_cast<unsigned long long>(dt));
-        atomicAdd(&t[(site & 255u) * 2 + 1], 1ull);
-    }
-}
-// all threads, before the first and after the last traced region (with __syncthreads around)
-__device__ __forceinline__ void trace_init() {
-    unsigned long long* t = trace_smem();
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) t[i] = 0ull;
-}
-__device__ __forceinline__ void trace_flush(unsigned int* status) {
-    unsigned long long* t = trace_smem();
-    unsigned long long* g = reinterpret_cast<unsigned long long*>(status + 2);
-    for (int i = threadIdx.x; i < 512; i += blockDim.x)
-        if (t[i]) atomicAdd(&g[i], t[i]);
-}
-#endif
-#ifdef EVO_TRACE
-// timeline of CTA 0 (trace builds): clock at (role, step, event), plain stores to global memory
-__device__ __forceinline__ void timeline(unsigned int* status, int role, int step, int evt) {
-    if (blockIdx.x == 0 && (threadIdx.x & 31u) == 0u && step < 64) {
-        unsigned long long* g = reinterpret_cast<unsigned long long*>(status + 2) + 512;
-        g[(role * 64 + step) * 8 + evt] = static_cast<unsigned long long>(clock64());
-    }
-}
-#define EVO_TL(status, role, step, evt) timeline((status), (role), (step), (evt))
-#define EVO_TRACE_INIT() trace_init()
-#define EVO_TRACE_FLUSH(status) trace_flush(status)
-#define EVO_T0() const long long evo_t0_ = clock64()
-#define EVO_T1(status, site) trace_add((status), (site), clock64() - evo_t0_)
-#define EVO_TS(var) const long long var = clock64()
-#define EVO_TE(var, status, site) trace_add((status), (site), clock64() - var)
-#else
-#define EVO_TL(status, role, step, evt) do {} while (0)
-#define EVO_TRACE_INIT() do {} while (0)
-#define EVO_TRACE_FLUSH(status) do {} while (0)
-#define EVO_T0() do {} while (0)
-#define EVO_T1(status, site) do {} while (0)
-#define EVO_TS(var) do {} while (0)
-#define EVO_TE(var, status, site) do {} while (0)
-#endif
-
 // Budget of one wait: an iteration limit and a wall-clock limit (try_wait may
 // itself block for a hardware-defined interval), whichever comes first.
 #ifndef EVO_WAIT_LIMIT
@@ -183,16 +110,11 @@ __device__ __forceinline__ uint64_t global_ns() {
 // Bounded wait on phase `parity` of `bar` with explicit limits (iterations, nanoseconds).
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, const WaitCtx& w,
                                                   uint32_t site, uint32_t max_iters, uint64_t max_ns) {
-    EVO_T0();
-    if (mbar_try_wait(bar, parity)) {
-        EVO_T1(w.status, site);
-        return true;
-    }
+    if (mbar_try_wait(bar, parity)) return true;
     uint64_t t0 = 0;
     for (uint32_t it = 0; it < max_iters; ++it) {
         if (mbar_try_wait(bar, parity)) {
-            EVO_T1(w.status, site);
-            return true;
+                return true;
         }
 #ifdef EVO_WAIT_BACKOFF_NS
         __nanosleep(EVO_WAIT_BACKOFF_NS);
@@ -231,17 +153,7 @@ __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffff
 // not wait for the warp's earlier shared-memory loads to return: measured on
 // B200, a warp's loads queued behind heavy barrier polling were still pending
 // when its arrive let the producer refill the buffer, and they returned the new
-// tile.  The fence makes lane 0 wait for the warp's outstanding loads (a load
-// instruction completes for all lanes together) before the arrive.
-__device__ __forceinline__ void mbar_release_after_reads(uint64_t* bar) {
-    __syncwarp();
-    if ((threadIdx.x & 31u) == 0u) {
-        __threadfence_block();
-        mbar_arrive(bar);
-    }
-}
-
-// The same hand-back without a fence.  `dep` must be computed FROM the values the last
+// tile.  `dep` must be computed FROM the values the last
 // loads of the buffer returned (any cheap combination of one register per load
 // instruction).  Lane 0 stores it to a scratch word before the arrive: the store
 // cannot issue before those loads have written their registers (a load instruction
@@ -266,16 +178,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t saddr) {
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr));
     return v;
 }
-__device__ __forceinline__ float4 lds128f(uint32_t saddr) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(saddr));
-    return v;
-}
-__device__ __forceinline__ float lds32f(uint32_t saddr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(saddr));
-    return v;
-}
 __device__ __forceinline__ uint32_t lds_u16(uint32_t saddr) {
     uint16_t v;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr));
@@ -283,9 +185,6 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t saddr) {
 }
 __device__ __forceinline__ void sts128(uint32_t saddr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-__device__ __forceinline__ void sts128f(uint32_t saddr, float4 v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 // ---- TMA --------------------------------------------------------------------
@@ -304,24 +203,6 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* m, uin
         " [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
           "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar,
-                                            int c0, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
-          "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* m, uint64_t* bar,
-                                            int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
-          "r"(c0), "r"(c1)
         : "memory");
 }
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, bytes % 16 == 0.
@@ -502,10 +383,6 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
     d |= static_cast<uint64_t>(swz & 7u) << 61;
     return d;
 }
-// Moving a descriptor by a byte offset only touches the start-address field.
-__device__ __forceinline__ uint64_t desc_advance(uint64_t d, uint32_t bytes) {
-    return d + static_cast<uint64_t>(bytes >> 4);
-}
 
 // Instruction descriptor for kind::f16 with bf16 A/B and fp32 accumulation:
 //   [4,6) D format (1 = f32)  [7,10) A format (1 = bf16)  [10,13) B format (1 = bf16)
@@ -637,11 +514,6 @@ __device__ __forceinline__ void quad_transpose(uint4 (&c)[4]) {
     swap_pair(c[2], c[3], b0, 1);
     swap_pair(c[0], c[2], b1, 2);
     swap_pair(c[1], c[3], b1, 2);
-}
-
-// Named barrier over `nthreads` threads (ids 1..15; 0 is __syncthreads).
-__device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
 // Register reallocation between warpgroups (all four warps of the warpgroup
