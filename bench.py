@@ -39,7 +39,7 @@ for _p in (ROOT, PKG):
 import evo_workloads as wl  # noqa: E402
 
 # DRAM bytes per S row of one evo_bwd_kernel launch, from the ncu capture summarised under profiles/
-# (160.77 MB read + 53.59 MB written at 128 rows of cfg2).
+# (110.18 MB read + 46.15 MB written at 128 rows of cfg2).
 NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.18e6 + 46.15e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"

@@ -1030,7 +1030,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.dq = static_cast<__nv_bfloat16*>(dq);
     p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
-    p.lay = lay_grad;          // the kernel's own stores are dK and dV
+    p.lay = lay_grad;          // D = 128: thread-level stores (D <= 64 stores through tensor maps)
     p.status = status_word();
     if (!p.status) return EVO_ERR_CUDA;
 

@@ -9,15 +9,14 @@
 // slice of the S rows and keeps the running sum in registers, so the only
 // traffic of the reduction is one write (or one vector atomic per slice) of the
 // finished tile.  S and dP are recomputed for that (the dQ/dK/dV kernel computes
-// them too); the recompute costs two small MMAs per step, and the elementwise
-// work runs without the shared-memory round trips the dQ/dK/dV kernel needs
-// for its operands.
+// them too): two small MMAs and the exponentials per step, with nothing written back
+// to shared or tensor memory.
 //
-//   warp NCW   (producer)  TMA per step (one S row): Q, dO tiles of q tile i,
-//                          K, V tiles of kv tile j, and the two extra tiles of the
-//                          step (per-row terms of i, per-column terms of j)
-//   warp NCW+1 (mma)       S' = Q K^T + (mask - LSE) / scale and dP' = dO V^T - delta
-//                          into one of two tensor memory buffers, so the MMAs of
+//   warps NCW, NCW+3       TMA per step (one S row): Q, dO tiles of q tile i and the
+//   (producers)            extra tile of its rows; K, V tiles of kv tile j and its
+//                          extra tile (per-row terms of i, per-column terms of j)
+//   warps NCW+1, NCW+2     S' = Q K^T + (mask - LSE) / scale; dP' = dO V^T - delta;
+//   (mma)                  into one of two tensor memory buffers, so the MMAs of
 //                          step n+1 overlap the elementwise work of step n.  The
 //                          additive terms ride in an extra contraction block
 //                          (evo_tiles.cuh), so the elementwise work is one fused
@@ -41,7 +40,7 @@ template <int DH, int NG>
 struct DbCfg {
     static constexpr int CW = TILE / NG;                  // kv columns per thread
     static constexpr int NCW = NG * 4;                    // compute warps
-    static constexpr int THREADS = (NCW + 4) * 32;        // + one warpgroup: producer, mma, two idle warps
+    static constexpr int THREADS = (NCW + 4) * 32;        // + one warpgroup: two producers, two mma issuers
     // setmaxnreg budgets.  The CTA's register pool is what it was launched with
     // (the per-thread cap ptxas derives from the launch bound, times THREADS); an
     // increase blocks until the pool has room, for ever if it never can.

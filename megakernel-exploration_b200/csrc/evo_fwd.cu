@@ -69,8 +69,8 @@ struct FwdParams {
 // (b, h, q tile), so one tile serves G streams; otherwise (few rows per batch, or too few items to
 // fill the SMs G at a time) every stream has its own items and its own ring slot.
 //
-// Measured against the kernel with two groups of 64 columns on one item (which runs D = 128): B=1, S=512,
-// N=384, H=8, D=32 0.371 -> 0.323 ms; S=256, N=768 0.650 -> 0.560; S=256, N=1024, H=4, D=64 0.700 -> 0.640.
+// Measured against one item at a time on two groups of 64 columns (what is below included; kernel alone, in one run):
+// B=1, S=512, N=384, H=8, D=32 0.358 -> 0.299 ms; S=256, N=768 0.638 -> 0.538; S=256, N=1024, H=4, D=64 0.677 -> 0.602.
 // A step takes about 2400 clocks of a CTA: 1024 for its exponentials, 1000 issue slots.  Also tried: the
 // epilogue on a warpgroup of its own (its registers cost the softmax warps more than it saves, 0.42 ms),
 // two streams in the exp2 pass at a time (0.365), none taking turns (0.39), two streams at D = 32 (0.375).
@@ -80,6 +80,10 @@ struct FwdParams {
 // Staged in buffers that the item no longer needs, sent by the MMA warp's TMA stores, and with what does
 // not depend on the last PV ahead of the wait for it: 2200 (the two shapes at D = 32 0.319 -> 0.295 and
 // 0.585 -> 0.540 ms).
+//
+// One maximum per 128 columns instead of one per 64 leaves one exact P a row and tile instead of two: O is 2 to 3 %
+// further from 64 bits (relative error 2.11e-3 -> 2.16e-3 at N = 264, D = 64, of which 1.66e-3 is its own bf16).  Two
+// maxima would take a second accumulator per stream, for which there is no tensor memory.
 //
 // The mask rides in an extra contraction block (evo_tiles.cuh, "EXTRA TILE"): the producer turns 128
 // mask values into a [128][8] tile (m/scale in three bf16 parts, exact to fp32), columns past N get
@@ -175,8 +179,8 @@ __device__ __forceinline__ uint2 mask_term(float m, float inv_scale) {
 // From this |m| of a row on (one, or the tiles of it so far, all masked by terms like -1e9 or -1e30) m log2e, rounded, is
 // off by 32 and more, and 2^(x log2e - m log2e) no exponential of x - m any longer.  But there the logits are multiples
 // of 32, so that all below m get nothing, whatever the base: with 2 instead of e, x - m is exact.
-// (Kernel alone, without any of it / this / x - m formed first in a branch for such rows: B=1, S=256, N=1024, H=4, D=64
-// 0.587 / 0.593 / 0.688 ms; S=512, N=384, H=8, D=32 0.288 / 0.291 / 0.299.)
+// (Kernel alone, without any of it / this: B=1, S=256, N=1024, H=4, D=64 0.600 / 0.602 ms; S=512, N=384, H=8, D=32
+// 0.293 / 0.299; x - m formed first, in a branch for such rows, cost the first 17 %.)
 constexpr float FWD_FAR = 536870912.f;         // 2^29
 
 // GATED: the epilogue also writes sigmoid(gate) * O.  tm_2: the rounding residual (GATED: the gated output).
@@ -774,8 +778,8 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         prof_end(0, st);
     } else {
         using C = FwdCfg<DH>;
-        // Streams share bias tiles (rows taken G at a time) when that leaves no SM with more rounds of work
-        // than separate items would.
+        // Streams share bias tiles (rows taken G at a time) when that leaves no SM with more than 1/16 more rounds of
+        // work than separate items would: a shared tile is loaded once instead of G times.
         const int sg = (d->S + C::G - 1) / C::G;
         const long units = static_cast<long>(d->B) * sg * QT * d->H;
         const long apart = (static_cast<long>(p.total_items) + static_cast<long>(C::G) * sms - 1) / (static_cast<long>(C::G) * sms);

@@ -18,8 +18,8 @@
 // softmax per tile), of which two are in flight, so 3000 clocks per tile against 1024 for its exponentials
 // and 1100 for its products; and 6000 clocks per item for the stores, which all SMs issue at about the same
 // time (128 KB each).  Measured against two groups of 64 columns on one item, which waited for each
-// other on every tile: B=1, S=128, N=768, H=4, D=128 0.350 -> 0.255 ms; S=1024, N=64, H=16 0.525 -> 0.395;
-// S=300, N=600, H=8, D=96 1.11 -> 0.92.  Without turns on the exp2 pass the streams fall into step and queue
+// other on every tile: B=1, S=128, N=768, H=4, D=128 0.301 -> 0.244 ms; S=1024, N=64, H=16 0.509 -> 0.358;
+// S=300, N=600, H=8, D=96 1.04 -> 0.83.  Without turns on the exp2 pass the streams fall into step and queue
 // for the tensor core together (0.272); handing the turn on halfway through the pass 0.279.
 #pragma once
 #include "evo_bias_ring.cuh"

@@ -478,8 +478,8 @@ class HostStreamedEvoAttention:
     def _rows_per_chunk(self, S, N, H, D):
         """At most chunk_rows; fewer so that there are four chunks (the link idles in one direction while the
         first comes in and the last goes out) of copies of one to six megabytes (below, the cost of a copy
-        shows; above, the idle ends do).  B=1, N=384, H=8, D=32, chunk_rows=64: S=128 3.37 -> 2.92 ms, S=512
-        10.8 -> 10.0 ms."""
+        shows; above, the idle ends do).  B=1, N=384, H=8, D=32, chunk_rows=64, against chunks of 64
+        rows in two buffer sets: S=128 3.26 -> 3.03 ms; S=512 10.5 ms."""
         one = -(-(1 << 20) // (2 * N * H * D))               # rows of a megabyte
         return max(1, min(self.chunk_rows, S, max(one, min(-(-S // 4), 6 * one))))
 
