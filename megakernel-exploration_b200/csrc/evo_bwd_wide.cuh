@@ -454,6 +454,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) { report_abort(wc); report_abort(WaitCtx{tmem_slot + 3, p.status}); }
     if (warp == C::W_MMA) tmem_dealloc(tmem, BWD_TMEM_COLS);
 }
 

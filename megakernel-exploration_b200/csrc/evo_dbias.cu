@@ -371,6 +371,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) { report_abort(wc); report_abort(WaitCtx{tmem_slot + 3, p.status}); }
     if (warp == NCW + 1) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 

@@ -513,6 +513,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) { report_abort(wc); report_abort(WaitCtx{tmem_slot + 3, p.status}); }
     if (warp == C::W_PROD) tmem_dealloc(tmem, C::TMEM_COLS);
 }
 

@@ -140,6 +140,7 @@ selftest_mma_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) report_abort(wc);
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
@@ -231,6 +232,7 @@ selftest_xt_kernel(const __grid_constant__ CUtensorMap tm_y, const __grid_consta
     }
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) report_abort(wc);
     if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
@@ -257,7 +259,7 @@ static int launch_selftest_xt(const void* y, const void* z, const void* a, const
 // the status word and raises the CTA's abort flag; warp 1 waits on a second such barrier
 // with the library's normal limits and must be released by the abort flag long before
 // those run out.  Then the kernel returns normally: no trap, no fault, no unbounded spin.
-__global__ void __launch_bounds__(64, 1) selftest_wait_kernel(unsigned long long limit_ns, unsigned int* status,
+__global__ void __launch_bounds__(64, 1) selftest_wait_kernel(uint32_t limit_ns, unsigned int* status,
                                                               unsigned int* released) {
     __shared__ uint64_t bars[2];
     __shared__ uint32_t abort_word;
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(64, 1) selftest_wait_kernel(unsigned long long
         if (!ok && tid == 32) *released = (*abort_flag != 0u) ? 1u : 0u;
     }
     __syncthreads();
+    if (tid == 0) report_abort(wc);
 }
 
 }  // namespace evo
@@ -290,7 +293,7 @@ extern "C" int evo_selftest_wait_timeout(unsigned long long limit_ns, unsigned i
     if (int rc = evo::ensure_context()) return rc;
     unsigned int* status = evo::status_word();
     if (!status) return EVO_ERR_CUDA;
-    evo::selftest_wait_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(limit_ns, status, released);
+    evo::selftest_wait_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<uint32_t>(limit_ns), status, released);
     return evo::cuda_err(cudaGetLastError());
 }
 
