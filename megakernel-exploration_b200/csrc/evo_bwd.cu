@@ -15,7 +15,7 @@
 //                         the main kernels need no edge predicates; zeroes the accumulators
 //   2. evo_dbias_kernel   dBias (evo_dbias.cu): one CTA per pair-bias tile keeps its
 //                         sum over the S rows in registers, no reduction traffic
-//   3. evo_bwd_kernel     dQ, dK, dV (below)
+//   3. evo_bwd_kernel     dQ, dK, dV (below; D <= 32: evo_bwd_halves.cuh, D > 64: evo_bwd_wide.cuh)
 //   4. bwd_finish_kernel  fp32 dQ accumulator -> bf16 dQ in the caller layout (and dBias,
 //                         summed over slices of S in fp32, to bf16 if the caller wants that)
 #include "evo_dbias.cuh"
@@ -50,6 +50,7 @@ struct BwdParams {
     size_t scratch_stride;
     float* dq_acc;             // the others: [B*S - acc_row0][N][H][DH], zeroed before the launch
     int acc_row0;              // their first S row
+    int seg_dj, seg_dp;        // from a CTA's single segment to its next: kv tiles, pairs (grid % NT, grid / NT)
     __nv_bfloat16* dq;    // activation layout `lay` (dq: of the whole pairs only)
     __nv_bfloat16* dk;
     __nv_bfloat16* dv;
@@ -94,14 +95,15 @@ struct Segments {
 };
 
 }  // namespace evo
+#include "evo_bwd_halves.cuh"
 #include "evo_bwd_wide.cuh"
 namespace evo {
 
 // ---------------------------------------------------------------------------
-// dQ, dK, dV.  One persistent CTA per SM walks segments (S row, head h, kv tile j of 128 residues); a
-// segment walks steps (q tile i).  Everything is formed TRANSPOSED, kv rows in the tensor-memory lanes,
-// so that P^T and dS^T are in place as A operands of the products that contract over q, without a trip
-// through shared memory:
+// dQ, dK, dV at D = 64, and what the dQ/dK/dV kernels share (D <= 32: evo_bwd_halves.cuh; D = 96, 128: evo_bwd_wide.cuh).
+// One persistent CTA per SM walks segments (S row, head h, kv tile j of 128 residues); a segment walks steps (q tile i).
+// Everything is formed TRANSPOSED, kv rows in the tensor-memory lanes, so that P^T and dS^T are in place as A operands of
+// the products that contract over q, without a trip through shared memory:
 //
 //   S'^T = K Q^T + extra block,  dP'^T = V dO^T + extra block         (evo_tiles.cuh, "EXTRA TILE")
 //   P^T = exp2(S'^T c1 + bias^T log2e),  dS^T = P^T o dP'^T           (thread = one kv row)
@@ -114,14 +116,12 @@ namespace evo {
 // because with eight the loads, multiplies and exponentials of a warp hardly overlapped (2000 clocks for
 // the same work).
 //
-//   D = 32: one phase.  P^T and dS^T have columns of their own, so S' and dP' of the next step are formed
-//     during the second half of this one's arithmetic.  (A share of the exponentials on the multiply-add
-//     pipe only costs here: 0.446 -> 0.514 ms.)
-//   D = 64: no columns for P^T and dS^T: they overwrite the columns they were computed from (ALIAS).  Two
-//     phases, P (from S') and dS (from dP'), each with its own barriers, so that the products of one are
-//     formed during the other: dV and S' of the next step while dS is computed, dK, dQ and dP' of the next
-//     step while its P is (B=1, S=256, N=1024, H=4: 1.30 -> 1.11 ms; at D = 32 the extra barriers cost more
-//     than they save).
+//   D = 64: no columns for P^T and dS^T: they overwrite the columns they were computed from.  Two phases, P (from
+//     S') and dS (from dP'), each with its own barriers, so that the products of one are formed during the other: dV
+//     and S' of the next step while dS is computed, dK, dQ and dP' of the next step while its P is (B=1, S=256,
+//     N=1024, H=4: 1.30 -> 1.11 ms).  The halves of the D <= 32 kernel measure the same here (1.13 and 1.12 ms) and lose
+//     where a pair has two q tiles or one S row (S=200, N=200, H=4 78 -> 84 us; B=4, S=1, N=1024, H=16 106 -> 121): one
+//     dQ accumulator and one K/V buffer are all that fits.
 //
 //   warps 0-15 (compute)  group g = warp / 4 owns q columns 32g .. 32g+31 of the tile
 //   warps 16-19 (drain)   after every step 32 rows of dQ each, after a segment dK and dV as bf16 stores
@@ -130,8 +130,8 @@ namespace evo {
 //   warps 21, 22, 23      MMA issuers, one chain family each: S'^T and dP'^T; dV and dK; dQ
 //
 // dQ is a sum over kv tiles.  A CTA takes all NT segments of a pair (S row, head) where it can, and so sees
-// the whole sum.  With one or two tiles it stays in tensor memory until the last segment; otherwise the drain
-// warps keep partial sums in a scratch area of the CTA, in L2 (written and added to by bulk copies: loads
+// the whole sum.  With few tiles (two here, four at D <= 32) it stays in tensor memory until the last segment; otherwise
+// the drain warps keep partial sums in a scratch area of the CTA, in L2 (written and added to by bulk copies: loads
 // and stores of their own held up the compute warps' shared-memory accesses), and the last segment's go out
 // as bf16.  Whole pairs fill whole rounds of the SMs; the pairs that are left over are dealt by segments, and
 // their partial sums meet in an fp32 accumulator in memory (TMA reduce-add), which costs a pass to zero it and
@@ -139,22 +139,18 @@ namespace evo {
 // D=32 182 -> 176 us; S=200, N=200, H=4 47 -> 44; S=1024, N=768, H=8 3333 -> 3255).
 //
 // Measured against one kernel with P and dS in shared memory and two compute groups (whole backward):
-// B=1, S=512, N=384, H=8, D=32 0.81 -> 0.71 ms; S=256, N=768 1.40 -> 1.28; S=256, N=1024, H=4, D=64 1.93 ->
-// 1.59; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
-// D = 128: evo_bwd_wide.cuh.
+// S=256, N=1024, H=4, D=64 1.93 -> 1.59 ms; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
 // ---------------------------------------------------------------------------
 template <int DH>
 struct BwdCfg {
-    static constexpr bool ALIAS = (DH == 64);
-    static constexpr bool TWO_PHASE = (DH == 64);
-    static_assert(DH == 32 || DH == 64, "evo_bwd_wide.cuh has D = 128");
+    static_assert(DH == 64, "D = 32 is in evo_bwd_halves.cuh, 128 in evo_bwd_wide.cuh");
     static constexpr int NG = 4;                       // compute groups
     static constexpr int CW = TILE / NG;               // q columns per group
     static constexpr int NCW = 4 * NG;
     static constexpr int W_DRAIN = NCW, W_PROD = NCW + 4, W_MMA = NCW + 5;
     static constexpr int THREADS = (NCW + 8) * 32;
-    static constexpr int QS = (DH == 32) ? 3 : 2;      // Q/dO stages
-    static constexpr int NKV = (DH == 32) ? 2 : 1;     // K/V buffers
+    static constexpr int QS = 2;                       // Q/dO stages
+    static constexpr int NKV = 1;                      // K/V buffers
     static constexpr int NB = 2;                       // bias tiles
     static constexpr int DQ_BUFS = 2;
     static constexpr uint32_t ROWT = RowTile<DH>::BYTES;
@@ -165,26 +161,22 @@ struct BwdCfg {
     static constexpr uint32_t OFF_KV = OFF_STAGE + QS * STAGE_BYTES;
     static constexpr uint32_t OFF_BIAS = OFF_KV + NKV * KV_BYTES;
     static constexpr uint32_t OFF_DS = OFF_BIAS + NB * SQ_BYTES;
-    // per drain warp: WSLOTS slots of [32 rows][32 fp32], for bulk copies of dQ, dK and dV
+    // per drain warp a slot of [32 rows][32 fp32], for bulk copies of dQ, dK and dV
     static constexpr uint32_t WQ_BYTES = 32 * 32 * 4;
-    static constexpr int WSLOTS = (DH == 32) ? 2 : 1;
     static constexpr uint32_t OFF_WSTG = OFF_DS + SQ_BYTES;
     // constant extra tiles, above every tile that refers to the zero tile
-    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WSLOTS * WQ_BYTES;            // row selector of -delta
+    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WQ_BYTES;            // row selector of -delta
     static constexpr uint32_t OFF_ZERO = OFF_XDP + XT_BYTES;
     static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr uint32_t NUM_BARS = 2 * QS + 2 * NKV + 2 * NB + 2 * DQ_BUFS + 9;
+    static constexpr uint32_t NUM_BARS = 2 * QS + 2 * NKV + 2 * NB + 2 * DQ_BUFS + 8;
     static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
     static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + alignment slack
     static constexpr uint32_t TMEM_S = 0, TMEM_DP = 128;
-    static constexpr uint32_t TMEM_P = 256;                                 // not ALIAS: P^T, then dS^T
-    static constexpr uint32_t TMEM_DQ = ALIAS ? 256 : 384;               // DQ_BUFS accumulators
+    static constexpr uint32_t TMEM_DQ = 256;                                // DQ_BUFS accumulators
     static constexpr uint32_t TMEM_DK = TMEM_DQ + 2 * DH, TMEM_DV = TMEM_DK + DH;
-    // column of contraction block kk (16 q) of P^T / dS^T: dense, or inside the columns of its own group
-    __device__ static __forceinline__ uint32_t p_col(int kk) {
-        return ALIAS ? TMEM_S + 32 * (kk >> 1) + 8 * (kk & 1) : TMEM_P + 8 * kk;
-    }
-    __device__ static __forceinline__ uint32_t ds_col(int kk) { return p_col(kk) + (ALIAS ? 128 : 64); }
+    // column of contraction block kk (16 q) of P^T / dS^T, inside the columns of its own group
+    __device__ static __forceinline__ uint32_t p_col(int kk) { return TMEM_S + 32 * (kk >> 1) + 8 * (kk & 1); }
+    __device__ static __forceinline__ uint32_t ds_col(int kk) { return p_col(kk) + 128; }
     static_assert(TMEM_DV + DH <= BWD_TMEM_COLS, "tensor memory budget");
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
     static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
@@ -214,12 +206,11 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     uint64_t* dq_full = bias_empty + NB;       // [DQB]
     uint64_t* dq_free = dq_full + DQB;         // [DQB]
     uint64_t* dp_full = dq_free + DQB;         // dP' complete
-    uint64_t* s_free = dp_full + 1;            // S', dP' are read (one phase)
-    uint64_t* p_ready = s_free + 1;            // P^T is written (two phases)
+    uint64_t* p_ready = dp_full + 1;           // P^T is written
     uint64_t* ds_ready = p_ready + 1;          // dS^T and the dS tile are written
     uint64_t* dv_done = ds_ready + 1;          // dV of the step is complete
     uint64_t* dk_done = dv_done + 1;           // dK
-    uint64_t* dq_done = dk_done + 1;           // dQ; one phase: dV, dK and dQ
+    uint64_t* dq_done = dk_done + 1;           // dQ
     uint64_t* dkv_full = dq_done + 1;          // dK, dV of the segment are complete
     uint64_t* dkv_free = dkv_full + 1;         // ... and read out
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
@@ -238,9 +229,8 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int i = 0; i < NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
         for (int i = 0; i < NB; ++i) { mbar_init(&s_full[i], 2); mbar_init(&bias_empty[i], C::NCW); }
         for (int i = 0; i < DQB; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
-        for (uint64_t* x : {s_free, p_ready, ds_ready}) mbar_init(x, C::NCW);
-        for (uint64_t* x : {dp_full, dv_done, dk_done, dkv_full}) mbar_init(x, 1);
-        mbar_init(dq_done, C::TWO_PHASE ? 1 : 2);
+        for (uint64_t* x : {p_ready, ds_ready}) mbar_init(x, C::NCW);
+        for (uint64_t* x : {dp_full, dv_done, dk_done, dq_done, dkv_full}) mbar_init(x, 1);
         mbar_init(dkv_free, 4);
         fence_mbar_init();
     }
@@ -349,8 +339,8 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (role == 0) {
                     ok = warp_all(mbar_wait(&st_full[st], (gs / QS) & 1, wc, 0x50));
                     if (ok && i == 0) ok = warp_all(mbar_wait(&kv_full[kb], (sg / NKV) & 1, wc, 0x51));
-                    // the columns are read, or (ALIAS) P^T in them is consumed
-                    if (ok && gs > 0) ok = warp_all(mbar_wait(C::ALIAS ? dv_done : s_free, (gs - 1) & 1, wc, 0x52));
+                    // P^T in the columns is consumed
+                    if (ok && gs > 0) ok = warp_all(mbar_wait(dv_done, (gs - 1) & 1, wc, 0x52));
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t d_xq = xt_desc(sb + C::ST_XQ, aZero);
@@ -362,10 +352,10 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                                 umma_ss(tmem + C::TMEM_S, RD::kmajor(k_lo, kk), RD::kmajor(q_lo, kk), IDESC_SDP, kk > 0);
                         // + (mask - LSE) / scale: the extra contraction block
                         umma_ss(tmem + C::TMEM_S, xt_desc(kvb + C::KV_XK, aZero), d_xq, IDESC_SDP, 1u);
-                        if (C::TWO_PHASE) umma_commit(&s_full[gs % NB]);
+                        umma_commit(&s_full[gs % NB]);
                     }
                     __syncwarp();
-                    if (C::TWO_PHASE && gs > 0) ok = warp_all(mbar_wait(dk_done, (gs - 1) & 1, wc, 0x59));
+                    if (gs > 0) ok = warp_all(mbar_wait(dk_done, (gs - 1) & 1, wc, 0x59));
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -376,7 +366,7 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                                 umma_ss(tmem + C::TMEM_DP, RD::kmajor(v_lo, kk), RD::kmajor(do_lo, kk), IDESC_SDP, kk > 0);
                         // - delta
                         umma_ss(tmem + C::TMEM_DP, xt_desc(smem_u32(smem + C::OFF_XDP), aZero), d_xq, IDESC_SDP, 1u);
-                        umma_commit(C::TWO_PHASE ? dp_full : &s_full[gs % NB]);
+                        umma_commit(dp_full);
                     }
                     __syncwarp();
                 } else if (role == 1) {
@@ -390,30 +380,22 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     auto dk = [&](int kk) {
                         umma_ts(tmem + C::TMEM_DK, tmem + C::ds_col(kk), RD::mnmajor(q_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
                     };
-                    if constexpr (C::TWO_PHASE) {
-                        if (ok) ok = warp_all(mbar_wait(p_ready, gs & 1, wc, 0x53));
-                        if (!ok) break;
-                        tc_fence_after();
-                        if (elect_one()) {
-#pragma unroll
-                            for (int kk = 0; kk < 8; ++kk) dv(kk);
-                            umma_commit(dv_done);
-                        }
-                        __syncwarp();
-                    }
-                    if (ok) ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5a));
+                    if (ok) ok = warp_all(mbar_wait(p_ready, gs & 1, wc, 0x53));
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        if constexpr (C::TWO_PHASE) {
 #pragma unroll
-                            for (int kk = 0; kk < 8; ++kk) dk(kk);
-                            umma_commit(dk_done);
-                        } else {
+                        for (int kk = 0; kk < 8; ++kk) dv(kk);
+                        umma_commit(dv_done);
+                    }
+                    __syncwarp();
+                    ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5a));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < 8; ++kk) { dv(kk); dk(kk); }      // two interleaved chains
-                            umma_commit(dq_done);
-                        }
+                        for (int kk = 0; kk < 8; ++kk) dk(kk);
+                        umma_commit(dk_done);
                         umma_commit(&st_empty[st]);
                         if (i == NT - 1) {
                             umma_commit(dkv_full);
@@ -449,20 +431,20 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int w4 = warp & 3;
         const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
-        uint8_t* const wslot = smem + C::OFF_WSTG + w4 * C::WSLOTS * C::WQ_BYTES;
-        // Where the next bulk copy (one group each) is staged, once the copy that used the place last has read it:
-        // two slots in turn, or with one slot its two halves for copies of half its size.
+        uint8_t* const wslot = smem + C::OFF_WSTG + w4 * C::WQ_BYTES;
+        // Where the next bulk copy (one group each) is staged, once the copy that used the place last has read it: the
+        // slot, or its halves in turn for copies of half its size.
         int pos = 0;
         bool last_half = false;
         auto next_slot = [&](bool half) -> uint8_t* {
             if (lane == 0) {
-                if (C::WSLOTS == 2 || (half && last_half)) tma_wait_group_read<1>();
+                if (half && last_half) tma_wait_group_read<1>();
                 else tma_wait_group_read<0>();
             }
             __syncwarp();
             last_half = half;
             pos ^= 1;
-            return wslot + (C::WSLOTS == 2 ? pos * C::WQ_BYTES : (half ? pos * (C::WQ_BYTES / 2) : 0));
+            return wslot + (half ? pos * (C::WQ_BYTES / 2) : 0);
         };
         // 32 columns of 32 rows as bf16, by a bulk tensor store (which clips rows past N and columns past Dt)
         auto store_rows = [&](const CUtensorMap* tm, const uint4 (&u)[4], int h, int row0, int col0, int bs) {
@@ -630,131 +612,73 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if constexpr (DBIAS_HERE != DBIAS_NO) seg.decode(sg, bs, h, j);
             for (int i = 0; i < NT && ok; ++i, ++gs) {
                 const int bb = gs % NB;
-                if constexpr (C::TWO_PHASE) {
-                    // ---- phase P: x = S' c1 + bias log2e (S' already carries mask and -LSE through the extra
-                    // contraction block), P = exp2(x), P^T (bf16) into tensor memory
-                    // (S' of this step waited for dV of the previous one: its columns are free)
-                    ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
-                    if (!ok) break;
-                    tc_fence_after();
-                    float2 p2[16];
-                    uint32_t dep = 0;
+                // ---- phase P: x = S' c1 + bias log2e (S' already carries mask and -LSE through the extra
+                // contraction block), P = exp2(x), P^T (bf16) into tensor memory
+                // (S' of this step waited for dV of the previous one: its columns are free)
+                ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
+                if (!ok) break;
+                tc_fence_after();
+                float2 p2[16];
+                uint32_t dep = 0;
 #pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
-                        uint32_t sv[16], bq[16];
-                        tmem_ld16(tS + 16 * ch, sv);
+                for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
+                    uint32_t sv[16], bq[16];
+                    tmem_ld16(tS + 16 * ch, sv);
 #pragma unroll
-                        for (int k = 0; k < 16; ++k)
-                            bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
-                        tmem_wait_ld();
-                        uint32_t pk[8];
+                    for (int k = 0; k < 16; ++k)
+                        bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
+                    tmem_wait_ld();
+                    uint32_t pk[8];
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
-                            const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
-                            const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
-                            p2[8 * ch + k] = e2;
-                            pk[k] = pack_bf16(e2.x, e2.y);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) dep ^= pk[k];      // depends on every bias value read
-                        tmem_st8(lane_base + C::p_col(2 * g + ch), pk);
+                    for (int k = 0; k < 8; ++k) {
+                        const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
+                        const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
+                        const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
+                        p2[8 * ch + k] = e2;
+                        pk[k] = pack_bf16(e2.x, e2.y);
                     }
-                    mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(p_ready);
-
-                    // ---- phase dS: dS = P dP' (dP' already carries -delta), dS^T into tensor memory and the tile.
-                    // Both are free once dK and dQ of the previous step are complete.
-                    if (gs == 0)
-                        ok = warp_all(mbar_wait(dp_full, 0, wc, 0x66));
-                    else                           // (dP' of this step waited for dK)
-                        ok = warp_all(mbar_wait_both(dp_full, gs & 1, dq_done, (gs - 1) & 1, wc, 0x66));
-                    if (!ok) break;
-                    tc_fence_after();
 #pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {
-                        uint32_t dv[16];
-                        tmem_ld16(tDP + 16 * ch, dv);
-                        tmem_wait_ld();
-                        uint32_t pkd[8];
-                        float2 dsv[8];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            dsv[k] = fmul2(p2[8 * ch + k], u2f2(dv[2 * k], dv[2 * k + 1]));
-                            pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
-                        }
-                        tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-                            sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
-                                   make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
-                        store_dbias(ch, i, j, bs, h, pkd, dsv);
-                    }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(ds_ready);
-                } else {
-                    // One phase: per element x = S' c1 + bias log2e (S' already carries mask and -LSE through the
-                    // extra contraction block), P = exp2(x), dS = P dP' (dP' already carries -delta).
-                    ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
-                    if (!ok) break;
-                    tc_fence_after();
-                    uint32_t dep = 0;
-#pragma unroll
-                    for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
-                        uint32_t sv[16], dv[16], bq[16];
-                        tmem_ld16(tS + 16 * ch, sv);
-                        tmem_ld16(tDP + 16 * ch, dv);
-#pragma unroll
-                        for (int k = 0; k < 16; ++k)
-                            bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
-                        tmem_wait_ld();
-                        if (ch == 1) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(s_free);
-                        }
-                        uint32_t pkp[8], pkd[8];
-                        float2 dsv[8];
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
-                            const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
-                            const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
-                            dsv[k] = fmul2(e2, u2f2(dv[2 * k], dv[2 * k + 1]));
-                            pkp[k] = pack_bf16(e2.x, e2.y);
-                            pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) dep ^= pkp[k];     // depends on every bias value read
-                        if (ch == 1) {
-                            mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
-                        } else if (gs > 0) {
-                            // P^T, dS^T and the dS tile are free once the previous step's MMAs are done
-                            ok = warp_all(mbar_wait(dq_done, (gs - 1) & 1, wc, 0x61));
-                            if (!ok) break;
-                            tc_fence_after();
-                        }
-                        tmem_st8(lane_base + C::p_col(2 * g + ch), pkp);
-                        tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-                            sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
-                                   make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
-                        store_dbias(ch, i, j, bs, h, pkd, dsv);
-                    }
-                    if (!ok) break;
-                    tmem_wait_st();
-                    tc_fence_before();
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(ds_ready);
+                    for (int k = 0; k < 8; ++k) dep ^= pk[k];      // depends on every bias value read
+                    tmem_st8(lane_base + C::p_col(2 * g + ch), pk);
                 }
+                mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_ready);
+
+                // ---- phase dS: dS = P dP' (dP' already carries -delta), dS^T into tensor memory and the tile.
+                // Both are free once dK and dQ of the previous step are complete.
+                if (gs == 0)
+                    ok = warp_all(mbar_wait(dp_full, 0, wc, 0x66));
+                else                           // (dP' of this step waited for dK)
+                    ok = warp_all(mbar_wait_both(dp_full, gs & 1, dq_done, (gs - 1) & 1, wc, 0x66));
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t dv[16];
+                    tmem_ld16(tDP + 16 * ch, dv);
+                    tmem_wait_ld();
+                    uint32_t pkd[8];
+                    float2 dsv[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        dsv[k] = fmul2(p2[8 * ch + k], u2f2(dv[2 * k], dv[2 * k + 1]));
+                        pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
+                    }
+                    tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
+                               make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
+                    store_dbias(ch, i, j, bs, h, pkd, dsv);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ds_ready);
             }
         }
     }
@@ -1016,7 +940,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tdo, d_o, BS, d->N, d->H, Dt, TILE, lay_do, RowTile<DH>::BOX_D))) return rc;
-    if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N))) return rc;
+    if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N, DH == 32 ? TILE / 2 : TILE))) return rc;
 
     BwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
@@ -1062,14 +986,17 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         const size_t acc_n = static_cast<size_t>(pairs - full / d->H * d->H) * d->N;
         if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > room) p.n_whole = 0;
     }
-    // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; two at D <= 64)
-    if (p.n_whole == pairs && NT > (DH == 128 ? 1 : 2) && std::min(pairs, use_sms) * n32 > room) p.n_whole = 0;
+    // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; two at D = 64, four at D <= 32)
+    constexpr int TILES_HELD = DH == 128 ? 1 : (DH == 64 ? BwdCfg<64>::DQ_BUFS : BwdHalvesCfg::DQ_BUFS);
+    if (p.n_whole == pairs && NT > TILES_HELD && std::min(pairs, use_sms) * n32 > room) p.n_whole = 0;
     p.pairs = pairs;
     p.acc_row0 = p.n_whole / d->H;
     const int rest_rows = p.n_whole < pairs ? BS - p.acc_row0 : 0;
     const int grid = static_cast<int>(std::min<long>(p.n_whole ? pairs : static_cast<long>(pairs) * NT, use_sms));
     // workspace: the partial sums of every CTA with whole pairs, then the accumulator of the rest
     p.scratch_stride = n32 * DH / 4;
+    p.seg_dj = grid % NT;
+    p.seg_dp = grid / NT;
     p.dq_scratch = dq_ws;
     p.dq_acc = dq_ws + (p.n_whole ? grid : 0) * p.scratch_stride * 4;
     if constexpr (DH <= 64) {
@@ -1149,6 +1076,11 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             auto kernel = mode == DBIAS_NO ? evo_bwd_wide_kernel<DH, W, DBIAS_NO>
                                            : (mode == DBIAS_BF16 ? evo_bwd_wide_kernel<DH, W, DBIAS_BF16> : evo_bwd_wide_kernel<DH, W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
+        } else if constexpr (DH == 32) {
+            using C = BwdHalvesCfg;
+            auto kernel = mode == DBIAS_NO ? evo_bwd_halves_kernel<W, DBIAS_NO>
+                                           : (mode == DBIAS_BF16 ? evo_bwd_halves_kernel<W, DBIAS_BF16> : evo_bwd_halves_kernel<W, DBIAS_F32>);
+            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         } else {
             using C = BwdCfg<DH>;
             auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<DH, W, DBIAS_NO>

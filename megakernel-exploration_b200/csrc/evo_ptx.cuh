@@ -183,6 +183,22 @@ __device__ __forceinline__ void sts128(uint32_t saddr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// Four 8 x 8 blocks of 16-bit values; lane 8 i + r gives the address of row r of block i.
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t saddr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
+}
+__device__ __forceinline__ void stmatrix4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// An 8 x 8 block of 16-bit values, transposed between the threads.
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+    uint32_t d;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+
 // ---- TMA --------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -332,6 +348,32 @@ __device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t (&r)[32]
           "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
+}
+// Fragments: 32 lanes x 32 columns dealt to the warp as 8 x 8 blocks, like the operands of ldmatrix.  Thread t
+// holds row t / 4 and columns 2 (t % 4), + 1 of each block; word 16 hb + 4 cb + 2 m + e is column e of block (rows
+// 16 hb + 8 m, columns 8 cb).  (16 lanes a load.)
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t addr, uint32_t (&r)[32]) {
+#pragma unroll
+    for (int hb = 0; hb < 2; ++hb)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[16 * hb + 0]), "=r"(r[16 * hb + 1]), "=r"(r[16 * hb + 2]), "=r"(r[16 * hb + 3]), "=r"(r[16 * hb + 4]),
+              "=r"(r[16 * hb + 5]), "=r"(r[16 * hb + 6]), "=r"(r[16 * hb + 7]), "=r"(r[16 * hb + 8]), "=r"(r[16 * hb + 9]),
+              "=r"(r[16 * hb + 10]), "=r"(r[16 * hb + 11]), "=r"(r[16 * hb + 12]), "=r"(r[16 * hb + 13]),
+              "=r"(r[16 * hb + 14]), "=r"(r[16 * hb + 15])
+            : "r"(addr + (static_cast<uint32_t>(16 * hb) << 16))
+            : "memory");
+}
+// The same blocks as pairs of bf16, two columns a word: 32 lanes x 16 words, word 8 hb + 2 cb + m.
+__device__ __forceinline__ void tmem_st_frag16(uint32_t addr, const uint32_t (&r)[16]) {
+#pragma unroll
+    for (int hb = 0; hb < 2; ++hb)
+        asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     ::"r"(addr + (static_cast<uint32_t>(16 * hb) << 16)), "r"(r[8 * hb + 0]), "r"(r[8 * hb + 1]),
+                       "r"(r[8 * hb + 2]), "r"(r[8 * hb + 3]), "r"(r[8 * hb + 4]), "r"(r[8 * hb + 5]), "r"(r[8 * hb + 6]),
+                       "r"(r[8 * hb + 7])
+                     : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

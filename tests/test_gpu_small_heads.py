@@ -1,0 +1,32 @@
+"""dQ, dK, dV (and dBias of one S row) at head dims 16 and 32, at the edges of the kernel's tiles, halves and walks.
+
+A tile is 128 kv rows by two halves of 64 q columns; dQ of a (row, head) pair stays in tensor memory for up to four
+tiles and goes through a scratch area from five on; with more pairs than SMs the last ones are dealt by segments.
+"""
+import pytest
+import torch
+
+from oracle import evo_ref
+from _util import assert_parity, oracle_on_rounded, run_layer
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [8, 64, 72, 128, 136, 192, 200, 256, 384, 392, 456, 512, 520, 648]
+
+
+@pytest.mark.parametrize("S", [1, 3])
+@pytest.mark.parametrize("N", SIZES)
+@pytest.mark.parametrize("D,bias_type", [(16, torch.float32), (32, torch.bfloat16), (32, torch.float32)])
+def test_tiles_and_halves(D, bias_type, N, S):
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(2, S, N, 2, D, 0.5, 1.0, "bernoulli0.9", seed=N + S)
+    got = run_layer(q, k, v, mask, bias, d_o, bias_type=bias_type)
+    assert_parity(oracle_on_rounded(q, k, v, mask, bias, d_o), got, dbias_type=bias_type, tag=f"N={N} S={S} D={D}")
+
+
+@pytest.mark.parametrize("N", [120, 264, 520])
+def test_pairs_left_over_after_full_rounds(N):
+    # whole pairs on every SM, then segments of the rest; two rounds of whole pairs before them at N = 120
+    S = 80 if N == 120 else 40
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(1, S, N, 4, 32, 0.5, 1.0, "tail0to32", seed=N)
+    got = run_layer(q, k, v, mask, bias, d_o)
+    assert_parity(oracle_on_rounded(q, k, v, mask, bias, d_o), got, tag=f"N={N} S={S}")
