@@ -82,9 +82,10 @@ struct FwdParams {
 // 0.585 -> 0.540 ms).
 //
 // The streams are at different places of their code at any time, and what they fetch competes for the instruction cache
-// (a warp in seven that could have issued waited for an instruction): short waits and one copy of the producer's loop for
-// all streams, 105 -> 61 KB of code at D = 32: B=1, S=512, N=384, H=8 0.302 -> 0.293 ms; S=200, N=200, H=4 45 -> 38 us; at
-// D = 64 S=256, N=1024, H=4 645 -> 562 us.  (Rolling the loops over a tile's chunks as well: no gain.)
+// (a warp in seven that could have issued waited for an instruction).  Short waits, 105 -> 83 KB of code: B=1, S=512, N=384,
+// H=8, D=32 0.302 -> 0.277 ms; S=200, N=200, H=4 44 -> 40 us; S=256, N=1024, H=4, D=64 640 -> 575.  The producer's loop stays
+// unrolled over the streams, its masks requested ahead: one copy of it for all streams was 0.298 ms at the first shape (one
+// warp is then too slow for three streams).  Rolling the loops over a tile's chunks: no gain.
 //
 // One maximum per 128 columns instead of one per 64 leaves one exact P a row and tile instead of two: O is 2 to 3 %
 // further from 64 bits (relative error 2.11e-3 -> 2.16e-3 at N = 264, D = 64, of which 1.66e-3 is its own bf16).  Two
@@ -276,22 +277,18 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Round r holds tile r of every stream (item r / NT, kv tile r % NT): the bias tile, then Q per
             // item, K and the mask tile.  (V is fetched by the stream's MMA warp, the first to know that its
             // buffer is free.)  The warp runs with all lanes and elects one to issue.
-            // Lane s keeps the state of stream s, so that the loop over streams stays one copy of its code (unrolled it
-            // was 39 of the kernel's 90 KB).
-            const int ls = lane < G ? lane : 0;
-            FwdItem item = items_of(ls);
-            int used = 0, qn = 0;    // tiles and items of the stream so far
+            int used[G], qn[G];      // tiles and items of the stream so far
+            FwdItem item[3] = {items_of(0), items_of(1), items_of(2)};      // the first G of them are walked
+#pragma unroll
+            for (int s = 0; s < G; ++s) used[s] = qn[s] = 0;
             bool ok = true;
             int r = 0;
             for (int it = 0; it < n_items && ok; ++it) {
                 for (int j = 0; j < NT && ok; ++j, ++r) {
-#pragma unroll 1
+#pragma unroll
                     for (int s = 0; s < G; ++s) {
-                        auto of = [&](int x) { return __shfl_sync(0xffffffffu, x, s); };
-                        const FwdItem cur{of(item.h), of(item.qt), of(item.row), of(item.b)};
-                        const int n = of(used), q = of(qn);
-                        if (!ok || !cur.valid(p)) continue;
-                        const int bs = cur.bs(p), qt = cur.qt, h = cur.h;
+                        if (!ok || !item[s].valid(p)) continue;
+                        const int bs = item[s].bs(p), qt = item[s].qt, h = item[s].h;
                         const FwdBars b(bars + s * C::BARS);
                         uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
                         // four mask values per lane, requested before the waits
@@ -299,8 +296,8 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         uint2 mw = make_uint2(0u, 0u);
                         if (c < p.N) mw = __ldg(reinterpret_cast<const uint2*>(p.mask + static_cast<size_t>(bs) * p.N + c));
                         if (j == 0) {
-                            const int qb = q % NQ, use = q / NQ;
-                            if (q >= NQ) ok = warp_all(mbar_wait(&b.q_empty[qb], (use - 1) & 1, wc, 0x10));
+                            const int qb = qn[s] % NQ, use = qn[s] / NQ;
+                            if (qn[s]++ >= NQ) ok = warp_all(mbar_wait(&b.q_empty[qb], (use - 1) & 1, wc, 0x10));
                             if (ok && elect_one()) {
                                 mbar_arrive_expect_tx(&b.q_full[qb], C::ROWT);
                                 tma_load_row_tile<DH>(sb + C::ST_Q + qb * C::ROWT, &tm_q, &b.q_full[qb], h, qt * TILE, bs);
@@ -308,8 +305,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             __syncwarp();
                         }
                         if (!ok) continue;
-                        if (lane == s) { ++used; qn += j == 0; }
-                        const int kb = n % NK;
+                        const int n = used[s]++, kb = n % NK;
                         if (n >= NK) ok = warp_all(mbar_wait(&b.k_empty[kb], ((n / NK) - 1) & 1, wc, 0x11));
                         if (!ok) continue;
                         if (elect_one()) {
@@ -335,23 +331,23 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             if (ok && elect_one()) {
                                 uint8_t* bt = smem + C::OFF_BIAS + slot * SQ_BYTES;
                                 mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
-                                tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, cur.b);
-                                tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, cur.b);
+                                tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, item[s].b);
+                                tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, item[s].b);
                             }
                             __syncwarp();
                         }
                     }
                 }
-                advance(item, ls);
+#pragma unroll
+                for (int s = 0; s < G; ++s) advance(item[s], s);
             }
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
-#pragma unroll 1
+#pragma unroll
             for (int s = 0; s < G; ++s) {
                 const FwdBars b(bars + s * C::BARS);
-                const int n = __shfl_sync(0xffffffffu, used, s), q = __shfl_sync(0xffffffffu, qn, s);
-                for (int k = (n > NK ? n - NK : 0); k < n; ++k) (void)mbar_wait(&b.k_full[k % NK], (k / NK) & 1, dc, 0x12);
-                for (int k = (q > NQ ? q - NQ : 0); k < q; ++k) (void)mbar_wait(&b.q_full[k % NQ], (k / NQ) & 1, dc, 0x13);
+                for (int k = (used[s] > NK ? used[s] - NK : 0); k < used[s]; ++k) (void)mbar_wait(&b.k_full[k % NK], (k / NK) & 1, dc, 0x12);
+                for (int k = (qn[s] > NQ ? qn[s] - NQ : 0); k < qn[s]; ++k) (void)mbar_wait(&b.q_full[k % NQ], (k / NQ) & 1, dc, 0x13);
             }
         } else if (warp - C::W_PROD - 1 < G) {
             // ------------------------------ MMA warp of one stream ------------------------------

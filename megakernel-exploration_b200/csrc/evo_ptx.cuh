@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t global_ns() {
 
 // Bounded wait on phase `parity` of `bar` with explicit limits (iterations, nanoseconds).  The code behind the first
 // probe is short because it is in every role of a kernel a dozen times, and roles at different places of their code
-// compete for the instruction cache (the forward at D = 32: 105 -> 90 KB of code, 0.302 -> 0.296 ms at B=1, S=512, N=384,
+// compete for the instruction cache (the forward at D = 32: 105 -> 83 KB of code, 0.302 -> 0.277 ms at B=1, S=512, N=384,
 // H=8); the status word is written once, when the kernel ends (report_abort).
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, const WaitCtx& w,
                                                   uint32_t site, uint32_t max_iters, uint32_t max_ns) {
