@@ -270,7 +270,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {          // S', then dP' of one half, then of the other
                         const int hf = t >> 1, part = t & 1;
-                        if (gs > 0 && part == 0) ok = warp_all(mbar_wait(&s_free[hf], (gs - 1) & 1, wc, 0x52));
+                        if (ok && gs > 0 && part == 0) ok = warp_all(mbar_wait(&s_free[hf], (gs - 1) & 1, wc, 0x52));
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {
