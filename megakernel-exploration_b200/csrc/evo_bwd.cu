@@ -224,7 +224,7 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
     if (tid == 0) {
         *abort_flag = 0;
-        tmem_slot[3] = 0;                      // the flag of the waits before exit: never set
+        tmem_slot[3] = 0;                      // the abort word of the waits before exit
         for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
         for (int i = 0; i < NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
         for (int i = 0; i < NB; ++i) { mbar_init(&s_full[i], 2); mbar_init(&bias_empty[i], C::NCW); }
@@ -313,8 +313,8 @@ evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
         // barrier with an MMA commit, which may then never come: a bounded pause instead).
         const WaitCtx dc{tmem_slot + 3, p.status};
-        for (int k = (n_st > QS ? n_st - QS : 0); k < n_st; ++k) (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, dc, 0x43);
-        for (int k = (n_kv > NKV ? n_kv - NKV : 0); k < n_kv; ++k) (void)mbar_wait(&kv_full[k % NKV], (k / NKV) & 1, dc, 0x45);
+        for (int k = (n_st > QS ? n_st - QS : 0); k < n_st; ++k) mbar_wait_landed(&st_full[k % QS], (k / QS) & 1, dc, 0x43);
+        for (int k = (n_kv > NKV ? n_kv - NKV : 0); k < n_kv; ++k) mbar_wait_landed(&kv_full[k % NKV], (k / NKV) & 1, dc, 0x45);
         if (!ok && n_bias > 0)
             for (int k = 0; k < 64; ++k) __nanosleep(1000);
     } else if (warp >= C::W_MMA) {

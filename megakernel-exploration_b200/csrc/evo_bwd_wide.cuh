@@ -86,7 +86,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
     if (tid == 0) {
         *abort_flag = 0;
-        tmem_slot[3] = 0;                      // the flag of the waits before exit: never set
+        tmem_slot[3] = 0;                      // the abort word of the waits before exit
         for (uint64_t* b : {do_full, do_empty, q_full, q_empty, kv_full, dv_done, dk_done, dq_full, dkv_full}) mbar_init(b, 1);
         for (uint64_t* b : {kv_empty, sdp_full}) mbar_init(b, 2);
         for (uint64_t* b : {bias_empty, pds_ready, dq_free, dkv_free}) mbar_init(b, C::NCW);
@@ -169,9 +169,9 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
         // barrier with an MMA commit, which may then never come: a bounded pause instead).
         const WaitCtx dc{tmem_slot + 3, p.status};
-        if (n_do > 0) (void)mbar_wait(do_full, (n_do - 1) & 1, dc, 0x43);
-        if (n_q > 0) (void)mbar_wait(q_full, (n_q - 1) & 1, dc, 0x47);
-        if (n_kv > 0) (void)mbar_wait(kv_full, (n_kv - 1) & 1, dc, 0x45);
+        if (n_do > 0) mbar_wait_landed(do_full, (n_do - 1) & 1, dc, 0x43);
+        if (n_q > 0) mbar_wait_landed(q_full, (n_q - 1) & 1, dc, 0x47);
+        if (n_kv > 0) mbar_wait_landed(kv_full, (n_kv - 1) & 1, dc, 0x45);
         if (!ok && n_bias > 0)
             for (int k = 0; k < 64; ++k) __nanosleep(1000);
     } else if (warp >= C::W_MMA) {

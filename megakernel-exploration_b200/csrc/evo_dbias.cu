@@ -117,7 +117,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
     if (tid == 0) {
         *abort_flag = 0;
-        tmem_slot[3] = 0;                   // the flag of the waits before exit: never set
+        tmem_slot[3] = 0;                   // the abort word of the waits before exit
         for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 2); mbar_init(&st_empty[i], 2); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sdp_full[i], 2); mbar_init(&sdp_free[i], NCW); }
         fence_mbar_init();
@@ -207,7 +207,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // of a stage may then never have been asked for: a bounded pause instead)
             const WaitCtx dc{tmem_slot + 3, p.status};
             if (ok && !*abort_flag)
-                for (int k = (ld > QS ? ld - QS : 0); k < ld; ++k) (void)mbar_wait(&st_full[k % QS], (k / QS) & 1, dc, 0x83);
+                for (int k = (ld > QS ? ld - QS : 0); k < ld; ++k) mbar_wait_landed(&st_full[k % QS], (k / QS) & 1, dc, 0x83);
             else
                 for (int k = 0; k < 64; ++k) __nanosleep(1000);
         } else if (warp == NCW + 1 || warp == NCW + 2) {

@@ -217,7 +217,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
     if (tid == 0) {
         *abort_flag = 0;
-        tmem_slot[3] = 0;                   // the flag of the waits before exit: never set
+        tmem_slot[3] = 0;                   // the abort word of the waits before exit
         for (int s = 0; s < G; ++s) {
             const FwdBars b(bars + s * C::BARS);
             for (int i = 0; i < NQ; ++i) { mbar_init(&b.q_full[i], 1); mbar_init(&b.q_empty[i], 1); }
@@ -346,8 +346,8 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int s = 0; s < G; ++s) {
                 const FwdBars b(bars + s * C::BARS);
-                for (int k = (used[s] > NK ? used[s] - NK : 0); k < used[s]; ++k) (void)mbar_wait(&b.k_full[k % NK], (k / NK) & 1, dc, 0x12);
-                for (int k = (qn[s] > NQ ? qn[s] - NQ : 0); k < qn[s]; ++k) (void)mbar_wait(&b.q_full[k % NQ], (k / NQ) & 1, dc, 0x13);
+                for (int k = (used[s] > NK ? used[s] - NK : 0); k < used[s]; ++k) mbar_wait_landed(&b.k_full[k % NK], (k / NK) & 1, dc, 0x12);
+                for (int k = (qn[s] > NQ ? qn[s] - NQ : 0); k < qn[s]; ++k) mbar_wait_landed(&b.q_full[k % NQ], (k / NQ) & 1, dc, 0x13);
             }
         } else if (warp - C::W_PROD - 1 < G) {
             // ------------------------------ MMA warp of one stream ------------------------------
@@ -470,7 +470,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             if (elect_one()) tma_wait_group<0>();
             __syncwarp();
-            if (loaded > 0) (void)mbar_wait(b.v_full, (loaded - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x26);
+            if (loaded > 0) mbar_wait_landed(b.v_full, (loaded - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x26);
         }
     } else {
         reg_inc<C::REGS_SOFTMAX>();

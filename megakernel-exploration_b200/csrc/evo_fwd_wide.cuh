@@ -89,7 +89,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
     if (tid == 0) {
         *abort_flag = 0;
-        tmem_slot[3] = 0;                   // the flag of the waits before exit: never set
+        tmem_slot[3] = 0;                   // the abort word of the waits before exit
         for (int i = 0; i < 2; ++i) {
             mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
             mbar_init(&v_full[i], 1);
@@ -214,11 +214,11 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
-            if (n_k0 > 0) (void)mbar_wait(&k_full[0], (n_k0 - 1) & 1, dc, 0x13);
-            if (n_k1 > 0) (void)mbar_wait(&k_full[1], (n_k1 - 1) & 1, dc, 0x13);
-            if (n_v > 0) (void)mbar_wait(v_full, (n_v - 1) & 1, dc, 0x14);
-            if (n_q0 > 0) (void)mbar_wait(&q_full[0], (n_q0 - 1) & 1, dc, 0x15);
-            if (n_q1 > 0) (void)mbar_wait(&q_full[1], (n_q1 - 1) & 1, dc, 0x15);
+            if (n_k0 > 0) mbar_wait_landed(&k_full[0], (n_k0 - 1) & 1, dc, 0x13);
+            if (n_k1 > 0) mbar_wait_landed(&k_full[1], (n_k1 - 1) & 1, dc, 0x13);
+            if (n_v > 0) mbar_wait_landed(v_full, (n_v - 1) & 1, dc, 0x14);
+            if (n_q0 > 0) mbar_wait_landed(&q_full[0], (n_q0 - 1) & 1, dc, 0x15);
+            if (n_q1 > 0) mbar_wait_landed(&q_full[1], (n_q1 - 1) & 1, dc, 0x15);
         } else if (warp == C::W_BIAS) {
             // ------------------------------ bias ------------------------------
             FwdItem cur0 = items_of(0), cur1 = items_of(1);
@@ -249,7 +249,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             const WaitCtx dc{tmem_slot + 3, p.status};
             for (int i = (n_loads > NF ? n_loads - NF : 0); i < n_loads; ++i)
-                (void)mbar_wait(&bias_full[i % NF], WideBiasRing::full_parity(i / NF), dc, 0x17);
+                mbar_wait_landed(&bias_full[i % NF], WideBiasRing::full_parity(i / NF), dc, 0x17);
         } else {
             // ------------------------------ MMA warp of one stream ------------------------------
             const int s = warp - C::W_MMA;
@@ -312,7 +312,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 advance(cur);
             }
-            if (n_v > 0) (void)mbar_wait(vf, (n_v - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x18);
+            if (n_v > 0) mbar_wait_landed(vf, (n_v - 1) & 1, WaitCtx{tmem_slot + 3, p.status}, 0x18);
         }
     } else {
         reg_inc<C::REGS_SOFTMAX>();

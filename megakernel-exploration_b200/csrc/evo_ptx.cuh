@@ -112,7 +112,9 @@ __device__ __forceinline__ uint32_t global_ns() {
 // Bounded wait on phase `parity` of `bar` with explicit limits (iterations, nanoseconds).  The code behind the first
 // probe is short because it is in every role of a kernel a dozen times, and roles at different places of their code
 // compete for the instruction cache (the forward at D = 32: 105 -> 83 KB of code, 0.302 -> 0.277 ms at B=1, S=512, N=384,
-// H=8); the status word is written once, when the kernel ends (report_abort).
+// H=8); the status word is written once, when the kernel ends (report_abort).  HEED: returns soon after any other wait
+// with the same abort word gave up.
+template <bool HEED = true>
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, const WaitCtx& w,
                                                   uint32_t site, uint32_t max_iters, uint32_t max_ns) {
     const uint32_t a = smem_u32(bar);
@@ -121,7 +123,7 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
     uint32_t it = 0;
 #pragma unroll 1
     while (!mbar_try_wait(a, parity))
-        if ((++it & 63u) == 0u && (*w.abort_flag || it >= max_iters || global_ns() - t0 > max_ns)) {
+        if ((++it & 63u) == 0u && ((HEED && *w.abort_flag) || it >= max_iters || global_ns() - t0 > max_ns)) {
             if (*w.abort_flag == 0u) *w.abort_flag = site | (ST_WAIT_TIMEOUT << 16);
             return false;
         }
@@ -132,6 +134,12 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtx& w,
                                           uint32_t site) {
     return mbar_wait_limited(bar, parity, w, site, EVO_WAIT_LIMIT, EVO_WAIT_NS);
+}
+
+// Before exit: for a load in flight, which must land before its CTA's shared memory is another's, whatever has given up.  Each
+// of these waits has limits of its own, also after one of them ran out.
+__device__ __forceinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity, const WaitCtx& w, uint32_t site) {
+    (void)mbar_wait_limited<false>(bar, parity, w, site, EVO_WAIT_LIMIT, EVO_WAIT_NS);
 }
 
 // Two barriers at once: both probes are in flight together, which costs a ready pair one latency.

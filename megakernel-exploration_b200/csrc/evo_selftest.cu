@@ -258,7 +258,8 @@ static int launch_selftest_xt(const void* y, const void* z, const void* a, const
 // nobody arrives at, gives up after `limit_ns`, records (ST_WAIT_TIMEOUT, site 0xee) in
 // the status word and raises the CTA's abort flag; warp 1 waits on a second such barrier
 // with the library's normal limits and must be released by the abort flag long before
-// those run out.  Then the kernel returns normally: no trap, no fault, no unbounded spin.
+// those run out; then it waits as for a load in flight, another `limit_ns`.  Then the kernel returns normally: no trap,
+// no fault, no unbounded spin.
 __global__ void __launch_bounds__(64, 1) selftest_wait_kernel(uint32_t limit_ns, unsigned int* status,
                                                               unsigned int* released) {
     __shared__ uint64_t bars[2];
@@ -280,6 +281,8 @@ __global__ void __launch_bounds__(64, 1) selftest_wait_kernel(uint32_t limit_ns,
         ok = warp_all(mbar_wait(&bars[1], 0, wc, 0xef));
         // released by the abort flag, not by its own limit: it never reports
         if (!ok && tid == 32) *released = (*abort_flag != 0u) ? 1u : 0u;
+        // ... and a wait for a load in flight lasts as long as its own limit all the same
+        if (!ok) (void)mbar_wait_limited<false>(&bars[1], 0, wc, 0xed, EVO_WAIT_LIMIT, limit_ns);
     }
     __syncthreads();
     if (tid == 0) report_abort(wc);

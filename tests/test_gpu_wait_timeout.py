@@ -36,6 +36,20 @@ def test_wait_runs_out_and_context_survives():
     assert_parity(oracle_on_rounded(q, k, v, mask, bias, d_o), got, tag="after time-out")
 
 
+def test_wait_before_exit_has_a_limit_of_its_own():
+    # the released warp then waits for a load that does not land: another 20 ms, not until the next look at the abort word
+    import _evoattn
+    released = torch.zeros(1, dtype=torch.int32, device="cuda")
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record()
+    _evoattn.selftest_wait_timeout(20_000_000, released, torch.cuda.current_stream().cuda_stream)
+    end.record()
+    with pytest.raises(_evoattn.EvoAttnError):
+        _evoattn.device_status()
+    assert released.item() == 1
+    assert 40 <= start.elapsed_time(end) < 1000
+
+
 def test_wait_limit_argument_is_checked():
     import _evoattn
     released = torch.zeros(1, dtype=torch.int32, device="cuda")
