@@ -498,34 +498,42 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         int gs = 0;
         const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
 
-        // one S row: a step's dS tile is the dBias tile (q tile i, kv tile j); kv 16 hb .. 16 hb + 15 of this warp
-        auto store_dbias = [&](int hb, int i, int j, int bs, int h, const uint32_t* pkd, const float2 (&dsv)[8]) {
+        // Word b of lane c of each four lanes goes to lane b as its word c.
+        auto quad_transpose = [&](uint32_t (&a)[4]) {
+            const bool odd = lane & 1, high = lane & 2;
+            const uint32_t s0 = __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 1);
+            const uint32_t s1 = __shfl_xor_sync(0xffffffffu, odd ? a[2] : a[3], 1);
+            const uint32_t n0 = odd ? s0 : a[0], n1 = odd ? a[1] : s0, n2 = odd ? s1 : a[2], n3 = odd ? a[3] : s1;
+            const uint32_t t0 = __shfl_xor_sync(0xffffffffu, high ? n0 : n2, 2);
+            const uint32_t t1 = __shfl_xor_sync(0xffffffffu, high ? n1 : n3, 2);
+            a[0] = high ? t0 : n0; a[1] = high ? t1 : n1; a[2] = high ? n2 : t0; a[3] = high ? n3 : t1;
+        };
+        // One S row: a step's dS tile is the dBias tile (q tile i, kv tile j).  Stored when the issuers have their operands, and
+        // by whole rows: four-lane transposes leave lane c with the block of kv 8 c .. 8 c + 7, so that a store takes 128 bytes
+        // of one q row (fp32) or 64 of eight (bf16).  Inside the arithmetic, and straight from the fragments, with 32 bytes of
+        // four or eight rows, the addresses and values did not fit the registers, and the stores were what a step waited for:
+        // B=4, S=1, N=1024, H=16, D=32 fp32 116 -> 91 us, bf16 85 -> 75 (one thread per kv row, as at D = 64: 101 and 82).
+        // out: this lane's place in q row 32 g of the tile
+        auto store_dbias = [&](auto* out, int q0, uint32_t (&pkd)[16], float2 (&dsv)[16]) {
             if constexpr (DBIAS_HERE != DBIAS_NO) {
-                const size_t head = (static_cast<size_t>(bs) * p.H + h) * p.N;
-                const int kv0 = j * TILE + 32 * w4 + 16 * hb, q0 = i * TILE + 32 * g;
-                if constexpr (DBIAS_HERE == DBIAS_F32) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int kv = kv0 + 8 * (k & 1) + (lane >> 2), q = q0 + 8 * (k >> 1) + 2 * (lane & 3);
-                        float* out = static_cast<float*>(p.dbias) + (head + q) * p.N + kv;
-                        if (kv < p.N && q < p.N) {       // (N is even)
-                            out[0] = dsv[k].x;
-                            out[p.N] = dsv[k].y;
-                        }
-                    }
-                } else {
-                    // blocks transposed back; lanes 2n and 2n + 1 then exchange words, so that each stores four kv of a
-                    // q row, the even one in the first block of a pair, the odd one in the second
-                    const bool odd = lane & 1;
-                    const int kv = kv0 + (odd ? 8 : 0) + 2 * (lane & 2);
+                for (int cb = 0; cb < 4; ++cb) {
+                    const bool rows = q0 + 8 * cb < p.N;          // (N is a multiple of 8)
+                    if constexpr (DBIAS_HERE == DBIAS_F32) {
+                        uint32_t x[2][4];
 #pragma unroll
-                    for (int cb = 0; cb < 4; ++cb) {
-                        const uint32_t w0 = movmatrix_trans(pkd[2 * cb]), w1 = movmatrix_trans(pkd[2 * cb + 1]);
-                        const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1);
-                        const int q = q0 + 8 * cb + (lane >> 2);
-                        if (kv < p.N && q < p.N)
-                            *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.dbias) + (head + q) * p.N + kv) =
-                                odd ? make_uint2(other, w1) : make_uint2(w0, other);
+                        for (int b = 0; b < 4; ++b) { x[0][b] = __float_as_uint(dsv[4 * cb + b].x); x[1][b] = __float_as_uint(dsv[4 * cb + b].y); }
+                        quad_transpose(x[0]);
+                        quad_transpose(x[1]);
+                        if (rows)
+#pragma unroll
+                            for (int r = 0; r < 8; ++r) out[static_cast<size_t>(8 * cb + r) * p.N] = __uint_as_float(x[r & 1][r >> 1]);
+                    } else {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) w[b] = movmatrix_trans(pkd[8 * (b >> 1) + 2 * cb + (b & 1)]);
+                        quad_transpose(w);
+                        if (rows) *reinterpret_cast<uint4*>(out + static_cast<size_t>(8 * cb) * p.N) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
             }
@@ -533,8 +541,17 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
 #pragma unroll 1
         for (int sg = 0; sg < n_segs && ok; ++sg) {
-            int bs = 0, h = 0, j = 0;
-            if constexpr (DBIAS_HERE != DBIAS_NO) seg.decode(sg, bs, h, j);
+            using DBias = std::conditional_t<DBIAS_HERE == DBIAS_F32, float, __nv_bfloat16>;
+            DBias* out = nullptr;
+            bool cols = false;
+            if constexpr (DBIAS_HERE != DBIAS_NO) {
+                int bs, h, j;
+                seg.decode(sg, bs, h, j);
+                const int kv0 = j * TILE + 32 * w4 + 8 * (lane & 3), r = lane >> 2;
+                cols = kv0 < p.N;
+                out = static_cast<DBias*>(p.dbias) + ((static_cast<size_t>(bs) * p.H + h) * p.N + 32 * g + (DBIAS_HERE == DBIAS_F32 ? 0 : r)) * p.N +
+                      kv0 + (DBIAS_HERE == DBIAS_F32 ? r : 0);
+            }
 #pragma unroll 1
             for (int i = 0; i < NT && ok; ++i, ++gs) {
                 // Per element x = S' c1 + bias log2e (S' already carries mask and -LSE through the extra contraction
@@ -544,6 +561,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t sv[32], dv[32], bq[4][4], pkp[16], pkd[16];
+                float2 dsv[16];
                 tmem_ld_frag32(tS, sv);
                 tmem_ld_frag32(tDP, dv);
 #pragma unroll
@@ -554,22 +572,23 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_free[hf]);
 #pragma unroll
-                for (int hb = 0; hb < 2; ++hb) {
-                    float2 dsv[8];
+                for (int cb = 0; cb < 4; ++cb) {              // 8 columns: four blocks of 8 kv
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {             // block (16 hb + 8 m, 8 cb) with k = 2 cb + m
-                        const int r = 16 * hb + 2 * k;
-                        const float2 b2 = fmul2(bf16x2_f2(bq[k >> 1][2 * hb + (k & 1)]), l2e2);
+                    for (int b = 0; b < 4; ++b) {             // block (8 b, 8 cb)
+                        const int r = 16 * (b >> 1) + 4 * cb + 2 * (b & 1), w = 8 * (b >> 1) + 2 * cb + (b & 1);
+                        const float2 b2 = fmul2(bf16x2_f2(bq[cb][b]), l2e2);
                         const float2 x2 = ffma2(u2f2(sv[r], sv[r + 1]), c1x2, b2);
                         const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
-                        dsv[k] = fmul2(e2, u2f2(dv[r], dv[r + 1]));
-                        pkp[8 * hb + k] = pack_bf16(e2.x, e2.y);
-                        pkd[8 * hb + k] = pack_bf16(dsv[k].x, dsv[k].y);
+                        const float2 d2 = fmul2(e2, u2f2(dv[r], dv[r + 1]));
+                        pkp[w] = pack_bf16(e2.x, e2.y);
+                        pkd[w] = pack_bf16(d2.x, d2.y);
+                        dsv[4 * cb + b] = d2;
                     }
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)               // formed here, not behind the wait below
-                        asm volatile("" : "+r"(pkp[8 * hb + k]), "+r"(pkd[8 * hb + k]));
-                    store_dbias(hb, i, j, bs, h, pkd + 8 * hb, dsv);
+                    for (int b = 0; b < 4; ++b) {             // formed here, not behind the wait below
+                        const int w = 8 * (b >> 1) + 2 * cb + (b & 1);
+                        asm volatile("" : "+r"(pkp[w]), "+r"(pkd[w]));
+                    }
                 }
                 mbar_release_after_loads(&bias_empty[slot], pkp[0] ^ pkp[2] ^ pkp[4] ^ pkp[6], scratch_w);
                 if (gs > 0) {
@@ -586,6 +605,10 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ds_ready[hf]);
+                if constexpr (DBIAS_HERE != DBIAS_NO) {
+                    store_dbias(out, cols ? i * TILE + 32 * g : p.N, pkd, dsv);
+                    out += static_cast<size_t>(TILE) * p.N;
+                }
             }
         }
     }

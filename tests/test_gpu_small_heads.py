@@ -30,3 +30,18 @@ def test_pairs_left_over_after_full_rounds(N):
     q, k, v, mask, bias, d_o = evo_ref.make_inputs(1, S, N, 4, 32, 0.5, 1.0, "tail0to32", seed=N)
     got = run_layer(q, k, v, mask, bias, d_o)
     assert_parity(oracle_on_rounded(q, k, v, mask, bias, d_o), got, tag=f"N={N} S={S}")
+
+
+# One S row: the kernel also writes dBias, from fragments.  148 SMs.
+@pytest.mark.parametrize("D,bias_type", [(16, torch.float32), (16, torch.bfloat16), (32, torch.float32), (32, torch.bfloat16)])
+@pytest.mark.parametrize("B,N,H", [
+    (38, 104, 8),      # 304 pairs of one tile, taken whole
+    (8, 512, 16),      # 128 pairs of four tiles, whole: dQ stays in tensor memory
+    (8, 640, 16),      # ... of five: dQ through scratch
+    (150, 200, 1),     # 148 whole, then the segments of two pairs
+    (38, 392, 8),      # 296 whole, then the segments of eight
+])
+def test_one_row(B, N, H, D, bias_type):
+    q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, 1, N, H, D, 0.5, 1.0, "bernoulli0.9", seed=B + N)
+    got = run_layer(q, k, v, mask, bias, d_o, bias_type=bias_type)
+    assert_parity(oracle_on_rounded(q, k, v, mask, bias, d_o), got, dbias_type=bias_type, tag=f"B={B} N={N} H={H} D={D}")
