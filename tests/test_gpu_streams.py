@@ -40,14 +40,16 @@ def test_forward_wide(B, S, N, H, D):
 
 
 # dQ/dK/dV kernel: whole items (every kv tile of a row and head in one CTA) where (rows x heads) fill the 148
-# SMs, single segments where they do not; one and two tiles keep dQ in tensor memory, more go through scratch
+# SMs, single segments where they do not; dQ of whole items stays in tensor memory for one tile at D = 128, up to two at D = 64
+# and up to four at D <= 32, with more it goes through scratch
 @pytest.mark.parametrize("bias_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,S,N,H,D", [
-    (1, 49, 264, 3, 32),     # whole, three ragged tiles
-    (1, 37, 328, 4, 64),
+    (1, 49, 264, 3, 32),     # whole, three ragged tiles, in tensor memory
+    (1, 49, 520, 3, 32),     # ... five, through scratch
+    (1, 37, 328, 4, 64),     # ... three
     (1, 37, 264, 4, 128),
     (1, 74, 200, 2, 96),     # two tiles
-    (1, 150, 136, 2, 32),    # ... and several items per CTA
+    (1, 150, 136, 2, 32),    # ... and two items per CTA, then the segments of four
     (1, 74, 200, 2, 64),
     (1, 160, 72, 2, 16),     # one tile
     (1, 150, 104, 2, 128),   # one tile
@@ -65,15 +67,17 @@ def test_backward_items(B, S, N, H, D, bias_type):
 # ... and pairs of a row and a head past the last full round of the 148 SMs, dealt by segments after the whole ones
 @pytest.mark.parametrize("bias_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,S,N,H,D", [
-    (1, 50, 200, 3, 32),     # 148 + 2; dQ of the whole ones stays in tensor memory
-    (1, 101, 136, 3, 64),    # 296 + 7
-    (1, 50, 264, 3, 32),     # 148 + 2, dQ of the whole ones goes through scratch
-    (1, 50, 392, 3, 64),
-    (2, 38, 520, 4, 16),     # 296 + 8
+    (1, 50, 200, 3, 32),     # 150: scratch and accumulator of whole rows do not fit, so all by segments
+    (1, 101, 136, 3, 64),    # 296 + 7; dQ of the whole ones stays in tensor memory
+    (1, 50, 264, 3, 32),     # 150: all by segments, three a CTA
+    (1, 99, 264, 3, 32),     # 296 + 1; three tiles in tensor memory
+    (1, 50, 392, 3, 64),     # 150: all by segments
+    (1, 99, 392, 3, 64),     # 296 + 1; dQ of the whole ones goes through scratch
+    (2, 38, 520, 4, 16),     # 296 + 8; through scratch
     (1, 20, 200, 16, 32),    # 296 + 24: the first of the rest lies in the middle of a row
-    (1, 19, 264, 8, 64),     # 152: the accumulator of whole rows does not fit, so all by segments
+    (1, 19, 264, 8, 64),     # 152: all by segments
     (1, 38, 264, 4, 128),    # D = 128: all of them by segments
-    (150, 1, 200, 1, 64),    # one row: the same kernel also writes dBias
+    (150, 1, 200, 1, 64),    # 148 + 2 of one row: the same kernel also writes dBias
 ])
 def test_backward_rest(B, S, N, H, D, bias_type):
     q, k, v, mask, bias, d_o = evo_ref.make_inputs(B, S, N, H, D, 1.0, 1.0, "bernoulli0.9", seed=7 * S + N)
@@ -107,12 +111,14 @@ def test_dbias_over_many_rows(S, D):
 
 # ... in the smallest workspace that is accepted, whose dQ area has no room for N rounded up to 32 rows per pair
 @pytest.mark.parametrize("B,S,N,H,D", [
-    (1, 5, 264, 3, 32),      # fewer pairs than SMs: scratch of all does not fit, so segments
-    (1, 5, 200, 3, 64),      # two tiles need no scratch
-    (1, 50, 264, 6, 32),     # 296 + 4
-    (1, 75, 264, 4, 64),     # 300 pairs
-    (1, 37, 264, 4, 128),    # D = 128, three tiles: 148 pairs
-    (1, 37, 104, 4, 96),     # ... one
+    (1, 5, 264, 3, 32),      # fewer pairs than SMs: segments
+    (1, 5, 200, 3, 64),
+    (1, 50, 264, 6, 32),     # 296 + 4; the whole ones need no scratch
+    (1, 50, 520, 6, 32),     # ... and do
+    (1, 49, 520, 3, 32),     # 147 pairs, whole but for the room: segments
+    (1, 75, 264, 4, 64),     # 296 + 4 through scratch
+    (1, 37, 264, 4, 128),    # D = 128, three tiles: 148 pairs, whole but for the room
+    (1, 37, 104, 4, 96),     # ... one tile: whole
 ])
 @pytest.mark.parametrize("gated", [False, True])
 def test_backward_smallest_workspace(B, S, N, H, D, gated):
