@@ -141,9 +141,8 @@ namespace evo {
 // Measured against one kernel with P and dS in shared memory and two compute groups (whole backward):
 // S=256, N=1024, H=4, D=64 1.93 -> 1.59 ms; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
 // ---------------------------------------------------------------------------
-template <int DH>
 struct BwdCfg {
-    static_assert(DH == 64, "D = 32 is in evo_bwd_halves.cuh, 128 in evo_bwd_wide.cuh");
+    static constexpr int DH = 64;
     static constexpr int NG = 4;                       // compute groups
     static constexpr int CW = TILE / NG;               // q columns per group
     static constexpr int NCW = 4 * NG;
@@ -182,14 +181,15 @@ struct BwdCfg {
     static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
 };
 
-template <int DH, int WALK, int DBIAS_HERE>
-__global__ void __launch_bounds__(BwdCfg<DH>::THREADS, 1)
+template <int WALK, int DBIAS_HERE>
+__global__ void __launch_bounds__(BwdCfg::THREADS, 1)
 evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_dq,
                const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                const __grid_constant__ CUtensorMap tm_acc, const BwdParams p) {
-    using C = BwdCfg<DH>;
+    using C = BwdCfg;
+    constexpr int DH = C::DH;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
     constexpr int QS = C::QS, NKV = C::NKV, NB = C::NB, DQB = C::DQ_BUFS;
@@ -987,7 +987,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > room) p.n_whole = 0;
     }
     // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; two at D = 64, four at D <= 32)
-    constexpr int TILES_HELD = DH == 128 ? 1 : (DH == 64 ? BwdCfg<64>::DQ_BUFS : BwdHalvesCfg::DQ_BUFS);
+    constexpr int TILES_HELD = DH == 128 ? 1 : (DH == 64 ? BwdCfg::DQ_BUFS : BwdHalvesCfg::DQ_BUFS);
     if (p.n_whole == pairs && NT > TILES_HELD && std::min(pairs, use_sms) * n32 > room) p.n_whole = 0;
     p.pairs = pairs;
     p.acc_row0 = p.n_whole / d->H;
@@ -1082,9 +1082,9 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
                                            : (mode == DBIAS_BF16 ? evo_bwd_halves_kernel<W, DBIAS_BF16> : evo_bwd_halves_kernel<W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         } else {
-            using C = BwdCfg<DH>;
-            auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<DH, W, DBIAS_NO>
-                                           : (mode == DBIAS_BF16 ? evo_bwd_kernel<DH, W, DBIAS_BF16> : evo_bwd_kernel<DH, W, DBIAS_F32>);
+            using C = BwdCfg;
+            auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<W, DBIAS_NO>
+                                           : (mode == DBIAS_BF16 ? evo_bwd_kernel<W, DBIAS_BF16> : evo_bwd_kernel<W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         }
     };

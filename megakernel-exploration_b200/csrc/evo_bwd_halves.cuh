@@ -21,14 +21,14 @@
 //     a scratch area, and the drain of the last kv tile (a bulk copy's completion, two fences and a read back per step)
 //     was slower than the step;
 //   - dK and dV are both read out before the first is packed and stored.
-// Kernel alone: B=1, S=512, N=384, H=8 441 -> 356 us; S=384, N=384, H=4 177 -> 152; S=256, N=768, H=8 845 -> 775;
-// S=256, N=256, H=8 106 -> 98; N = 128 and 200 the same.
+// Kernel alone: B=1, S=512, N=384, H=8 441 -> 349 us; S=384, N=384, H=4 177 -> 148; S=256, N=768, H=8 848 -> 765;
+// S=256, N=512, H=8 387 -> 304; S=256, N=256, H=8 108 -> 96; S=200, N=200, H=4 48 -> 46; N = 128 the same (70).
 //
-// Tried: two dS tiles (428 at the first shape, for 356: issuers and LSU then meet on shared memory more often, the
+// Tried, against 356 at the first shape then: two dS tiles (428: issuers and LSU then meet on shared memory more often, the
 // matrix unit has its operands first and loads take five times as long); half-steps of all warps with the next one
 // prefetched into registers (637: twice the barriers); one issuer for dV, dK and dQ (433); loops around the issuers'
 // MMAs instead of straight code (404); the waits' slow path as it was (373: two halves at different places of the code
-// compete for the instruction cache).
+// compete for the instruction cache; with the short one 0.4 warps a scheduler wait for instructions per issue).
 #pragma once
 
 namespace evo {
@@ -68,8 +68,8 @@ struct BwdHalvesCfg {
     // setmaxnreg budgets: the CTA's register pool is the launch count (the cap ptxas derives from the
     // launch bound) times the threads; an increase that the pool cannot satisfy blocks for ever
     static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
-    static constexpr int REGS_COMPUTE = 88, REGS_DRAIN = 80, REGS_OTHER = 48;
-    static_assert((REGS_COMPUTE * NCW + (REGS_DRAIN + REGS_OTHER) * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
+    static constexpr int REGS_COMPUTE = 88, REGS_OTHER = 48;       // drain warps: as launched
+    static_assert((REGS_COMPUTE * NCW + (REGS_LAUNCH + REGS_OTHER) * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
     static constexpr int QS = 3;                       // Q/dO stages
     static constexpr int NKV = 2;                      // K/V buffers
     static constexpr int NB = 4;                       // halves of bias tiles
@@ -345,8 +345,9 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
     }
     } else if (warp >= C::W_DRAIN) {
-        if constexpr (C::REGS_DRAIN < C::REGS_LAUNCH) reg_dec<C::REGS_DRAIN>();
         // ------------------------------ drain warps ------------------------------
+        // (The loops over DH / 32 run once.  Written without them the mixed walk spills in other places, and is slower with
+        // one S row: B=38, N=392, H=8 83 -> 89 us.)
         const int w4 = warp & 3;
         const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
@@ -397,8 +398,8 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     const bool final_sum = whole && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
                     float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
                     float4 old[8];
-                    // The bulk copy that last wrote this part of the scratch area, NT >= 3 steps ago, is complete
-                    // before the sum is added to or read: at least two were issued after it.
+                    // The bulk copy that last wrote this part of the scratch area, a segment ago, is complete
+                    // before the sum is added to or read: two or more were issued after it (NT > DQB).
                     if (whole && j > 0 && !resident) {
                         if (lane == 0) tma_wait_group<2>();
                         if (add) fence_async_all();
@@ -407,7 +408,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
                     if (!ok) break;
                     tc_fence_after();
-    #pragma unroll
+#pragma unroll
                     for (int rd = 0; rd < DH / 32; ++rd) {
                         float dqv[32];
                         tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
@@ -419,9 +420,9 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
                         if (final_sum) {
                             if (add) {
-    #pragma unroll
+#pragma unroll
                                 for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + (rd * 8 + c) * 32 + lane);
-    #pragma unroll
+#pragma unroll
                                 for (int c = 0; c < 8; ++c) {
                                     dqv[4 * c] += old[c].x; dqv[4 * c + 1] += old[c].y;
                                     dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
@@ -434,7 +435,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         }
                         uint8_t* wq = next_slot();
                         const float sc = whole ? 1.0f : p.scale;
-    #pragma unroll
+#pragma unroll
                         for (int c = 0; c < 8; ++c)
                             *reinterpret_cast<float4*>(wq + (whole ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
                                 make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
@@ -457,9 +458,9 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 tc_fence_after();
                 const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
                 uint4 u[2][DH / 32][4];
-    #pragma unroll
+#pragma unroll
                 for (int t = 0; t < 2; ++t)                     // dK, then dV
-    #pragma unroll
+#pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
                         float v[32];
                         __syncwarp();
@@ -469,9 +470,9 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dkv_free);
-    #pragma unroll
+#pragma unroll
                 for (int t = 0; t < 2; ++t)
-    #pragma unroll
+#pragma unroll
                     for (int c = 0; c < DH / 32; ++c)
                         if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[t][c], h, j * TILE + wrow0, c * 32, bs);
             }

@@ -1,5 +1,5 @@
-// dQ, dK, dV at D = 96 and 128 (evo_bwd.cu has the interface, the D <= 64 kernel and what the two share:
-// transposed products, whole pairs or single segments).  Tensor memory holds S', dP', dK and dV and
+// dQ, dK, dV at D = 96 and 128 (evo_bwd.cu has the interface and what the dQ/dK/dV kernels share: transposed
+// products, whole pairs or single segments).  Tensor memory holds S', dP', dK and dV and
 // nothing else: P^T and dS^T overwrite the columns they were computed from, and dQ takes the columns of S'
 // once dV, which reads P^T from them, is complete.  A step is then one chain
 //
@@ -19,7 +19,7 @@ namespace evo {
 
 template <int DH>
 struct BwdWideCfg {
-    static_assert(DH == 128, "the D <= 64 kernel is in evo_bwd.cu");
+    static_assert(DH == 128, "D <= 32 is in evo_bwd_halves.cuh, 64 in evo_bwd.cu");
     static constexpr int NG = 4;                       // compute groups
     static constexpr int NCW = 4 * NG;
     static constexpr int W_PROD = NCW, W_MMA = NCW + 1;

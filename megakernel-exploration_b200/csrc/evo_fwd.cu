@@ -70,8 +70,8 @@ struct FwdParams {
 // fill the SMs G at a time) every stream has its own items and its own ring slot.
 //
 // Measured against one item at a time on two groups of 64 columns (what is below included; kernel alone, in one run):
-// B=1, S=512, N=384, H=8, D=32 0.358 -> 0.299 ms; S=256, N=768 0.638 -> 0.538; S=256, N=1024, H=4, D=64 0.677 -> 0.602.
-// A step takes about 2400 clocks of a CTA: 1024 for its exponentials, 1000 issue slots.  Also tried: the
+// B=1, S=512, N=384, H=8, D=32 0.358 -> 0.278 ms; S=256, N=768 0.638 -> 0.522; S=256, N=1024, H=4, D=64 0.677 -> 0.585.
+// A step takes about 2200 clocks of a CTA: 1024 for its exponentials, 1000 issue slots.  Also tried: the
 // epilogue on a warpgroup of its own (its registers cost the softmax warps more than it saves, 0.42 ms),
 // two streams in the exp2 pass at a time (0.365), none taking turns (0.39), two streams at D = 32 (0.375).
 //
@@ -82,10 +82,11 @@ struct FwdParams {
 // 0.585 -> 0.540 ms).
 //
 // The streams are at different places of their code at any time, and what they fetch competes for the instruction cache
-// (a warp in seven that could have issued waited for an instruction).  Short waits, 105 -> 83 KB of code: B=1, S=512, N=384,
+// (1.1 warps a scheduler wait for instructions per issue; 0.7 with short waits).  Short waits, 105 -> 83 KB of code: B=1, S=512, N=384,
 // H=8, D=32 0.302 -> 0.277 ms; S=200, N=200, H=4 44 -> 40 us; S=256, N=1024, H=4, D=64 640 -> 575.  The producer's loop stays
 // unrolled over the streams, its masks requested ahead: one copy of it for all streams was 0.298 ms at the first shape (one
-// warp is then too slow for three streams).  Rolling the loops over a tile's chunks: no gain.
+// warp is then too slow for three streams).  With two streams, D = 64, the one copy was the quicker (B=4, S=1, N=512, H=16
+// 18.4 -> 16.6 us): the number of copies could go by G, which is not done.  Rolling the loops over a tile's chunks: no gain.
 //
 // One maximum per 128 columns instead of one per 64 leaves one exact P a row and tile instead of two: O is 2 to 3 %
 // further from 64 bits (relative error 2.11e-3 -> 2.16e-3 at N = 264, D = 64, of which 1.66e-3 is its own bf16).  Two
