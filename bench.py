@@ -38,9 +38,9 @@ for _p in (ROOT, PKG):
 
 import evo_workloads as wl  # noqa: E402
 
-# DRAM bytes per S row of one evo_bwd_kernel launch, from the ncu capture summarised under profiles/
-# (110.18 MB read + 46.15 MB written at 128 rows of cfg2).
-NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.18e6 + 46.15e6) / 128}
+# DRAM bytes per S row of one evo_bwd_halves_kernel launch, from the ncu capture summarised under profiles/
+# (110.21 MB read + 43.95 MB written at 128 rows of cfg2).
+NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.21e6 + 43.95e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"
 UNIT = "TFLOP/s"
@@ -410,7 +410,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     bwd_avg_ms = bwd_ms / max(bwd_n, 1)
     achieved = bwd_flops_launch / (bwd_avg_ms * 1e-3) / 1e12 if bwd_n else None
     roofline = {
-        "kernel": "evo_bwd_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["burst"], "unit": "TFLOP/s",
+        "kernel": "evo_bwd_halves_kernel" if D <= 32 else "evo_bwd_kernel" if D <= 64 else "evo_bwd_wide_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["burst"], "unit": "TFLOP/s",
         "frac": (achieved / peaks["burst"]) if achieved else None,
         "frac_of_sustained_peak": (achieved / peaks["sustained"]) if achieved else None,
         "traffic": (NCU_DRAM_BYTES_PER_ROW[name] * rows) if name in NCU_DRAM_BYTES_PER_ROW else None,
