@@ -410,7 +410,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     bwd_avg_ms = bwd_ms / max(bwd_n, 1)
     achieved = bwd_flops_launch / (bwd_avg_ms * 1e-3) / 1e12 if bwd_n else None
     roofline = {
-        "kernel": "evo_bwd_halves_kernel" if D <= 32 else "evo_bwd_kernel" if D <= 64 else "evo_bwd_wide_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["burst"], "unit": "TFLOP/s",
+        "kernel": "evo_bwd_halves_kernel" if D <= 64 else "evo_bwd_wide_kernel", "bound": "tensor", "achieved": achieved, "peak": peaks["burst"], "unit": "TFLOP/s",
         "frac": (achieved / peaks["burst"]) if achieved else None,
         "frac_of_sustained_peak": (achieved / peaks["sustained"]) if achieved else None,
         "traffic": (NCU_DRAM_BYTES_PER_ROW[name] * rows) if name in NCU_DRAM_BYTES_PER_ROW else None,

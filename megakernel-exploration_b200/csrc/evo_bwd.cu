@@ -15,7 +15,7 @@
 //                         the main kernels need no edge predicates; zeroes the accumulators
 //   2. evo_dbias_kernel   dBias (evo_dbias.cu): one CTA per pair-bias tile keeps its
 //                         sum over the S rows in registers, no reduction traffic
-//   3. evo_bwd_kernel     dQ, dK, dV (below; D <= 32: evo_bwd_halves.cuh, D > 64: evo_bwd_wide.cuh)
+//   3. evo_bwd_halves_kernel, evo_bwd_wide_kernel   dQ, dK, dV (D <= 64: evo_bwd_halves.cuh, above: evo_bwd_wide.cuh)
 //   4. bwd_finish_kernel  fp32 dQ accumulator -> bf16 dQ in the caller layout (and dBias,
 //                         summed over slices of S in fp32, to bf16 if the caller wants that)
 #include "evo_dbias.cuh"
@@ -94,600 +94,33 @@ struct Segments {
     }
 };
 
-}  // namespace evo
-#include "evo_bwd_halves.cuh"
-#include "evo_bwd_wide.cuh"
-namespace evo {
-
 // ---------------------------------------------------------------------------
-// dQ, dK, dV at D = 64, and what the dQ/dK/dV kernels share (D <= 32: evo_bwd_halves.cuh; D = 96, 128: evo_bwd_wide.cuh).
+// What the dQ/dK/dV kernels share (D <= 64: evo_bwd_halves.cuh; D = 96, 128: evo_bwd_wide.cuh).
 // One persistent CTA per SM walks segments (S row, head h, kv tile j of 128 residues); a segment walks steps (q tile i).
-// Everything is formed TRANSPOSED, kv rows in the tensor-memory lanes, so that P^T and dS^T are in place as A operands of
+// Everything is formed TRANSPOSED, kv rows in the tensor-memory lanes, so that P^T (and dS^T) are in place as A operands of
 // the products that contract over q, without a trip through shared memory:
 //
 //   S'^T = K Q^T + extra block,  dP'^T = V dO^T + extra block         (evo_tiles.cuh, "EXTRA TILE")
 //   P^T = exp2(S'^T c1 + bias^T log2e),  dS^T = P^T o dP'^T           (thread = one kv row)
-//   dV += P^T dO,  dK += dS^T Q      A from tensor memory: 16 clocks per K = 16 block at N = 32, where an
-//                                    A tile in shared memory costs 40 (it is read at 128 bytes a clock)
+//   dV += P^T dO,  dK += dS^T Q
 //   dQ = dS K                        A = dS from shared memory (M = q: MN-major), the one tile written there
 //
-// What bounds a step is the work of the compute warps, about 1400 issue slots and 1024 clocks of
-// exponentials per scheduler, and the chain of barriers and products around it.  Sixteen compute warps,
-// because with eight the loads, multiplies and exponentials of a warp hardly overlapped (2000 clocks for
-// the same work).
-//
-//   D = 64: no columns for P^T and dS^T: they overwrite the columns they were computed from.  Two phases, P (from
-//     S') and dS (from dP'), each with its own barriers, so that the products of one are formed during the other: dV
-//     and S' of the next step while dS is computed, dK, dQ and dP' of the next step while its P is (B=1, S=256,
-//     N=1024, H=4: 1.30 -> 1.11 ms).  The halves of the D <= 32 kernel measure the same here (1.13 and 1.12 ms) and lose
-//     where a pair has two q tiles or one S row (S=200, N=200, H=4 78 -> 84 us; B=4, S=1, N=1024, H=16 106 -> 121): one
-//     dQ accumulator and one K/V buffer are all that fits.
-//
-//   warps 0-15 (compute)  group g = warp / 4 owns q columns 32g .. 32g+31 of the tile
-//   warps 16-19 (drain)   after every step 32 rows of dQ each, after a segment dK and dV as bf16 stores
-//   warp 20 (producer)    TMA: per step Q, dO, the extra tile of the q rows, the pair-bias tile; per
-//                         segment K, V and the extra tile of the kv rows
-//   warps 21, 22, 23      MMA issuers, one chain family each: S'^T and dP'^T; dV and dK; dQ
+// Sixteen compute warps, because with eight the loads, multiplies and exponentials of a warp hardly overlapped (2000 clocks
+// for the same work).
 //
 // dQ is a sum over kv tiles.  A CTA takes all NT segments of a pair (S row, head) where it can, and so sees
-// the whole sum.  With few tiles (two here, four at D <= 32) it stays in tensor memory until the last segment; otherwise
-// the drain warps keep partial sums in a scratch area of the CTA, in L2 (written and added to by bulk copies: loads
-// and stores of their own held up the compute warps' shared-memory accesses), and the last segment's go out
-// as bf16.  Whole pairs fill whole rounds of the SMs; the pairs that are left over are dealt by segments, and
+// the whole sum.  With few tiles (four at D <= 32) it stays in tensor memory until the last segment; otherwise
+// partial sums go to a scratch area of the CTA, in L2, and the last segment's go out as bf16.  Whole pairs fill whole rounds
+// of the SMs; the pairs that are left over are dealt by segments, and
 // their partial sums meet in an fp32 accumulator in memory (TMA reduce-add), which costs a pass to zero it and
 // a pass to convert it, of those pairs only (against all pairs whole, or none, the kernel alone: S=384, N=384, H=4,
 // D=32 182 -> 176 us; S=200, N=200, H=4 47 -> 44; S=1024, N=768, H=8 3333 -> 3255).
-//
-// Measured against one kernel with P and dS in shared memory and two compute groups (whole backward):
-// S=256, N=1024, H=4, D=64 1.93 -> 1.59 ms; B=4, S=1, N=1024, H=16, D=64 0.24 -> 0.15.
 // ---------------------------------------------------------------------------
-struct BwdCfg {
-    static constexpr int DH = 64;
-    static constexpr int NG = 4;                       // compute groups
-    static constexpr int CW = TILE / NG;               // q columns per group
-    static constexpr int NCW = 4 * NG;
-    static constexpr int W_DRAIN = NCW, W_PROD = NCW + 4, W_MMA = NCW + 5;
-    static constexpr int THREADS = (NCW + 8) * 32;
-    static constexpr int QS = 2;                       // Q/dO stages
-    static constexpr int NKV = 1;                      // K/V buffers
-    static constexpr int NB = 2;                       // bias tiles
-    static constexpr int DQ_BUFS = 2;
-    static constexpr uint32_t ROWT = RowTile<DH>::BYTES;
-    static constexpr uint32_t ST_Q = 0, ST_DO = ROWT, ST_XQ = 2 * ROWT;
-    static constexpr uint32_t STAGE_BYTES = 2 * ROWT + XT_BYTES;
-    static constexpr uint32_t KV_K = 0, KV_V = ROWT, KV_XK = 2 * ROWT, KV_BYTES = 2 * ROWT + XT_BYTES;
-    static constexpr uint32_t OFF_STAGE = 0;
-    static constexpr uint32_t OFF_KV = OFF_STAGE + QS * STAGE_BYTES;
-    static constexpr uint32_t OFF_BIAS = OFF_KV + NKV * KV_BYTES;
-    static constexpr uint32_t OFF_DS = OFF_BIAS + NB * SQ_BYTES;
-    // per drain warp a slot of [32 rows][32 fp32], for bulk copies of dQ, dK and dV
-    static constexpr uint32_t WQ_BYTES = 32 * 32 * 4;
-    static constexpr uint32_t OFF_WSTG = OFF_DS + SQ_BYTES;
-    // constant extra tiles, above every tile that refers to the zero tile
-    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WQ_BYTES;            // row selector of -delta
-    static constexpr uint32_t OFF_ZERO = OFF_XDP + XT_BYTES;
-    static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr uint32_t NUM_BARS = 2 * QS + 2 * NKV + 2 * NB + 2 * DQ_BUFS + 8;
-    static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
-    static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + alignment slack
-    static constexpr uint32_t TMEM_S = 0, TMEM_DP = 128;
-    static constexpr uint32_t TMEM_DQ = 256;                                // DQ_BUFS accumulators
-    static constexpr uint32_t TMEM_DK = TMEM_DQ + 2 * DH, TMEM_DV = TMEM_DK + DH;
-    // column of contraction block kk (16 q) of P^T / dS^T, inside the columns of its own group
-    __device__ static __forceinline__ uint32_t p_col(int kk) { return TMEM_S + 32 * (kk >> 1) + 8 * (kk & 1); }
-    __device__ static __forceinline__ uint32_t ds_col(int kk) { return p_col(kk) + 128; }
-    static_assert(TMEM_DV + DH <= BWD_TMEM_COLS, "tensor memory budget");
-    static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-    static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
-};
 
-template <int WALK, int DBIAS_HERE>
-__global__ void __launch_bounds__(BwdCfg::THREADS, 1)
-evo_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-               const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_dq,
-               const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-               const __grid_constant__ CUtensorMap tm_acc, const BwdParams p) {
-    using C = BwdCfg;
-    constexpr int DH = C::DH;
-    using RT = RowTile<DH>;
-    using RD = RowDesc<DH>;
-    constexpr int QS = C::QS, NKV = C::NKV, NB = C::NB, DQB = C::DQ_BUFS;
-
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BARS);
-    uint64_t* st_full = bars;                  // [QS]
-    uint64_t* st_empty = st_full + QS;         // [QS]
-    uint64_t* kv_full = st_empty + QS;         // [NKV]
-    uint64_t* kv_empty = kv_full + NKV;        // [NKV]
-    uint64_t* s_full = kv_empty + NKV;         // [NB]: S' complete and the bias tile landed
-    uint64_t* bias_empty = s_full + NB;        // [NB]
-    uint64_t* dq_full = bias_empty + NB;       // [DQB]
-    uint64_t* dq_free = dq_full + DQB;         // [DQB]
-    uint64_t* dp_full = dq_free + DQB;         // dP' complete
-    uint64_t* p_ready = dp_full + 1;           // P^T is written
-    uint64_t* ds_ready = p_ready + 1;          // dS^T and the dS tile are written
-    uint64_t* dv_done = ds_ready + 1;          // dV of the step is complete
-    uint64_t* dk_done = dv_done + 1;           // dK
-    uint64_t* dq_done = dk_done + 1;           // dQ
-    uint64_t* dkv_full = dq_done + 1;          // dK, dV of the segment are complete
-    uint64_t* dkv_free = dkv_full + 1;         // ... and read out
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::OFF_MISC);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-
-    const int tid = threadIdx.x;
-    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // uniform
-    const int lane = tid & 31;
-    const int NT = p.NT;
-    WaitCtx wc{abort_flag, p.status};
-
-    if (tid == 0) {
-        *abort_flag = 0;
-        tmem_slot[3] = 0;                      // the abort word of the waits before exit
-        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
-        for (int i = 0; i < NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
-        for (int i = 0; i < NB; ++i) { mbar_init(&s_full[i], 2); mbar_init(&bias_empty[i], C::NCW); }
-        for (int i = 0; i < DQB; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
-        for (uint64_t* x : {p_ready, ds_ready}) mbar_init(x, C::NCW);
-        for (uint64_t* x : {dp_full, dv_done, dk_done, dq_done, dkv_full}) mbar_init(x, 1);
-        mbar_init(dkv_free, 4);
-        fence_mbar_init();
-    }
-    if (warp == C::W_MMA) {
-        tmem_alloc(tmem_slot, BWD_TMEM_COLS);
-        tmem_relinquish();
-    }
-    if (warp == C::W_PROD && lane == 0) {
-        prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do);
-        prefetch_tmap(&tm_bias); prefetch_tmap(&tm_dq); prefetch_tmap(&tm_dk); prefetch_tmap(&tm_dv);
-        prefetch_tmap(&tm_acc);
-    }
-    // constant extra tiles: row n of the -delta selector is (0,0,0,0,1,1,0,0); the zero tile
-    if (tid < 128) {
-        *reinterpret_cast<uint4*>(smem + C::OFF_XDP + tid * 16) = make_uint4(0u, 0u, 0x3f803f80u, 0u);
-        *reinterpret_cast<uint4*>(smem + C::OFF_ZERO + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-
-    const Segments<WALK> seg(p);
-    const int n_segs = seg.n;
-    const bool res_ok = NT <= DQB;       // dQ of a whole pair stays in tensor memory
-    // dQ accumulators in order of use: one per step, or (resident) one per q tile of a pair
-    auto dq_event = [&](bool resident, int sg, int j, int i) {
-        return resident ? (sg - j) + i : sg * NT + i - (res_ok ? seg.n_ws * (NT - 1) : 0);
-    };
-
-    if (warp == C::W_PROD) {
-        // ------------------------------ producer ------------------------------
-        bool ok = true;
-        int gs = 0, n_st = 0, n_bias = 0, n_kv = 0;      // steps; loads issued
-        for (int sg = 0; sg < n_segs && ok; ++sg) {
-            int bs, h, j;
-            seg.decode(sg, bs, h, j);
-            const int b = bs / p.S;
-            const __nv_bfloat16* xq = p.xq + (static_cast<size_t>(bs) * p.H + h) * p.NTP * 8;
-            {
-                const int kb = sg % NKV;
-                if (sg >= NKV) ok = warp_all(mbar_wait(&kv_empty[kb], ((sg / NKV) - 1) & 1, wc, 0x40));
-                if (!ok) break;
-                if (elect_one()) {
-                    uint8_t* kvb = smem + C::OFF_KV + kb * C::KV_BYTES;
-                    mbar_arrive_expect_tx(&kv_full[kb], C::KV_BYTES);
-                    tma_load_row_tile<DH>(kvb + C::KV_K, &tm_k, &kv_full[kb], h, j * TILE, bs);
-                    tma_load_row_tile<DH>(kvb + C::KV_V, &tm_v, &kv_full[kb], h, j * TILE, bs);
-                    bulk_load(kvb + C::KV_XK, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &kv_full[kb]);
-                }
-                __syncwarp();
-                ++n_kv;
-            }
-            for (int i = 0; i < NT && ok; ++i, ++gs) {
-                const int st = gs % QS, bb = gs % NB;
-                uint8_t* sb = smem + C::OFF_STAGE + st * C::STAGE_BYTES;
-                if (gs >= QS) ok = warp_all(mbar_wait(&st_empty[st], ((gs / QS) - 1) & 1, wc, 0x42));
-                if (!ok) break;
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&st_full[st], C::STAGE_BYTES);
-                    tma_load_row_tile<DH>(sb + C::ST_Q, &tm_q, &st_full[st], h, i * TILE, bs);
-                    tma_load_row_tile<DH>(sb + C::ST_DO, &tm_do, &st_full[st], h, i * TILE, bs);
-                    bulk_load(sb + C::ST_XQ, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &st_full[st]);
-                }
-                __syncwarp();
-                ++n_st;
-                if (gs >= NB) ok = warp_all(mbar_wait(&bias_empty[bb], ((gs / NB) - 1) & 1, wc, 0x41));
-                if (!ok) break;
-                if (elect_one()) {
-                    uint8_t* bt = smem + C::OFF_BIAS + bb * SQ_BYTES;
-                    mbar_arrive_expect_tx(&s_full[bb], SQ_BYTES);
-                    tma_load_4d(bt, &tm_bias, &s_full[bb], j * TILE, i * TILE, h, b);
-                    tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &s_full[bb], j * TILE + 64, i * TILE, h, b);
-                }
-                __syncwarp();
-                ++n_bias;
-            }
-        }
-        // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
-        // barrier with an MMA commit, which may then never come: a bounded pause instead).
-        const WaitCtx dc{tmem_slot + 3, p.status};
-        for (int k = (n_st > QS ? n_st - QS : 0); k < n_st; ++k) mbar_wait_landed(&st_full[k % QS], (k / QS) & 1, dc, 0x43);
-        for (int k = (n_kv > NKV ? n_kv - NKV : 0); k < n_kv; ++k) mbar_wait_landed(&kv_full[k % NKV], (k / NKV) & 1, dc, 0x45);
-        if (!ok && n_bias > 0)
-            for (int k = 0; k < 64; ++k) __nanosleep(1000);
-    } else if (warp >= C::W_MMA) {
-        // ------------------------------ mma issuers ------------------------------
-        // Each warp runs its loop with all lanes (uniform control flow: operand descriptors stay in
-        // uniform registers) and elects one lane to issue.
-        constexpr uint32_t IDESC_SDP = make_idesc_bf16(128, 128, 0, 0);
-        // N = the head-dim columns that hold data (the rest of a wider kernel's tile is zero fill)
-        const uint32_t IDESC_DKV = make_idesc_bf16(128, 16 * p.KB, 0, 1);
-        const uint32_t IDESC_DQ = make_idesc_bf16(128, 16 * p.KB, 1, 1);
-        const uint32_t aSt = smem_u32(smem + C::OFF_STAGE), aKV = smem_u32(smem + C::OFF_KV);
-        const uint32_t aZero = smem_u32(smem + C::OFF_ZERO);
-        const int role = warp - C::W_MMA;          // 0: S/dP, 1: dV/dK, 2: dQ
-        bool ok = true;
-        int gs = 0;
-        for (int sg = 0; sg < n_segs && ok; ++sg) {
-            const int kb = sg % NKV;
-            const uint32_t kvb = aKV + kb * C::KV_BYTES;
-            for (int i = 0; i < NT && ok; ++i, ++gs) {
-                const int st = gs % QS;
-                const uint32_t sb = aSt + st * C::STAGE_BYTES;
-                if (role == 0) {
-                    ok = warp_all(mbar_wait(&st_full[st], (gs / QS) & 1, wc, 0x50));
-                    if (ok && i == 0) ok = warp_all(mbar_wait(&kv_full[kb], (sg / NKV) & 1, wc, 0x51));
-                    // P^T in the columns is consumed
-                    if (ok && gs > 0) ok = warp_all(mbar_wait(dv_done, (gs - 1) & 1, wc, 0x52));
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t d_xq = xt_desc(sb + C::ST_XQ, aZero);
-                    if (elect_one()) {
-                        const uint32_t q_lo = RD::kmajor_lo(sb + C::ST_Q), k_lo = RD::kmajor_lo(kvb + C::KV_K);
-#pragma unroll
-                        for (int kk = 0; kk < RT::KBLOCKS; ++kk)
-                            if (kk < p.KB)      // the others are zero-filled blocks past the true head dim
-                                umma_ss(tmem + C::TMEM_S, RD::kmajor(k_lo, kk), RD::kmajor(q_lo, kk), IDESC_SDP, kk > 0);
-                        // + (mask - LSE) / scale: the extra contraction block
-                        umma_ss(tmem + C::TMEM_S, xt_desc(kvb + C::KV_XK, aZero), d_xq, IDESC_SDP, 1u);
-                        umma_commit(&s_full[gs % NB]);
-                    }
-                    __syncwarp();
-                    if (gs > 0) ok = warp_all(mbar_wait(dk_done, (gs - 1) & 1, wc, 0x59));
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t do_lo = RD::kmajor_lo(sb + C::ST_DO), v_lo = RD::kmajor_lo(kvb + C::KV_V);
-#pragma unroll
-                        for (int kk = 0; kk < RT::KBLOCKS; ++kk)
-                            if (kk < p.KB)
-                                umma_ss(tmem + C::TMEM_DP, RD::kmajor(v_lo, kk), RD::kmajor(do_lo, kk), IDESC_SDP, kk > 0);
-                        // - delta
-                        umma_ss(tmem + C::TMEM_DP, xt_desc(smem_u32(smem + C::OFF_XDP), aZero), d_xq, IDESC_SDP, 1u);
-                        umma_commit(dp_full);
-                    }
-                    __syncwarp();
-                } else if (role == 1) {
-                    const uint32_t acc = (i > 0) ? 1u : 0u;
-                    // the first MMA of a segment overwrites dK / dV: the previous one's must be out
-                    if (i == 0 && sg > 0) ok = warp_all(mbar_wait(dkv_free, (sg - 1) & 1, wc, 0x55));
-                    const uint32_t q_lo = RD::mnmajor_lo(sb + C::ST_Q), do_lo = RD::mnmajor_lo(sb + C::ST_DO);
-                    auto dv = [&](int kk) {
-                        umma_ts(tmem + C::TMEM_DV, tmem + C::p_col(kk), RD::mnmajor(do_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
-                    };
-                    auto dk = [&](int kk) {
-                        umma_ts(tmem + C::TMEM_DK, tmem + C::ds_col(kk), RD::mnmajor(q_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
-                    };
-                    if (ok) ok = warp_all(mbar_wait(p_ready, gs & 1, wc, 0x53));
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) dv(kk);
-                        umma_commit(dv_done);
-                    }
-                    __syncwarp();
-                    ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5a));
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) dk(kk);
-                        umma_commit(dk_done);
-                        umma_commit(&st_empty[st]);
-                        if (i == NT - 1) {
-                            umma_commit(dkv_full);
-                            umma_commit(&kv_empty[kb]);
-                        }
-                    }
-                    __syncwarp();
-                } else {
-                    const bool whole = seg.whole(sg), resident = whole && res_ok;
-                    const int j = whole ? sg % NT : 0, ev = dq_event(resident, sg, j, i);
-                    if (ev >= DQB && !(resident && j > 0)) ok = warp_all(mbar_wait(&dq_free[ev % DQB], ((ev / DQB) - 1) & 1, wc, 0x54));
-                    if (ok) ok = warp_all(mbar_wait(ds_ready, gs & 1, wc, 0x5b));
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t ds_lo = SqDesc::mnmajor_lo(smem_u32(smem + C::OFF_DS));
-                        const uint32_t k_lo = RD::mnmajor_lo(kvb + C::KV_K);
-                        const uint32_t t_dq = tmem + C::TMEM_DQ + (ev % DQB) * DH;
-                        const uint32_t acc = (resident && j > 0) ? 1u : 0u;
-#pragma unroll
-                        for (int kk = 0; kk < 8; ++kk)
-                            umma_ss(t_dq, SqDesc::mnmajor(ds_lo, kk), RD::mnmajor(k_lo, kk), IDESC_DQ, kk > 0 ? 1u : acc);
-                        umma_commit(dq_done);
-                        if (!resident || j == NT - 1) umma_commit(&dq_full[ev % DQB]);
-                        if (i == NT - 1) umma_commit(&kv_empty[kb]);
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-    } else if (warp >= C::W_DRAIN) {
-        // ------------------------------ drain warps ------------------------------
-        const int w4 = warp & 3;
-        const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp
-        const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
-        uint8_t* const wslot = smem + C::OFF_WSTG + w4 * C::WQ_BYTES;
-        // Where the next bulk copy (one group each) is staged, once the copy that used the place last has read it: the
-        // slot, or its halves in turn for copies of half its size.
-        int pos = 0;
-        bool last_half = false;
-        auto next_slot = [&](bool half) -> uint8_t* {
-            if (lane == 0) {
-                if (half && last_half) tma_wait_group_read<1>();
-                else tma_wait_group_read<0>();
-            }
-            __syncwarp();
-            last_half = half;
-            pos ^= 1;
-            return wslot + (half ? pos * (C::WQ_BYTES / 2) : 0);
-        };
-        // 32 columns of 32 rows as bf16, by a bulk tensor store (which clips rows past N and columns past Dt)
-        auto store_rows = [&](const CUtensorMap* tm, const uint4 (&u)[4], int h, int row0, int col0, int bs) {
-            uint8_t* sl = next_slot(true);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sl + swz_off<64>(lane, c)) = u[c];
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-                tma_store_4d(tm, sl, col0, h, row0, bs);
-                tma_commit_group();
-            }
-        };
-        auto pack_rows = [](uint4 (&u)[4], const float (&v)[32], float sc) {
-#pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8)
-                u[c8] = make_uint4(pack_bf16(v[c8 * 8 + 0] * sc, v[c8 * 8 + 1] * sc), pack_bf16(v[c8 * 8 + 2] * sc, v[c8 * 8 + 3] * sc),
-                                   pack_bf16(v[c8 * 8 + 4] * sc, v[c8 * 8 + 5] * sc), pack_bf16(v[c8 * 8 + 6] * sc, v[c8 * 8 + 7] * sc));
-        };
-        // whole pairs: the partial sums of this CTA, in units of 4 KB: 32 rows x 32 columns as [16-byte word][row]
-        float4* part = reinterpret_cast<float4*>(p.dq_scratch) + static_cast<size_t>(blockIdx.x) * p.scratch_stride;
-        bool ok = true;
-        auto drain = [&](auto whole_c, int sg0, int sg1) {
-            constexpr bool whole = decltype(whole_c)::value;
-            for (int sg = sg0; sg < sg1 && ok; ++sg) {
-                int bs, h, j;
-                seg.decode(sg, bs, h, j);
-                const bool resident = whole && res_ok;
-                for (int i = 0; i < NT && ok; ++i) {
-                    if (resident && j < NT - 1) continue;          // dQ is still being summed
-                    const int ev = dq_event(resident, sg, j, i), b = ev % DQB;
-                    const bool rows = i * TILE + wrow0 < p.N;     // warp-uniform: some row of this warp exists
-                    const bool final_sum = whole && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
-                    float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
-                    float4 old[8];
-                    // The bulk copy that last wrote this part of the scratch area, NT >= 3 steps ago, is complete
-                    // before the sum is added to or read: at least two were issued after it.
-                    if (whole && j > 0 && !resident) {
-                        if (lane == 0) tma_wait_group<2>();
-                        if (add) fence_async_all();
-                        __syncwarp();
-                    }
-                    ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
-                    if (!ok) break;
-                    tc_fence_after();
-    #pragma unroll
-                    for (int rd = 0; rd < DH / 32; ++rd) {
-                        float dqv[32];
-                        tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
-                        if (rd == DH / 32 - 1) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&dq_free[b]);
-                        }
-                        if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
-                        if (final_sum) {
-                            if (add) {
-    #pragma unroll
-                                for (int c = 0; c < 8; ++c) old[c] = __ldcg(ps + (rd * 8 + c) * 32 + lane);
-    #pragma unroll
-                                for (int c = 0; c < 8; ++c) {
-                                    dqv[4 * c] += old[c].x; dqv[4 * c + 1] += old[c].y;
-                                    dqv[4 * c + 2] += old[c].z; dqv[4 * c + 3] += old[c].w;
-                                }
-                            }
-                            uint4 u[4];
-                            pack_rows(u, dqv, p.scale);
-                            store_rows(&tm_dq, u, h, i * TILE + wrow0, rd * 32, bs);
-                            continue;
-                        }
-                        uint8_t* wq = next_slot(false);
-                        const float sc = whole ? 1.0f : p.scale;
-    #pragma unroll
-                        for (int c = 0; c < 8; ++c)
-                            *reinterpret_cast<float4*>(wq + (whole ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
-                                make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
-                        fence_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            if (!whole)
-                                tma_reduce_add_4d(&tm_acc, wq, rd * 32, h, i * TILE + wrow0, bs - p.acc_row0);
-                            else if (j == 0)
-                                bulk_store(ps + rd * 8 * 32, wq, C::WQ_BYTES);
-                            else
-                                bulk_reduce_add_f32(ps + rd * 8 * 32, wq, C::WQ_BYTES);
-                            tma_commit_group();
-                        }
-                    }
-                }
-                if (!ok) break;
-                ok = warp_all(mbar_wait(dkv_full, sg & 1, wc, 0x69));
-                if (!ok) break;
-                tc_fence_after();
-                const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
-    #pragma unroll
-                for (int t = 0; t < 2; ++t) {                   // dK, then dV
-                    uint4 u[DH / 32][4];
-    #pragma unroll
-                    for (int c = 0; c < DH / 32; ++c) {
-                        float v[32];
-                        __syncwarp();
-                        tmem_ld_f32<32>(lane_base + (t ? C::TMEM_DV : C::TMEM_DK) + c * 32, v);
-                        pack_rows(u[c], v, t ? 1.0f : p.scale);
-                    }
-                    if (t == 1) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(dkv_free);
-                    }
-    #pragma unroll
-                    for (int c = 0; c < DH / 32; ++c)
-                        if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[c], h, j * TILE + wrow0, c * 32, bs);
-                }
-            }
-        };
-        if (WALK != WALK_SEGMENTS) drain(std::true_type{}, 0, seg.n_ws);
-        if (WALK != WALK_WHOLE) drain(std::false_type{}, seg.n_ws, n_segs);
-        if (lane == 0) tma_wait_group<0>();
-    } else {
-        // ------------------------------ compute groups ------------------------------
-        const int g = warp >> 2;             // q columns 32g .. 32g+31 of the tile
-        const int row = tid & 127;           // kv row within the tile == TMEM lane
-        const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-        const uint32_t tS = lane_base + C::TMEM_S + 32 * g, tDP = lane_base + C::TMEM_DP + 32 * g;
-        const uint32_t aDS = smem_u32(smem + C::OFF_DS);
-        // this thread's column of the bias tile ([q][kv], swizzled by q & 7), first row of the group
-        const uint32_t aBias = smem_u32(smem + C::OFF_BIAS) + (row >> 6) * SQ_SUB_BYTES + 32 * g * 128 + (row & 7) * 2;
-        const uint32_t bchunk = (row & 63) >> 3;
-        const uint32_t scratch_w = smem_u32(tmem_slot + 2);       // a word nobody reads
-        bool ok = true;
-        int gs = 0;
-        const float2 c1x2 = make_float2(p.c1, p.c1), l2e2 = make_float2(LOG2E, LOG2E);
-
-        // one S row: a step's dS tile is the dBias tile (q tile i, kv tile j); columns 16 ch .. of this group
-        auto store_dbias = [&](int ch, int i, int j, int bs, int h, const uint32_t (&pkd)[8], const float2 (&dsv)[8]) {
-            if constexpr (DBIAS_HERE != DBIAS_NO) {
-                // one S row: this step's dS tile is the dBias tile (q tile i, kv tile j)
-                const int kv = j * TILE + row, q0 = i * TILE + 32 * g + 16 * ch;
-                const size_t at = ((static_cast<size_t>(bs) * p.H + h) * p.N + q0) * p.N + kv;
-                if constexpr (DBIAS_HERE == DBIAS_F32) {
-                    float* out = static_cast<float*>(p.dbias) + at;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        if (kv < p.N && q0 + 2 * k < p.N) out[static_cast<size_t>(2 * k) * p.N] = dsv[k].x;
-                        if (kv < p.N && q0 + 2 * k + 1 < p.N) out[static_cast<size_t>(2 * k + 1) * p.N] = dsv[k].y;
-                    }
-                } else {
-                    // lanes 2n and 2n+1 exchange halves: the even one stores both kv of the even q row, the
-                    // odd one those of the odd row
-                    const bool odd = lane & 1;
-                    uint32_t* out = reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.dbias) + at - (odd ? 1 : 0));
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const uint32_t other = __shfl_xor_sync(0xffffffffu, pkd[k], 1);
-                        const uint32_t w = odd ? __byte_perm(other, pkd[k], 0x7632) : __byte_perm(pkd[k], other, 0x5410);
-                        const int q = q0 + 2 * k + (odd ? 1 : 0);
-                        if (kv < p.N && q < p.N) out[static_cast<size_t>(2 * k + (odd ? 1 : 0)) * (p.N >> 1)] = w;
-                    }
-                }
-            }
-        };
-
-        for (int sg = 0; sg < n_segs && ok; ++sg) {
-            int bs = 0, h = 0, j = 0;
-            if constexpr (DBIAS_HERE != DBIAS_NO) seg.decode(sg, bs, h, j);
-            for (int i = 0; i < NT && ok; ++i, ++gs) {
-                const int bb = gs % NB;
-                // ---- phase P: x = S' c1 + bias log2e (S' already carries mask and -LSE through the extra
-                // contraction block), P = exp2(x), P^T (bf16) into tensor memory
-                // (S' of this step waited for dV of the previous one: its columns are free)
-                ok = warp_all(mbar_wait(&s_full[bb], (gs / NB) & 1, wc, 0x63));
-                if (!ok) break;
-                tc_fence_after();
-                float2 p2[16];
-                uint32_t dep = 0;
-#pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {          // 16 columns at a time
-                    uint32_t sv[16], bq[16];
-                    tmem_ld16(tS + 16 * ch, sv);
-#pragma unroll
-                    for (int k = 0; k < 16; ++k)
-                        bq[k] = lds_u16(aBias + bb * SQ_BYTES + (16 * ch + k) * 128 + ((bchunk ^ (k & 7)) << 4));
-                    tmem_wait_ld();
-                    uint32_t pk[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float2 b2 = fmul2(make_float2(__uint_as_float(bq[2 * k] << 16), __uint_as_float(bq[2 * k + 1] << 16)), l2e2);
-                        const float2 x2 = ffma2(u2f2(sv[2 * k], sv[2 * k + 1]), c1x2, b2);
-                        const float2 e2 = make_float2(ex2(x2.x), ex2(x2.y));
-                        p2[8 * ch + k] = e2;
-                        pk[k] = pack_bf16(e2.x, e2.y);
-                    }
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) dep ^= pk[k];      // depends on every bias value read
-                    tmem_st8(lane_base + C::p_col(2 * g + ch), pk);
-                }
-                mbar_release_after_loads(&bias_empty[bb], dep, scratch_w);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_ready);
-
-                // ---- phase dS: dS = P dP' (dP' already carries -delta), dS^T into tensor memory and the tile.
-                // Both are free once dK and dQ of the previous step are complete.
-                if (gs == 0)
-                    ok = warp_all(mbar_wait(dp_full, 0, wc, 0x66));
-                else                           // (dP' of this step waited for dK)
-                    ok = warp_all(mbar_wait_both(dp_full, gs & 1, dq_done, (gs - 1) & 1, wc, 0x66));
-                if (!ok) break;
-                tc_fence_after();
-#pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t dv[16];
-                    tmem_ld16(tDP + 16 * ch, dv);
-                    tmem_wait_ld();
-                    uint32_t pkd[8];
-                    float2 dsv[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        dsv[k] = fmul2(p2[8 * ch + k], u2f2(dv[2 * k], dv[2 * k + 1]));
-                        pkd[k] = pack_bf16(dsv[k].x, dsv[k].y);
-                    }
-                    tmem_st8(lane_base + C::ds_col(2 * g + ch), pkd);
-#pragma unroll
-                    for (int c = 0; c < 2; ++c)
-                        sts128(aDS + sq_chunk_off(row, 4 * g + 2 * ch + c),
-                               make_uint4(pkd[4 * c], pkd[4 * c + 1], pkd[4 * c + 2], pkd[4 * c + 3]));
-                    store_dbias(ch, i, j, bs, h, pkd, dsv);
-                }
-                tmem_wait_st();
-                tc_fence_before();
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(ds_ready);
-            }
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) { report_abort(wc); report_abort(WaitCtx{tmem_slot + 3, p.status}); }
-    if (warp == C::W_MMA) tmem_dealloc(tmem, BWD_TMEM_COLS);
-}
+}  // namespace evo
+#include "evo_bwd_halves.cuh"
+#include "evo_bwd_wide.cuh"
+namespace evo {
 
 // ---------------------------------------------------------------------------
 // prep: delta = rowsum(dO o O) (replaces evo_bwd_prep_ker, tk_evoattention.cu:352-416),
@@ -940,7 +373,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     if ((rc = make_tmap_qkv(&tk, k, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tv, v, BS, d->N, d->H, Dt, TILE, lay_in, RowTile<DH>::BOX_D))) return rc;
     if ((rc = make_tmap_qkv(&tdo, d_o, BS, d->N, d->H, Dt, TILE, lay_do, RowTile<DH>::BOX_D))) return rc;
-    if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N, DH == 32 ? TILE / 2 : TILE))) return rc;
+    if ((rc = make_tmap_bias(&tb, bias, d->B, d->H, d->N, DH <= 64 ? TILE / 2 : TILE))) return rc;
 
     BwdParams p{};
     p.B = d->B; p.S = d->S; p.N = d->N; p.H = d->H;
@@ -986,8 +419,8 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         const size_t acc_n = static_cast<size_t>(pairs - full / d->H * d->H) * d->N;
         if (p.n_whole < pairs && static_cast<size_t>(full ? use_sms : 0) * n32 + acc_n > room) p.n_whole = 0;
     }
-    // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; two at D = 64, four at D <= 32)
-    constexpr int TILES_HELD = DH == 128 ? 1 : (DH == 64 ? BwdCfg::DQ_BUFS : BwdHalvesCfg::DQ_BUFS);
+    // all whole: partial sums of every CTA, unless they stay in tensor memory (one tile; four at D <= 32)
+    constexpr int TILES_HELD = DH == 128 ? 1 : BwdHalvesCfg<DH == 128 ? 64 : DH>::DQ_BUFS;
     if (p.n_whole == pairs && NT > TILES_HELD && std::min(pairs, use_sms) * n32 > room) p.n_whole = 0;
     p.pairs = pairs;
     p.acc_row0 = p.n_whole / d->H;
@@ -1076,15 +509,10 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             auto kernel = mode == DBIAS_NO ? evo_bwd_wide_kernel<DH, W, DBIAS_NO>
                                            : (mode == DBIAS_BF16 ? evo_bwd_wide_kernel<DH, W, DBIAS_BF16> : evo_bwd_wide_kernel<DH, W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
-        } else if constexpr (DH == 32) {
-            using C = BwdHalvesCfg;
-            auto kernel = mode == DBIAS_NO ? evo_bwd_halves_kernel<W, DBIAS_NO>
-                                           : (mode == DBIAS_BF16 ? evo_bwd_halves_kernel<W, DBIAS_BF16> : evo_bwd_halves_kernel<W, DBIAS_F32>);
-            return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         } else {
-            using C = BwdCfg;
-            auto kernel = mode == DBIAS_NO ? evo_bwd_kernel<W, DBIAS_NO>
-                                           : (mode == DBIAS_BF16 ? evo_bwd_kernel<W, DBIAS_BF16> : evo_bwd_kernel<W, DBIAS_F32>);
+            using C = BwdHalvesCfg<DH>;
+            auto kernel = mode == DBIAS_NO ? evo_bwd_halves_kernel<DH, W, DBIAS_NO>
+                                           : (mode == DBIAS_BF16 ? evo_bwd_halves_kernel<DH, W, DBIAS_BF16> : evo_bwd_halves_kernel<DH, W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
         }
     };

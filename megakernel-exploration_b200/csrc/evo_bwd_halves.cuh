@@ -1,4 +1,4 @@
-// dQ, dK, dV at D <= 32 (evo_bwd.cu has the interface, and what the dQ/dK/dV kernels share: transposed products, whole
+// dQ, dK, dV at D <= 64 (evo_bwd.cu has the interface, and what the dQ/dK/dV kernels share: transposed products, whole
 // pairs or single segments, the drain of dQ).
 //
 //   warps 0-15 (compute)  group g = warp / 4 owns q columns 32g .. 32g+31 of the tile; groups 0 and 1 are the first half
@@ -24,7 +24,19 @@
 // Kernel alone: B=1, S=512, N=384, H=8 441 -> 349 us; S=384, N=384, H=4 177 -> 148; S=256, N=768, H=8 848 -> 765;
 // S=256, N=512, H=8 387 -> 304; S=256, N=256, H=8 108 -> 96; S=200, N=200, H=4 48 -> 46; N = 128 the same (70).
 //
-// Tried, against 356 at the first shape then: two dS tiles (428: issuers and LSU then meet on shared memory more often, the
+// D = 64.  A kernel with two phases of sixteen warps a step (P, then dS) measured the same as halves that shared its loads:
+// what bounded both was that two Q/dO stages and one K/V buffer were freed by a step's last products, 1900 clocks before what
+// replaced them had landed (a wait of 1500 clocks a step for Q and dO and of 3900 a segment for K and V), and the drain warps,
+// which staged the partial sums of dQ for bulk copies (3400 of a step's 4300 clocks).  Here Q, dO, K and V have rings and
+// barriers of their own (dO is free with dV, V with the last dP', so that two and one buffers do), a half hands its bias back
+// as soon as it is in registers, and the partial sums of a whole pair go from registers to the CTA's scratch area as vector
+// reductions, coalesced and unstaged.  With one dQ accumulator there is room for P^T beside S'; pairs of two tiles then use the
+// scratch area, which costs them less than a second accumulator over S' did.  Kernel alone: B=1, S=256, N=1024, H=4 1147 -> 999 us
+// (37 rows 166 -> 140); S=74, N=640 137 -> 120, N=384 66 -> 56; S=148, N=256 58 -> 52; S=200, N=200 77 -> 73; B=4, S=1, N=1024,
+// H=16 109 -> 106, with an fp32 bias 124 -> 112.  D = 32 with more than four tiles, for the reductions: S=256, N=768, H=8
+// 784 -> 718.  (D = 32 with rings of their own for Q, dO, K and V: S=200, N=200, H=4 46 -> 51, N=384 350 -> 360; it keeps the pairs.)
+//
+// Tried at D = 32, against 356 at the first shape then: two dS tiles (428: issuers and LSU then meet on shared memory more often, the
 // matrix unit has its operands first and loads take five times as long); half-steps of all warps with the next one
 // prefetched into registers (637: twice the barriers); one issuer for dV, dK and dQ (433); loops around the issuers'
 // MMAs instead of straight code (404); the waits' slow path as it was (373: two halves at different places of the code
@@ -59,8 +71,10 @@ struct SegmentWalk {
 };
 
 
+template <int DH_>
 struct BwdHalvesCfg {
-    static constexpr int DH = 32;
+    static constexpr int DH = DH_;
+    static_assert(DH == 32 || DH == 64, "D = 96 and 128 are in evo_bwd_wide.cuh");
     static constexpr int NG = 4;                       // compute groups
     static constexpr int NCW = 4 * NG;
     static constexpr int W_DRAIN = NCW, W_PROD = NCW + 4, W_MMA = NCW + 5;
@@ -70,58 +84,59 @@ struct BwdHalvesCfg {
     static constexpr int REGS_LAUNCH = (65536 / THREADS) & ~7;
     static constexpr int REGS_COMPUTE = 88, REGS_OTHER = 48;       // drain warps: as launched
     static_assert((REGS_COMPUTE * NCW + (REGS_LAUNCH + REGS_OTHER) * 4) * 32 <= REGS_LAUNCH * THREADS, "register pool");
-    static constexpr int QS = 3;                       // Q/dO stages
-    static constexpr int NKV = 2;                      // K/V buffers
-    static constexpr int NB = 4;                       // halves of bias tiles
-    static constexpr int DQ_BUFS = 4;
+    // Buffers of Q (with the extra tile of its rows), dO, K (with its extra tile), V, halves of bias tiles.  D = 32: Q and
+    // dO, and K and V, come and go together, which is fewer barriers for the producer; D = 64 has no room for that.
+    static constexpr bool PAIRED = DH == 32;
+    static constexpr int NQ = 3, NDO = PAIRED ? NQ : 2, NK = 2, NV = PAIRED ? NK : 1, NB = (DH == 32) ? 4 : 2;
+    static constexpr int DQ_BUFS = (DH == 32) ? 4 : 1;             // dQ accumulators
     static constexpr uint32_t ROWT = RowTile<DH>::BYTES;
-    static constexpr uint32_t ST_Q = 0, ST_DO = ROWT, ST_XQ = 2 * ROWT;
-    static constexpr uint32_t STAGE_BYTES = 2 * ROWT + XT_BYTES;
-    static constexpr uint32_t KV_K = 0, KV_V = ROWT, KV_XK = 2 * ROWT, KV_BYTES = 2 * ROWT + XT_BYTES;
-    static constexpr uint32_t OFF_STAGE = 0;
-    static constexpr uint32_t OFF_KV = OFF_STAGE + QS * STAGE_BYTES;
-    static constexpr uint32_t OFF_BIAS = OFF_KV + NKV * KV_BYTES;
+    static constexpr uint32_t OFF_Q = 0, OFF_DO = OFF_Q + NQ * ROWT, OFF_K = OFF_DO + NDO * ROWT, OFF_V = OFF_K + NK * ROWT;
+    static constexpr uint32_t OFF_BIAS = OFF_V + NV * ROWT;
     static constexpr uint32_t OFF_DS = OFF_BIAS + NB * SQ_SUB_BYTES;
     // per drain warp: WSLOTS slots of [32 rows][32 fp32], for bulk copies of dQ, dK and dV
     static constexpr uint32_t WQ_BYTES = 32 * 32 * 4;
-    static constexpr int WSLOTS = 2;
+    static constexpr int WSLOTS = (DH == 32) ? 2 : 1;
     static constexpr uint32_t OFF_WSTG = OFF_DS + SQ_BYTES;
+    static constexpr uint32_t OFF_XQ = OFF_WSTG + 4 * WSLOTS * WQ_BYTES, OFF_XK = OFF_XQ + NQ * XT_BYTES;
     // constant extra tiles, above every tile that refers to the zero tile
-    static constexpr uint32_t OFF_XDP = OFF_WSTG + 4 * WSLOTS * WQ_BYTES;            // row selector of -delta
+    static constexpr uint32_t OFF_XDP = OFF_XK + NK * XT_BYTES;            // row selector of -delta
     static constexpr uint32_t OFF_ZERO = OFF_XDP + XT_BYTES;
     static constexpr uint32_t OFF_BARS = OFF_ZERO + XT_BYTES;
-    static constexpr uint32_t NUM_BARS = 2 * QS + 2 * NKV + 2 * NB + 2 * DQ_BUFS + 9;
+    static constexpr uint32_t NUM_BARS = 2 * (NQ + NDO + NK + NV + NB + DQ_BUFS) + 9;
     static constexpr uint32_t OFF_MISC = OFF_BARS + NUM_BARS * 8;
     static constexpr uint32_t SMEM_BYTES = OFF_MISC + 16 + 1024;            // + alignment slack
     static constexpr uint32_t TMEM_S = 0, TMEM_DP = 128, TMEM_P = 256;       // S', dP', P^T (bf16)
-    static constexpr uint32_t TMEM_DQ = 320;                                // DQ_BUFS accumulators
+    static constexpr uint32_t TMEM_DQ = 320;                                // accumulators
     static constexpr uint32_t TMEM_DK = TMEM_DQ + DQ_BUFS * DH, TMEM_DV = TMEM_DK + DH;
     static_assert(TMEM_DV + DH <= BWD_TMEM_COLS, "tensor memory budget");
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-    static_assert(STAGE_BYTES % 1024 == 0 && KV_BYTES % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
+    static_assert(ROWT % 1024 == 0 && WQ_BYTES % 1024 == 0, "tile alignment");
 };
 
-template <int WALK, int DBIAS_HERE>
-__global__ void __launch_bounds__(BwdHalvesCfg::THREADS, 1)
+template <int DH, int WALK, int DBIAS_HERE>
+__global__ void __launch_bounds__(BwdHalvesCfg<DH>::THREADS, 1)
 evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_bias, const __grid_constant__ CUtensorMap tm_dq,
                const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                const __grid_constant__ CUtensorMap tm_acc, const BwdParams p) {
-    using C = BwdHalvesCfg;
-    constexpr int DH = C::DH;
+    using C = BwdHalvesCfg<DH>;
     using RT = RowTile<DH>;
     using RD = RowDesc<DH>;
-    constexpr int QS = C::QS, NKV = C::NKV, NB = C::NB, DQB = C::DQ_BUFS;
+    constexpr int NQ = C::NQ, NDO = C::NDO, NK = C::NK, NV = C::NV, NB = C::NB, DQB = C::DQ_BUFS;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::OFF_BARS);
-    uint64_t* st_full = bars;                  // [QS]
-    uint64_t* st_empty = st_full + QS;         // [QS]
-    uint64_t* kv_full = st_empty + QS;         // [NKV]
-    uint64_t* kv_empty = kv_full + NKV;        // [NKV]
-    uint64_t* bias_full = kv_empty + NKV;      // [NB]
+    uint64_t* q_full = bars;                   // [NQ]: Q and the extra tile of its rows
+    uint64_t* q_empty = q_full + NQ;           // [NQ]
+    uint64_t* do_full = q_empty + NQ;          // [NDO]
+    uint64_t* do_empty = do_full + NDO;        // [NDO]
+    uint64_t* k_full = do_empty + NDO;         // [NK]: K and the extra tile of its rows
+    uint64_t* k_empty = k_full + NK;           // [NK]
+    uint64_t* v_full = k_empty + NK;           // [NV]
+    uint64_t* v_empty = v_full + NV;           // [NV]
+    uint64_t* bias_full = v_empty + NV;       // [NB]
     uint64_t* bias_empty = bias_full + NB;     // [NB]
     uint64_t* dq_full = bias_empty + NB;       // [DQB]
     uint64_t* dq_free = dq_full + DQB;         // [DQB]
@@ -144,8 +159,10 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (tid == 0) {
         *abort_flag = 0;
         tmem_slot[3] = 0;                      // the abort word of the waits before exit
-        for (int i = 0; i < QS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
-        for (int i = 0; i < NKV; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
+        for (int i = 0; i < NQ; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
+        for (int i = 0; i < NDO; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
+        for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+        for (int i = 0; i < NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for (int i = 0; i < NB; ++i) { mbar_init(&bias_full[i], 1); mbar_init(&bias_empty[i], C::NCW / 2); }
         for (int i = 0; i < DQB; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
         mbar_init(ds_free, 2);
@@ -187,7 +204,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (warp == C::W_PROD) {
         // ------------------------------ producer ------------------------------
         bool ok = true;
-        int gs = 0, n_st = 0, n_bias = 0, n_kv = 0;      // steps; loads issued
+        int gs = 0, n_q = 0, n_do = 0, n_k = 0, n_v = 0, n_bias = 0;      // steps; loads issued
         SegmentWalk<WALK> at(seg, 0);
 #pragma unroll 1
         for (int sg = 0; sg < n_segs && ok; ++sg) {
@@ -195,34 +212,51 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const int bs = at.bs, h = at.h, j = at.j;
             const int b = bs / p.S;
             const __nv_bfloat16* xq = p.xq + (static_cast<size_t>(bs) * p.H + h) * p.NTP * 8;
-            {
-                const int kb = sg % NKV;
-                if (sg >= NKV) ok = warp_all(mbar_wait(&kv_empty[kb], ((sg / NKV) - 1) & 1, wc, 0x40));
-                if (!ok) break;
-                if (elect_one()) {
-                    uint8_t* kvb = smem + C::OFF_KV + kb * C::KV_BYTES;
-                    mbar_arrive_expect_tx(&kv_full[kb], C::KV_BYTES);
-                    tma_load_row_tile<DH>(kvb + C::KV_K, &tm_k, &kv_full[kb], h, j * TILE, bs);
-                    tma_load_row_tile<DH>(kvb + C::KV_V, &tm_v, &kv_full[kb], h, j * TILE, bs);
-                    bulk_load(kvb + C::KV_XK, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &kv_full[kb]);
-                }
-                __syncwarp();
-                ++n_kv;
+            const int kb = sg % NK, vb = sg % NV;
+            if (sg >= NK) ok = warp_all(mbar_wait(&k_empty[kb], ((sg / NK) - 1) & 1, wc, 0x40));
+            if (!ok) break;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&k_full[kb], (C::PAIRED ? 2 : 1) * C::ROWT + XT_BYTES);
+                tma_load_row_tile<DH>(smem + C::OFF_K + kb * C::ROWT, &tm_k, &k_full[kb], h, j * TILE, bs);
+                if (C::PAIRED) tma_load_row_tile<DH>(smem + C::OFF_V + kb * C::ROWT, &tm_v, &k_full[kb], h, j * TILE, bs);
+                bulk_load(smem + C::OFF_XK + kb * XT_BYTES, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &k_full[kb]);
             }
+            __syncwarp();
+            ++n_k;
 #pragma unroll 1
             for (int i = 0; i < NT && ok; ++i, ++gs) {
-                const int st = gs % QS;
-                uint8_t* sb = smem + C::OFF_STAGE + st * C::STAGE_BYTES;
-                if (gs >= QS) ok = warp_all(mbar_wait(&st_empty[st], ((gs / QS) - 1) & 1, wc, 0x42));
+                const int qb = gs % NQ, db = gs % NDO;
+                if (gs >= NQ) ok = warp_all(mbar_wait(&q_empty[qb], ((gs / NQ) - 1) & 1, wc, 0x42));
                 if (!ok) break;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&st_full[st], C::STAGE_BYTES);
-                    tma_load_row_tile<DH>(sb + C::ST_Q, &tm_q, &st_full[st], h, i * TILE, bs);
-                    tma_load_row_tile<DH>(sb + C::ST_DO, &tm_do, &st_full[st], h, i * TILE, bs);
-                    bulk_load(sb + C::ST_XQ, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &st_full[st]);
+                    mbar_arrive_expect_tx(&q_full[qb], (C::PAIRED ? 2 : 1) * C::ROWT + XT_BYTES);
+                    tma_load_row_tile<DH>(smem + C::OFF_Q + qb * C::ROWT, &tm_q, &q_full[qb], h, i * TILE, bs);
+                    if (C::PAIRED) tma_load_row_tile<DH>(smem + C::OFF_DO + qb * C::ROWT, &tm_do, &q_full[qb], h, i * TILE, bs);
+                    bulk_load(smem + C::OFF_XQ + qb * XT_BYTES, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &q_full[qb]);
                 }
                 __syncwarp();
-                ++n_st;
+                ++n_q;
+                if constexpr (!C::PAIRED) {
+                    if (gs >= NDO) ok = warp_all(mbar_wait(&do_empty[db], ((gs / NDO) - 1) & 1, wc, 0x46));
+                    if (!ok) break;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&do_full[db], C::ROWT);
+                        tma_load_row_tile<DH>(smem + C::OFF_DO + db * C::ROWT, &tm_do, &do_full[db], h, i * TILE, bs);
+                    }
+                    __syncwarp();
+                    ++n_do;
+                    if (i == 0) {
+                        // V is free with the last dP' of its segment, K with the last dQ
+                        if (sg >= NV) ok = warp_all(mbar_wait(&v_empty[vb], ((sg / NV) - 1) & 1, wc, 0x47));
+                        if (!ok) break;
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(&v_full[vb], C::ROWT);
+                            tma_load_row_tile<DH>(smem + C::OFF_V + vb * C::ROWT, &tm_v, &v_full[vb], h, j * TILE, bs);
+                        }
+                        __syncwarp();
+                        ++n_v;
+                    }
+                }
 #pragma unroll 1
                 for (int hf = 0; hf < 2 && ok; ++hf, ++n_bias) {
                     const int bb = n_bias % NB;
@@ -240,8 +274,11 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         // the last loads have landed before the CTA exits, also if a wait gave up
         const WaitCtx dc{tmem_slot + 3, p.status};
-        for (int k = (n_st > QS ? n_st - QS : 0); k < n_st; ++k) mbar_wait_landed(&st_full[k % QS], (k / QS) & 1, dc, 0x43);
-        for (int k = (n_kv > NKV ? n_kv - NKV : 0); k < n_kv; ++k) mbar_wait_landed(&kv_full[k % NKV], (k / NKV) & 1, dc, 0x45);
+        for (int k = (n_q > NQ ? n_q - NQ : 0); k < n_q; ++k) mbar_wait_landed(&q_full[k % NQ], (k / NQ) & 1, dc, 0x43);
+        // (n_do, n_v: 0 where they come with Q and K)
+        for (int k = (n_do > NDO ? n_do - NDO : 0); k < n_do; ++k) mbar_wait_landed(&do_full[k % NDO], (k / NDO) & 1, dc, 0x48);
+        for (int k = (n_k > NK ? n_k - NK : 0); k < n_k; ++k) mbar_wait_landed(&k_full[k % NK], (k / NK) & 1, dc, 0x45);
+        for (int k = (n_v > NV ? n_v - NV : 0); k < n_v; ++k) mbar_wait_landed(&v_full[k % NV], (k / NV) & 1, dc, 0x49);
         for (int k = (n_bias > NB ? n_bias - NB : 0); k < n_bias; ++k) mbar_wait_landed(&bias_full[k % NB], (k / NB) & 1, dc, 0x44);
     } else {
         // ------------------------------ mma issuers ------------------------------
@@ -251,42 +288,41 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // N = the head-dim columns that hold data (the rest of a wider kernel's tile is zero fill)
         const uint32_t IDESC_DKV = make_idesc_bf16(128, 16 * p.KB, 0, 1);
         const uint32_t IDESC_DQ = make_idesc_bf16(128, 16 * p.KB, 1, 1);
-        const uint32_t aSt = smem_u32(smem + C::OFF_STAGE), aKV = smem_u32(smem + C::OFF_KV);
+        const uint32_t aQ = smem_u32(smem + C::OFF_Q), aDO = smem_u32(smem + C::OFF_DO), aK = smem_u32(smem + C::OFF_K);
         const uint32_t aZero = smem_u32(smem + C::OFF_ZERO);
         const int role = warp - C::W_MMA;          // 0: S/dP, 1: dV/dK, 2: dQ
         bool ok = true;
         int gs = 0;
 #pragma unroll 1
         for (int sg = 0; sg < n_segs && ok; ++sg) {
-            const int kb = sg % NKV;
-            const uint32_t kvb = aKV + kb * C::KV_BYTES;
+            const int kb = sg % NK, vb = sg % NV;
 #pragma unroll 1
             for (int i = 0; i < NT && ok; ++i, ++gs) {
-                const int st = gs % QS;
-                const uint32_t sb = aSt + st * C::STAGE_BYTES;
+                const int qb = gs % NQ, db = gs % NDO;
                 if (role == 0) {
-                    ok = warp_all(mbar_wait(&st_full[st], (gs / QS) & 1, wc, 0x50));
-                    if (ok && i == 0) ok = warp_all(mbar_wait(&kv_full[kb], (sg / NKV) & 1, wc, 0x51));
+                    ok = warp_all(mbar_wait(&q_full[qb], (gs / NQ) & 1, wc, 0x50));
+                    if (ok && i == 0) ok = warp_all(mbar_wait(&k_full[kb], (sg / NK) & 1, wc, 0x51));
 #pragma unroll
                     for (int t = 0; t < 4; ++t) {          // S', then dP' of one half, then of the other
                         const int hf = t >> 1, part = t & 1;
                         if (ok && gs > 0 && part == 0) ok = warp_all(mbar_wait(&s_free[hf], (gs - 1) & 1, wc, 0x52));
+                        if (!C::PAIRED && ok && t == 1) ok = warp_all(mbar_wait(&do_full[db], (gs / NDO) & 1, wc, 0x56));
+                        if (!C::PAIRED && ok && t == 1 && i == 0) ok = warp_all(mbar_wait(&v_full[vb], (sg / NV) & 1, wc, 0x57));
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {
-                            // K and V, and Q and dO, lie side by side
-                            static_assert(C::KV_V == C::KV_K + C::ROWT && C::ST_DO == C::ST_Q + C::ROWT, "order of the tiles");
-                            const uint32_t a_lo = RD::kmajor_lo(kvb + C::KV_K + part * C::ROWT);
-                            const uint32_t b_lo = RD::kmajor_lo(sb + C::ST_Q + part * C::ROWT + hf * 64 * RT::ROW_BYTES);
+                            const uint32_t a_lo = RD::kmajor_lo(part ? smem_u32(smem + C::OFF_V) + vb * C::ROWT : aK + kb * C::ROWT);
+                            const uint32_t b_lo = RD::kmajor_lo((part ? aDO + db * C::ROWT : aQ + qb * C::ROWT) + hf * 64 * RT::ROW_BYTES);
                             const uint32_t d = tmem + C::TMEM_S + 128 * part + 64 * hf;
 #pragma unroll
                             for (int kk = 0; kk < RT::KBLOCKS; ++kk)
                                 if (kk < p.KB)      // the others are zero-filled blocks past the true head dim
                                     umma_ss(d, RD::kmajor(a_lo, kk), RD::kmajor(b_lo, kk), IDESC_SDP, kk > 0);
                             // the extra contraction block: + (mask - LSE) / scale, - delta
-                            umma_ss(d, xt_desc(part ? smem_u32(smem + C::OFF_XDP) : kvb + C::KV_XK, aZero),
-                                    xt_desc(sb + C::ST_XQ + hf * 64 * 16, aZero), IDESC_SDP, 1u);
+                            umma_ss(d, xt_desc(part ? smem_u32(smem + C::OFF_XDP) : smem_u32(smem + C::OFF_XK) + kb * XT_BYTES, aZero),
+                                    xt_desc(smem_u32(smem + C::OFF_XQ) + qb * XT_BYTES + hf * 64 * 16, aZero), IDESC_SDP, 1u);
                             if (part) umma_commit(&s_full[hf]);
+                            if (!C::PAIRED && t == 3 && i == NT - 1) umma_commit(&v_empty[vb]);
                         }
                         __syncwarp();
                     }
@@ -295,49 +331,47 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     if (i == 0 && sg > 0) ok = warp_all(mbar_wait(dkv_free, (sg - 1) & 1, wc, 0x55));
 #pragma unroll 1
                     for (int hf = 0; hf < 2; ++hf) {
-                        if (ok) ok = warp_all(mbar_wait(&ds_ready[hf], gs & 1, wc, 0x5a));
+                        if (ok) ok = warp_all(mbar_wait(&ds_ready[hf], gs & 1, wc, 0x5a));      // (Q and dO have landed: dP' read them)
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {
                             const uint32_t row0 = hf * 64 * RT::ROW_BYTES;
-                            const uint32_t do_lo = RD::mnmajor_lo(sb + C::ST_DO + row0), q_lo = RD::mnmajor_lo(sb + C::ST_Q + row0);
+                            const uint32_t do_lo = RD::mnmajor_lo(aDO + db * C::ROWT + row0), q_lo = RD::mnmajor_lo(aQ + qb * C::ROWT + row0);
                             const uint32_t ds_lo = SqDesc::kmajor_lo(smem_u32(smem + C::OFF_DS) + hf * SQ_SUB_BYTES);
                             const uint32_t t_p = tmem + C::TMEM_P + 32 * hf, acc = (hf > 0 || i > 0) ? 1u : 0u;
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk)
                                 umma_ts(tmem + C::TMEM_DV, t_p + 8 * kk, RD::mnmajor(do_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
+                            if (!C::PAIRED && hf == 1) umma_commit(&do_empty[db]);
 #pragma unroll
                             for (int kk = 0; kk < 4; ++kk)
                                 umma_ss(tmem + C::TMEM_DK, SqDesc::kmajor(ds_lo, kk), RD::mnmajor(q_lo, kk), IDESC_DKV, kk > 0 ? 1u : acc);
                             if (hf == 1) {
                                 umma_commit(ds_free);
-                                umma_commit(&st_empty[st]);
-                                if (i == NT - 1) {
-                                    umma_commit(dkv_full);
-                                    umma_commit(&kv_empty[kb]);
-                                }
+                                umma_commit(&q_empty[qb]);
+                                if (i == NT - 1) umma_commit(dkv_full);
                             }
                         }
                         __syncwarp();
                     }
                 } else {
                     const bool whole = seg.whole(sg), resident = whole && res_ok;
-                    const int j = whole ? sg % NT : 0, ev = dq_event(resident, sg, j, i);
-                    if (ev >= DQB && !(resident && j > 0)) ok = warp_all(mbar_wait(&dq_free[ev % DQB], ((ev / DQB) - 1) & 1, wc, 0x54));
+                    const int j = whole ? sg % NT : 0, ev = dq_event(resident, sg, j, i), buf = ev % DQB, use = ev / DQB;
+                    if (use > 0 && !(resident && j > 0)) ok = warp_all(mbar_wait(&dq_free[buf], (use - 1) & 1, wc, 0x54));
                     if (ok) ok = warp_all(mbar_wait_both(&ds_ready[0], gs & 1, &ds_ready[1], gs & 1, wc, 0x5b));
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
                         const uint32_t ds_lo = SqDesc::mnmajor_lo(smem_u32(smem + C::OFF_DS));
-                        const uint32_t k_lo = RD::mnmajor_lo(kvb + C::KV_K);
-                        const uint32_t t_dq = tmem + C::TMEM_DQ + (ev % DQB) * DH;
+                        const uint32_t k_lo = RD::mnmajor_lo(aK + kb * C::ROWT);
+                        const uint32_t t_dq = tmem + C::TMEM_DQ + buf * DH;
                         const uint32_t acc = (resident && j > 0) ? 1u : 0u;
 #pragma unroll
                         for (int kk = 0; kk < 8; ++kk)
                             umma_ss(t_dq, SqDesc::mnmajor(ds_lo, kk), RD::mnmajor(k_lo, kk), IDESC_DQ, kk > 0 ? 1u : acc);
                         umma_commit(ds_free);
-                        if (!resident || j == NT - 1) umma_commit(&dq_full[ev % DQB]);
-                        if (i == NT - 1) umma_commit(&kv_empty[kb]);
+                        if (!resident || j == NT - 1) umma_commit(&dq_full[buf]);
+                        if (i == NT - 1) umma_commit(&k_empty[kb]);
                     }
                     __syncwarp();
                 }
@@ -352,17 +386,23 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(wrow0) << 16);
         uint8_t* const wslot = smem + C::OFF_WSTG + w4 * C::WSLOTS * C::WQ_BYTES;
-        // where the next bulk copy (one group each) is staged: two slots in turn, once the copy before last has read its own
+        // Where the next bulk copy (one group each) is staged: two slots in turn, once the copy before last has read its own;
+        // or one slot, or its halves in turn for copies of half its size.
         int pos = 0;
-        auto next_slot = [&]() -> uint8_t* {
-            if (lane == 0) tma_wait_group_read<1>();
+        bool last_half = false;
+        auto next_slot = [&](bool half) -> uint8_t* {
+            if (lane == 0) {
+                if (C::WSLOTS == 2 || (half && last_half)) tma_wait_group_read<1>();
+                else tma_wait_group_read<0>();
+            }
             __syncwarp();
+            last_half = half;
             pos ^= 1;
-            return wslot + pos * C::WQ_BYTES;
+            return wslot + (C::WSLOTS == 2 ? pos * C::WQ_BYTES : (half ? pos * (C::WQ_BYTES / 2) : 0));
         };
         // 32 columns of 32 rows as bf16, by a bulk tensor store (which clips rows past N and columns past Dt)
         auto store_rows = [&](const CUtensorMap* tm, const uint4 (&u)[4], int h, int row0, int col0, int bs) {
-            uint8_t* sl = next_slot();
+            uint8_t* sl = next_slot(true);
 #pragma unroll
             for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sl + swz_off<64>(lane, c)) = u[c];
             fence_async_smem();
@@ -393,29 +433,22 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll 1
                 for (int i = 0; i < NT && ok; ++i) {
                     if (resident && j < NT - 1) break;             // dQ is still being summed
-                    const int ev = dq_event(resident, sg, j, i), b = ev % DQB;
+                    const int ev = dq_event(resident, sg, j, i), buf = ev % DQB;
                     const bool rows = i * TILE + wrow0 < p.N;     // warp-uniform: some row of this warp exists
                     const bool final_sum = whole && j == NT - 1, add = final_sum && j > 0 && !resident && rows;
                     float4* ps = part + static_cast<size_t>(i * 4 + w4) * (DH / 4) * 32;
                     float4 old[8];
-                    // The bulk copy that last wrote this part of the scratch area, a segment ago, is complete
-                    // before the sum is added to or read: two or more were issued after it (NT > DQB).
-                    if (whole && j > 0 && !resident) {
-                        if (lane == 0) tma_wait_group<2>();
-                        if (add) fence_async_all();
-                        __syncwarp();
-                    }
-                    ok = warp_all(mbar_wait(&dq_full[b], (ev / DQB) & 1, wc, 0x68));
+                    ok = warp_all(mbar_wait(&dq_full[buf], (ev / DQB) & 1, wc, 0x68));
                     if (!ok) break;
                     tc_fence_after();
 #pragma unroll
                     for (int rd = 0; rd < DH / 32; ++rd) {
                         float dqv[32];
-                        tmem_ld_f32<32>(lane_base + C::TMEM_DQ + b * DH + rd * 32, dqv);
+                        tmem_ld_f32<32>(lane_base + C::TMEM_DQ + buf * DH + rd * 32, dqv);
                         if (rd == DH / 32 - 1) {
                             tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) mbar_arrive(&dq_free[b]);
+                            if (lane == 0) mbar_arrive(&dq_free[buf]);
                         }
                         if (!rows || rd * 32 >= p.Dt) continue;    // warp-uniform
                         if (final_sum) {
@@ -433,21 +466,25 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                             store_rows(&tm_dq, u, h, i * TILE + wrow0, rd * 32, bs);
                             continue;
                         }
-                        uint8_t* wq = next_slot();
-                        const float sc = whole ? 1.0f : p.scale;
+                        if (whole) {
+                            // (the thread that reads the sum in the last segment is the same)
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) {
+                                float4* at = ps + (rd * 8 + c) * 32 + lane;
+                                if (j == 0) __stcg(at, make_float4(dqv[c * 4], dqv[c * 4 + 1], dqv[c * 4 + 2], dqv[c * 4 + 3]));
+                                else red_add_v4(reinterpret_cast<float*>(at), dqv[c * 4], dqv[c * 4 + 1], dqv[c * 4 + 2], dqv[c * 4 + 3]);
+                            }
+                            continue;
+                        }
+                        uint8_t* wq = next_slot(false);
 #pragma unroll
                         for (int c = 0; c < 8; ++c)
-                            *reinterpret_cast<float4*>(wq + (whole ? (c * 32 + lane) * 16 : swz_off<128>(lane, c))) =
-                                make_float4(dqv[c * 4 + 0] * sc, dqv[c * 4 + 1] * sc, dqv[c * 4 + 2] * sc, dqv[c * 4 + 3] * sc);
+                            *reinterpret_cast<float4*>(wq + swz_off<128>(lane, c)) =
+                                make_float4(dqv[c * 4 + 0] * p.scale, dqv[c * 4 + 1] * p.scale, dqv[c * 4 + 2] * p.scale, dqv[c * 4 + 3] * p.scale);
                         fence_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            if (!whole)
-                                tma_reduce_add_4d(&tm_acc, wq, rd * 32, h, i * TILE + wrow0, bs - p.acc_row0);
-                            else if (j == 0)
-                                bulk_store(ps + rd * 8 * 32, wq, C::WQ_BYTES);
-                            else
-                                bulk_reduce_add_f32(ps + rd * 8 * 32, wq, C::WQ_BYTES);
+                            tma_reduce_add_4d(&tm_acc, wq, rd * 32, h, i * TILE + wrow0, bs - p.acc_row0);
                             tma_commit_group();
                         }
                     }
@@ -458,8 +495,13 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 tc_fence_after();
                 const bool some = j * TILE + wrow0 < p.N;      // warp-uniform
                 uint4 u[2][DH / 32][4];
+                auto store = [&](int t) {
 #pragma unroll
-                for (int t = 0; t < 2; ++t)                     // dK, then dV
+                    for (int c = 0; c < DH / 32; ++c)
+                        if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[t][c], h, j * TILE + wrow0, c * 32, bs);
+                };
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {                   // dK, then dV
 #pragma unroll
                     for (int c = 0; c < DH / 32; ++c) {
                         float v[32];
@@ -467,14 +509,13 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         tmem_ld_f32<32>(lane_base + (t ? C::TMEM_DV : C::TMEM_DK) + c * 32, v);
                         pack_rows(u[t][c], v, t ? 1.0f : p.scale);
                     }
+                    if (DH == 64 && t == 0) store(0);          // (no registers for both)
+                }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(dkv_free);
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-#pragma unroll
-                    for (int c = 0; c < DH / 32; ++c)
-                        if (some && c * 32 < p.Dt) store_rows(t ? &tm_dv : &tm_dk, u[t][c], h, j * TILE + wrow0, c * 32, bs);
+                if (DH == 32) store(0);
+                store(1);
             }
         };
         if (WALK != WALK_SEGMENTS) drain(std::true_type{}, 0, seg.n_ws);
@@ -572,6 +613,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_free[hf]);
+                if (DH == 64) mbar_release_after_loads(&bias_empty[slot], bq[0][0] ^ bq[1][0] ^ bq[2][0] ^ bq[3][0], scratch_w);
 #pragma unroll
                 for (int cb = 0; cb < 4; ++cb) {              // 8 columns: four blocks of 8 kv
 #pragma unroll
@@ -591,7 +633,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         asm volatile("" : "+r"(pkp[w]), "+r"(pkd[w]));
                     }
                 }
-                mbar_release_after_loads(&bias_empty[slot], pkp[0] ^ pkp[2] ^ pkp[4] ^ pkp[6], scratch_w);
+                if (DH != 64) mbar_release_after_loads(&bias_empty[slot], pkp[0] ^ pkp[2] ^ pkp[4] ^ pkp[6], scratch_w);
                 if (gs > 0) {
                     ok = warp_all(mbar_wait(ds_free, (gs - 1) & 1, wc, 0x61));
                     if (!ok) break;
