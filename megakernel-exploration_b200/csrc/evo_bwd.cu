@@ -55,6 +55,7 @@ struct BwdParams {
     __nv_bfloat16* dk;
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
+    int release;          // the next kernel on the stream may take SMs early (not if some are kept free for other work)
     unsigned int* status;
 };
 
@@ -175,6 +176,7 @@ constexpr int prep_blocks() { return U == 1 ? 5 : 3; }      // per SM: 48 and 80
 template <int LANES, bool GATED, int U>
 __global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const PrepParams p) {
     constexpr uint32_t ONES = 0x3f803f80u;     // bf16 (1, 1)
+    chain_wait_and_release();
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int N = p.N, H = p.H, NTP = p.NTP;
@@ -300,6 +302,7 @@ __device__ __forceinline__ uint4 cvt8(const float* src) {
 }
 template <int DH>
 __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
+    chain_wait_and_release();
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     for (size_t i = t0; i < p.n8; i += gstride) {
@@ -389,6 +392,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.dq = static_cast<__nv_bfloat16*>(dq);
     p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
     p.lay = lay_grad;          // D = 128: thread-level stores (D <= 64 stores through tensor maps)
+    p.release = reserved_sms <= 0;
     p.status = status_word();
     if (!p.status) return EVO_ERR_CUDA;
 
@@ -487,7 +491,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;
         if (!dbias_here && (rc = launch_dbias(d, tq, tk, tv, tdo, bias, xq, xk, dbias_acc,
-                                              (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, st)))
+                                              (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, both, st)))
             return rc;
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
@@ -498,9 +502,9 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         const int e = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
         if (e) return e;
         prof_begin(1, st);
-        kernel<<<grid, threads, smem, st>>>(maps..., p);
+        const int e2 = launch_chained(both, kernel, grid, threads, smem, st, maps..., p);
         prof_end(1, st);
-        return cuda_err(cudaGetLastError());
+        return e2;
     };
     auto launch = [&](auto walk_c) -> int {
         constexpr int W = decltype(walk_c)::value;
@@ -532,8 +536,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     f.dbias_acc = convert_dbias ? dbias_acc : nullptr;
     f.dbias = static_cast<__nv_bfloat16*>(dbias_out);
     f.nb8 = db_elems / 8;
-    bwd_finish_kernel<DH><<<sms * 8, 256, 0, st>>>(f);
-    return cuda_err(cudaGetLastError());
+    return launch_chained(both, bwd_finish_kernel<DH>, sms * 8, 256, 0, st, f);
 }
 
 }  // namespace evo

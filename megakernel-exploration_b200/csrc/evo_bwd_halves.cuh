@@ -190,6 +190,8 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
+    if (p.release) chain_release();
 
     const Segments<WALK> seg(p);
     const int n_segs = seg.n;

@@ -110,6 +110,8 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
+    if (p.release) chain_release();
 
     static_assert(WALK != WALK_BOTH, "all pairs whole, or none");
     const Segments<WALK> seg(p);

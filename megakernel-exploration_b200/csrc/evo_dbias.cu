@@ -140,6 +140,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait_and_release();
 
     const int first = blockIdx.x;
     const int stride = gridDim.x;
@@ -402,7 +403,7 @@ int dbias_slices(const EvoDims* d, int sms) {
 template <int DH>
 static int launch_dbias_t(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                           const CUtensorMap& tdo, const void* bias, const void* xq, const void* xk, float* dbias,
-                          void* dbias16, int slices, float scale, int sms, cudaStream_t st) {
+                          void* dbias16, int slices, float scale, int sms, bool chained, cudaStream_t st) {
     constexpr int NG = DBIAS_GROUPS<DH>;
     using C = DbCfg<DH, NG>;
     const int NT = (d->N + TILE - 1) / TILE;
@@ -428,16 +429,16 @@ static int launch_dbias_t(const EvoDims* d, const CUtensorMap& tq, const CUtenso
         return rc;
     const int grid = p.total_items < sms ? p.total_items : sms;
     prof_begin(2, st);
-    evo_dbias_kernel<DH, NG><<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tdo, p);
+    rc = launch_chained(chained, evo_dbias_kernel<DH, NG>, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tdo, p);
     prof_end(2, st);
-    return cuda_err(cudaGetLastError());
+    return rc;
 }
 
 int launch_dbias(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                  const void* bias, const void* xq, const void* xk, float* dbias, void* dbias16, int slices, float scale, int sms,
-                 cudaStream_t st) {
+                 bool chained, cudaStream_t st) {
     auto f = d->D <= 32 ? launch_dbias_t<32> : (d->D <= 64 ? launch_dbias_t<64> : launch_dbias_t<128>);
-    return f(d, tq, tk, tv, tdo, bias, xq, xk, dbias, dbias16, slices, scale, sms, st);
+    return f(d, tq, tk, tv, tdo, bias, xq, xk, dbias, dbias16, slices, scale, sms, chained, st);
 }
 
 }  // namespace evo

@@ -14,6 +14,6 @@ int dbias_slices(const EvoDims* d, int sms);
 // [B*S][H][NTP][8] with the per-row terms and bf16 [B*S][NTP][8] with the per-column terms.
 int launch_dbias(const EvoDims* d, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                  const void* bias, const void* xq, const void* xk, float* dbias, void* dbias16, int slices, float scale, int sms,
-                 cudaStream_t st);
+                 bool chained, cudaStream_t st);
 
 }  // namespace evo

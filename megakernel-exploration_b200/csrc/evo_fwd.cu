@@ -246,6 +246,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait_and_release();
 
     // Items.  h fastest, then q tile, then row (or group of G rows), so that CTAs side by side touch the
     // same 128-byte lines of q/k/v.  Every stream counts the same number of items; the last ones of a
@@ -782,7 +783,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_wide_kernel<true> : evo_fwd_wide_kernel<false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, p);
+        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, p);
         prof_end(0, st);
     } else {
         using C = FwdCfg<DH>;
@@ -808,10 +809,10 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_kernel<DH, true> : evo_fwd_kernel<DH, false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(tq, tk, tv, tb, to, t2, p);
+        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, to, t2, p);
         prof_end(0, st);
     }
-    return cuda_err(cudaGetLastError());
+    return rc;
 }
 
 }  // namespace evo

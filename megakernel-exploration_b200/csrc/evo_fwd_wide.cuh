@@ -116,6 +116,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait_and_release();
 
     // Items: (head, pair of q tiles, row, batch), or single ones dealt to the streams in turn (OWN).
     const int first = blockIdx.x, stride = gridDim.x, per_cta = stride * (own ? 2 : 1);

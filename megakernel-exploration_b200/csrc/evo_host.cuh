@@ -71,4 +71,25 @@ int set_max_smem_once(const void* func, int bytes);
 void prof_begin(int kernel, cudaStream_t st);
 void prof_end(int kernel, cudaStream_t st);
 
+// Launches a kernel that begins with chain_wait_and_release (evo_ptx.cuh).  chained: its blocks may be placed, and wait there,
+// as soon as those of the kernel before it on the stream have all started.  (Not between the two phases of a backward with a
+// collective beside it: blocks that wait would take the SMs that are kept free for that.  Nor the prep kernel: its blocks, three
+// or five to an SM, then go to the SMs in the order in which these become free, and read a step's tensors slower: B=1, S=512,
+// N=384, H=8, D=32 a step 862 -> 885 us.  The four others each take 1 to 4 us off a step: the same one 862 -> 854; S=200, N=200,
+// H=4 115.5 -> 108.7; a forward of B=4, S=1, N=512, H=16, D=64 behind another 18.4 -> 16.2.)
+template <typename... P, typename... A>
+int launch_chained(bool chained, void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cuda_err(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 }  // namespace evo

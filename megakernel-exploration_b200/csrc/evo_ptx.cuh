@@ -51,6 +51,18 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// ---- kernels of a chain -------------------------------------------------------
+// Every kernel of a step is launched so that its blocks may start when all blocks of the kernel before it have (launch_chained):
+// what they set up for themselves then runs while that kernel's last blocks finish.  wait: the kernel before, and all that it
+// waited for, is complete and its writes are visible; no global memory is touched ahead of it.  release: the next one may start
+// (at once: its blocks only fit where one of ours has ended).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait_and_release() {
+    chain_wait();
+    chain_release();
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
