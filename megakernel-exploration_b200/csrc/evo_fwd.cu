@@ -83,10 +83,10 @@ struct FwdParams {
 //
 // The streams are at different places of their code at any time, and what they fetch competes for the instruction cache
 // (1.1 warps a scheduler wait for instructions per issue; 0.7 with short waits).  Short waits, 105 -> 83 KB of code: B=1, S=512, N=384,
-// H=8, D=32 0.302 -> 0.277 ms; S=200, N=200, H=4 44 -> 40 us; S=256, N=1024, H=4, D=64 640 -> 575.  The producer's loop stays
-// unrolled over the streams, its masks requested ahead: one copy of it for all streams was 0.298 ms at the first shape (one
-// warp is then too slow for three streams).  With two streams, D = 64, the one copy was the quicker (B=4, S=1, N=512, H=16
-// 18.4 -> 16.6 us): the number of copies could go by G, which is not done.  Rolling the loops over a tile's chunks: no gain.
+// H=8, D=32 0.302 -> 0.277 ms; S=200, N=200, H=4 44 -> 40 us; S=256, N=1024, H=4, D=64 640 -> 575.  The producer's loop is
+// unrolled over three streams, its masks requested ahead: one copy of it was 0.298 ms at the first shape (one warp is then too slow for
+// three streams).  Over two streams, D = 64, one copy is the quicker: S=256, N=1024, H=4 597 -> 582 us, S=300, N=128 34.2 -> 32.7,
+// B=4, S=1, N=1024, H=16 54.7 -> 53.6.  Rolling the loops over a tile's chunks: no gain.
 //
 // One maximum per 128 columns instead of one per 64 leaves one exact P a row and tile instead of two: O is 2 to 3 %
 // further from 64 bits (relative error 2.11e-3 -> 2.16e-3 at N = 264, D = 64, of which 1.66e-3 is its own bf16).  Two
@@ -279,6 +279,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Round r holds tile r of every stream (item r / NT, kv tile r % NT): the bias tile, then Q per
             // item, K and the mask tile.  (V is fetched by the stream's MMA warp, the first to know that its
             // buffer is free.)  The warp runs with all lanes and elects one to issue.
+            constexpr int COPIES = G == 3 ? G : 1;      // of the loop over streams (see above)
             int used[G], qn[G];      // tiles and items of the stream so far
             FwdItem item[3] = {items_of(0), items_of(1), items_of(2)};      // the first G of them are walked
 #pragma unroll
@@ -287,7 +288,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             int r = 0;
             for (int it = 0; it < n_items && ok; ++it) {
                 for (int j = 0; j < NT && ok; ++j, ++r) {
-#pragma unroll
+#pragma unroll COPIES
                     for (int s = 0; s < G; ++s) {
                         if (!ok || !item[s].valid(p)) continue;
                         const int bs = item[s].bs(p), qt = item[s].qt, h = item[s].h;
@@ -340,7 +341,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         }
                     }
                 }
-#pragma unroll
+#pragma unroll COPIES
                 for (int s = 0; s < G; ++s) advance(item[s], s);
             }
             // the last loads have landed before the CTA exits (also if a wait gave up)
