@@ -8,6 +8,14 @@
 // so what bounds it is that chain, and the 16 compute warps, idle while the products are formed, read
 // out dQ (32 columns each, a 600-clock pass; four drain warps took 2900) and, after a segment, dK and dV.
 //
+// A step takes 8000 clocks (B=1, S=128, N=768, H=4).  Measured in it: 1400 of arithmetic, 3400 in which the compute warps wait for
+// their reductions of dQ (64 KB a step; an SM sends them at 18 bytes a clock in rows of 64 bytes, 25 contiguous), 2100 for dQ.
+// Without its reductions it is 11 % shorter, no more.  What takes their place is shared memory: 270 KB of operands a step at 128
+// bytes a clock beside 100 KB of loads and the compute warps' accesses.  Tried, kernel alone at that shape against 552 us: the reductions
+// on four drain warps (554); with that, Q in halves through a ring of three, K and V on barriers of their own and the bias by ldmatrix
+// (586); and with that, dQ in the columns of dP', so that S' waits for dV alone, dK from the dS tile, and 32 columns of dQ read by the
+// compute warps (589).
+//
 //   warps 0-15 (compute)  group g = warp / 4 owns q columns 32g .. 32g+31 of the tile, and head-dim columns
 //                         32g .. 32g+31 of dQ, dK and dV
 //   warp 16 (producer)    TMA: dO with the extra tile of the q rows, Q, the pair-bias tile per step; K, V and
@@ -19,7 +27,7 @@ namespace evo {
 
 template <int DH>
 struct BwdWideCfg {
-    static_assert(DH == 128, "D <= 32 is in evo_bwd_halves.cuh, 64 in evo_bwd.cu");
+    static_assert(DH == 128, "D <= 64 is in evo_bwd_halves.cuh");
     static constexpr int NG = 4;                       // compute groups
     static constexpr int NCW = 4 * NG;
     static constexpr int W_PROD = NCW, W_MMA = NCW + 1;
