@@ -279,70 +279,78 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Round r holds tile r of every stream (item r / NT, kv tile r % NT): the bias tile, then Q per
             // item, K and the mask tile.  (V is fetched by the stream's MMA warp, the first to know that its
             // buffer is free.)  The warp runs with all lanes and elects one to issue.
-            constexpr int COPIES = G == 3 ? G : 1;      // of the loop over streams (see above)
             int used[G], qn[G];      // tiles and items of the stream so far
             FwdItem item[3] = {items_of(0), items_of(1), items_of(2)};      // the first G of them are walked
 #pragma unroll
             for (int s = 0; s < G; ++s) used[s] = qn[s] = 0;
             bool ok = true;
             int r = 0;
+            // one copy of the code per stream, or (D = 64) for both (see above)
+            auto each_stream = [&](auto&& f) {
+                if constexpr (G == 3) {
+#pragma unroll
+                    for (int s = 0; s < G; ++s) f(s);
+                } else {
+#pragma unroll 1
+                    for (int s = 0; s < G; ++s) f(s);
+                }
+            };
+            auto load_tile = [&](int s, int j, int r) {
+                if (!ok || !item[s].valid(p)) return;
+                const int bs = item[s].bs(p), qt = item[s].qt, h = item[s].h;
+                const FwdBars b(bars + s * C::BARS);
+                uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
+                // four mask values per lane, requested before the waits
+                const int c = j * TILE + 4 * lane;
+                uint2 mw = make_uint2(0u, 0u);
+                if (c < p.N) mw = __ldg(reinterpret_cast<const uint2*>(p.mask + static_cast<size_t>(bs) * p.N + c));
+                if (j == 0) {
+                    const int qb = qn[s] % NQ, use = qn[s] / NQ;
+                    if (qn[s]++ >= NQ) ok = warp_all(mbar_wait(&b.q_empty[qb], (use - 1) & 1, wc, 0x10));
+                    if (ok && elect_one()) {
+                        mbar_arrive_expect_tx(&b.q_full[qb], C::ROWT);
+                        tma_load_row_tile<DH>(sb + C::ST_Q + qb * C::ROWT, &tm_q, &b.q_full[qb], h, qt * TILE, bs);
+                    }
+                    __syncwarp();
+                }
+                if (!ok) return;
+                const int n = used[s]++, kb = n % NK;
+                if (n >= NK) ok = warp_all(mbar_wait(&b.k_empty[kb], ((n / NK) - 1) & 1, wc, 0x11));
+                if (!ok) return;
+                if (elect_one()) {
+                    mbar_expect_tx(&b.k_full[kb], C::ROWT);
+                    tma_load_row_tile<DH>(sb + C::ST_K + kb * C::ROWT, &tm_k, &b.k_full[kb], h, j * TILE, bs);
+                }
+                __syncwarp();
+                const float mv[4] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y)};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint2 w = mask_term(c < p.N ? mv[e] : -INFINITY, p.inv_scale);
+                    *reinterpret_cast<uint4*>(sb + C::ST_XK + kb * XT_BYTES + (4 * lane + e) * 16) = make_uint4(w.x, w.y, 0u, 0u);
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (elect_one()) mbar_arrive(&b.k_full[kb]);
+                __syncwarp();
+                // the bias tile: once per round if the streams share it (stream 0 always has the item)
+                if (!shared_bias || s == 0) {
+                    int slot; uint32_t ph;
+                    bias_slot(s, r, slot, ph);
+                    if (r >= (shared_bias ? NR : 1)) ok = warp_all(mbar_wait(&bias_empty[slot], ph ^ 1u, wc, 0x14));
+                    if (ok && elect_one()) {
+                        uint8_t* bt = smem + C::OFF_BIAS + slot * SQ_BYTES;
+                        mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
+                        tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, item[s].b);
+                        tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, item[s].b);
+                    }
+                    __syncwarp();
+                }
+            };
             for (int it = 0; it < n_items && ok; ++it) {
                 for (int j = 0; j < NT && ok; ++j, ++r) {
-#pragma unroll COPIES
-                    for (int s = 0; s < G; ++s) {
-                        if (!ok || !item[s].valid(p)) continue;
-                        const int bs = item[s].bs(p), qt = item[s].qt, h = item[s].h;
-                        const FwdBars b(bars + s * C::BARS);
-                        uint8_t* sb = smem + C::OFF_STREAM + s * C::STREAM_BYTES;
-                        // four mask values per lane, requested before the waits
-                        const int c = j * TILE + 4 * lane;
-                        uint2 mw = make_uint2(0u, 0u);
-                        if (c < p.N) mw = __ldg(reinterpret_cast<const uint2*>(p.mask + static_cast<size_t>(bs) * p.N + c));
-                        if (j == 0) {
-                            const int qb = qn[s] % NQ, use = qn[s] / NQ;
-                            if (qn[s]++ >= NQ) ok = warp_all(mbar_wait(&b.q_empty[qb], (use - 1) & 1, wc, 0x10));
-                            if (ok && elect_one()) {
-                                mbar_arrive_expect_tx(&b.q_full[qb], C::ROWT);
-                                tma_load_row_tile<DH>(sb + C::ST_Q + qb * C::ROWT, &tm_q, &b.q_full[qb], h, qt * TILE, bs);
-                            }
-                            __syncwarp();
-                        }
-                        if (!ok) continue;
-                        const int n = used[s]++, kb = n % NK;
-                        if (n >= NK) ok = warp_all(mbar_wait(&b.k_empty[kb], ((n / NK) - 1) & 1, wc, 0x11));
-                        if (!ok) continue;
-                        if (elect_one()) {
-                            mbar_expect_tx(&b.k_full[kb], C::ROWT);
-                            tma_load_row_tile<DH>(sb + C::ST_K + kb * C::ROWT, &tm_k, &b.k_full[kb], h, j * TILE, bs);
-                        }
-                        __syncwarp();
-                        const float mv[4] = {bf16_lo(mw.x), bf16_hi(mw.x), bf16_lo(mw.y), bf16_hi(mw.y)};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint2 w = mask_term(c < p.N ? mv[e] : -INFINITY, p.inv_scale);
-                            *reinterpret_cast<uint4*>(sb + C::ST_XK + kb * XT_BYTES + (4 * lane + e) * 16) = make_uint4(w.x, w.y, 0u, 0u);
-                        }
-                        fence_async_smem();
-                        __syncwarp();
-                        if (elect_one()) mbar_arrive(&b.k_full[kb]);
-                        __syncwarp();
-                        // the bias tile: once per round if the streams share it (stream 0 always has the item)
-                        if (!shared_bias || s == 0) {
-                            int slot; uint32_t ph;
-                            bias_slot(s, r, slot, ph);
-                            if (r >= (shared_bias ? NR : 1)) ok = warp_all(mbar_wait(&bias_empty[slot], ph ^ 1u, wc, 0x14));
-                            if (ok && elect_one()) {
-                                uint8_t* bt = smem + C::OFF_BIAS + slot * SQ_BYTES;
-                                mbar_arrive_expect_tx(&bias_full[slot], SQ_BYTES);
-                                tma_load_4d(bt, &tm_bias, &bias_full[slot], j * TILE, qt * TILE, h, item[s].b);
-                                tma_load_4d(bt + SQ_SUB_BYTES, &tm_bias, &bias_full[slot], j * TILE + 64, qt * TILE, h, item[s].b);
-                            }
-                            __syncwarp();
-                        }
-                    }
+                    each_stream([&](int s) { load_tile(s, j, r); });
                 }
-#pragma unroll COPIES
-                for (int s = 0; s < G; ++s) advance(item[s], s);
+                each_stream([&](int s) { advance(item[s], s); });
             }
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
@@ -773,6 +781,10 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
 
     int sms = 0;
     if ((rc = sm_count(&sms))) return rc;
+    // Placed early (launch_chained) where start-up is a good part of it: up to 64 tiles an SM (B=4, S=1, N=512, H=16, D=64, seven:
+    // 18.4 -> 16.4 us).  Longer ones gain nothing: the order in which the SMs become free then decides which blocks lie side by
+    // side (S=512, N=384, H=8, 249 tiles: 289.4 -> 291.3 us, twice).
+    const bool chained = static_cast<long>(p.total_items) * QT <= 64L * sms;
     if constexpr (WIDE) {
         using C = FwdWideCfg;
         // pairs of q tiles; with one q tile per row, items dealt to the two streams of a CTA in turn
@@ -784,7 +796,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_wide_kernel<true> : evo_fwd_wide_kernel<false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, p);
+        rc = launch_chained(chained, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, p);
         prof_end(0, st);
     } else {
         using C = FwdCfg<DH>;
@@ -810,7 +822,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_kernel<DH, true> : evo_fwd_kernel<DH, false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, to, t2, p);
+        rc = launch_chained(chained, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, to, t2, p);
         prof_end(0, st);
     }
     return rc;
