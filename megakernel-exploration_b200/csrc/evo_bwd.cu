@@ -452,9 +452,6 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     // one S row and the whole backward in this call: the dQ/dK/dV kernel writes dBias (= dS) itself
     const bool both = (phases & EVO_BWD_PHASE_DBIAS) && (phases & EVO_BWD_PHASE_DQKV);
     const bool dbias_here = (d->S == 1) && both;
-    // Placed early (launch_chained), but for long steps at D = 128, which are slower for it (B=1, S=128, N=768, H=4, 125 tiles
-    // an SM: 1102 -> 1109 us).
-    const bool chained = both && (DH != 128 || static_cast<long>(pairs) * NT * NT <= 64L * sms);
     p.dbias = dbias_out;
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
@@ -494,7 +491,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;
         if (!dbias_here && (rc = launch_dbias(d, tq, tk, tv, tdo, bias, xq, xk, dbias_acc,
-                                              (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, chained, st)))
+                                              (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, both, st)))
             return rc;
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
@@ -505,7 +502,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         const int e = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
         if (e) return e;
         prof_begin(1, st);
-        const int e2 = launch_chained(chained, kernel, grid, threads, smem, st, maps..., p);
+        const int e2 = launch_chained(both, kernel, grid, threads, smem, st, maps..., p);
         prof_end(1, st);
         return e2;
     };
@@ -539,7 +536,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     f.dbias_acc = convert_dbias ? dbias_acc : nullptr;
     f.dbias = static_cast<__nv_bfloat16*>(dbias_out);
     f.nb8 = db_elems / 8;
-    return launch_chained(chained, bwd_finish_kernel<DH>, sms * 8, 256, 0, st, f);
+    return launch_chained(both, bwd_finish_kernel<DH>, sms * 8, 256, 0, st, f);
 }
 
 }  // namespace evo

@@ -781,10 +781,6 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
 
     int sms = 0;
     if ((rc = sm_count(&sms))) return rc;
-    // Placed early (launch_chained) where start-up is a good part of it: up to 64 tiles an SM (B=4, S=1, N=512, H=16, D=64, seven:
-    // 18.4 -> 16.4 us).  Longer ones gain nothing: the order in which the SMs become free then decides which blocks lie side by
-    // side (S=512, N=384, H=8, 249 tiles: 289.4 -> 291.3 us, twice).
-    const bool chained = static_cast<long>(p.total_items) * QT <= 64L * sms;
     if constexpr (WIDE) {
         using C = FwdWideCfg;
         // pairs of q tiles; with one q tile per row, items dealt to the two streams of a CTA in turn
@@ -796,7 +792,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_wide_kernel<true> : evo_fwd_wide_kernel<false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        rc = launch_chained(chained, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, p);
+        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, p);
         prof_end(0, st);
     } else {
         using C = FwdCfg<DH>;
@@ -822,7 +818,7 @@ static int launch_fwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto kernel = gate ? evo_fwd_kernel<DH, true> : evo_fwd_kernel<DH, false>;
         if ((rc = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(C::SMEM_BYTES)))) return rc;
         prof_begin(0, st);
-        rc = launch_chained(chained, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, to, t2, p);
+        rc = launch_chained(true, kernel, grid, C::THREADS, C::SMEM_BYTES, st, tq, tk, tv, tb, to, t2, p);
         prof_end(0, st);
     }
     return rc;
