@@ -556,7 +556,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // by whole rows: four-lane transposes leave lane c with the block of kv 8 c .. 8 c + 7, so that a store takes 128 bytes
         // of one q row (fp32) or 64 of eight (bf16).  Inside the arithmetic, and straight from the fragments, with 32 bytes of
         // four or eight rows, the addresses and values did not fit the registers, and the stores were what a step waited for:
-        // B=4, S=1, N=1024, H=16, D=32 fp32 116 -> 91 us, bf16 85 -> 75 (one thread per kv row, as at D = 64: 101 and 82).
+        // B=4, S=1, N=1024, H=16, D=32 fp32 116 -> 91 us, bf16 85 -> 75 (one thread per kv row: 101 and 82).
         // out: this lane's place in q row 32 g of the tile
         auto store_dbias = [&](auto* out, int q0, uint32_t (&pkd)[16], float2 (&dsv)[16]) {
             if constexpr (DBIAS_HERE != DBIAS_NO) {

@@ -52,7 +52,7 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- kernels of a chain -------------------------------------------------------
-// Every kernel of a step is launched so that its blocks may start when all blocks of the kernel before it have (launch_chained):
+// Every kernel of a step but the prep kernel is launched so that its blocks may start when all blocks of the kernel before it have (launch_chained):
 // what they set up for themselves then runs while that kernel's last blocks finish.  wait: the kernel before, and all that it
 // waited for, is complete and its writes are visible; no global memory is touched ahead of it.  release: the next one may start
 // (at once: its blocks only fit where one of ours has ended).
