@@ -55,7 +55,7 @@ struct BwdParams {
     __nv_bfloat16* dk;
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
-    int release;          // the next kernel on the stream may take SMs early (not if some are kept free for other work)
+    int release;          // the next kernel on the stream may be placed early (not if some SMs are kept free for other work)
     unsigned int* status;
 };
 
@@ -176,7 +176,6 @@ constexpr int prep_blocks() { return U == 1 ? 5 : 3; }      // per SM: 48 and 80
 template <int LANES, bool GATED, int U>
 __global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const PrepParams p) {
     constexpr uint32_t ONES = 0x3f803f80u;     // bf16 (1, 1)
-    chain_wait_and_release();
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int N = p.N, H = p.H, NTP = p.NTP;
@@ -302,7 +301,7 @@ __device__ __forceinline__ uint4 cvt8(const float* src) {
 }
 template <int DH>
 __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
-    chain_wait_and_release();
+    chain_wait();
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     for (size_t i = t0; i < p.n8; i += gstride) {

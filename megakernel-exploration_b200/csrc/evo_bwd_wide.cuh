@@ -119,7 +119,6 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     chain_wait();
-    if (p.release) chain_release();
 
     static_assert(WALK != WALK_BOTH, "all pairs whole, or none");
     const Segments<WALK> seg(p);
@@ -176,6 +175,7 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 ++n_q;
             }
         }
+        if (p.release) chain_release();
         // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
         // barrier with an MMA commit, which may then never come: a bounded pause instead).
         const WaitCtx dc{tmem_slot + 3, p.status};

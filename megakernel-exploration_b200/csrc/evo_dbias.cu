@@ -140,7 +140,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    chain_wait_and_release();
+    chain_wait();
 
     const int first = blockIdx.x;
     const int stride = gridDim.x;
@@ -204,6 +204,7 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     }
                 }
             }
+            chain_release();
             // the most recent loads have landed before the CTA exits (also if a wait gave up; the other producer's half
             // of a stage may then never have been asked for: a bounded pause instead)
             const WaitCtx dc{tmem_slot + 3, p.status};

@@ -246,7 +246,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    chain_wait_and_release();
+    chain_wait();
 
     // Items.  h fastest, then q tile, then row (or group of G rows), so that CTAs side by side touch the
     // same 128-byte lines of q/k/v.  Every stream counts the same number of items; the last ones of a
@@ -352,6 +352,7 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 each_stream([&](int s) { advance(item[s], s); });
             }
+            chain_release();
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
 #pragma unroll

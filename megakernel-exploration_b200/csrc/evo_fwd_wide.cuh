@@ -116,7 +116,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    chain_wait_and_release();
+    chain_wait();
 
     // Items: (head, pair of q tiles, row, batch), or single ones dealt to the streams in turn (OWN).
     const int first = blockIdx.x, stride = gridDim.x, per_cta = stride * (own ? 2 : 1);
@@ -213,6 +213,7 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 if (ok && r > 0) load_v(vx, vj);
             }
+            chain_release();
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
             if (n_k0 > 0) mbar_wait_landed(&k_full[0], (n_k0 - 1) & 1, dc, 0x13);
