@@ -55,7 +55,6 @@ struct BwdParams {
     __nv_bfloat16* dk;
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
-    int release;          // the next kernel on the stream may be placed early (not if some SMs are kept free for other work)
     unsigned int* status;
 };
 
@@ -391,7 +390,6 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.dq = static_cast<__nv_bfloat16*>(dq);
     p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
     p.lay = lay_grad;          // D = 128: thread-level stores (D <= 64 stores through tensor maps)
-    p.release = reserved_sms <= 0;
     p.status = status_word();
     if (!p.status) return EVO_ERR_CUDA;
 

@@ -273,7 +273,6 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
             }
         }
-        if (p.release) chain_release();
         // the last loads have landed before the CTA exits, also if a wait gave up
         const WaitCtx dc{tmem_slot + 3, p.status};
         for (int k = (n_q > NQ ? n_q - NQ : 0); k < n_q; ++k) mbar_wait_landed(&q_full[k % NQ], (k / NQ) & 1, dc, 0x43);

@@ -175,7 +175,6 @@ evo_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 ++n_q;
             }
         }
-        if (p.release) chain_release();
         // The last loads have landed before the CTA exits, also if a wait gave up (a bias load shares its
         // barrier with an MMA commit, which may then never come: a bounded pause instead).
         const WaitCtx dc{tmem_slot + 3, p.status};

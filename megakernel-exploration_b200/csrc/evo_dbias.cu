@@ -204,7 +204,6 @@ evo_dbias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     }
                 }
             }
-            chain_release();
             // the most recent loads have landed before the CTA exits (also if a wait gave up; the other producer's half
             // of a stage may then never have been asked for: a bounded pause instead)
             const WaitCtx dc{tmem_slot + 3, p.status};

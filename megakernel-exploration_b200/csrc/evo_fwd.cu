@@ -352,7 +352,6 @@ evo_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 each_stream([&](int s) { advance(item[s], s); });
             }
-            chain_release();
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
 #pragma unroll

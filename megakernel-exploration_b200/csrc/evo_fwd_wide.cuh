@@ -213,7 +213,6 @@ evo_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 if (ok && r > 0) load_v(vx, vj);
             }
-            chain_release();
             // the last loads have landed before the CTA exits (also if a wait gave up)
             const WaitCtx dc{tmem_slot + 3, p.status};
             if (n_k0 > 0) mbar_wait_landed(&k_full[0], (n_k0 - 1) & 1, dc, 0x13);

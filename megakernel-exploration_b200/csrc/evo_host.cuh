@@ -71,18 +71,18 @@ int set_max_smem_once(const void* func, int bytes);
 void prof_begin(int kernel, cudaStream_t st);
 void prof_end(int kernel, cudaStream_t st);
 
-// Launches a kernel that calls chain_wait ahead of its first access to global memory (evo_ptx.cuh).  chained: its blocks may be placed,
-// and wait there, wherever there is room, as soon as all of the kernel before it on the stream have called chain_release or ended.
-// The forward, dBias and dQ/dK/dV kernels release (dQ/dK/dV not where SMs are kept free for other work); behind any other kernel that does
-// not, the prep and finish kernels and those of other libraries included, only the launch itself is early.
-// Not chained: the two phases of a backward with a collective beside it, whose SMs blocks that wait would take.  Nor the prep kernel: its
-// blocks, three or five to an SM, then go to the SMs in the order in which these become free, and read a step's tensors slower: B=1,
-// S=512, N=384, H=8, D=32 a step 862 -> 885 us.
-// Steps queued back to back, not chained / released at the start of each kernel / when its last loads are asked for: that step
-// 857 / 855 / 848 us, D=64 S=200, N=200, H=4 156.4 / 150.4 / 148.5, B=4, S=1, N=512, H=16 63.9 / 58.1 / 57.9, D=32 S=32, N=64, H=4 35.1 / 28.7 /
-// 26.8, D=128 S=128, N=768, H=4 1091.1 / 1094.2 / 1090.7.  A 4 MB elementwise kernel of a second stream beside them: 35 / 148 / 35 us beside
-// the first step, 33 / 116 / 34 at D=64, S=128, N=1024, H=4, 26 / 65 / 26 at D=128, S=64, N=768; beside short kernels, whose ends are much of them, it
-// keeps some of the difference (D=32 S=200, N=200 11 / 22 / 14, D=64 B=4, S=1, N=1024 15 / 34 / 19: steps that are 6 and 5 us shorter).
+// Launches a kernel that calls chain_wait ahead of its first access to global memory (evo_ptx.cuh).  chained: as a programmatic launch, whose
+// blocks may be placed as soon as those of the kernel before it on the stream, whichever that is, have all ended, without the rest of a
+// launch's latency.  No kernel releases the next one ahead of its end (griddepcontrol.launch_dependents): blocks that wait take every SM that
+// becomes free, ahead of another stream's of the same priority, and steps are no shorter for it.
+// Steps queued back to back, not chained / released at the start of each kernel / chained as it is: B=1, S=512, N=384, H=8, D=32
+// 857 / 853 / 847 us; S=32, N=64, H=4 33.9 / 28.1 / 26.1; D=64: S=200, N=200, H=4 156 / 151 / 149, B=4, S=1, N=512, H=16 63.0 / 55.6 / 55.2; D=128:
+// S=128, N=768, H=4 1092 / 1095 / 1084 (released when a block has asked for its last loads: 847, 26.2, 149, 55.5, 1091).  A 4 MB elementwise
+// kernel of a second stream beside them: 35 / 148 / 35 us beside the first, 33 / 116 / 34 at D=64, S=128, N=1024, H=4, 26 / 65 / 26 at D=128, S=64,
+// N=768; beside short kernels, of whose gaps it lived, 11 / 22 / 13 (D=32, S=200, N=200, a step 118 / 111 / 111) and 15 / 34 / 19 (D=64, B=4, S=1,
+// N=1024, 162 / 156 / 157).
+// Not chained: the two phases of a backward with a collective beside it.  Nor the prep kernel, whose blocks, three or five to an SM, went to
+// the SMs in the order in which these became free when its predecessor released it, and read a step's tensors slower: the first step 862 -> 885 us.
 template <typename... P, typename... A>
 int launch_chained(bool chained, void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute at{};

@@ -52,14 +52,10 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- kernels of a chain -------------------------------------------------------
-// Every kernel of a step but the prep kernel is launched so that its blocks may be placed when every block of the kernel before it has
-// released them or ended (launch_chained): what they set up for themselves then runs while that kernel's last blocks finish.  wait: the
-// kernel before, and all that it waited for, is complete and its writes are visible; no global memory is touched ahead of it.  release:
-// issued when a block has asked for its last loads, a few microseconds before its end.  From then on the next kernel's blocks queue for every SM
-// that becomes free, ahead of another stream's of the same priority: released at the start of a kernel they kept those out for
-// all of it, the SMs included that its last round leaves idle (launch_chained has the figures).
+// Every kernel of a step but the prep kernel is launched so that its launch is under way when the kernel before it ends
+// (launch_chained).  wait: the kernel before, and all that it waited for, is complete and its writes are visible; no global memory is
+// touched ahead of it.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

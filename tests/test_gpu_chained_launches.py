@@ -1,4 +1,4 @@
-"""Kernels of a step whose blocks may be placed before the kernel ahead of them has ended (programmatic launches).
+"""Kernels of a step are programmatic launches: a wait of their own is what orders them behind the kernel ahead of them.
 
 Calls are queued without a wait, each on what the one before wrote and with no other kernel in between, into buffers that hold NaN until
 then; the other arm waits after every call and takes the backward in its two phases, whose kernels are launched in full order.  O, LSE, dK and dV are
@@ -55,7 +55,7 @@ def test_forwards_without_a_wait(B, S, N, H, D):
 @pytest.mark.parametrize("B,S,N,H,D", [
     (2, 1, 128, 4, 64),      # one S row: forward, prep, dQ/dK/dV
     (2, 8, 64, 2, 32),       # one tile: no finish kernel
-    (1, 6, 200, 4, 32),      # segments, finish kernel ahead of the next forward
+    (1, 6, 200, 4, 32),      # segments: the finish kernel is ahead of the next forward
     (1, 40, 200, 4, 64),     # whole pairs and segments
     (1, 150, 136, 2, 16),
     (1, 5, 256, 2, 128),
