@@ -39,8 +39,8 @@ for _p in (ROOT, PKG):
 import evo_workloads as wl  # noqa: E402
 
 # DRAM bytes per S row of one evo_bwd_halves_kernel launch, from the ncu capture summarised under profiles/
-# (110.21 MB read + 43.95 MB written at 128 rows of cfg2).
-NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.17e6 + 41.48e6) / 128}
+# (110.16 MB read + 43.55 MB written at 128 rows of cfg2).
+NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.16e6 + 43.55e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"
 UNIT = "TFLOP/s"

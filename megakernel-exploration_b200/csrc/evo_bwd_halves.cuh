@@ -381,7 +381,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
     } else if (warp >= C::W_DRAIN) {
         // ------------------------------ drain warps ------------------------------
-        // (The loops over DH / 32 run once.  Written without them the mixed walk spills in other places, and is slower with
+        // (The loops over DH / 32 run once at D = 32, twice at 64.  Written without them for D = 32 the mixed walk spills in other places, and is slower with
         // one S row: B=38, N=392, H=8 83 -> 89 us.)
         const int w4 = warp & 3;
         const int wrow0 = w4 * 32;           // tensor-memory lanes (tile rows) of this warp

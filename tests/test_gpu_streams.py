@@ -40,7 +40,7 @@ def test_forward_wide(B, S, N, H, D):
 
 
 # dQ/dK/dV kernel: whole items (every kv tile of a row and head in one CTA) where (rows x heads) fill the 148
-# SMs, single segments where they do not; dQ of whole items stays in tensor memory for one tile at D = 128, up to two at D = 64
+# SMs, single segments where they do not; dQ of whole items stays in tensor memory for one tile at D = 64 and 128
 # and up to four at D <= 32, with more it goes through scratch
 @pytest.mark.parametrize("bias_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,S,N,H,D", [
@@ -68,7 +68,7 @@ def test_backward_items(B, S, N, H, D, bias_type):
 @pytest.mark.parametrize("bias_type", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("B,S,N,H,D", [
     (1, 50, 200, 3, 32),     # 150: scratch and accumulator of whole rows do not fit, so all by segments
-    (1, 101, 136, 3, 64),    # 296 + 7; dQ of the whole ones stays in tensor memory
+    (1, 101, 136, 3, 64),    # 296 + 7; dQ of the whole ones goes through scratch
     (1, 50, 264, 3, 32),     # 150: all by segments, three a CTA
     (1, 99, 264, 3, 32),     # 296 + 1; three tiles in tensor memory
     (1, 50, 392, 3, 64),     # 150: all by segments
