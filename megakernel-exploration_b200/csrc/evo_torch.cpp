@@ -11,6 +11,8 @@
 // reference's own assertion); it never falls back to another implementation of the math.
 #include <torch/extension.h>
 
+#include <ATen/core/CachingHostAllocator.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -299,8 +301,73 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
     return f.out;
 }
 
+// The chunks of HostStreamedEvoAttention.run (tk_evo_attention_layer.py has what they are): rows [s0, s0 + r) of batch b in,
+// through the kernels and out, on three streams and three sets of device buffers.  ins: q, k, v, dO, mask and outs: o, dq,
+// dk, dv in host memory, contiguous; a set: q, k, v, do, mask, o, ores, dq, dk, dv, lse, dbias, ws for at least the rows
+// of a chunk.  Through torch's Python operators a chunk was about 200 us of host time, so that a step of eight chunks was
+// bound by it.
+void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunks, const std::vector<Tensor>& ins, const Tensor& bias,
+                 const Tensor& dbias, const std::vector<Tensor>& outs, const std::vector<std::vector<Tensor>>& sets,
+                 const std::vector<std::tuple<int64_t, int64_t, int64_t>>& streams) {
+    TORCH_CHECK(ins.size() == 5 && outs.size() == 4 && sets.size() == 3 && streams.size() == 3, "host_chunks: wrong number of arguments");
+    const int64_t S = ins[0].size(1), N = ins[0].size(2), H = ins[0].size(3), D = ins[0].size(4);
+    auto stream_of = [&](int i) {
+        const auto& [id, index, type] = streams[i];
+        return c10::cuda::CUDAStream::unpack3(id, static_cast<c10::DeviceIndex>(index), static_cast<c10::DeviceType>(type));
+    };
+    const c10::cuda::CUDAStream s_in = stream_of(0), s_cmp = stream_of(1), s_out = stream_of(2);
+    const c10::cuda::CUDAGuard guard(bias.device());
+    const size_t act = static_cast<size_t>(2 * N * H * D), mask_row = static_cast<size_t>(2 * N);     // bytes of a row
+    auto copy = [](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, const c10::cuda::CUDAStream& s) {
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, s.stream());
+        TORCH_CHECK(e == cudaSuccess, "HostStreamedEvoAttention: a copy failed: ", cudaGetErrorString(e));
+    };
+    // whatever happens, pinned memory is not handed out again before the copies queued so far are done
+    struct Hold {
+        const std::vector<Tensor>*ins, *outs;
+        c10::Stream in, out;
+        ~Hold() {
+            for (const Tensor& t : *ins) at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), in);
+            for (const Tensor& t : *outs) at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), out);
+        }
+    } const hold{&ins, &outs, s_in.unwrap(), s_out.unwrap()};
+    at::cuda::CUDAEvent ev_in[3], ev_cmp[3], ev_out[3];
+    for (size_t c = 0; c < chunks.size(); ++c) {
+        const auto [b, s0, r] = chunks[c];
+        const std::vector<Tensor>& st = sets[c % 3];
+        const size_t row = static_cast<size_t>(b * S + s0);
+        if (c >= 3) ev_out[c % 3].block(s_in);               // this set's previous results are out
+        for (int i = 0; i < 5; ++i) {
+            const size_t bytes = i < 4 ? act : mask_row;
+            copy(st[i].data_ptr(), static_cast<const char*>(ins[i].const_data_ptr()) + row * bytes, r * bytes, cudaMemcpyHostToDevice, s_in);
+        }
+        ev_in[c % 3].record(s_in);
+        ev_in[c % 3].block(s_cmp);
+        // a chunk with fewer rows than its set uses the leading rows of the (contiguous) buffers
+        const EvoDims dims{1, static_cast<int32_t>(r), static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(D)};
+        const void* bias_b = static_cast<const char*>(bias.const_data_ptr()) + b * 2 * H * N * N;
+        float* lse = static_cast<float*>(st[10].data_ptr());
+        check(evo_fwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
+                      st[6].data_ptr(), lse, 0.f, s_cmp.stream()), "evo_fwd");
+        check(evo_bwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
+                      st[6].data_ptr(), lse, st[3].data_ptr(), st[7].data_ptr(), st[8].data_ptr(), st[9].data_ptr(),
+                      static_cast<float*>(st[11].data_ptr()), st[12].data_ptr(), static_cast<size_t>(st[12].numel()), 0.f,
+                      s_cmp.stream()), "evo_bwd");
+        {
+            const c10::cuda::CUDAStreamGuard on(s_cmp);
+            dbias.select(0, b).add_(st[11].select(0, 0));
+        }
+        ev_cmp[c % 3].record(s_cmp);
+        ev_cmp[c % 3].block(s_out);
+        for (int i = 0; i < 4; ++i)
+            copy(static_cast<char*>(outs[i].data_ptr()) + row * act, st[i == 0 ? 5 : 6 + i].data_ptr(), r * act, cudaMemcpyDeviceToHost, s_out);
+        ev_out[c % 3].record(s_out);
+    }
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("apply", &apply, "EvoAttention with its autograd node; None if the call is not one of the plain kind");
+    m.def("host_chunks", &host_chunks, "The chunks of HostStreamedEvoAttention.run", pybind11::call_guard<pybind11::gil_scoped_release>());
 }

@@ -466,6 +466,9 @@ class HostStreamedEvoAttention:
     full pair_bias; d_pair_bias is all-reduced before it is copied out.
     """
 
+    # a buffer set, in the order of host_chunks
+    NAMES = ("q", "k", "v", "do", "mask", "o", "ores", "dq", "dk", "dv", "lse", "dbias", "ws")
+
     def __init__(self, device, chunk_rows: int = 64, process_group=None):
         self.dev = torch.device(device)
         if self.dev.type != "cuda":
@@ -475,13 +478,34 @@ class HostStreamedEvoAttention:
         self.s_in, self.s_cmp, self.s_out = (torch.cuda.Stream(self.dev) for _ in range(3))
         self._key, self._rows = None, 0
 
-    def _rows_per_chunk(self, S, N, H, D):
-        """At most chunk_rows; fewer so that there are four chunks (the link idles in one direction while the
-        first comes in and the last goes out) of copies of one to six megabytes (below, the cost of a copy
-        shows; above, the idle ends do).  B=1, N=384, H=8, D=32, chunk_rows=64, against chunks of 64
-        rows in two buffer sets: S=128 3.26 -> 3.03 ms; S=512 10.5 ms."""
-        one = -(-(1 << 20) // (2 * N * H * D))               # rows of a megabyte
-        return max(1, min(self.chunk_rows, S, max(one, min(-(-S // 4), 6 * one))))
+    def _chunks(self, B, S, N, H, D):
+        """(batch, first row, rows) of every chunk: at most chunk_rows rows, copies of one to six megabytes and at least four
+        chunks in a batch (below, the cost of a copy shows; above, the time in which the link idles in one direction,
+        while the first chunk comes in and the last goes out).  So the first chunks also grow, by twos from copies of
+        1.5 megabytes, and the last shrink to them: B=1, S=128, N=384, H=8, D=32, chunk_rows=64, 3.08-3.32 ms in four equal
+        chunks, 2.96-3.14 in [8, 16, 27, 27, 26, 16, 8], 3.02-3.30 from copies of one megabyte on (both directions at once,
+        a small copy takes several times as long)."""
+        row = 2 * N * H * D
+        one, r0 = -(-(1 << 20) // row), -(-(3 << 19) // row)
+        most = max(1, min(self.chunk_rows, S, max(one, min(-(-S // 4), 6 * one))))
+        out = []
+        for b in range(B):
+            head, tail, left, r = [], [], S, r0
+            while r < most and left > 2 * r:
+                if b == 0:
+                    head.append(r)
+                    left -= r
+                if b == B - 1:
+                    tail.append(r)
+                    left -= r
+                r *= 2
+            n = -(-left // most)
+            rows = head + [left // n + (i < left % n) for i in range(n)] + tail[::-1]
+            s0 = 0
+            for r in rows:
+                out.append((b, s0, r))
+                s0 += r
+        return out
 
     def _buffers(self, B, N, H, D, R):
         key = (B, N, H, D)
@@ -513,8 +537,8 @@ class HostStreamedEvoAttention:
         bias = pair_bias.reshape(B, H, N, N)
         assert mask.dtype == torch.bfloat16 and bias.dtype == torch.bfloat16
         dbias_out = out["dbias"].reshape(B, H, N, N)
-        R = self._rows_per_chunk(S, N, H, D)
-        self._buffers(B, N, H, D, R)
+        chunks = self._chunks(B, S, N, H, D)
+        self._buffers(B, N, H, D, max(r for _, _, r in chunks))
         cur = torch.cuda.current_stream(self.dev)
         for s_ in (self.s_in, self.s_cmp, self.s_out):
             s_.wait_stream(cur)
@@ -522,36 +546,15 @@ class HostStreamedEvoAttention:
             self.bias.copy_(bias, non_blocking=True)
         with torch.cuda.stream(self.s_cmp):
             self.dbias.zero_()
-        c = 0
-        for b in range(B):
-            for s0 in range(0, S, R):
-                r = min(R, S - s0)
-                st = self.sets[c % 3]
-                dims = _evoattn.EvoDims(1, r, N, H, D)
-                with torch.cuda.stream(self.s_in):
-                    if c >= 3:
-                        self.s_in.wait_event(st["ev_out"])      # this set's previous results are out
-                    for n, h in (("q", q), ("k", k), ("v", v), ("do", d_o)):
-                        st[n][:, :r].copy_(h[b:b + 1, s0:s0 + r], non_blocking=True)
-                    st["mask"][:, :r].copy_(mask[b:b + 1, s0:s0 + r], non_blocking=True)
-                    st["ev_in"].record(self.s_in)
-                with torch.cuda.stream(self.s_cmp):
-                    self.s_cmp.wait_event(st["ev_in"])
-                    h_ = self.s_cmp.cuda_stream
-                    # a chunk with fewer rows uses the leading rows of the (contiguous) buffers
-                    _evoattn.fwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
-                                 st["ores"], st["lse"], 0.0, h_)
-                    _evoattn.bwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
-                                 st["ores"], st["lse"], st["do"], st["dq"], st["dk"], st["dv"], st["dbias"],
-                                 st["ws"], 0.0, h_)
-                    self.dbias[b:b + 1].add_(st["dbias"])
-                    st["ev_cmp"].record(self.s_cmp)
-                with torch.cuda.stream(self.s_out):
-                    self.s_out.wait_event(st["ev_cmp"])
-                    for n in ("o", "dq", "dk", "dv"):
-                        out[n][b:b + 1, s0:s0 + r].copy_(st[n][:, :r], non_blocking=True)
-                    st["ev_out"].record(self.s_out)
-                c += 1
+        _native()
+        native = sys.modules.get("_evo_torch")
+        ins, outs = (q, k, v, d_o, mask), [out[n] for n in ("o", "dq", "dk", "dv")]
+        if native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
+                t.shape == q.shape and t.dtype == torch.bfloat16 and t.is_contiguous() and not t.is_cuda for t in outs):
+            native.host_chunks(chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
+                               [(s_.stream_id, s_.device_index, s_.device_type) for s_ in (self.s_in, self.s_cmp, self.s_out)])
+        else:
+            self._run_chunks(chunks, q, k, v, mask, d_o, out)
         with torch.cuda.stream(self.s_cmp):
             if self.pg is not None:
                 import torch.distributed as dist
@@ -559,3 +562,33 @@ class HostStreamedEvoAttention:
             dbias_out.copy_(self.dbias, non_blocking=True)
         for s_ in (self.s_in, self.s_cmp, self.s_out):
             cur.wait_stream(s_)
+
+    def _run_chunks(self, chunks, q, k, v, mask, d_o, out):
+        """host_chunks of csrc/evo_torch.cpp for tensors that lie otherwise in host memory, or without the native host path."""
+        N, H, D = q.shape[2:]
+        for c, (b, s0, r) in enumerate(chunks):
+            st = self.sets[c % 3]
+            dims = _evoattn.EvoDims(1, r, N, H, D)
+            with torch.cuda.stream(self.s_in):
+                if c >= 3:
+                    self.s_in.wait_event(st["ev_out"])      # this set's previous results are out
+                for n, h in (("q", q), ("k", k), ("v", v), ("do", d_o)):
+                    st[n][:, :r].copy_(h[b:b + 1, s0:s0 + r], non_blocking=True)
+                st["mask"][:, :r].copy_(mask[b:b + 1, s0:s0 + r], non_blocking=True)
+                st["ev_in"].record(self.s_in)
+            with torch.cuda.stream(self.s_cmp):
+                self.s_cmp.wait_event(st["ev_in"])
+                h_ = self.s_cmp.cuda_stream
+                # a chunk with fewer rows uses the leading rows of the (contiguous) buffers
+                _evoattn.fwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
+                             st["ores"], st["lse"], 0.0, h_)
+                _evoattn.bwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
+                             st["ores"], st["lse"], st["do"], st["dq"], st["dk"], st["dv"], st["dbias"],
+                             st["ws"], 0.0, h_)
+                self.dbias[b:b + 1].add_(st["dbias"])
+                st["ev_cmp"].record(self.s_cmp)
+            with torch.cuda.stream(self.s_out):
+                self.s_out.wait_event(st["ev_cmp"])
+                for n in ("o", "dq", "dk", "dv"):
+                    out[n][b:b + 1, s0:s0 + r].copy_(st[n][:, :r], non_blocking=True)
+                st["ev_out"].record(self.s_out)

@@ -191,6 +191,32 @@ def test_host_streamed_matches_layer():
     assert (out["dbias"].float() - ref["dbias"].float()).abs().max().item() <= 1e-3
 
 
+def test_host_streamed_native_and_python_chunks_agree():
+    """The chunk loop in native code and the Python one, which tensors with other strides in host memory take, run the same
+    kernels on the same chunks (growing and shrinking ones here): O, dK and dV bit for bit, dQ and dBias but for the order of
+    their fp32 sums."""
+    from tk_evo_attention_layer import HostStreamedEvoAttention
+    B, S, N, H, D = 1, 60, 384, 8, 32
+    bf = torch.bfloat16
+    q, k, v, mask, bias, d_o = (t.to(bf) for t in evo_ref.make_inputs(B, S, N, H, D, 0.5, 1.0, "tail0to32", seed=12))
+    eng = HostStreamedEvoAttention("cuda", chunk_rows=64)
+    sizes = [r for _, _, r in eng._chunks(B, S, N, H, D)]
+    assert sizes[0] < max(sizes) > sizes[-1]
+    outs = []
+    for view in (lambda t: t, lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)):
+        out = {n: torch.empty((B, S, N, H, D), dtype=bf).pin_memory() for n in ("o", "dq", "dk", "dv")}
+        out["dbias"] = torch.empty((B, 1, H, N, N), dtype=torch.float32).pin_memory()
+        eng.run(view(q), view(k), view(v), mask, bias, view(d_o), out)
+        torch.cuda.synchronize()
+        outs.append(out)
+    a, b = outs
+    for n in ("o", "dk", "dv"):
+        assert torch.equal(a[n], b[n]), n
+    # sums of fp32 terms in another order, dQ rounded to bf16 behind them: one step of the largest value
+    assert (a["dq"].float() - b["dq"].float()).abs().max() <= 2.0 ** -7 * a["dq"].float().abs().max()
+    assert (a["dbias"] - b["dbias"]).abs().max() <= 1e-5 * a["dbias"].abs().max()
+
+
 @pytest.mark.parametrize("case", [
     # (B, S, N, H, D, storage order as a permutation of (B, S, N, H, D) axes)
     (1, 24, 200, 2, 32, (0, 2, 1, 3, 4)),     # "ending node": stored [B][N_CTX][N_SEQ][H][D]
