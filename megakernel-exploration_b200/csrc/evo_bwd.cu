@@ -14,7 +14,8 @@
 //                         core (evo_tiles.cuh, "EXTRA TILE"), padded to whole tiles so
 //                         the main kernels need no edge predicates; zeroes the accumulators
 //   2. evo_dbias_kernel   dBias (evo_dbias.cu): one CTA per pair-bias tile keeps its
-//                         sum over the S rows in registers, no reduction traffic
+//                         sum over the S rows in registers, no reduction traffic.  Not with one
+//                         S row or a small problem: kernel 3 then writes dBias (DbiasHere)
 //   3. evo_bwd_halves_kernel, evo_bwd_wide_kernel   dQ, dK, dV (D <= 64: evo_bwd_halves.cuh, above: evo_bwd_wide.cuh)
 //   4. bwd_finish_kernel  fp32 dQ accumulator -> bf16 dQ in the caller layout (and dBias,
 //                         summed over slices of S in fp32, to bf16 if the caller wants that)
@@ -45,7 +46,9 @@ struct BwdParams {
     const __nv_bfloat16* xq;   // [B*S][H][NTP][8] extra tiles of the q rows  (bwd_prep_kernel)
     const __nv_bfloat16* xk;   // [B*S][NTP][8]    extra tiles of the kv rows
     const __nv_bfloat16* bias; // [B][H][N][N]
-    void* dbias;               // [B][H][N][N], fp32 or bf16 (written by this kernel only when S = 1)
+    void* dbias;               // [B][H][N][N], fp32 or bf16 (written by this kernel only: S = 1, or DBIAS_ADD)
+    float* dbias_acc;          // DBIAS_ADD: the fp32 sum, zeroed before the launch
+    int* dbias_done;           // DBIAS_ADD: rows added so far to each [32 x 32] part of dBias, zeroed; nullptr: the sum is the result
     float* dq_scratch;         // whole pairs: per CTA scratch_stride 16-byte words, partial sums of dQ
     size_t scratch_stride;
     float* dq_acc;             // the others: [B*S - acc_row0][N][H][DH], zeroed before the launch
@@ -61,7 +64,9 @@ struct BwdParams {
 // DBIAS_HERE (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
 // dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
 // per item) is not launched.
-enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2 };
+// DBIAS_ADD (small problems): the compute groups add their dS to an fp32 sum in memory, whole rows at a time.  That takes a CTA
+// about 1.3 us per step of a full tile, and saves the dBias kernel, 5 us and more with its launch and the second computation of S and dP.
+enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2, DBIAS_ADD = 3 };
 
 // What a CTA of the dQ/dK/dV kernels walks: the segments (kv tiles) of whole pairs (S row, head) one after another,
 // single segments, or the one and then the other.  A template parameter: chosen at run time it costs the drain warps,
@@ -327,6 +332,12 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
         for (size_t i = t0; i < p.nb8; i += gstride) reinterpret_cast<uint4*>(p.dbias)[i] = cvt8(p.dbias_acc + 8 * i);
 }
 
+// dBias is added up in memory (DBIAS_ADD) if the fullest CTA has no more steps than this.  Forward and backward queued back to
+// back, dBias kernel / added up, us, by steps of the fullest CTA: 1 (S=32, N=64, H=4, D=32) 25.9 / 20.8; 4 (S=64, N=128, H=8, D=32) 41.7 / 37.2,
+// (S=4, N=512, H=8, D=64) 43.7 / 40.9; 6 (S=100, N=128, H=8, D=64) 69.0 / 61.1, (S=3, N=768, H=4, D=64) 48.3 / 47.3; 7 (S=128, N=128, H=8, D=32)
+// 59.5 / 57.0; 8 (S=32, N=256, H=8, D=64) 67.1 / 64.5, but (S=2, N=1024, H=4, D=64) 56.0 / 57.6.
+constexpr int DBIAS_ADD_STEPS = 7;
+
 struct BwdWorkspace {
     size_t off_xq, off_xk, off_do, off_db, off_dq, least, total;
 };
@@ -450,10 +461,23 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const bool both = (phases & EVO_BWD_PHASE_DBIAS) && (phases & EVO_BWD_PHASE_DQKV);
     const bool dbias_here = (d->S == 1) && both;
     p.dbias = dbias_out;
+    // with few steps a CTA they add it up in memory
+    const long steps = p.n_whole == pairs ? static_cast<long>((pairs + use_sms - 1) / use_sms) * NT * NT : t_seg * NT;
+    // (D <= 32: of whole pairs only.  A quarter of the dBias kernel's exponentials are polynomials there, 7e-5 from these, and the smallest
+    // problems of several tiles have dBias from that kernel whether their backward is one call or two phases.)
+    const bool dbias_add = DH <= 64 && both && !dbias_here && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS;
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
-    const bool convert_dbias = dbias_bf16 && !dbias_here && slices > 1;
+    // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
+    // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the
+    // launch costs a caller as much as anything (S=32, N=64, H=4, D=32: the kernels 20.8 us either way, the whole step, host
+    // work, 85.6 -> 83 with the finish kernel and -> 81 without); with four steps the finish kernel is the better (37.2 us for 43.2).
+    const size_t parts = static_cast<size_t>(d->B) * d->H * NT * NT * 16;
+    const bool count = dbias_add && dbias_bf16 && steps <= 1 && p.n_whole == pairs && NT <= TILES_HELD && parts <= room * DH;
+    const bool convert_dbias = dbias_bf16 && !dbias_here && (dbias_add ? !count : slices > 1);
+    p.dbias_acc = dbias_acc;
+    p.dbias_done = count ? reinterpret_cast<int*>(dq_ws) : nullptr;
     if (phases & EVO_BWD_PHASE_DBIAS) {
         PrepParams r;
         r.o = static_cast<const __nv_bfloat16*>(o);
@@ -467,9 +491,9 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         r.do_att = reinterpret_cast<__nv_bfloat16*>(ws + w.off_do);
         r.d_gate = static_cast<__nv_bfloat16*>(d_gate);
         r.zero[0] = reinterpret_cast<uint4*>(dbias_acc);
-        r.n_zero[0] = (!dbias_here && slices > 1) ? db_elems / 4 : 0;
-        r.zero[1] = reinterpret_cast<uint4*>(p.dq_acc);
-        r.n_zero[1] = both ? acc_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
+        r.n_zero[0] = (!dbias_here && (dbias_add || slices > 1)) ? db_elems / 4 : 0;
+        r.zero[1] = reinterpret_cast<uint4*>(count ? dq_ws : p.dq_acc);
+        r.n_zero[1] = count ? parts / 4 : both ? acc_bytes / 16 : 0;      // a separate second phase zeroes its own accumulator
         r.inv_scale = 1.0f / p.scale;
         r.BS = BS; r.N = d->N; r.H = d->H; r.NTP = p.NTP; r.Dt = Dt;
         r.lay = lay_out;
@@ -487,14 +511,14 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         };
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;
-        if (!dbias_here && (rc = launch_dbias(d, tq, tk, tv, tdo, bias, xq, xk, dbias_acc,
+        if (!dbias_here && !dbias_add && (rc = launch_dbias(d, tq, tk, tv, tdo, bias, xq, xk, dbias_acc,
                                               (dbias_bf16 && !convert_dbias) ? dbias_out : nullptr, slices, p.scale, sms, both, st)))
             return rc;
     }
     if (!(phases & EVO_BWD_PHASE_DQKV)) return EVO_OK;
 
     if (!both && rest_rows && (rc = cuda_err(cudaMemsetAsync(p.dq_acc, 0, acc_bytes, st)))) return rc;
-    const int mode = !dbias_here ? DBIAS_NO : (dbias_bf16 ? DBIAS_BF16 : DBIAS_F32);
+    const int mode = dbias_add ? DBIAS_ADD : !dbias_here ? DBIAS_NO : (dbias_bf16 ? DBIAS_BF16 : DBIAS_F32);
     auto run = [&](auto kernel, int threads, uint32_t smem, auto... maps) -> int {
         const int e = set_max_smem_once(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
         if (e) return e;
@@ -512,6 +536,9 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
         } else {
             using C = BwdHalvesCfg<DH>;
+            if constexpr (W == WALK_WHOLE || (W == WALK_SEGMENTS && DH == 64)) {
+                if (mode == DBIAS_ADD) return run(evo_bwd_halves_kernel<DH, W, DBIAS_ADD>, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
+            }
             auto kernel = mode == DBIAS_NO ? evo_bwd_halves_kernel<DH, W, DBIAS_NO>
                                            : (mode == DBIAS_BF16 ? evo_bwd_halves_kernel<DH, W, DBIAS_BF16> : evo_bwd_halves_kernel<DH, W, DBIAS_F32>);
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);

@@ -562,7 +562,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
                 for (int cb = 0; cb < 4; ++cb) {
                     const bool rows = q0 + 8 * cb < p.N;          // (N is a multiple of 8)
-                    if constexpr (DBIAS_HERE == DBIAS_F32) {
+                    if constexpr (DBIAS_HERE != DBIAS_BF16) {
                         uint32_t x[2][4];
 #pragma unroll
                         for (int b = 0; b < 4; ++b) { x[0][b] = __float_as_uint(dsv[4 * cb + b].x); x[1][b] = __float_as_uint(dsv[4 * cb + b].y); }
@@ -570,7 +570,11 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         quad_transpose(x[1]);
                         if (rows)
 #pragma unroll
-                            for (int r = 0; r < 8; ++r) out[static_cast<size_t>(8 * cb + r) * p.N] = __uint_as_float(x[r & 1][r >> 1]);
+                            for (int r = 0; r < 8; ++r) {
+                                const float v = __uint_as_float(x[r & 1][r >> 1]);
+                                if constexpr (DBIAS_HERE == DBIAS_ADD) red_add(&out[static_cast<size_t>(8 * cb + r) * p.N], v);
+                                else out[static_cast<size_t>(8 * cb + r) * p.N] = v;
+                            }
                     } else {
                         uint32_t w[4];
 #pragma unroll
@@ -582,18 +586,44 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             }
         };
 
+        // DBIAS_ADD: this warp's part of the tile has one row more; with the last one it becomes the bf16 result.
+        auto count_row = [&](const float* at, int part, int q0) {
+            if constexpr (DBIAS_HERE == DBIAS_ADD) {
+                if (p.dbias_done == nullptr) return;
+                __threadfence();
+                __syncwarp();
+                int before = 0;
+                if (lane == 0) before = atomicAdd(p.dbias_done + part, 1);
+                if (__shfl_sync(0xffffffffu, before, 0) != p.S - 1) return;
+                __threadfence();
+                __nv_bfloat16* res = static_cast<__nv_bfloat16*>(p.dbias) + (at - p.dbias_acc);
+                if (q0 >= p.N) return;
+                const int rows = p.N - q0 < 32 ? p.N - q0 : 32;
+                float v[32];                                  // (all loads in flight at once)
+#pragma unroll
+                for (int r = 0; r < 32; ++r) v[r] = __ldcg(at + static_cast<size_t>(r < rows ? r : 0) * p.N);
+#pragma unroll
+                for (int r = 0; r < 32; ++r)
+                    if (r < rows) res[static_cast<size_t>(r) * p.N] = __float2bfloat16_rn(v[r]);
+            }
+        };
+
 #pragma unroll 1
         for (int sg = 0; sg < n_segs && ok; ++sg) {
-            using DBias = std::conditional_t<DBIAS_HERE == DBIAS_F32, float, __nv_bfloat16>;
+            using DBias = std::conditional_t<DBIAS_HERE != DBIAS_BF16, float, __nv_bfloat16>;
             DBias* out = nullptr;
             bool cols = false;
+            int part = 0;
             if constexpr (DBIAS_HERE != DBIAS_NO) {
                 int bs, h, j;
                 seg.decode(sg, bs, h, j);
+                if (DBIAS_HERE == DBIAS_ADD) bs /= p.S;             // (else S = 1)
+                part = ((bs * p.H + h) * NT * NT + j) * 16 + warp;
                 const int kv0 = j * TILE + 32 * w4 + 8 * (lane & 3), r = lane >> 2;
                 cols = kv0 < p.N;
-                out = static_cast<DBias*>(p.dbias) + ((static_cast<size_t>(bs) * p.H + h) * p.N + 32 * g + (DBIAS_HERE == DBIAS_F32 ? 0 : r)) * p.N +
-                      kv0 + (DBIAS_HERE == DBIAS_F32 ? r : 0);
+                constexpr bool BF = DBIAS_HERE == DBIAS_BF16;
+                out = static_cast<DBias*>(DBIAS_HERE == DBIAS_ADD ? p.dbias_acc : p.dbias) +
+                      ((static_cast<size_t>(bs) * p.H + h) * p.N + 32 * g + (BF ? r : 0)) * p.N + kv0 + (BF ? 0 : r);
             }
 #pragma unroll 1
             for (int i = 0; i < NT && ok; ++i, ++gs) {
@@ -651,6 +681,7 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (lane == 0) mbar_arrive(&ds_ready[hf]);
                 if constexpr (DBIAS_HERE != DBIAS_NO) {
                     store_dbias(out, cols ? i * TILE + 32 * g : p.N, pkd, dsv);
+                    if (DBIAS_HERE == DBIAS_ADD) count_row(reinterpret_cast<float*>(out), part + i * NT * 16, cols ? i * TILE + 32 * g : p.N);
                     out += static_cast<size_t>(TILE) * p.N;
                 }
             }

@@ -215,6 +215,9 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }
 
+__device__ __forceinline__ void red_add(float* at, float x) {
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(at), "f"(x) : "memory");
+}
 __device__ __forceinline__ void red_add_v4(float* at, float x, float y, float z, float w) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
