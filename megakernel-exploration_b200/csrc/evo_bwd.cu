@@ -59,6 +59,11 @@ struct BwdParams {
     __nv_bfloat16* dv;
     ActLayout lay;        // element strides of the activation tensors
     unsigned int* status;
+    // own_prep: there is no prep kernel ahead, the drain warps form the extra tiles of the CTA's one step (D <= 64)
+    int own_prep;
+    const __nv_bfloat16 *o, *o_resid, *d_o, *mask;
+    const float* lse;
+    ActLayout lay_out;    // of o, o_resid, d_o
 };
 
 // DBIAS_HERE (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
@@ -122,6 +127,14 @@ struct Segments {
 // D=32 182 -> 176 us; S=200, N=200, H=4 47 -> 44; S=1024, N=768, H=8 3333 -> 3255).
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ uint32_t split_bf16(float v) {
+    // (head, remainder) as a bf16 pair, head in the low half
+    v = fminf(fmaxf(v, -1e30f), 1e30f);
+    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+    const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
+    return static_cast<uint32_t>(__bfloat16_as_ushort(hi)) | (static_cast<uint32_t>(__bfloat16_as_ushort(lo)) << 16);
+}
+
 }  // namespace evo
 #include "evo_bwd_halves.cuh"
 #include "evo_bwd_wide.cuh"
@@ -144,13 +157,6 @@ namespace evo {
 // uses O to about 16 bits instead of 8: the rounding of O otherwise puts an
 // error of order 2^-9 |dO||O| on every dS, which adds up over the S rows of dBias.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t split_bf16(float v) {
-    // (head, remainder) as a bf16 pair, head in the low half
-    v = fminf(fmaxf(v, -1e30f), 1e30f);
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-    return static_cast<uint32_t>(__bfloat16_as_ushort(hi)) | (static_cast<uint32_t>(__bfloat16_as_ushort(lo)) << 16);
-}
 
 // With a gate (evo_bwd_gated) d_o is the gradient of the GATED output: the kernel then also forms
 // sig = sigmoid(gate), writes the gradient that enters the attention, bf16(d_o * sig), to do_att
@@ -478,7 +484,19 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const bool convert_dbias = dbias_bf16 && !dbias_here && (dbias_add ? !count : slices > 1);
     p.dbias_acc = dbias_acc;
     p.dbias_done = count ? reinterpret_cast<int*>(dq_ws) : nullptr;
-    if (phases & EVO_BWD_PHASE_DBIAS) {
+    // One S row of one tile, at most one pair a CTA: the dQ/dK/dV kernel is all of the backward.  (Forward and backward queued back to back,
+    // with the prep kernel / without: B=4, N=128, H=16, D=64 20.7 / 18.7 us, D=32 18.7 / 15.2.  A sum over S rows needs its zeros written first,
+    // and with more tiles every segment would form all of its pair's terms again.)
+    p.own_prep = DH <= 64 && dbias_here && !gate && NT == 1 && pairs <= use_sms;
+    if (p.own_prep) {
+        p.o = static_cast<const __nv_bfloat16*>(o);
+        p.o_resid = static_cast<const __nv_bfloat16*>(o_resid);
+        p.d_o = static_cast<const __nv_bfloat16*>(d_o);
+        p.mask = static_cast<const __nv_bfloat16*>(mask);
+        p.lse = lse;
+        p.lay_out = lay_out;
+    }
+    if ((phases & EVO_BWD_PHASE_DBIAS) && !p.own_prep) {
         PrepParams r;
         r.o = static_cast<const __nv_bfloat16*>(o);
         r.o_resid = static_cast<const __nv_bfloat16*>(o_resid);

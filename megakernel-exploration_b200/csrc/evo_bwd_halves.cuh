@@ -154,14 +154,16 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // uniform
     const int lane = tid & 31;
     const int NT = p.NT;
+    const bool own_prep = WALK == WALK_WHOLE && (DBIAS_HERE == DBIAS_F32 || DBIAS_HERE == DBIAS_BF16) && p.own_prep;
     WaitCtx wc{abort_flag, p.status};
 
     if (tid == 0) {
         *abort_flag = 0;
         tmem_slot[3] = 0;                      // the abort word of the waits before exit
-        for (int i = 0; i < NQ; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
+        const uint32_t full = own_prep ? 5 : 1;      // the loads, and the drain warps for the extra tiles
+        for (int i = 0; i < NQ; ++i) { mbar_init(&q_full[i], full); mbar_init(&q_empty[i], 1); }
         for (int i = 0; i < NDO; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
-        for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+        for (int i = 0; i < NK; ++i) { mbar_init(&k_full[i], full); mbar_init(&k_empty[i], 1); }
         for (int i = 0; i < NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for (int i = 0; i < NB; ++i) { mbar_init(&bias_full[i], 1); mbar_init(&bias_empty[i], C::NCW / 2); }
         for (int i = 0; i < DQB; ++i) { mbar_init(&dq_full[i], 1); mbar_init(&dq_free[i], 4); }
@@ -217,10 +219,10 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (sg >= NK) ok = warp_all(mbar_wait(&k_empty[kb], ((sg / NK) - 1) & 1, wc, 0x40));
             if (!ok) break;
             if (elect_one()) {
-                mbar_arrive_expect_tx(&k_full[kb], (C::PAIRED ? 2 : 1) * C::ROWT + XT_BYTES);
+                mbar_arrive_expect_tx(&k_full[kb], (C::PAIRED ? 2 : 1) * C::ROWT + (own_prep ? 0 : XT_BYTES));
                 tma_load_row_tile<DH>(smem + C::OFF_K + kb * C::ROWT, &tm_k, &k_full[kb], h, j * TILE, bs);
                 if (C::PAIRED) tma_load_row_tile<DH>(smem + C::OFF_V + kb * C::ROWT, &tm_v, &k_full[kb], h, j * TILE, bs);
-                bulk_load(smem + C::OFF_XK + kb * XT_BYTES, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &k_full[kb]);
+                if (!own_prep) bulk_load(smem + C::OFF_XK + kb * XT_BYTES, p.xk + (static_cast<size_t>(bs) * p.NTP + j * TILE) * 8, XT_BYTES, &k_full[kb]);
             }
             __syncwarp();
             ++n_k;
@@ -230,10 +232,10 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (gs >= NQ) ok = warp_all(mbar_wait(&q_empty[qb], ((gs / NQ) - 1) & 1, wc, 0x42));
                 if (!ok) break;
                 if (elect_one()) {
-                    mbar_arrive_expect_tx(&q_full[qb], (C::PAIRED ? 2 : 1) * C::ROWT + XT_BYTES);
+                    mbar_arrive_expect_tx(&q_full[qb], (C::PAIRED ? 2 : 1) * C::ROWT + (own_prep ? 0 : XT_BYTES));
                     tma_load_row_tile<DH>(smem + C::OFF_Q + qb * C::ROWT, &tm_q, &q_full[qb], h, i * TILE, bs);
                     if (C::PAIRED) tma_load_row_tile<DH>(smem + C::OFF_DO + qb * C::ROWT, &tm_do, &q_full[qb], h, i * TILE, bs);
-                    bulk_load(smem + C::OFF_XQ + qb * XT_BYTES, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &q_full[qb]);
+                    if (!own_prep) bulk_load(smem + C::OFF_XQ + qb * XT_BYTES, xq + static_cast<size_t>(i) * TILE * 8, XT_BYTES, &q_full[qb]);
                 }
                 __syncwarp();
                 ++n_q;
@@ -519,6 +521,54 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 store(1);
             }
         };
+        if (own_prep && n_segs > 0) {
+            // what the prep kernel does (evo_bwd.cu), for the one step of this CTA: thread = row
+            int bs, h, j;
+            seg.decode(0, bs, h, j);
+            const int row = wrow0 + lane;
+            const float inv_scale = 1.0f / p.scale;
+            uint4 xq = make_uint4(0x3f803f80u, split_bf16(-1e30f), 0u, 0u), xk = make_uint4(split_bf16(-1e30f), 0x3f803f80u, 0u, 0u);
+            if (row < p.N) {
+                const size_t off = bs * p.lay_out.row + row * p.lay_out.n + h * p.lay_out.h;
+                const float lse = __ldg(p.lse + (static_cast<size_t>(bs) * p.H + h) * p.N + row);
+                const float m = __bfloat162float(p.mask[static_cast<size_t>(bs) * p.N + row]);
+                float s[DH / 8];                   // by chunks of eight columns, and these in pairs: the prep kernel's sum to the bit
+#pragma unroll
+                for (int c0 = 0; c0 < DH; c0 += 32) {
+                    uint4 a[4], b[4], r[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        a[c] = b[c] = r[c] = make_uint4(0u, 0u, 0u, 0u);
+                        if (c0 + 8 * c >= p.Dt) continue;
+                        a[c] = __ldg(reinterpret_cast<const uint4*>(p.o + off + c0 + 8 * c));
+                        b[c] = __ldg(reinterpret_cast<const uint4*>(p.d_o + off + c0 + 8 * c));
+                        if (p.o_resid) r[c] = __ldg(reinterpret_cast<const uint4*>(p.o_resid + off + c0 + 8 * c));
+                    }
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t aw[4] = {a[c].x, a[c].y, a[c].z, a[c].w}, bw[4] = {b[c].x, b[c].y, b[c].z, b[c].w}, rw[4] = {r[c].x, r[c].y, r[c].z, r[c].w};
+                        float& sc = s[c0 / 8 + c];
+                        sc = 0.f;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            sc = fmaf(bf16_lo(aw[e]) + bf16_lo(rw[e]), bf16_lo(bw[e]), sc);
+                            sc = fmaf(bf16_hi(aw[e]) + bf16_hi(rw[e]), bf16_hi(bw[e]), sc);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int w = 1; w < DH / 8; w *= 2)
+#pragma unroll
+                    for (int c = 0; c < DH / 8; c += 2 * w) s[c] += s[c + w];
+                xq = make_uint4(0x3f803f80u, split_bf16(-lse * inv_scale), split_bf16(-s[0]), 0u);
+                xk.x = split_bf16(m * inv_scale);
+            }
+            *reinterpret_cast<uint4*>(smem + C::OFF_XQ + row * 16) = xq;
+            *reinterpret_cast<uint4*>(smem + C::OFF_XK + row * 16) = xk;
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(&q_full[0]); mbar_arrive(&k_full[0]); }
+        }
         if (WALK != WALK_SEGMENTS) drain(std::true_type{}, 0, seg.n_ws);
         if (WALK != WALK_WHOLE) drain(std::false_type{}, seg.n_ws, n_segs);
         if (lane == 0) tma_wait_group<0>();
