@@ -185,6 +185,7 @@ template <int U>
 constexpr int prep_blocks() { return U == 1 ? 5 : 3; }      // per SM: 48 and 80 registers
 template <int LANES, bool GATED, int U>
 __global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const PrepParams p) {
+    chain_wait();
     constexpr uint32_t ONES = 0x3f803f80u;     // bf16 (1, 1)
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t t0 = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -522,10 +523,8 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             constexpr int U = G ? 2 : 4;
             // one row per thread where a single pass takes all of them (B=1, S=32, N=64, H=4, D=32: 4 us less)
             if (static_cast<size_t>(BS) * d->N * d->H * L <= static_cast<size_t>(sms) * prep_blocks<1>() * 256)
-                bwd_prep_kernel<L, G, 1><<<sms * prep_blocks<1>(), 256, 0, st>>>(r);
-            else
-                bwd_prep_kernel<L, G, U><<<sms * prep_blocks<U>(), 256, 0, st>>>(r);
-            return cuda_err(cudaGetLastError());
+                return launch_chained(both, bwd_prep_kernel<L, G, 1>, sms * prep_blocks<1>(), 256, 0, st, r);
+            return launch_chained(both, bwd_prep_kernel<L, G, U>, sms * prep_blocks<U>(), 256, 0, st, r);
         };
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;

@@ -81,8 +81,9 @@ void prof_end(int kernel, cudaStream_t st);
 // kernel of a second stream beside them: 35 / 148 / 35 us beside the first, 33 / 116 / 34 at D=64, S=128, N=1024, H=4, 26 / 65 / 26 at D=128, S=64,
 // N=768; beside short kernels, of whose gaps it lived, 11 / 22 / 13 (D=32, S=200, N=200, a step 118 / 111 / 111) and 15 / 34 / 19 (D=64, B=4, S=1,
 // N=1024, 162 / 156 / 157).
-// Not chained: the two phases of a backward with a collective beside it.  Nor the prep kernel, whose blocks, three or five to an SM, went to
-// the SMs in the order in which these became free when its predecessor released it, and read a step's tensors slower: the first step 862 -> 885 us.
+// Not chained: the two phases of a backward with a collective beside it.  The prep kernel read a step's tensors slower when its predecessor released it
+// early (its blocks, three or five to an SM, went to the SMs as these became free: the first step 862 -> 885 us); behind a predecessor that has ended it
+// is chained like the others (not chained / chained: the first step 845.5 / 842.3 us, S=200, N=200, H=4, D=32 106.1 / 103.4, S=384, N=384 349.9 / 347.6).
 template <typename... P, typename... A>
 int launch_chained(bool chained, void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchAttribute at{};
