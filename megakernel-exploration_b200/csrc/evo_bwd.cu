@@ -178,13 +178,13 @@ struct PrepParams {
     int BS, N, H, NTP, Dt;
     ActLayout lay;
 };
-// LANES per row: the power of two at or above Dt / 8.  U rows per thread at a time, their loads in flight
-// together.  All blocks are resident: with a grid that the registers cut into two waves, as it was, the
-// second wave held half of the threads (B=1, S=512, N=384, H=8, D=32 82 -> 61 us, 50 at the rate of a copy).
-template <int U>
-constexpr int prep_blocks() { return U == 1 ? 5 : 3; }      // per SM: 48 and 80 registers
-template <int LANES, bool GATED, int U>
-__global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const PrepParams p) {
+// LANES per row: the power of two at or above Dt / 8.  All blocks are resident, six to an SM (40 registers): with one row per thread
+// at a time, more threads keep more loads in flight than more rows per thread do.  Three blocks of four rows a thread (gated: two)
+// / five of one / six of one, us: B=1, S=512, N=384, H=8, D=32 60.1 / 59.8 / 57.9 (50 at the rate of a copy); S=256, N=1024, H=4, D=64 80.0 / 78.8 / 77.6;
+// S=128, N=768, H=4, D=128 87.5 / 88.7 / 86.6; S=384, N=384, H=4, D=32, gated 46.3 / 41.4 / 40.3 (36).
+constexpr int PREP_BLOCKS = 6;      // per SM
+template <int LANES, bool GATED>
+__global__ void __launch_bounds__(256, PREP_BLOCKS) bwd_prep_kernel(const PrepParams p) {
     chain_wait();
     constexpr uint32_t ONES = 0x3f803f80u;     // bf16 (1, 1)
     const size_t gstride = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -214,63 +214,54 @@ __global__ void __launch_bounds__(256, prep_blocks<U>()) bwd_prep_kernel(const P
         return At{n_inner ? out_ : in_, n_inner ? in_ : out_, h};
     };
     // (whole warps run the same number of iterations: the shuffles need all lanes)
-    for (size_t r0 = (t0 - (threadIdx.x & 31)) / LANES; r0 < rows; r0 += U * rstride) {
-        uint4 a[U], b[U], rr[U], g4[GATED ? U : 1];
-        float lse[U];
-        size_t off[U], ro[U], att[GATED ? U : 1];
-        bool live[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const size_t r = r0 + (threadIdx.x & 31) / LANES + u * rstride;
-            live[u] = r < rows;
-            a[u] = b[u] = rr[u] = make_uint4(0u, 0u, 0u, 0u);
-            lse[u] = 0.f;
-            if constexpr (GATED) g4[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (!live[u]) continue;
+    for (size_t r0 = (t0 - (threadIdx.x & 31)) / LANES; r0 < rows; r0 += rstride) {
+        const size_t r = r0 + (threadIdx.x & 31) / LANES;
+        const bool live = r < rows;
+        uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a, rr = a, g4 = a;
+        float lse = 0.f;
+        size_t off = 0, ro = 0, att = 0;
+        if (live) {
             const At x = at(r);
-            off[u] = x.bs * p.lay.row + x.n * p.lay.n + x.h * p.lay.h + c * 8;
-            ro[u] = (x.bs * H + x.h) * NTP + x.n;
-            if constexpr (GATED) att[u] = ((x.bs * N + x.n) * H + x.h) * static_cast<size_t>(p.Dt) + c * 8;
+            off = x.bs * p.lay.row + x.n * p.lay.n + x.h * p.lay.h + c * 8;
+            ro = (x.bs * H + x.h) * NTP + x.n;
+            if constexpr (GATED) att = ((x.bs * N + x.n) * H + x.h) * static_cast<size_t>(p.Dt) + c * 8;
             if (have) {
-                a[u] = __ldg(reinterpret_cast<const uint4*>(p.o + off[u]));
-                b[u] = __ldg(reinterpret_cast<const uint4*>(p.d_o + off[u]));
-                if (p.o_resid) rr[u] = __ldg(reinterpret_cast<const uint4*>(p.o_resid + off[u]));
-                if constexpr (GATED) g4[u] = __ldg(reinterpret_cast<const uint4*>(p.gate + off[u]));
+                a = __ldg(reinterpret_cast<const uint4*>(p.o + off));
+                b = __ldg(reinterpret_cast<const uint4*>(p.d_o + off));
+                if (p.o_resid) rr = __ldg(reinterpret_cast<const uint4*>(p.o_resid + off));
+                if constexpr (GATED) g4 = __ldg(reinterpret_cast<const uint4*>(p.gate + off));
             }
-            if (c == 0) lse[u] = __ldg(p.lse + (x.bs * H + x.h) * N + x.n);
+            if (c == 0) lse = __ldg(p.lse + (x.bs * H + x.h) * N + x.n);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, rw[4] = {rr[u].x, rr[u].y, rr[u].z, rr[u].w};
-            if constexpr (GATED) {
-                const uint32_t gw[4] = {g4[u].x, g4[u].y, g4[u].z, g4[u].w}, dw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
-                uint32_t aw2[4], gg[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
-                    const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
-                    const float d0 = bf16_lo(dw[e]), d1 = bf16_hi(dw[e]);
-                    const float o0 = bf16_lo(aw[e]) + bf16_lo(rw[e]), o1 = bf16_hi(aw[e]) + bf16_hi(rw[e]);
-                    aw2[e] = pack_bf16(d0 * s0, d1 * s1);
-                    gg[e] = pack_bf16(d0 * o0 * s0 * (1.0f - s0), d1 * o1 * s1 * (1.0f - s1));
-                }
-                b[u] = make_uint4(aw2[0], aw2[1], aw2[2], aw2[3]);
-                if (live[u] && have) {
-                    *reinterpret_cast<uint4*>(p.do_att + att[u]) = b[u];
-                    *reinterpret_cast<uint4*>(p.d_gate + off[u]) = make_uint4(gg[0], gg[1], gg[2], gg[3]);
-                }
-            }
-            const uint32_t bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
-            float s = 0.f;
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, rw[4] = {rr.x, rr.y, rr.z, rr.w};
+        if constexpr (GATED) {
+            const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, dw[4] = {b.x, b.y, b.z, b.w};
+            uint32_t aw2[4], gg[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s = fmaf(bf16_lo(aw[e]) + bf16_lo(rw[e]), bf16_lo(bw[e]), s);
-                s = fmaf(bf16_hi(aw[e]) + bf16_hi(rw[e]), bf16_hi(bw[e]), s);
+                const float s0 = 1.0f / (1.0f + ex2(-bf16_lo(gw[e]) * LOG2E));
+                const float s1 = 1.0f / (1.0f + ex2(-bf16_hi(gw[e]) * LOG2E));
+                const float d0 = bf16_lo(dw[e]), d1 = bf16_hi(dw[e]);
+                const float o0 = bf16_lo(aw[e]) + bf16_lo(rw[e]), o1 = bf16_hi(aw[e]) + bf16_hi(rw[e]);
+                aw2[e] = pack_bf16(d0 * s0, d1 * s1);
+                gg[e] = pack_bf16(d0 * o0 * s0 * (1.0f - s0), d1 * o1 * s1 * (1.0f - s1));
             }
-#pragma unroll
-            for (int d = 1; d < LANES; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
-            if (live[u] && c == 0) p.xq[ro[u]] = make_uint4(ONES, split_bf16(-lse[u] * p.inv_scale), split_bf16(-s), 0u);
+            b = make_uint4(aw2[0], aw2[1], aw2[2], aw2[3]);
+            if (live && have) {
+                *reinterpret_cast<uint4*>(p.do_att + att) = b;
+                *reinterpret_cast<uint4*>(p.d_gate + off) = make_uint4(gg[0], gg[1], gg[2], gg[3]);
+            }
         }
+        const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
+        float s = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            s = fmaf(bf16_lo(aw[e]) + bf16_lo(rw[e]), bf16_lo(bw[e]), s);
+            s = fmaf(bf16_hi(aw[e]) + bf16_hi(rw[e]), bf16_hi(bw[e]), s);
+        }
+#pragma unroll
+        for (int d = 1; d < LANES; d *= 2) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (live && c == 0) p.xq[ro] = make_uint4(ONES, split_bf16(-lse * p.inv_scale), split_bf16(-s), 0u);
     }
     // padding of the per-row tiles, and the per-column tiles
     const int pad = NTP - N;
@@ -520,11 +511,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto prep = [&](auto lanes_c, auto gated_c) -> int {
             constexpr int L = decltype(lanes_c)::value;
             constexpr bool G = decltype(gated_c)::value;
-            constexpr int U = G ? 2 : 4;
-            // one row per thread where a single pass takes all of them (B=1, S=32, N=64, H=4, D=32: 4 us less)
-            if (static_cast<size_t>(BS) * d->N * d->H * L <= static_cast<size_t>(sms) * prep_blocks<1>() * 256)
-                return launch_chained(both, bwd_prep_kernel<L, G, 1>, sms * prep_blocks<1>(), 256, 0, st, r);
-            return launch_chained(both, bwd_prep_kernel<L, G, U>, sms * prep_blocks<U>(), 256, 0, st, r);
+            return launch_chained(both, bwd_prep_kernel<L, G>, sms * PREP_BLOCKS, 256, 0, st, r);
         };
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;
