@@ -304,8 +304,8 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
 // The chunks of HostStreamedEvoAttention.run (tk_evo_attention_layer.py has what they are): rows [s0, s0 + r) of batch b in,
 // through the kernels and out, on three streams and three sets of device buffers.  ins: q, k, v, dO, mask and outs: o, dq,
 // dk, dv in host memory, contiguous; a set: q, k, v, do, mask, o, ores, dq, dk, dv, lse, dbias, ws for at least the rows
-// of a chunk.  Through torch's Python operators a chunk was about 200 us of host time, so that a step of eight chunks was
-// bound by it.
+// of a chunk.  Through torch's Python operators a chunk was about 200 us of host time, and small steps
+// were bound by it.
 void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunks, const std::vector<Tensor>& ins, const Tensor& bias,
                  const Tensor& dbias, const std::vector<Tensor>& outs, const std::vector<std::vector<Tensor>>& sets,
                  const std::vector<std::tuple<int64_t, int64_t, int64_t>>& streams) {

@@ -479,33 +479,15 @@ class HostStreamedEvoAttention:
         self._key, self._rows = None, 0
 
     def _chunks(self, B, S, N, H, D):
-        """(batch, first row, rows) of every chunk: at most chunk_rows rows, copies of one to six megabytes and at least four
-        chunks in a batch (below, the cost of a copy shows; above, the time in which the link idles in one direction,
-        while the first chunk comes in and the last goes out).  So the first chunks also grow, by twos from copies of
-        1.5 megabytes, and the last shrink to them: B=1, S=128, N=384, H=8, D=32, chunk_rows=64, 3.08-3.32 ms in four equal
-        chunks, 2.96-3.14 in [8, 16, 27, 27, 26, 16, 8], 3.02-3.30 from copies of one megabyte on (both directions at once,
-        a small copy takes several times as long)."""
-        row = 2 * N * H * D
-        one, r0 = -(-(1 << 20) // row), -(-(3 << 19) // row)
-        most = max(1, min(self.chunk_rows, S, max(one, min(-(-S // 4), 6 * one))))
-        out = []
-        for b in range(B):
-            head, tail, left, r = [], [], S, r0
-            while r < most and left > 2 * r:
-                if b == 0:
-                    head.append(r)
-                    left -= r
-                if b == B - 1:
-                    tail.append(r)
-                    left -= r
-                r *= 2
-            n = -(-left // most)
-            rows = head + [left // n + (i < left % n) for i in range(n)] + tail[::-1]
-            s0 = 0
-            for r in rows:
-                out.append((b, s0, r))
-                s0 += r
-        return out
+        """(batch, first row, rows) of every chunk: at most chunk_rows rows; fewer so that there are four chunks (the link idles in
+        one direction while the first comes in and the last goes out) of copies of one to six megabytes (below, the cost of a
+        copy shows; above, the idle ends do).  B=1, N=384, H=8, D=32, chunk_rows=64, against chunks of 64 rows in two buffer
+        sets: S=128 3.26 -> 3.03 ms; S=512 10.5 ms.  Chunks that grow from copies of 1.5 megabytes and shrink to them at the
+        end are no gain, for all that the ends are shorter (both directions at once, a small copy takes several
+        times as long): in turn in one process 3085 / 3044 us there, S=512 10751 / 10845, S=300, N=200, H=4, D=64 3425 / 3489."""
+        one = -(-(1 << 20) // (2 * N * H * D))               # rows of a megabyte
+        R = max(1, min(self.chunk_rows, S, max(one, min(-(-S // 4), 6 * one))))
+        return [(b, s0, min(R, S - s0)) for b in range(B) for s0 in range(0, S, R)]
 
     def _buffers(self, B, N, H, D, R):
         key = (B, N, H, D)

@@ -193,15 +193,13 @@ def test_host_streamed_matches_layer():
 
 def test_host_streamed_native_and_python_chunks_agree():
     """The chunk loop in native code and the Python one, which tensors with other strides in host memory take, run the same
-    kernels on the same chunks (growing and shrinking ones here): O, dK and dV bit for bit, dQ and dBias but for the order of
+    kernels on the same chunks: O, dK and dV bit for bit, dQ and dBias but for the order of
     their fp32 sums."""
     from tk_evo_attention_layer import HostStreamedEvoAttention
-    B, S, N, H, D = 1, 60, 384, 8, 32
+    B, S, N, H, D = 2, 21, 200, 2, 32
     bf = torch.bfloat16
     q, k, v, mask, bias, d_o = (t.to(bf) for t in evo_ref.make_inputs(B, S, N, H, D, 0.5, 1.0, "tail0to32", seed=12))
-    eng = HostStreamedEvoAttention("cuda", chunk_rows=64)
-    sizes = [r for _, _, r in eng._chunks(B, S, N, H, D)]
-    assert sizes[0] < max(sizes) > sizes[-1]
+    eng = HostStreamedEvoAttention("cuda", chunk_rows=4)
     outs = []
     for view in (lambda t: t, lambda t: t.transpose(1, 2).contiguous().transpose(1, 2)):
         out = {n: torch.empty((B, S, N, H, D), dtype=bf).pin_memory() for n in ("o", "dq", "dk", "dv")}
