@@ -331,6 +331,7 @@ void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunk
             for (const Tensor& t : *outs) at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), out);
         }
     } const hold{&ins, &outs, s_in.unwrap(), s_out.unwrap()};
+    for (const Tensor& t : outs) t.unsafeGetTensorImpl()->bump_version();
     at::cuda::CUDAEvent ev_in[3], ev_cmp[3], ev_out[3];
     for (size_t c = 0; c < chunks.size(); ++c) {
         const auto [b, s0, r] = chunks[c];
