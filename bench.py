@@ -40,7 +40,7 @@ import evo_workloads as wl  # noqa: E402
 
 # DRAM bytes per S row of one evo_bwd_halves_kernel launch, from the ncu capture summarised under profiles/
 # (110.16 MB read + 43.55 MB written at 128 rows of cfg2).
-NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.16e6 + 43.55e6) / 128}
+NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.23e6 + 43.04e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"
 UNIT = "TFLOP/s"
