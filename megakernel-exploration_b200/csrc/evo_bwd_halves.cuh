@@ -643,9 +643,13 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 __threadfence();
                 __syncwarp();
                 int before = 0;
-                if (lane == 0) before = atomicAdd(p.dbias_done + part, 1);
-                if (__shfl_sync(0xffffffffu, before, 0) != p.S - 1) return;
-                __threadfence();
+                if (lane == 0) {
+                    before = atomicAdd(p.dbias_done + part, 1);
+                    __threadfence();                          // behind the counts of the other warps, for all lanes:
+                }
+                before = __shfl_sync(0xffffffffu, before, 0);
+                __syncwarp();                                 // a shuffle orders no memory
+                if (before != p.S - 1) return;
                 __nv_bfloat16* res = static_cast<__nv_bfloat16*>(p.dbias) + (at - p.dbias_acc);
                 if (q0 >= p.N) return;
                 const int rows = p.N - q0 < 32 ? p.N - q0 : 32;
