@@ -70,7 +70,8 @@ struct BwdParams {
 // dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
 // per item) is not launched.
 // DBIAS_ADD (small problems): the compute groups add their dS to an fp32 sum in memory, whole rows at a time.  That takes a CTA
-// about 1.3 us per step of a full tile, and saves the dBias kernel, 5 us and more with its launch and the second computation of S and dP.
+// about 1.3 us per step of a full tile (D = 32: 2, with the dBias kernel's polynomials), and saves the dBias kernel, 5 us and more with its launch and the
+// second computation of S and dP.
 enum DbiasHere { DBIAS_NO = 0, DBIAS_F32 = 1, DBIAS_BF16 = 2, DBIAS_ADD = 3 };
 
 // What a CTA of the dQ/dK/dV kernels walks: the segments (kv tiles) of whole pairs (S row, head) one after another,
@@ -331,10 +332,12 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
 }
 
 // dBias is added up in memory (DBIAS_ADD) if the fullest CTA has no more steps than this.  Forward and backward queued back to
-// back, dBias kernel / added up, us, by steps of the fullest CTA: 1 (S=32, N=64, H=4, D=32) 25.9 / 20.8; 4 (S=64, N=128, H=8, D=32) 41.7 / 37.2,
-// (S=4, N=512, H=8, D=64) 43.7 / 40.9; 6 (S=100, N=128, H=8, D=64) 69.0 / 61.1, (S=3, N=768, H=4, D=64) 48.3 / 47.3; 7 (S=128, N=128, H=8, D=32)
-// 59.5 / 57.0; 8 (S=32, N=256, H=8, D=64) 67.1 / 64.5, but (S=2, N=1024, H=4, D=64) 56.0 / 57.6.
-constexpr int DBIAS_ADD_STEPS = 7;
+// back, dBias kernel / added up, us, bf16 dBias, by steps of the fullest CTA.  D = 32, where the dBias kernel's polynomials come on top (and the second
+// computation of S and dP is cheap): 1 (S=32, N=64, H=4) 23.6 / 20.0, (S=18, N=128, H=8) 27.4 / 22.2; 2 (S=30, N=128, H=8) 28.8 / 24.9; 3 (S=32, N=128, H=12)
+// 32.8 / 30.0; 4 (S=32, N=128, H=16) 39.3 / 37.6, (S=16, N=256, H=8) 35.6 / 34.1; 5 (H=20) 43.2 / 42.4, (N=64) 39.6 / 39.6; 6 (H=24) 47.2 / 48.1; 7 (H=32) 55.9 / 58.7.
+// D = 64: 1 (S=32, N=64, H=4) 25.6 / 20.0; 4 (S=32, N=128, H=16) 49.0 / 41.7; 6 (H=24) 65.6 / 57.3, by segments (S=3, N=768, H=1) 42.3 / 40.8; 7 (H=32) 82.4 / 72.0;
+// 8 (S=32, N=256, H=8) 64.1 / 61.7, but (S=2, N=1024, H=4) 56.0 / 57.6.
+template <int DH> constexpr int DBIAS_ADD_STEPS = (DH == 32) ? 4 : 7;
 
 struct BwdWorkspace {
     size_t off_xq, off_xk, off_do, off_db, off_dq, least, total;
@@ -461,11 +464,10 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     p.dbias = dbias_out;
     // with few steps a CTA they add it up in memory
     const long steps = p.n_whole == pairs ? static_cast<long>((pairs + use_sms - 1) / use_sms) * NT * NT : t_seg * NT;
-    // (D <= 32: of whole pairs only.  A quarter of the dBias kernel's exponentials are polynomials there, 7e-5 from these, and the smallest
-    // problems of several tiles have dBias from that kernel whether their backward is one call or two phases.)
-    const bool dbias_add = DH <= 64 && both && !dbias_here && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS;
+    // (D <= 32: of whole pairs only)
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
+    const bool dbias_add = DH <= 64 && both && !dbias_here && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS<DH>;
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
     // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the

@@ -711,6 +711,15 @@ evo_bwd_halves_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         pkp[w] = pack_bf16(e2.x, e2.y);
                         pkd[w] = pack_bf16(d2.x, d2.y);
                         dsv[4 * cb + b] = d2;
+                        if constexpr (DBIAS_HERE == DBIAS_ADD && DBIAS_POLY_EVERY<DH> > 0) {
+                            // dBias from the dBias kernel's exponentials: polynomials in the same kv columns, this thread's rows
+                            const float2 a2 = ex2_poly2<3>(x2);
+                            const bool poly = use_poly<DBIAS_POLY_EVERY<DH>>(lane >> 3);
+                            float2 p2 = make_float2(poly ? a2.x : e2.x, poly ? a2.y : e2.y);
+                            asm volatile("" : "+f"(p2.x), "+f"(p2.y));      // chosen here: 40 bytes of spills, 184 with the choice put off
+                            dsv[4 * cb + b] = fmul2(p2, u2f2(dv[r], dv[r + 1]));
+                            asm volatile("" : "+f"(dsv[4 * cb + b].x), "+f"(dsv[4 * cb + b].y));
+                        }
                     }
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {             // formed here, not behind the wait below

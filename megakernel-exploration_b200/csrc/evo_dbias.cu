@@ -32,10 +32,6 @@
 
 namespace evo {
 
-// D = 32, whose arithmetic is little more than the exp2: every fourth column pair takes its exp2 on the
-// fused-multiply-add pipe (see ex2_poly2; 0.187 -> 0.180 ms at B=1, S=512, N=384, H=8).
-template <int DH> constexpr int DBIAS_POLY_EVERY = (DH == 32) ? 4 : 0;
-
 template <int DH, int NG>
 struct DbCfg {
     static constexpr int CW = TILE / NG;                  // kv columns per thread

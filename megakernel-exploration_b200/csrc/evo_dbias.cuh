@@ -5,6 +5,11 @@
 
 namespace evo {
 
+// D = 32, whose arithmetic is little more than the exp2: every fourth pair of kv columns takes its exp2 on the
+// fused-multiply-add pipe (see ex2_poly2; 0.187 -> 0.180 ms at B=1, S=512, N=384, H=8).  Whatever else forms dBias as a sum over rows
+// takes the same columns' there (evo_bwd_halves.cuh), so that dBias does not depend on which kernel a call gets.
+template <int DH> constexpr int DBIAS_POLY_EVERY = (DH == 32) ? 4 : 0;
+
 // Slices of S that the launcher cuts the sum into (1: every dBias tile is one CTA's whole sum).
 int dbias_slices(const EvoDims* d, int sms);
 
