@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
 // computation of S and dP is cheap): 1 (S=32, N=64, H=4) 23.6 / 20.0, (S=18, N=128, H=8) 27.4 / 22.2; 2 (S=30, N=128, H=8) 28.8 / 24.9; 3 (S=32, N=128, H=12)
 // 32.8 / 30.0; 4 (S=32, N=128, H=16) 39.3 / 37.6, (S=16, N=256, H=8) 35.6 / 34.1; 5 (H=20) 43.2 / 42.4, (N=64) 39.6 / 39.6; 6 (H=24) 47.2 / 48.1; 7 (H=32) 55.9 / 58.7.
 // D = 64: 1 (S=32, N=64, H=4) 25.6 / 20.0; 4 (S=32, N=128, H=16) 49.0 / 41.7; 6 (H=24) 65.6 / 57.3, by segments (S=3, N=768, H=1) 42.3 / 40.8; 7 (H=32) 82.4 / 72.0;
-// 8 (S=32, N=256, H=8) 64.1 / 61.7, but (S=2, N=1024, H=4) 56.0 / 57.6.
+// at 8 (S=32, N=256, H=8) the gain is down to 64.1 / 61.7, and left.
 template <int DH> constexpr int DBIAS_ADD_STEPS = (DH == 32) ? 4 : 7;
 
 struct BwdWorkspace {
@@ -462,12 +462,13 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const bool both = (phases & EVO_BWD_PHASE_DBIAS) && (phases & EVO_BWD_PHASE_DQKV);
     const bool dbias_here = (d->S == 1) && both;
     p.dbias = dbias_out;
-    // with few steps a CTA they add it up in memory
+    // with few steps a CTA they add it up in memory, unless the dBias kernel has the sum in registers or in two slices: then it comes out
+    // the same in every call, which a sum of three or more in any order does not; and without several slices that kernel needs neither zeros nor a conversion
     const long steps = p.n_whole == pairs ? static_cast<long>((pairs + use_sms - 1) / use_sms) * NT * NT : t_seg * NT;
     // (D <= 32: of whole pairs only)
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
-    const bool dbias_add = DH <= 64 && both && !dbias_here && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS<DH>;
+    const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS<DH>;
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
     // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the

@@ -35,3 +35,20 @@ def test_one_call_equals_two_phases(B, S, N, H, D):
     1e-5 of the largest entry with terms that hardly cancel in it."""
     one, two = _one_call_and_phases(B, S, N, H, D)
     assert (one - two).abs().max() <= 1e-5 * two.abs().max()
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("B,S,N,H", [
+    (8, 4, 128, 16),        # 128 tiles of dBias: a slice for each; four steps
+    (8, 8, 128, 8),
+    (1, 4, 512, 8),         # ... by segments at D = 64
+    (1, 3, 768, 4),
+    (2, 2, 136, 3),         # two slices: two terms onto zero, in either order
+    (4, 3, 128, 16),
+])
+def test_few_slices_repeat(B, S, N, H, D):
+    """Where the dBias kernel has a dBias tile's sum in one slice of S, or in two, dBias is the same bit for bit in every call,
+    and in two phases."""
+    *calls, phased = _one_call_and_phases(B, S, N, H, D, calls=4)
+    for x in calls:
+        assert torch.equal(x, phased)
