@@ -338,6 +338,11 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
 // D = 64: 1 (S=32, N=64, H=4) 25.6 / 20.0; 4 (S=32, N=128, H=16) 49.0 / 41.7; 6 (H=24) 65.6 / 57.3, by segments (S=3, N=768, H=1) 42.3 / 40.8; 7 (H=32) 82.4 / 72.0;
 // at 8 (S=32, N=256, H=8) the gain is down to 64.1 / 61.7, and left.
 template <int DH> constexpr int DBIAS_ADD_STEPS = (DH == 32) ? 4 : 7;
+// ... and if no more rows meet in a sum than this.  Where the sum lies within a few KB of something that the kernel reads (an fp32 dBias between the
+// pair bias and the mask, as the allocator places small tensors), an add now and then takes 0.2 us per row of the sum: over some 200
+// placements, dBias kernel / added up, median and worst: S=512, N=40, H=1, D=32 41 / 34 and 149; S=518, N=64, H=2, D=64 68 / 62 and 99; S=100, N=40, H=8, D=64
+// 54 / 49 and 68; S=60, N=200, H=1, D=64 33 / 27 and 39; S=48 31 / 26 and 34; S=32 30 / 25 and 29, N=64, H=4 24.6 / 19.6 and 19.6, N=40, H=8 28 / 24 and (one of 240) 32.
+constexpr int DBIAS_ADD_ROWS = 32;
 
 struct BwdWorkspace {
     size_t off_xq, off_xk, off_do, off_db, off_dq, least, total;
@@ -468,7 +473,8 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     // (D <= 32: of whole pairs only)
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
-    const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) && steps <= DBIAS_ADD_STEPS<DH>;
+    const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) &&
+                           steps <= DBIAS_ADD_STEPS<DH> && d->S <= DBIAS_ADD_ROWS;
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
     // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the

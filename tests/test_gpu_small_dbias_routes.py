@@ -52,3 +52,24 @@ def test_few_slices_repeat(B, S, N, H, D):
     *calls, phased = _one_call_and_phases(B, S, N, H, D, calls=4)
     for x in calls:
         assert torch.equal(x, phased)
+
+
+@pytest.mark.parametrize("B,S,N,H,D,added", [
+    (1, 32, 64, 4, 32, True), (1, 32, 64, 4, 64, True), (1, 3, 128, 8, 16, True),
+    (1, 33, 64, 4, 32, False), (1, 33, 64, 4, 64, False), (1, 512, 40, 1, 64, False),       # rows that meet in a sum
+    (1, 32, 128, 16, 32, True), (1, 30, 128, 20, 32, False),                                # four steps a CTA, five
+    (1, 32, 128, 32, 64, True), (1, 32, 128, 33, 64, False),                                # seven, eight
+    (1, 4, 512, 8, 64, False), (2, 2, 136, 3, 64, False),                                   # one slice, two
+    (1, 4, 128, 4, 128, False),
+])
+def test_which_kernel_forms_dbias(B, S, N, H, D, added):
+    import _evoattn
+    _evoattn.profile_enable(True)
+    for k in range(3):
+        _evoattn.profile_read(k)
+    try:
+        _one_call_and_phases(B, S, N, H, D)
+    finally:
+        _evoattn.profile_enable(False)
+    launches = [_evoattn.profile_read(k)[1] for k in range(3)]
+    assert launches == [1, 2, 1 if added else 2]              # (the phased call has one of its own)
