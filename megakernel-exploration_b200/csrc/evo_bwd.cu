@@ -468,12 +468,13 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     const bool dbias_here = (d->S == 1) && both;
     p.dbias = dbias_out;
     // with few steps a CTA they add it up in memory, unless the dBias kernel has the sum in registers or in two slices: then it comes out
-    // the same in every call, which a sum of three or more in any order does not; and without several slices that kernel needs neither zeros nor a conversion
+    // the same in every call, which a sum of three or more in any order does not; and without several slices that kernel needs neither zeros nor a conversion.
+    // By segments D = 32, dBias kernel / added up: S=9, N=200, H=4 28.9 / 25.2 us, S=25, N=256, H=1 27.6 / 24.3, S=20, N=384, H=2 34.0 / 31.0, S=8, N=392, H=2 34.9 / 34.8.
+    // (Not where a CTA walks whole pairs and segments: that is six steps and more, and an instantiation that spills at D = 64.)
     const long steps = p.n_whole == pairs ? static_cast<long>((pairs + use_sms - 1) / use_sms) * NT * NT : t_seg * NT;
-    // (D <= 32: of whole pairs only)
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
-    const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || (DH == 64 && p.n_whole == 0)) &&
+    const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || p.n_whole == 0) &&
                            steps <= DBIAS_ADD_STEPS<DH> && d->S <= DBIAS_ADD_ROWS;
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
@@ -549,7 +550,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
             return run(kernel, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb);
         } else {
             using C = BwdHalvesCfg<DH>;
-            if constexpr (W == WALK_WHOLE || (W == WALK_SEGMENTS && DH == 64)) {
+            if constexpr (W != WALK_BOTH) {
                 if (mode == DBIAS_ADD) return run(evo_bwd_halves_kernel<DH, W, DBIAS_ADD>, C::THREADS, C::SMEM_BYTES, tq, tk, tv, tdo, tb, tdq, tdk, tdv, tacc);
             }
             auto kernel = mode == DBIAS_NO ? evo_bwd_halves_kernel<DH, W, DBIAS_NO>

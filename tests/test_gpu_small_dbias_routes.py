@@ -28,7 +28,7 @@ def _one_call_and_phases(B, S, N, H, D, calls=1):
 
 
 @pytest.mark.parametrize("D", [16, 32, 64])
-@pytest.mark.parametrize("B,S,N,H", [(1, 32, 64, 4), (1, 3, 128, 8), (2, 17, 40, 2), (4, 8, 128, 4), (1, 16, 256, 8), (1, 9, 200, 4), (1, 32, 128, 16)])
+@pytest.mark.parametrize("B,S,N,H", [(1, 32, 64, 4), (1, 3, 128, 8), (2, 17, 40, 2), (4, 8, 128, 4), (1, 16, 256, 8), (1, 9, 200, 4), (1, 32, 128, 16), (1, 3, 256, 4), (1, 8, 392, 2)])
 def test_one_call_equals_two_phases(B, S, N, H, D):
     """The same exponentials on both routes (at D <= 32 polynomials in the same columns, 7.5e-5 from the others): what is left are products
     and sums of up to 32 fp32 terms rounded in another order, below 32 * 2^-23 of the sum of their absolute values; at
@@ -60,6 +60,7 @@ def test_few_slices_repeat(B, S, N, H, D):
     (1, 32, 128, 16, 32, True), (1, 30, 128, 20, 32, False),                                # four steps a CTA, five
     (1, 32, 128, 32, 64, True), (1, 32, 128, 33, 64, False),                                # seven, eight
     (1, 4, 512, 8, 64, False), (2, 2, 136, 3, 64, False),                                   # one slice, two
+    (1, 9, 200, 4, 32, True), (1, 9, 200, 4, 64, True), (1, 8, 392, 2, 16, True), (1, 4, 640, 1, 32, False),      # by segments
     (1, 4, 128, 4, 128, False),
 ])
 def test_which_kernel_forms_dbias(B, S, N, H, D, added):
