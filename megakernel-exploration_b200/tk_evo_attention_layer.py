@@ -520,7 +520,7 @@ class HostStreamedEvoAttention:
         assert mask.dtype == torch.bfloat16 and bias.dtype == torch.bfloat16
         dbias_out = out["dbias"].reshape(B, H, N, N)
         chunks = self._chunks(B, S, N, H, D)
-        self._buffers(B, N, H, D, max(r for _, _, r in chunks))
+        self._buffers(B, N, H, D, max((r for _, _, r in chunks), default=1))      # (a rank without rows takes part in the all-reduce)
         cur = torch.cuda.current_stream(self.dev)
         for s_ in (self.s_in, self.s_cmp, self.s_out):
             s_.wait_stream(cur)
@@ -531,7 +531,7 @@ class HostStreamedEvoAttention:
         _native()
         native = sys.modules.get("_evo_torch")
         ins, outs = (q, k, v, d_o, mask), [out[n] for n in ("o", "dq", "dk", "dv")]
-        if native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
+        if chunks and native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
                 t.shape == q.shape and t.dtype == torch.bfloat16 and t.is_contiguous() and not t.is_cuda and not t.requires_grad
                 and not t.is_inference() for t in outs):
             native.host_chunks(chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
