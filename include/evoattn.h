@@ -104,8 +104,11 @@ int evo_bwd_strided(const EvoDims* dims, const EvoStrides* strides, const void* 
  *                        order), and leaves `reserved_sms` SMs unused
  * so that the caller can start the all-reduce of dbias on another stream between the
  * two calls and have it run on the reserved SMs next to the second phase.  Both bits
- * and reserved_sms = 0 is evo_bwd_strided. */
-enum { EVO_BWD_PHASE_DBIAS = 1, EVO_BWD_PHASE_DQKV = 2 };
+ * and reserved_sms = 0 is evo_bwd_strided.
+ *   EVO_BWD_BESIDE_COPIES  besides the phases: copies between host and device run on other
+ *                        streams meanwhile and matter more than the call's latency.  The same
+ *                        results; the first kernel is launched in full order. */
+enum { EVO_BWD_PHASE_DBIAS = 1, EVO_BWD_PHASE_DQKV = 2, EVO_BWD_BESIDE_COPIES = 4 };
 int evo_bwd_phased(const EvoDims* dims, const EvoStrides* strides, const void* q, const void* k,
                    const void* v, const void* pair_bias, const void* res_mask, const void* o,
                    const void* o_resid, const float* lse, const void* d_o, void* dq, void* dk, void* dv,

@@ -130,7 +130,7 @@ def bwd_strided(dims: EvoDims, strides: EvoStrides, q, k, v, bias, mask, o, o_re
                                 float(scale), stream), "evo_bwd_strided")
 
 
-BWD_PHASE_DBIAS, BWD_PHASE_DQKV = 1, 2
+BWD_PHASE_DBIAS, BWD_PHASE_DQKV, BWD_BESIDE_COPIES = 1, 2, 4
 
 
 def bwd_phased(dims: EvoDims, strides, q, k, v, bias, mask, o, o_resid, lse, d_o, dq, dk, dv, dbias, workspace,

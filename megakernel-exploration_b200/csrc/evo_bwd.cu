@@ -521,7 +521,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
         auto prep = [&](auto lanes_c, auto gated_c) -> int {
             constexpr int L = decltype(lanes_c)::value;
             constexpr bool G = decltype(gated_c)::value;
-            return launch_chained(both, bwd_prep_kernel<L, G>, sms * PREP_BLOCKS, 256, 0, st, r);
+            return launch_chained(both && !(phases & EVO_BWD_BESIDE_COPIES), bwd_prep_kernel<L, G>, sms * PREP_BLOCKS, 256, 0, st, r);
         };
         auto prep_lanes = [&](auto lanes_c) -> int { return gate ? prep(lanes_c, std::true_type{}) : prep(lanes_c, std::false_type{}); };
         if ((rc = Dt <= 16 ? prep_lanes(std::integral_constant<int, 2>{}) : prep_lanes(std::integral_constant<int, LANES>{}))) return rc;

@@ -350,10 +350,10 @@ void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunk
         float* lse = static_cast<float*>(st[10].data_ptr());
         check(evo_fwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
                       st[6].data_ptr(), lse, 0.f, s_cmp.stream()), "evo_fwd");
-        check(evo_bwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
-                      st[6].data_ptr(), lse, st[3].data_ptr(), st[7].data_ptr(), st[8].data_ptr(), st[9].data_ptr(),
-                      static_cast<float*>(st[11].data_ptr()), st[12].data_ptr(), static_cast<size_t>(st[12].numel()), 0.f,
-                      s_cmp.stream()), "evo_bwd");
+        check(evo_bwd_phased(&dims, nullptr, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
+                             st[6].data_ptr(), lse, st[3].data_ptr(), st[7].data_ptr(), st[8].data_ptr(), st[9].data_ptr(),
+                             static_cast<float*>(st[11].data_ptr()), st[12].data_ptr(), static_cast<size_t>(st[12].numel()), 0.f,
+                             EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV | EVO_BWD_BESIDE_COPIES, 0, s_cmp.stream()), "evo_bwd_phased");
         {
             const c10::cuda::CUDAStreamGuard on(s_cmp);
             dbias.select(0, b).add_(st[11].select(0, 0));

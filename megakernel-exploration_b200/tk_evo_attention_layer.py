@@ -565,9 +565,9 @@ class HostStreamedEvoAttention:
                 # a chunk with fewer rows uses the leading rows of the (contiguous) buffers
                 _evoattn.fwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
                              st["ores"], st["lse"], 0.0, h_)
-                _evoattn.bwd(dims, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
-                             st["ores"], st["lse"], st["do"], st["dq"], st["dk"], st["dv"], st["dbias"],
-                             st["ws"], 0.0, h_)
+                _evoattn.bwd_phased(dims, None, st["q"], st["k"], st["v"], self.bias[b:b + 1], st["mask"], st["o"],
+                                    st["ores"], st["lse"], st["do"], st["dq"], st["dk"], st["dv"], st["dbias"], st["ws"], 0.0,
+                                    _evoattn.BWD_PHASE_DBIAS | _evoattn.BWD_PHASE_DQKV | _evoattn.BWD_BESIDE_COPIES, 0, h_)
                 self.dbias[b:b + 1].add_(st["dbias"])
                 st["ev_cmp"].record(self.s_cmp)
             with torch.cuda.stream(self.s_out):
