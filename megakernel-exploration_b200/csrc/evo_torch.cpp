@@ -305,8 +305,8 @@ std::optional<Tensor> apply(const Tensor& Q, const Tensor& K, const Tensor& V, c
 // through the kernels and out, on three streams and three sets of device buffers.  ins: q, k, v, dO, mask and outs: o, dq,
 // dk, dv in host memory, contiguous; a set: q, k, v, do, mask, o, ores, dq, dk, dv, lse, dbias, ws for at least the rows
 // of a chunk.  Through torch's Python operators a chunk was about 200 us of host time, and small steps
-// were bound by it.
-void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunks, const std::vector<Tensor>& ins, const Tensor& bias,
+// were bound by it.  What the library refuses comes back as its error code and the name of the call, EVO_OK otherwise.
+std::pair<int, std::string> host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunks, const std::vector<Tensor>& ins, const Tensor& bias,
                  const Tensor& dbias, const std::vector<Tensor>& outs, const std::vector<std::vector<Tensor>>& sets,
                  const std::vector<std::tuple<int64_t, int64_t, int64_t>>& streams) {
     TORCH_CHECK(ins.size() == 5 && outs.size() == 4 && sets.size() == 3 && streams.size() == 3, "host_chunks: wrong number of arguments");
@@ -348,12 +348,14 @@ void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunk
         const EvoDims dims{1, static_cast<int32_t>(r), static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(D)};
         const void* bias_b = static_cast<const char*>(bias.const_data_ptr()) + b * 2 * H * N * N;
         float* lse = static_cast<float*>(st[10].data_ptr());
-        check(evo_fwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
-                      st[6].data_ptr(), lse, 0.f, s_cmp.stream()), "evo_fwd");
-        check(evo_bwd_phased(&dims, nullptr, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
-                             st[6].data_ptr(), lse, st[3].data_ptr(), st[7].data_ptr(), st[8].data_ptr(), st[9].data_ptr(),
-                             static_cast<float*>(st[11].data_ptr()), st[12].data_ptr(), static_cast<size_t>(st[12].numel()), 0.f,
-                             EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV | EVO_BWD_BESIDE_COPIES, 0, s_cmp.stream()), "evo_bwd_phased");
+        int rc = evo_fwd(&dims, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
+                         st[6].data_ptr(), lse, 0.f, s_cmp.stream());
+        if (rc != EVO_OK) return {rc, "evo_fwd"};
+        rc = evo_bwd_phased(&dims, nullptr, st[0].data_ptr(), st[1].data_ptr(), st[2].data_ptr(), bias_b, st[4].data_ptr(), st[5].data_ptr(),
+                            st[6].data_ptr(), lse, st[3].data_ptr(), st[7].data_ptr(), st[8].data_ptr(), st[9].data_ptr(),
+                            static_cast<float*>(st[11].data_ptr()), st[12].data_ptr(), static_cast<size_t>(st[12].numel()), 0.f,
+                            EVO_BWD_PHASE_DBIAS | EVO_BWD_PHASE_DQKV | EVO_BWD_BESIDE_COPIES, 0, s_cmp.stream());
+        if (rc != EVO_OK) return {rc, "evo_bwd_phased"};
         {
             const c10::cuda::CUDAStreamGuard on(s_cmp);
             dbias.select(0, b).add_(st[11].select(0, 0));
@@ -364,6 +366,7 @@ void host_chunks(const std::vector<std::tuple<int64_t, int64_t, int64_t>>& chunk
             copy(static_cast<char*>(outs[i].data_ptr()) + row * act, st[i == 0 ? 5 : 6 + i].data_ptr(), r * act, cudaMemcpyDeviceToHost, s_out);
         ev_out[c % 3].record(s_out);
     }
+    return {EVO_OK, ""};
 }
 
 }  // namespace

@@ -534,8 +534,9 @@ class HostStreamedEvoAttention:
         if chunks and native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
                 t.shape == q.shape and t.dtype == torch.bfloat16 and t.is_contiguous() and not t.is_cuda and not t.requires_grad
                 and not t.is_inference() for t in outs):
-            native.host_chunks(chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
-                               [(s_.stream_id, s_.device_index, s_.device_type) for s_ in (self.s_in, self.s_cmp, self.s_out)])
+            _evoattn.check(*native.host_chunks(
+                chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
+                [(s_.stream_id, s_.device_index, s_.device_type) for s_ in (self.s_in, self.s_cmp, self.s_out)]))
         else:
             self._run_chunks(chunks, q, k, v, mask, d_o, out)
         with torch.cuda.stream(self.s_cmp):
