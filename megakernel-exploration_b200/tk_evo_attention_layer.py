@@ -529,12 +529,12 @@ class HostStreamedEvoAttention:
         with torch.cuda.stream(self.s_cmp):
             self.dbias.zero_()
         _native()
-        native = sys.modules.get("_evo_torch")
+        native = getattr(sys.modules.get("_evo_torch"), "host_chunks", None)       # (None: not loaded, or built from earlier sources)
         ins, outs = (q, k, v, d_o, mask), [out[n] for n in ("o", "dq", "dk", "dv")]
         if chunks and native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
                 t.shape == q.shape and t.dtype == torch.bfloat16 and t.is_contiguous() and not t.is_cuda and not t.requires_grad
                 and not t.is_inference() for t in outs):
-            _evoattn.check(*native.host_chunks(
+            _evoattn.check(*native(
                 chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
                 [(s_.stream_id, s_.device_index, s_.device_type) for s_ in (self.s_in, self.s_cmp, self.s_out)]))
         else:
