@@ -442,6 +442,13 @@ class EvoAttention(torch.nn.Module):
         return TKEvoAttention.apply(Q, K, V, res_mask, pair_bias, self.process_group)
 
 
+def _host_bytes(t):
+    """Are the bytes of `t`'s storage in host memory, in order, its values?  (Not so for a subclass, a negated view, a zero or a
+    meta tensor, which a copy through torch's operators serves or refuses.)"""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and t.device.type == "cpu" and t.layout == torch.strided and t.is_contiguous()
+            and not t.is_neg() and not t._is_zerotensor())
+
+
 class HostStreamedEvoAttention:
     """Forward + backward for callers whose tensors live in HOST memory.
 
@@ -531,9 +538,8 @@ class HostStreamedEvoAttention:
         _native()
         native = getattr(sys.modules.get("_evo_torch"), "host_chunks", None)       # (None: not loaded, or built from earlier sources)
         ins, outs = (q, k, v, d_o, mask), [out[n] for n in ("o", "dq", "dk", "dv")]
-        if chunks and native is not None and all(t.is_contiguous() for t in ins) and not mask.is_cuda and all(
-                t.shape == q.shape and t.dtype == torch.bfloat16 and t.is_contiguous() and not t.is_cuda and not t.requires_grad
-                and not t.is_inference() for t in outs):
+        if chunks and native is not None and all(_host_bytes(t) for t in (*ins, *outs)) and all(
+                t.shape == q.shape and t.dtype == torch.bfloat16 and not t.requires_grad and not t.is_inference() for t in outs):
             _evoattn.check(*native(
                 chunks, ins, self.bias, self.dbias, outs, [[s_[n] for n in self.NAMES] for s_ in self.sets],
                 [(s_.stream_id, s_.device_index, s_.device_type) for s_ in (self.s_in, self.s_cmp, self.s_out)]))

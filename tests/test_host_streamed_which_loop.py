@@ -57,3 +57,64 @@ def _loops(monkeypatch, x, out, module):
                          ids=["built", "built from earlier sources", "not loaded"])
 def test_module(monkeypatch, module, loop):
     assert _loops(monkeypatch, *_call(), module) == [loop]
+
+
+def _subclass(t):
+    class Tagged(torch.Tensor):
+        pass
+    return t.as_subclass(Tagged)
+
+
+def _transposed(t):
+    return t.transpose(1, 2).contiguous().transpose(1, 2)
+
+
+@pytest.mark.parametrize("name", ["q", "d_o", "o", "dv"])
+@pytest.mark.parametrize("form,loop", [
+    (lambda t: t, "native"),
+    (lambda t: torch.cat([t, t])[1:], "native"),                     # at an offset of its storage
+    (lambda t: torch.nn.Parameter(t, requires_grad=False), "native"),
+    (_transposed, "python"),
+    (lambda t: torch._neg_view(t), "python"),                        # its bytes have the other sign
+    (_subclass, "python"),
+    (lambda t: torch._efficientzerotensor(t.shape, dtype=t.dtype), "python"),      # has no bytes
+    (lambda t: t.to("meta"), "python"),
+], ids=["plain", "offset", "parameter", "transposed", "negated", "subclass", "zero", "meta"])
+def test_form(monkeypatch, name, form, loop):
+    x, out = _call()
+    where = x if name in x else out
+    where[name] = form(where[name])
+    assert _loops(monkeypatch, x, out, types.SimpleNamespace(host_chunks=None)) == [loop]
+
+
+@pytest.mark.parametrize("form", [lambda t: t.requires_grad_(), lambda t: t.float(), lambda t: t[:, :, :, :1].expand(t.shape)],
+                         ids=["carries gradients", "fp32", "expanded"])
+def test_form_of_a_result(monkeypatch, form):
+    x, out = _call()
+    out["dq"] = form(out["dq"])
+    assert _loops(monkeypatch, x, out, types.SimpleNamespace(host_chunks=None)) == ["python"]
+
+
+@pytest.mark.gpu
+def test_on_the_device(monkeypatch):
+    """With the extension that was built: contiguous tensors take the native loop, transposed and negated ones the Python loop, and
+    the results are the same."""
+    from tk_evo_attention_layer import HostStreamedEvoAttention as Host
+    taken = []
+    run_chunks = Host._run_chunks
+    monkeypatch.setattr(Host, "_run_chunks", lambda self, *args: taken.append("python") or run_chunks(self, *args))
+    outs = []
+    for form, loops in ((lambda t: t, []), (_transposed, ["python"]), (lambda t: torch._neg_view(-t), ["python"])):
+        x, out = _call()
+        gen = torch.Generator().manual_seed(1)
+        for n in ("q", "k", "v", "d_o"):
+            x[n] = form(torch.randn((B, S, N, H, D), generator=gen).to(torch.bfloat16))
+        taken.clear()
+        Host("cuda").run(x["q"], x["k"], x["v"], x["mask"], x["bias"], x["d_o"], out)
+        torch.cuda.synchronize()
+        assert taken == loops
+        outs.append(out)
+    for other in outs[1:]:
+        for n in ("o", "dq", "dk", "dv", "dbias"):       # (one tile, one chunk of three rows: dBias three fp32 terms in any order)
+            a, b = outs[0][n], other[n]
+            assert torch.equal(a, b) if n != "dbias" else (a - b).abs().max() <= 1e-6 * a.abs().max(), n
