@@ -39,7 +39,7 @@ for _p in (ROOT, PKG):
 import evo_workloads as wl  # noqa: E402
 
 # DRAM bytes per S row of one evo_bwd_halves_kernel launch, from the ncu capture summarised under profiles/
-# (110.16 MB read + 43.55 MB written at 128 rows of cfg2).
+# (110.23 MB read + 43.04 MB written at 128 rows of cfg2).
 NCU_DRAM_BYTES_PER_ROW = {"cfg2_msa_row": (110.23e6 + 43.04e6) / 128}
 
 METRIC = "EvoAttention fwd+bwd TFLOP/s"
@@ -358,6 +358,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     fwd_ms, fwd_n = _evoattn.profile_read(0)
     bwd_ms, bwd_n = _evoattn.profile_read(1)
     db_ms, db_n = _evoattn.profile_read(2)
+    launches_per_step = _evoattn.profile_read(_evoattn.PROFILE_ALL)[1] // prof_steps
     _evoattn.device_status()
 
     e2e_steps = max(3, min(args.steps, 10))
@@ -444,8 +445,8 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "bytes_are": "per rank (the value is the whole job)",
                     "ms_per_step": ms_e2e / e2e_steps, "steps": e2e_steps},
-            # forward; backward: prep, dBias, dQ/dK/dV, conversion of fp32 sums (with a pair of one tile a CTA: no dBias kernel, no conversion)
-            "gpu_launches": (3 if N <= 128 and B * rows * H <= 148 else 5) * args.steps,
+            # this rank's; per step as counted by the library over the profiled steps
+            "gpu_launches": launches_per_step * args.steps,
             "graph_replay": bool(args.graph),
             "roofline": roofline,
         }

@@ -58,8 +58,8 @@ enum {
 };
 
 /* Library ABI version (major*100 + minor).  Minor 4 added evo_bwd_ex and
- * evo_bwd_ex_workspace_bytes. */
-#define EVO_ABI_VERSION 104
+ * evo_bwd_ex_workspace_bytes, minor 5 EVO_BWD_BESIDE_COPIES and EVO_PROFILE_ALL. */
+#define EVO_ABI_VERSION 105
 int evo_version(void);
 const char* evo_strerror(int code);
 /* cudaError_t of the most recent failing runtime call on this thread (0 if none). */
@@ -240,7 +240,9 @@ int evo_device_status(uint32_t* raw);
  * kept), evo_profile_enable(0) stops.  evo_profile_read waits for the recorded
  * events, returns the summed milliseconds and the launch count of
  * kernel 0 (forward), 1 (backward dQ/dK/dV kernel) or 2 (backward dBias kernel),
- * and clears that record. */
+ * and clears that record.  EVO_PROFILE_ALL: how many kernels of the library were launched
+ * for forwards and backwards while recording, of whichever kind (no time). */
+enum { EVO_PROFILE_ALL = 3 };
 int evo_profile_enable(int on);
 int evo_profile_read(int kernel, float* total_ms, int* launches);
 

@@ -12,7 +12,7 @@ import threading
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libevoattn.so")
 
-ABI_VERSION = 104
+ABI_VERSION = 105
 
 
 class EvoDims(C.Structure):
@@ -220,12 +220,16 @@ def device_status() -> int:
     return 0
 
 
+PROFILE_ALL = 3
+
+
 def profile_enable(on: bool) -> None:
     check(lib().evo_profile_enable(1 if on else 0), "evo_profile_enable")
 
 
 def profile_read(kernel: int):
-    """(total milliseconds, launches) of kernel 0 (forward) / 1 (backward dQ,dK,dV) / 2 (backward dBias)."""
+    """(total milliseconds, launches) of kernel 0 (forward) / 1 (backward dQ,dK,dV) / 2 (backward dBias); PROFILE_ALL: (0, launches of
+    every kernel)."""
     ms, n = C.c_float(0.0), C.c_int(0)
     check(lib().evo_profile_read(kernel, C.byref(ms), C.byref(n)), "evo_profile_read")
     return ms.value, n.value

@@ -4,6 +4,7 @@
 
 #include <cstdio>
 #include <memory>
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -225,7 +226,8 @@ struct ProfRec {
     bool armed = false;      // prof_begin pushed a pair that prof_end has not closed yet
 };
 std::mutex g_prof_mu;
-bool g_prof_on = false;
+std::atomic<bool> g_prof_on{false};
+std::atomic<int> g_prof_launches{0};
 ProfRec g_prof[3];
 constexpr size_t PROF_MAX = 4096;
 }  // namespace
@@ -257,6 +259,10 @@ void prof_end(int kernel, cudaStream_t st) {
     if (!r.armed) return;        // the matching prof_begin recorded nothing (off, full, or failed)
     cudaEventRecord(r.stop.back(), st);
     r.armed = false;
+}
+
+void prof_count() {
+    if (g_prof_on) ++g_prof_launches;
 }
 
 // ---- per-device launch constants and the tensor-map cache ---------------------------
@@ -338,7 +344,12 @@ int evo_profile_enable(int on) {
 }
 
 int evo_profile_read(int kernel, float* total_ms, int* launches) {
-    if (kernel < 0 || kernel > 2 || !total_ms || !launches) return EVO_ERR_NULL_PTR;
+    if (kernel < 0 || kernel > EVO_PROFILE_ALL || !total_ms || !launches) return EVO_ERR_NULL_PTR;
+    if (kernel == EVO_PROFILE_ALL) {
+        *total_ms = 0.f;
+        *launches = evo::g_prof_launches.exchange(0);
+        return EVO_OK;
+    }
     std::lock_guard<std::mutex> lock(evo::g_prof_mu);
     evo::ProfRec& r = evo::g_prof[kernel];
     float sum = 0.f;

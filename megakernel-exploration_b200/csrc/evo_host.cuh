@@ -70,6 +70,8 @@ int set_max_smem_once(const void* func, int bytes);
 // Event pairs around the main kernels when profiling is enabled (no-ops otherwise).
 void prof_begin(int kernel, cudaStream_t st);
 void prof_end(int kernel, cudaStream_t st);
+// A kernel has been launched (counted while profiling is enabled).
+void prof_count();
 
 // Launches a kernel that calls chain_wait ahead of its first access to global memory (evo_ptx.cuh).  chained: as a programmatic launch, whose
 // blocks may be placed as soon as those of the kernel before it on the stream, whichever that is, have all ended, without the rest of a
@@ -100,7 +102,9 @@ int launch_chained(bool chained, void (*kernel)(P...), int grid, int threads, si
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = chained ? 1 : 0;
-    return cuda_err(cudaLaunchKernelEx(&cfg, kernel, args...));
+    const int rc = cuda_err(cudaLaunchKernelEx(&cfg, kernel, args...));
+    if (rc == EVO_OK) prof_count();
+    return rc;
 }
 
 }  // namespace evo
