@@ -123,6 +123,11 @@ size_t evo_bwd_workspace_bytes(const EvoDims* dims);
 /* Backward.  Replaces evoattention_backward (tk_evoattention.cu:1051-1197):
  * recomputes P from LSE; dq = scale * dS k, dk = scale * dS^T q, dv = P^T d_o,
  * dbias = sum over S of dS (unscaled, tk_evoattention.cu:824-833), dS = P o (dP - delta).
+ * dQ and dBias are fp32 sums; where three or more parts of one meet in memory they do so in
+ * any order, and two calls may differ by the rounding of fp32 (O, LSE, dK and dV never do): dQ of
+ * three and more tiles of 128 kv rows whose segments go to several CTAs, dBias summed over S by
+ * three and more CTAs.  With one row of S and D <= 32 the dBias of one call and of two phases
+ * may differ by 1e-4 of its largest entry (other exponentials); otherwise by that rounding.
  * dq/dk/dv are written as bf16 in the caller layout (the reference returns
  * padded fp32, tk_evoattention.cu:1109-1112); dbias (fp32) is overwritten, not
  * accumulated into.  o_resid is the optional residual written by evo_fwd (NULL:

@@ -66,7 +66,7 @@ struct BwdParams {
     ActLayout lay_out;    // of o, o_resid, d_o
 };
 
-// DBIAS_HERE (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
+// DBIAS_F32, DBIAS_BF16 (S = 1 only): dBias is dS itself, no sum over rows, so the compute groups store their
 // dS straight to d_pair_bias and the dBias kernel (which would recompute S and dP for one step
 // per item) is not launched.
 // DBIAS_ADD (small problems): the compute groups add their dS to an fp32 sum in memory, whole rows at a time.  That takes a CTA
@@ -479,15 +479,15 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
     // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the
-    // launch costs a caller as much as anything (S=32, N=64, H=4, D=32: the kernels 20.8 us either way, the whole step, host
-    // work, 85.6 -> 83 with the finish kernel and -> 81 without); with four steps the finish kernel is the better (37.2 us for 43.2).
+    // launch costs a caller's host 3 us and the device little (finish kernel / last adder, S=32, N=64, H=4: D=32 19.5 / 20.0 us, D=64 20.7 / 20.2; S=18, N=128, H=8
+    // 21.1 / 22.2, 22.7 / 23.2); from two steps on the finish kernel is the better (S=30, N=128, H=8: D=32 24.7 / 28.1, D=64 26.8 / 29.2; S=32, H=16 38.2 / 45.1, 42.3 / 46.4).
     const size_t parts = static_cast<size_t>(d->B) * d->H * NT * NT * 16;
     const bool count = dbias_add && dbias_bf16 && steps <= 1 && p.n_whole == pairs && NT <= TILES_HELD && parts <= room * DH;
     const bool convert_dbias = dbias_bf16 && !dbias_here && (dbias_add ? !count : slices > 1);
     p.dbias_acc = dbias_acc;
     p.dbias_done = count ? reinterpret_cast<int*>(dq_ws) : nullptr;
     // One S row of one tile, at most one pair a CTA: the dQ/dK/dV kernel is all of the backward.  (Forward and backward queued back to back,
-    // with the prep kernel / without: B=4, N=128, H=16, D=64 20.7 / 18.7 us, D=32 18.7 / 15.2.  A sum over S rows needs its zeros written first,
+    // with the prep kernel / without: B=4, N=128, H=16, D=64 17.7 / 17.1 us, D=32 15.8 / 14.1, B=1, N=64, H=4 16.2 / 14.5, 15.1 / 12.4; and a launch of host work.  A sum over S rows needs its zeros written first,
     // and with more tiles every segment would form all of its pair's terms again.)
     p.own_prep = DH <= 64 && dbias_here && !gate && NT == 1 && pairs <= use_sms;
     if (p.own_prep) {

@@ -84,9 +84,9 @@ void prof_count();
 // N=768; beside short kernels, of whose gaps it lived, 11 / 22 / 13 (D=32, S=200, N=200, a step 118 / 111 / 111) and 15 / 34 / 19 (D=64, B=4, S=1,
 // N=1024, 162 / 156 / 157).
 // Not chained: the two phases of a backward with a collective beside it.  The prep kernel read a step's tensors slower when its predecessor released it
-// early (its blocks, three or five to an SM, went to the SMs as these became free: the first step 862 -> 885 us); behind a predecessor that has ended it
+// early (its blocks, then three or five to an SM, went to the SMs as these became free: the first step 862 -> 885 us); behind a predecessor that has ended it
 // is chained like the others (not chained / chained: the first step 845.5 / 842.3 us, S=200, N=200, H=4, D=32 106.1 / 103.4, S=384, N=384 349.9 / 347.6).
-// Not so beside copies between host and device (EVO_BWD_BESIDE_COPIES), which its early blocks, more of them than of any other kernel, slow down: steps of
+// Not so beside copies between host and device (EVO_BWD_BESIDE_COPIES), which take longer with it, for a reason that is not known: steps of
 // HostStreamedEvoAttention, three engines in turn, not chained / chained: S=128, N=384, H=8, D=32 2958-2975 / 2987-3050 us (with half of its blocks 3000-3017),
 // S=64, N=384, H=4, D=128 2897-2908 / 2923-2967, S=300, N=200, H=4, D=64 3437-3446 / 3423-3426, S=48, N=256, H=4 551-555 / 551-556, S=16, N=128, H=4
 // 157 / 157.  With no kernel chained 2977, 2925, 3507, 545 and 159.

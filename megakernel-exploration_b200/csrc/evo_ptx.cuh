@@ -52,8 +52,8 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- kernels of a chain -------------------------------------------------------
-// Every kernel of a step is launched so that its launch is under way when the kernel before it ends
-// (launch_chained).  wait: the kernel before, and all that it waited for, is complete and its writes are visible; no global memory is
+// The kernels of a step are launched so that their launch is under way when the kernel before them ends
+// (launch_chained, which has the exceptions).  wait: the kernel before, and all that it waited for, is complete and its writes are visible; no global memory is
 // touched ahead of it.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
