@@ -339,10 +339,12 @@ __global__ void __launch_bounds__(256) bwd_finish_kernel(const FinishParams p) {
 // at 8 (S=32, N=256, H=8) the gain is down to 64.1 / 61.7, and left.
 template <int DH> constexpr int DBIAS_ADD_STEPS = (DH == 32) ? 4 : 7;
 // ... and if no more rows meet in a sum than this.  Where the sum lies within a few KB of something that the kernel reads (an fp32 dBias between the
-// pair bias and the mask, as the allocator places small tensors), an add now and then takes 0.2 us per row of the sum: over some 200
+// pair bias and the mask, as the allocator places small tensors), an add now and then takes 0.2 us per row of the sum: over 200 to 700
 // placements, dBias kernel / added up, median and worst: S=512, N=40, H=1, D=32 41 / 34 and 149; S=518, N=64, H=2, D=64 68 / 62 and 99; S=100, N=40, H=8, D=64
-// 54 / 49 and 68; S=60, N=200, H=1, D=64 33 / 27 and 39; S=48 31 / 26 and 34; S=32 30 / 25 and 29, N=64, H=4 24.6 / 19.6 and 19.6, N=40, H=8 28 / 24 and (one of 240) 32.
-constexpr int DBIAS_ADD_ROWS = 32;
+// 54 / 49 and 68; S=128, N=192, H=1, D=64 39 / 34 and 45; S=60, N=200 33 / 27 and 39; S=48 31 / 26 and 34; S=32 30 / 25 and 29, N=64, H=4 24.6 / 19.6 and 19.6,
+// N=40, H=8 28 / 24 and (one of 240) 32.  Sums of whole tiles hardly show it: N=128, H=8, D=64 S=64 48.1 / 42.0 and 42.2, S=100 64.5 / 58.2 and 58.6, S=128 80.3 / 71.6
+// and 72.2, H=4 48.1 / 41.8 and 42.5, D=32 38.6 / 37.4 and 37.6; N=256, H=1 40.0 / 34.8 and 35.6; S=1036, N=128, H=1 84 / 73 and 81.
+constexpr int dbias_add_rows(int N) { return N % TILE == 0 ? 128 : 32; }
 
 struct BwdWorkspace {
     size_t off_xq, off_xk, off_do, off_db, off_dq, least, total;
@@ -475,7 +477,7 @@ static int launch_bwd(const EvoDims* d, const ActLayout& lay_in, const ActLayout
     // otherwise the dBias kernel does: in one piece, or as an fp32 sum of slices of S
     const int slices = dbias_slices(d, sms);
     const bool dbias_add = DH <= 64 && both && !dbias_here && slices > 2 && (p.n_whole == pairs || p.n_whole == 0) &&
-                           steps <= DBIAS_ADD_STEPS<DH> && d->S <= DBIAS_ADD_ROWS;
+                           steps <= DBIAS_ADD_STEPS<DH> && d->S <= dbias_add_rows(d->N);
     float* dbias_acc = (dbias_bf16 && !dbias_here) ? reinterpret_cast<float*>(ws + w.off_db) : static_cast<float*>(dbias_out);
     // An fp32 sum for a bf16 result is converted by the finish kernel, or by the warps that add the last row to each part of it.
     // That needs counters, where whole pairs need no scratch, and a fence behind every step's adds: with one step a CTA, where the

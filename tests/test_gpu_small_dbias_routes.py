@@ -28,10 +28,10 @@ def _one_call_and_phases(B, S, N, H, D, calls=1):
 
 
 @pytest.mark.parametrize("D", [16, 32, 64])
-@pytest.mark.parametrize("B,S,N,H", [(1, 32, 64, 4), (1, 3, 128, 8), (2, 17, 40, 2), (4, 8, 128, 4), (1, 16, 256, 8), (1, 9, 200, 4), (1, 32, 128, 16), (1, 3, 256, 4), (1, 8, 392, 2)])
+@pytest.mark.parametrize("B,S,N,H", [(1, 32, 64, 4), (1, 3, 128, 8), (2, 17, 40, 2), (4, 8, 128, 4), (1, 16, 256, 8), (1, 9, 200, 4), (1, 32, 128, 16), (1, 3, 256, 4), (1, 8, 392, 2), (1, 128, 128, 4)])
 def test_one_call_equals_two_phases(B, S, N, H, D):
     """The same exponentials on both routes (at D <= 32 polynomials in the same columns, 7.5e-5 from the others): what is left are products
-    and sums of up to 32 fp32 terms rounded in another order, below 32 * 2^-23 of the sum of their absolute values; at
+    and sums of up to 128 fp32 terms rounded in another order, below 128 * 2^-23 of the sum of their absolute values; at
     1e-5 of the largest entry with terms that hardly cancel in it."""
     one, two = _one_call_and_phases(B, S, N, H, D)
     assert (one - two).abs().max() <= 1e-5 * two.abs().max()
@@ -57,6 +57,7 @@ def test_few_slices_repeat(B, S, N, H, D):
 @pytest.mark.parametrize("B,S,N,H,D,added", [
     (1, 32, 64, 4, 32, True), (1, 32, 64, 4, 64, True), (1, 3, 128, 8, 16, True),
     (1, 33, 64, 4, 32, False), (1, 33, 64, 4, 64, False), (1, 512, 40, 1, 64, False),       # rows that meet in a sum
+    (1, 128, 128, 8, 64, True), (1, 100, 128, 2, 32, True), (1, 129, 128, 4, 64, False), (1, 64, 120, 2, 64, False),      # ... of whole tiles
     (1, 32, 128, 16, 32, True), (1, 30, 128, 20, 32, False),                                # four steps a CTA, five
     (1, 32, 128, 32, 64, True), (1, 32, 128, 33, 64, False),                                # seven, eight
     (1, 4, 512, 8, 64, False), (2, 2, 136, 3, 64, False),                                   # one slice, two
